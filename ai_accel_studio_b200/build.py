@@ -14,8 +14,8 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libqgemv_b200.so"
-# (source, extra defines, object name).  The two tensor-core-assisted kernels are compiled once per bit
-# width so that the objects build in parallel.
+# (source, extra defines, object name).  The tensor-core-assisted kernels are compiled in parts (per bit width; per
+# path and activation type) so that the objects build in parallel.
 UNITS = [
     ("qgemv_api.cu", [], "qgemv_api.o"),
     ("qgemv_simt.cu", [], "qgemv_simt.o"),
@@ -26,6 +26,8 @@ UNITS = [
     ("qgemv_mma.cu", ["-DQGEMV_INST_BITS=4"], "qgemv_mma_int4.o"),
     ("qgemv_pipe.cu", ["-DQGEMV_INST_BITS=2"], "qgemv_pipe_int2.o"),
     ("qgemv_pipe.cu", ["-DQGEMV_INST_BITS=4"], "qgemv_pipe_int4.o"),
+    ("qgemv_plan.cu", [], "qgemv_plan.o"),
+    *(("qgemv_stream.cu", [f"-DQGEMV_STREAM_MODE={m}", f"-DQGEMV_STREAM_BF16={b}"], f"qgemv_stream_{m}{b}.o") for m in range(3) for b in range(2)),
 ]
 OBJDIR = CSRC / "build"
 NVCC_FLAGS = [
@@ -42,11 +44,11 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or install the CUDA toolkit (12.8 or newer for sm_100a)")
 
 
-def _stale() -> bool:
-    if not LIB.exists():
+def _stale(target: Path = LIB, patterns=("*.cu", "*.cuh")) -> bool:
+    if not target.exists():
         return True
-    t = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list((PKG.parent / "include").glob("*.h"))
+    t = target.stat().st_mtime
+    deps = [d for pat in patterns for d in CSRC.glob(pat)] + list((PKG.parent / "include").glob("*.h"))
     return any(d.stat().st_mtime > t for d in deps)
 
 

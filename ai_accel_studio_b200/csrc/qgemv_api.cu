@@ -2,7 +2,7 @@
 #include <cstdarg>
 #include <cstdio>
 
-#include "qgemv_common.cuh"
+#include "qgemv_stream.cuh"
 
 namespace qgemv {
 
@@ -38,10 +38,10 @@ int simt_unit_bytes(const qgemv_problem& p) {
     return 1;
 }
 
-int validate(const qgemv_problem* p, size_t need) {
+int validate(const qgemv_problem* p, size_t need, int max_m = QGEMV_MAX_M) {
     if (!p) { set_error("qgemv_run: problem is NULL"); return QGEMV_ERR_BAD_ARG; }
     if (p->bits != 2 && p->bits != 4) { set_error("qgemv_run: bits must be 2 or 4 (got %d)", p->bits); return QGEMV_ERR_BAD_ARG; }
-    if (p->m < 1 || p->m > QGEMV_MAX_M) { set_error("qgemv_run: M must be 1..%d (got %d); larger batches use the dequantise + GEMM path", QGEMV_MAX_M, p->m); return QGEMV_ERR_BAD_ARG; }
+    if (p->m < 1 || p->m > max_m) { set_error("qgemv_run: M must be 1..%d (got %d); larger batches use the dequantise + GEMM path", max_m, p->m); return QGEMV_ERR_BAD_ARG; }
     if (p->n < 1 || p->k_padded < 1 || p->k_original < 1 || p->k_original > p->k_padded) { set_error("qgemv_run: bad N / K (n=%d, k_padded=%d, k_original=%d)", p->n, p->k_padded, p->k_original); return QGEMV_ERR_BAD_ARG; }
     if (!p->x || !p->packed || !p->scales || !p->y) { set_error("qgemv_run: x, packed, scales and y must be non-null"); return QGEMV_ERR_BAD_ARG; }
     if (p->act < QGEMV_ACT_NONE || p->act > QGEMV_ACT_SILU_MUL) { set_error("qgemv_run: unknown activation %d", p->act); return QGEMV_ERR_BAD_ARG; }
@@ -53,7 +53,7 @@ int validate(const qgemv_problem* p, size_t need) {
     const int cpb = 8 / p->bits;
     if (p->group < cpb || p->group % cpb || p->k_padded % p->group) { set_error("qgemv_run: group=%d must be a multiple of %d and divide k_padded=%d", p->group, cpb, p->k_padded); return QGEMV_ERR_SHAPE; }
     if (p->act == QGEMV_ACT_SILU_MUL && p->n % 16) { set_error("qgemv_run: the gated-pair activation needs N to be a multiple of 16 (got %d)", p->n); return QGEMV_ERR_SHAPE; }
-    if (p->ldx < p->k_padded || p->ldy < (p->act == QGEMV_ACT_SILU_MUL ? p->n / 2 : p->n) || p->ldp < (int64_t)p->k_padded / cpb || p->lds < p->k_padded / p->group) { set_error("qgemv_run: a leading dimension is smaller than its row"); return QGEMV_ERR_SHAPE; }
+    if (p->ldx < (max_m > QGEMV_MAX_M ? p->k_original : p->k_padded) || p->ldy < (p->act == QGEMV_ACT_SILU_MUL ? p->n / 2 : p->n) || p->ldp < (int64_t)p->k_padded / cpb || p->lds < p->k_padded / p->group) { set_error("qgemv_run: a leading dimension is smaller than its row"); return QGEMV_ERR_SHAPE; }
     if (p->outliers > 0 && p->ldow < p->outliers) { set_error("qgemv_run: ldow < outliers"); return QGEMV_ERR_SHAPE; }
     if (p->rank > 0 && (p->ldu < p->rank || p->ldv < p->k_original)) { set_error("qgemv_run: ldu < rank or ldv < k_original"); return QGEMV_ERR_SHAPE; }
     if (!aligned(p->x, 2) || !aligned(p->y, 2) || !aligned(p->scales, 2)) { set_error("qgemv_run: 16-bit tensors must be 2-byte aligned"); return QGEMV_ERR_ALIGN; }
@@ -296,4 +296,63 @@ extern "C" int qgemv_workspace_status(const void* workspace, void* stream, int32
 
 extern "C" int qgemv_run(const qgemv_problem* p, void* stream) {
     return run_checked(p, stream, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), kMaxPartialFloats);
+}
+
+// ---- prepared launches, up to 16 rows ------------------------------------------------------------------
+
+namespace {
+struct Prepared {                                  // what qgemv_prepare writes into the caller's buffer
+    qgemv_problem problem;
+    StreamPlan plan;                               // ok == false: as qgemv_run, four rows at a time
+};
+}  // namespace
+
+extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
+
+// The streaming kernel takes what qgemv_run cannot take in one launch -- more than four rows, and x whose rows are not
+// padded to k_padded columns or not 16-byte aligned -- and leaves one to four aligned rows to the kernels above: those
+// launches last about as long as their code takes to arrive in the instruction caches (some 3.5 clocks per instruction on
+// a first pass), and the streaming kernel has more of it (4096 x 4096 INT4, M = 1: 10.8 against 7.1 us).
+extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
+    const size_t need = qgemv_workspace_bytes(0, 0, 0, 0, 0, 0);
+    const int v = validate(p, need, QGEMV_MAX_BATCH);
+    if (v != QGEMV_OK) return v;
+    if (!prepared) { set_error("qgemv_prepare: prepared is NULL"); return QGEMV_ERR_BAD_ARG; }
+    Prepared* q = static_cast<Prepared*>(prepared);
+    q->problem = *p;
+    q->plan = StreamPlan{};
+    const bool padded = p->ldx >= p->k_padded && (p->k_padded == p->k_original || p->m > QGEMV_MAX_BATCH);
+    const qgemv_problem* one = p;
+    if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8) &&
+        plan_stream(&one, 1, kMaxPartialFloats, &q->plan))
+        return QGEMV_OK;
+    q->plan = StreamPlan{};
+    if (p->ldx < p->k_padded || p->k_padded != p->k_original) { set_error("qgemv_prepare: this shape needs x padded to k_padded columns"); return QGEMV_ERR_ALIGN; }
+    bool missing = false;
+    qgemv_problem part = *p;
+    part.m = p->m < QGEMV_MAX_M ? p->m : QGEMV_MAX_M;
+    (void)choose(part, kMaxPartialFloats, &missing);
+    if (missing) { set_error("qgemv_prepare: no kernel of the requested family takes this shape"); return QGEMV_ERR_SHAPE; }
+    return QGEMV_OK;
+}
+
+extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspace, int ordered, void* stream) {
+    Prepared* q = static_cast<Prepared*>(prepared);
+    if (!q || !x || !y || !workspace) { set_error("qgemv_launch_prepared: null pointer"); return QGEMV_ERR_BAD_ARG; }
+    if (q->plan.ok) {
+        if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
+        q->plan.args.x = x;
+        q->plan.args.seg[0].y = y;
+        return launch_stream(q->plan, q->problem.x_dtype == QGEMV_BF16, !ordered, workspace, static_cast<cudaStream_t>(stream));
+    }
+    qgemv_problem p = q->problem;
+    p.workspace = workspace;
+    for (int lo = 0; lo < q->problem.m; lo += QGEMV_MAX_M) {
+        p.m = q->problem.m - lo < QGEMV_MAX_M ? q->problem.m - lo : QGEMV_MAX_M;
+        p.x = static_cast<const char*>(x) + (size_t)lo * p.ldx * 2;
+        p.y = static_cast<char*>(y) + (size_t)lo * p.ldy * 2;
+        const int r = run_checked(&p, stream, 0, kMaxPartialFloats);
+        if (r != QGEMV_OK) return r;
+    }
+    return QGEMV_OK;
 }

@@ -18,9 +18,10 @@ namespace qgemv {
 constexpr int    kMaxRank        = 64;
 constexpr size_t kWsTOff         = 0;
 constexpr size_t kWsCounterOff   = 1024;
-constexpr int    kWsMaxCounters  = 16384;          // the last four entries are not tile counters:
+constexpr int    kWsMaxCounters  = 16384;          // the last entries are not tile counters:
 constexpr int    kWsStatusIdx    = kWsMaxCounters - 1;   //   wait-timeout status word
 constexpr int    kWsDoneIdx      = kWsMaxCounters - 3;   //   CTAs that finished the current launch
+constexpr int    kWsStreamEpochIdx = kWsMaxCounters - 6;  // 64-bit count of streaming launches with residual projections, times 256
 constexpr int    kWsEpochIdx     = kWsMaxCounters - 4;   //   launches completed so far (tag of in-kernel residual projections)
 constexpr size_t kWsPartialOff   = kWsCounterOff + sizeof(int) * kWsMaxCounters;   // 66560, 256-aligned
 constexpr int    kMaxTParts      = 8;              // K-parts of an in-kernel residual projection

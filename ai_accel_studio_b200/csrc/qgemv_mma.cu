@@ -773,7 +773,7 @@ MmaPlan plan_mma(const qgemv_problem& p, size_t partial_floats) {
     pl.ng = p.k_padded / p.group;
     pl.nch = (pl.ng + cg - 1) / cg;
     pl.nt = (p.n + kTileRows - 1) / kTileRows;
-    if (pl.nt > kWsMaxCounters - 4) return pl;          // the last four counters are status / residual bookkeeping
+    if (pl.nt > kWsMaxCounters - 6) return pl;          // the last six counters are status / residual bookkeeping
     if ((long long)pl.nt * pl.nch > 0x3fffffff) return pl;
     const int sms = sm_count();
     // Runs: consecutive chunks of one tile.  One chunk per run unless a CTA would then need more

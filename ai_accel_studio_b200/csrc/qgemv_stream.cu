@@ -1,0 +1,1212 @@
+// Streaming fused GEMV for packed groupwise INT2 / INT4 (and 16-bit) weights, up to 16 activation rows, sm_100a.
+//
+// A decode GEMV is a few microseconds of weight stream wrapped in a chain of short dependent phases; the chain, not HBM,
+// is what bounds it.  This kernel keeps the chain short and the instruction count per weight low:
+//
+//  * Everything that does not depend on x happens before the dependency wait.  Each warp owns a ring of 1 KB slots
+//    (16 weight rows x 64 bytes) filled by cp.async and has it full before `griddepcontrol.wait`.  A CTA takes half an
+//    SM's shared memory and registers, so the next launch of a decode loop is resident beside the running one and
+//    its first ~10 MB of weights are in shared memory when x arrives.
+//  * The warps cut K between them and keep the activations of the 128 columns they work on in registers (mma B fragments),
+//    used for up to four 16-row tiles.  There is no CTA barrier inside the main loop.
+//  * One or two activation rows run on integer tensor cores (mma.m16n8k32, u8 x s8 -> s32; as fast per instruction as the
+//    fp16 one and twice the K).  x is staged as four signed base-256 digits of a 31-bit fixed-point number per 128 columns
+//    -- exact for every element above 2^-20 of the block's largest -- and the digits are columns of B.  A code byte
+//    needs one AND (INT4: `w & 0x0f0f0f0f` and `w & 0xf0f0f0f0`), four codes per instruction; sums are exact integers; the
+//    level offset is the C operand of the first mma; adding 1.5 * 2^23 to the same operand makes the integer result a
+//    float after one subtraction.  About 40 instructions per 16 x 128 weights, where fp16 fragments need about 70.
+//  * 3 - 16 rows run on fp16 tensor cores: `word & mask` leaves one code in the low mantissa bits of each 16-bit half, an
+//    fp16 subnormal worth code * radix^c * 2^-24.  The position classes c accumulate apart and are weighed by radix^-c in
+//    fp32 once per scale group, so x needs no pre-scaling.  Sums of x per group come from the same instruction with an
+//    all-ones A.  bf16 activations become fp16 with a power of two per 128 columns (exact).
+//  * Outlier columns (16-bit weights against the gathered x) are two more mma per tile and 32 columns at the end; the
+//    residual's projections V.x are computed by single warps of a few CTAs and travel as {value, launch tag} words.
+//  * The main loop is kept below the instruction cache of an SM partition (a body of about 16 KB measured 1.8 of 5.8
+//    cycles per instruction waiting for instructions).
+//
+// Replaces _decode_gemv (ai_accel_lab/kernels/decode_int2.py:43-96) and _decode_int4_gemv
+// (ai_accel_lab/kernels/groupwise_int4.py:85-107) of the reference project.
+#include <type_traits>
+
+#include "qgemv_stream.cuh"
+
+namespace qgemv {
+namespace {
+
+// ---------------------------------------------------------------------------------------------
+// PTX helpers
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// 16-byte asynchronous copy that brings the whole 128-byte line to L2; z: only `valid` bytes are read, the rest is zero.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16z(uint32_t dst, const void* src, int valid) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+template <int BYTES> __device__ __forceinline__ void cp_async_small(uint32_t dst, const void* src) {
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global.L2::128B [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait_n() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_async_wait_depth(int depth) {  // all but the newest depth - 1 groups have landed (depth 2 - 4)
+    if (depth == 2) cp_async_wait_n<1>();
+    else if (depth == 3) cp_async_wait_n<2>();
+    else cp_async_wait_n<3>();
+}
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// D = A.B + C with C kept: a chain starts from a register quad that is set up once (a zero literal would be copied into
+// four registers before every chain).
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const float (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const int (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Shared-window loads by 32-bit address: compile-time offsets fold into the instruction.
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v; asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory"); return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v; asm("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory"); return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v; asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory"); return v;
+}
+__device__ __forceinline__ float lds_half(uint32_t a) {
+    uint16_t v; asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory"); return __half2float(__ushort_as_half(v));
+}
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+    unsigned long long v; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory"); return v;
+}
+__device__ __forceinline__ uint32_t lo16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5410); }
+__device__ __forceinline__ uint32_t hi16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+
+// 16-byte piece c of weight row r of a slot sits at piece position c ^ row_swizzle(r): the rows a shared-memory read
+// touches together (2 for 16-byte, 4 for 8-byte, 8 for 4-byte reads) then fall into different banks.
+__device__ __forceinline__ int row_swizzle(int r) { return ((r & 1) << 2) | (r & 2) | ((r >> 2) & 1); }
+// The same for piece p of a staged fp16 activation row (lanes t and t + 2 of a quad read pieces 8 apart).
+__device__ __forceinline__ int x_swizzle(int p) { return p ^ ((p >> 3) & 1); }
+
+constexpr uint32_t kOnesF16 = 0x3C003C00u, kOnesU8 = 0x01010101u;
+constexpr int kMagic = 0x4B400000;                    // 1.5 * 2^23: int sums below 2^22 in magnitude become floats by one subtraction
+constexpr float kMagicF = 12582912.0f;
+
+// kI8: one or two activation rows, integer digits; kF16 / kF16x2: up to 8 / 16 rows.
+enum Mode { kI8 = 0, kF16 = 1, kF16x2 = 2 };
+template <int MODE> struct ModeOf { static constexpr int NB = MODE == kF16x2 ? 2 : 1; };
+
+template <int FMT> struct Fmt {
+    static constexpr bool kPacked = FMT != kDense16;
+    static constexpr int BITS = FMT <= kInt2G64 ? 2 : 4;
+    static constexpr int NG = FMT == kInt2G64 || FMT == kInt4G64 ? 2 : FMT == kInt4G32 ? 4 : 1;   // scale groups per 128 columns
+    static constexpr int KB = BITS == 2 ? 4 : 2;                  // 128-column blocks per slot
+    static constexpr int W = BITS == 2 ? 2 : 4;                   // code words per lane, row and block
+    static constexpr int WG = W / NG;                             // ... per scale group
+};
+
+// ---------------------------------------------------------------------------------------------
+// fp16 path (3 - 16 activation rows)
+// ---------------------------------------------------------------------------------------------
+// Activations of one 128-column block as B fragments (staged in fragment order).  xrow: shared address of the lane's
+// activation row at the block.
+template <int FMT>
+__device__ __forceinline__ void load_frags(uint32_t xrow, int t, uint32_t (&fr)[16]) {
+    using F = Fmt<FMT>;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        int piece;                                    // a block starts at a multiple of 16 pieces: the swizzle depends on the lane alone
+        if constexpr (F::NG == 1) piece = t * 4 + q;
+        else if constexpr (F::NG == 2) piece = (q >> 1) * 8 + t * 2 + (q & 1);
+        else piece = q * 4 + t;
+        const uint4 v = lds128(xrow + (uint32_t)x_swizzle(piece) * 16);
+        fr[q * 4] = v.x; fr[q * 4 + 1] = v.y; fr[q * 4 + 2] = v.z; fr[q * 4 + 3] = v.w;
+    }
+}
+// Two 16-byte pieces of x (16 consecutive columns) in fragment order: INT4 pairs columns (j, j+4) of each piece, INT2 pairs
+// (j, j+8) of both, which is how the codes sit in the two halves of a masked word.
+template <int BITS>
+__device__ __forceinline__ void to_frag_order(uint4& a, uint4& b) {
+    if constexpr (BITS == 4) {
+        a = make_uint4(lo16(a.x, a.z), lo16(a.y, a.w), hi16(a.x, a.z), hi16(a.y, a.w));
+        b = make_uint4(lo16(b.x, b.z), lo16(b.y, b.w), hi16(b.x, b.z), hi16(b.y, b.w));
+    } else {
+        const uint4 p = make_uint4(lo16(a.x, b.x), lo16(a.z, b.z), hi16(a.x, b.x), hi16(a.z, b.z));
+        b = make_uint4(lo16(a.y, b.y), lo16(a.w, b.w), hi16(a.y, b.y), hi16(a.w, b.w));
+        a = p;
+    }
+}
+
+// Sum of x over each scale group of the block, for this lane's activation columns 2t and 2t+1.
+template <int FMT>
+__device__ __forceinline__ void group_sums(const uint32_t (&fr)[16], const float (&zero)[4], float2 (&sx)[Fmt<FMT>::NG]) {
+    constexpr int PER = 8 / Fmt<FMT>::NG;             // B pairs per group
+#pragma unroll
+    for (int j = 0; j < Fmt<FMT>::NG; ++j) {
+        float a[4];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const uint32_t b0 = fr[(j * PER + i) * 2], b1 = fr[(j * PER + i) * 2 + 1];
+            if (i == 0) mma_f16(a, kOnesF16, kOnesF16, kOnesF16, kOnesF16, b0, b1, zero);
+            else mma_f16(a, kOnesF16, kOnesF16, kOnesF16, kOnesF16, b0, b1);
+        }
+        sx[j] = make_float2(a[0], a[1]);
+    }
+}
+
+// y += scale * (level sum) of one tile, block and group of 8 activation rows.
+template <int FMT, bool BF16>
+__device__ __forceinline__ void tile_block(const uint32_t (&w0)[Fmt<FMT>::W], const uint32_t (&w1)[Fmt<FMT>::W], const uint32_t (&fr)[16],
+                                           const float (&zero)[4], const float2 (&sx)[Fmt<FMT>::NG], const float (&s0)[Fmt<FMT>::NG],
+                                           const float (&s1)[Fmt<FMT>::NG], float2 up, float (&y)[4]) {
+    using F = Fmt<FMT>;
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        float c[4];
+        if constexpr (F::BITS == 4) {
+            float a0[4], a1[4];
+#pragma unroll
+            for (int i = 0; i < F::WG; ++i) {
+                constexpr uint32_t M0 = 0x000f000fu, M1 = 0x00f000f0u;
+                const int q = j * F::WG + i;
+                const uint32_t u0 = w0[q], u1 = w1[q], h0 = u0 >> 8, h1 = u1 >> 8;
+                if (i == 0) {
+                    mma_f16(a0, u0 & M0, u1 & M0, h0 & M0, h1 & M0, fr[q * 4], fr[q * 4 + 1], zero);
+                    mma_f16(a1, u0 & M1, u1 & M1, h0 & M1, h1 & M1, fr[q * 4 + 2], fr[q * 4 + 3], zero);
+                } else {
+                    mma_f16(a0, u0 & M0, u1 & M0, h0 & M0, h1 & M0, fr[q * 4], fr[q * 4 + 1]);
+                    mma_f16(a1, u0 & M1, u1 & M1, h0 & M1, h1 & M1, fr[q * 4 + 2], fr[q * 4 + 3]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[e] = fmaf(a1[e], 1.0f / 16.0f, a0[e]);
+        } else {
+            float a[4][4];
+#pragma unroll
+            for (int i = 0; i < F::WG; ++i) {
+                const int q = j * F::WG + i;
+                const uint32_t u0 = w0[q], u1 = w1[q], h0 = u0 >> 8, h1 = u1 >> 8;
+#pragma unroll
+                for (int cl = 0; cl < 4; ++cl) {
+                    const uint32_t mk = 0x00030003u << (2 * cl);
+                    if (i == 0) mma_f16(a[cl], u0 & mk, u1 & mk, h0 & mk, h1 & mk, fr[q * 8 + cl * 2], fr[q * 8 + cl * 2 + 1], zero);
+                    else mma_f16(a[cl], u0 & mk, u1 & mk, h0 & mk, h1 & mk, fr[q * 8 + cl * 2], fr[q * 8 + cl * 2 + 1]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                c[e] = fmaf(fmaf(fmaf(a[3][e], 0.25f, a[2][e]), 0.25f, a[1][e]), 0.25f, a[0][e]);
+        }
+        // INT2 levels are (2c - 3) / 3, INT4 levels c - 8; codes carry the subnormal unit 2^-24
+        constexpr float kUnit = F::BITS == 4 ? 16777216.0f : 16777216.0f * (2.0f / 3.0f);
+        const float oa = F::BITS == 4 ? 8.0f * sx[j].x : sx[j].x, ob = F::BITS == 4 ? 8.0f * sx[j].y : sx[j].y;
+        float t0 = fmaf(c[0], kUnit, -oa), t1 = fmaf(c[1], kUnit, -ob), t2 = fmaf(c[2], kUnit, -oa), t3 = fmaf(c[3], kUnit, -ob);
+        if constexpr (BF16) { t0 *= up.x; t1 *= up.y; t2 *= up.x; t3 *= up.y; }
+        y[0] = fmaf(s0[j], t0, y[0]); y[1] = fmaf(s0[j], t1, y[1]);
+        y[2] = fmaf(s1[j], t2, y[2]); y[3] = fmaf(s1[j], t3, y[3]);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// integer path (1 - 2 activation rows): column 4 m + d of B is base-256 digit d of activation row m
+// ---------------------------------------------------------------------------------------------
+// kfac: what a unit of the integer sum is worth (INT4 sums 16 c - 128 or, in groups of 32, c - 8; INT2 sums 4 c - 6).
+template <int FMT> __device__ __forceinline__ constexpr float digit_unit() {
+    return Fmt<FMT>::BITS == 2 ? 1.0f / 6.0f : FMT == kInt4G32 ? 1.0f : 1.0f / 16.0f;
+}
+// Digits of 16 consecutive columns, by digit plane, in the order the code bytes meet them: B register pairs side by side.
+// ORDER 2: INT2, position classes 0, 2, 1, 3 of a word's bytes; 4: INT4, the even codes of two words, then the odd ones;
+// 32: INT4 in groups of 32, even and odd codes of each word.
+template <int ORDER>
+__device__ __forceinline__ void digit_planes(const float (&f)[16], float down, uint4 (&plane)[4]) {
+    uint32_t z[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) z[i] = ((uint32_t)__float2int_rn(f[i] * down) + 0x00808080u) ^ 0x00808080u;      // signed bytes
+    uint32_t r[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int o = ORDER == 2 ? (q & 1) * 2 + (q >> 1) : ORDER == 4 ? (q & 1) * 8 + (q >> 1) : (q >> 1) * 8 + (q & 1);
+        const int step = ORDER == 2 ? 4 : 2;
+        const uint32_t a = z[o], b = z[o + step], c = z[o + 2 * step], d = z[o + 3 * step];
+        const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(a, b, 0x7362), t2 = __byte_perm(c, d, 0x5140), t3 = __byte_perm(c, d, 0x7362);
+        r[0][q] = __byte_perm(t0, t2, 0x5410); r[1][q] = __byte_perm(t0, t2, 0x7632);
+        r[2][q] = __byte_perm(t1, t3, 0x5410); r[3][q] = __byte_perm(t1, t3, 0x7632);
+    }
+#pragma unroll
+    for (int d = 0; d < 4; ++d) plane[d] = make_uint4(r[d][0], r[d][1], r[d][2], r[d][3]);
+}
+// Position of 16-column unit u of a block inside a column's 128 bytes.
+__device__ __forceinline__ int digit_unit_pos(int u, int col) { return (u ^ (col & 1)) * 16; }
+
+template <int FMT>
+__device__ __forceinline__ void load_digits(uint32_t xcol, int col, int t, uint32_t (&fr)[8]) {
+    using F = Fmt<FMT>;
+    if constexpr (F::NG == 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint2 v = lds64(xcol + (uint32_t)(digit_unit_pos(j * 2 + (t >> 1), col) + (t & 1) * 8));
+            fr[j * 2] = v.x; fr[j * 2 + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const uint4 v = lds128(xcol + (uint32_t)digit_unit_pos(F::NG == 1 ? t * 2 + q : q * 4 + t, col));
+            fr[q * 4] = v.x; fr[q * 4 + 1] = v.y; fr[q * 4 + 2] = v.z; fr[q * 4 + 3] = v.w;
+        }
+    }
+}
+// C operand of each group's chain: magic - offset * (sum of the digits), for columns 2t and 2t+1.
+template <int FMT>
+__device__ __forceinline__ void digit_offsets(const uint32_t (&fr)[8], const int (&zero)[4], int (&ci)[Fmt<FMT>::NG][4]) {
+    using F = Fmt<FMT>;
+    constexpr int PER = 4 / F::NG, OFF = F::BITS == 2 ? 6 : FMT == kInt4G32 ? 8 : 128;
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        int a[4];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const uint32_t b0 = fr[(j * PER + i) * 2], b1 = fr[(j * PER + i) * 2 + 1];
+            if (i == 0) mma_s8(a, kOnesU8, kOnesU8, kOnesU8, kOnesU8, b0, b1, zero);
+            else mma_s8(a, kOnesU8, kOnesU8, kOnesU8, kOnesU8, b0, b1);
+        }
+        ci[j][0] = ci[j][2] = kMagic - OFF * a[0];
+        ci[j][1] = ci[j][3] = kMagic - OFF * a[1];
+    }
+}
+template <int FMT>
+__device__ __forceinline__ void tile_block_s8(const uint32_t (&w0)[Fmt<FMT>::W], const uint32_t (&w1)[Fmt<FMT>::W], const uint32_t (&fr)[8],
+                                              const int (&zero)[4], const int (&ci)[Fmt<FMT>::NG][4], const float (&s0)[Fmt<FMT>::NG],
+                                              const float (&s1)[Fmt<FMT>::NG], float up, float (&y)[4]) {
+    using F = Fmt<FMT>;
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        int v[4];
+        if constexpr (FMT == kInt4G32) {
+            constexpr uint32_t L = 0x0f0f0f0fu;
+            mma_s8(v, w0[j] & L, w1[j] & L, (w0[j] >> 4) & L, (w1[j] >> 4) & L, fr[j * 2], fr[j * 2 + 1], ci[j]);
+        } else if constexpr (F::BITS == 4) {
+            constexpr uint32_t L = 0x0f0f0f0fu, H = 0xf0f0f0f0u;
+            int a0[4];
+#pragma unroll
+            for (int i = 0; i < F::WG; i += 2) {
+                const int q = j * F::WG + i;
+                if (i == 0) {
+                    mma_s8(a0, w0[q] & L, w1[q] & L, w0[q + 1] & L, w1[q + 1] & L, fr[q * 2], fr[q * 2 + 1], zero);
+                    mma_s8(v, w0[q] & H, w1[q] & H, w0[q + 1] & H, w1[q + 1] & H, fr[q * 2 + 2], fr[q * 2 + 3], ci[j]);
+                } else {
+                    mma_s8(a0, w0[q] & L, w1[q] & L, w0[q + 1] & L, w1[q + 1] & L, fr[q * 2], fr[q * 2 + 1]);
+                    mma_s8(v, w0[q] & H, w1[q] & H, w0[q + 1] & H, w1[q + 1] & H, fr[q * 2 + 2], fr[q * 2 + 3]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] += a0[e] << 4;
+        } else {
+            constexpr uint32_t A = 0x03030303u, B = 0x0c0c0c0cu;
+            int a0[4];
+#pragma unroll
+            for (int i = 0; i < F::WG; ++i) {
+                const int q = j * F::WG + i;
+                const uint32_t h0 = w0[q] >> 4, h1 = w1[q] >> 4;
+                if (i == 0) {
+                    mma_s8(a0, w0[q] & A, w1[q] & A, h0 & A, h1 & A, fr[q * 4], fr[q * 4 + 1], zero);
+                    mma_s8(v, w0[q] & B, w1[q] & B, h0 & B, h1 & B, fr[q * 4 + 2], fr[q * 4 + 3], ci[j]);
+                } else {
+                    mma_s8(a0, w0[q] & A, w1[q] & A, h0 & A, h1 & A, fr[q * 4], fr[q * 4 + 1]);
+                    mma_s8(v, w0[q] & B, w1[q] & B, h0 & B, h1 & B, fr[q * 4 + 2], fr[q * 4 + 3]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] += a0[e] << 2;
+        }
+        const float u0 = s0[j] * up, u1 = s1[j] * up;
+        y[0] = fmaf(u0, __int_as_float(v[0]) - kMagicF, y[0]); y[1] = fmaf(u0, __int_as_float(v[1]) - kMagicF, y[1]);
+        y[2] = fmaf(u1, __int_as_float(v[2]) - kMagicF, y[2]); y[3] = fmaf(u1, __int_as_float(v[3]) - kMagicF, y[3]);
+    }
+}
+
+// Byte offsets of this lane's code words in a slot row, for block 0 (block kb: XOR kb * W * 16, the bits do not overlap).
+template <int FMT>
+__device__ __forceinline__ void code_offsets(int t, int sw, uint32_t (&o)[Fmt<FMT>::NG]) {
+    using F = Fmt<FMT>;
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        const int byte = F::WG == 4 ? t * 16 : F::WG == 2 ? j * 32 + t * 8 : j * 16 + t * 4;
+        o[j] = (uint32_t)((((byte >> 4) ^ sw) << 4) + (byte & 15));
+    }
+}
+// Code words of one tile and block: rows g (w0) and g + 8 (w1).
+template <int FMT>
+__device__ __forceinline__ void load_codes(uint32_t row0, const uint32_t (&o)[Fmt<FMT>::NG], uint32_t block, uint32_t (&w0)[Fmt<FMT>::W], uint32_t (&w1)[Fmt<FMT>::W]) {
+    using F = Fmt<FMT>;
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        const uint32_t at = row0 + (o[j] ^ block);
+        if constexpr (F::WG == 4) {
+            const uint4 a = lds128(at), b = lds128(at + 8 * kSlotRowBytes);
+            w0[0] = a.x; w0[1] = a.y; w0[2] = a.z; w0[3] = a.w;
+            w1[0] = b.x; w1[1] = b.y; w1[2] = b.z; w1[3] = b.w;
+        } else if constexpr (F::WG == 2) {
+            const uint2 a = lds64(at), b = lds64(at + 8 * kSlotRowBytes);
+            w0[j * 2] = a.x; w0[j * 2 + 1] = a.y;
+            w1[j * 2] = b.x; w1[j * 2 + 1] = b.y;
+        } else {
+            w0[j] = lds32(at);
+            w1[j] = lds32(at + 8 * kSlotRowBytes);
+        }
+    }
+}
+
+struct Ctx {                                          // what a warp needs in its main loop
+    uint32_t ring, x, up;
+    unsigned char* sx;                                // this warp's table of group sums (fp16 path)
+    int lane, g, t, sw;
+    int tiles, rows, row0, nrb;                       // this warp's tiles and rows, first row inside the CTA, row blocks
+    int s0, s1, sbase;                                // this warp's weight slots, first slot of the CTA's K slice
+    int rowbase;                                      // first row of the CTA in the matrix
+    int M;
+};
+
+// Rare producer paths, out of line and by value (the main loop has to stay inside the instruction cache, and a pointer to
+// the producer would move it to local memory).
+// A batch at the edge of the matrix: rows past `left` (counted from this lane's first row) and pieces past the row's end are zero.
+__device__ __noinline__ void edge_batch(uint32_t d, const uint8_t* src, size_t step, const uint8_t* any, int n, int left, bool piece_ok) {
+    const uint32_t even = d, odd = d ^ 16u;
+    for (int i = 0; i < n; ++i) {
+        const bool ok = piece_ok && i * 4 < left;
+        cp_async16z(((i & 1) ? odd : even) + i * (4 * kSlotRowBytes), ok ? src : any, ok ? 16 : 0);
+        src += step;
+    }
+}
+// Scales of a row whose copies are not aligned, or that run past the row's end.
+__device__ __noinline__ void odd_scales(uint32_t d, const __half* src, int count, int left) {
+    for (int i = 0; i < count; ++i) {
+        const unsigned short v = i < left ? __half_as_ushort(__ldg(src + i)) : 0;
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(d + i * 2), "h"(v) : "memory");
+    }
+}
+
+// Producer side of a warp's ring: batches in the order (row block, slot); a batch is one slot (16 rows x 128 bytes and their
+// scales) per tile of the row block.  The fields the hot path uses are copied out of the kernel parameter: indexed by the
+// segment, a parameter read is a load with a latency of its own.
+template <int FMT, int T>
+struct Producer {
+    using F = Fmt<FMT>;
+    static constexpr int EPS = F::KB * F::NG;         // scale groups per slot (groups of 64 and less, or 128)
+    static constexpr int BATCH = T * kSlotBytes;
+    const uint8_t* src;                               // row lane/8 of the row block, piece lane%8, next slot
+    size_t step;                                      // four rows
+    size_t block_step;                                // from the end of a row block's slots to the start of the next one
+    const __half* sp;                                 // scale row of row `lane` of the row block
+    long long sc_step;                                // scale elements per row block
+    int left;                                         // batches still to be requested
+    int s, s0, s1, rows;                              // rows: of this warp from the row block on
+    int s_lim, s_whole;                               // slots in which this lane's piece / the whole slot lies inside the row
+    int gshift, ng, lane, sc_count, sc_mask;          // scale groups a slot needs, and the mask that aligns the first one
+    bool sc_fast;
+    uint32_t dst, sc_dst, at, end;                    // ring offset of the next batch, size of the ring
+
+    __device__ __forceinline__ Producer(const Ctx& c, const StreamSeg& sg) {
+        const int r = c.lane >> 3, piece = c.lane & 7;
+        src = sg.w + (size_t)(c.rowbase + c.row0 + r) * sg.ldw + piece * 16 + (size_t)c.s0 * kSlotRowBytes;
+        step = (size_t)4 * sg.ldw;
+        block_step = (size_t)(T * 4) * step - (size_t)(c.s1 - c.s0) * kSlotRowBytes;
+        s = c.s0; s0 = c.s0; s1 = c.s1; rows = c.rows; lane = c.lane;
+        left = c.nrb * (c.s1 - c.s0);
+        s_lim = (sg.row_bytes - piece * 16 + kSlotRowBytes - 1) / kSlotRowBytes;
+        s_whole = sg.row_bytes / kSlotRowBytes;
+        gshift = sg.gshift; ng = sg.ng;
+        sc_fast = (sg.flags & kSegScaleAligned) != 0;
+        sc_count = max(2, EPS >> gshift);              // at least the 4 bytes of the smallest copy
+        sc_mask = sc_count > (EPS >> gshift) ? ~1 : ~0;
+        dst = c.ring + (uint32_t)(r * kSlotRowBytes + ((piece ^ row_swizzle(r)) << 4));
+        sp = sg.sc + (size_t)(c.rowbase + c.row0 + c.lane) * sg.lds;
+        sc_step = sg.lds * (T * kStreamTileRows);
+        sc_dst = c.ring + T * kTileBytes + c.lane * 16;
+        at = 0; end = (uint32_t)(sg.depth * BATCH);
+    }
+
+    __device__ __forceinline__ void issue(const StreamSeg& sg) {
+        if (left > 0) {
+            const uint32_t d = dst + at;
+            const uint8_t* from = src;
+            if (rows >= T * kStreamTileRows && s < s_whole) {
+#pragma unroll
+                for (int i = 0; i < 4 * T; ++i) {                          // rows 4 i + lane / 8: the swizzle of row + 4 flips one piece bit
+                    cp_async16(((i & 1) ? d ^ 16u : d) + i * (4 * kSlotRowBytes), from);
+                    from += step;
+                }
+            } else {
+                edge_batch(d, from, step, sg.w, 4 * T, rows - (lane >> 3), s < s_lim);
+            }
+            if constexpr (F::kPacked) {
+                const int e = (F::NG > 1 ? s * EPS : (s * F::KB) >> gshift) & sc_mask;        // first scale group of the copy
+                if (lane < min(T * kStreamTileRows, rows)) {
+                    if (sc_fast && e + sc_count <= ng) {
+                        if (EPS >= 8 && sc_count == 8) cp_async_small<16>(sc_dst + at, sp + e);
+                        else if (EPS >= 4 && sc_count == 4) cp_async_small<8>(sc_dst + at, sp + e);
+                        else cp_async_small<4>(sc_dst + at, sp + e);
+                    } else {
+                        odd_scales(sc_dst + at, sp + e, sc_count, ng - e);
+                    }
+                }
+            }
+            --left;
+            src += kSlotRowBytes;
+            at = at + BATCH == end ? 0u : at + BATCH;
+            if (++s == s1) {
+                s = s0;
+                src += block_step;
+                sp += sc_step;
+                rows -= T * kStreamTileRows;
+            }
+        }
+        cp_async_commit();
+    }
+};
+
+// Main loop of one warp over its share of one matrix, for one weight format and T tiles per row block.  The tiles are
+// straight-line code (their loads and mma chains overlap), the blocks of a slot a loop: the body has to stay well inside
+// the 512 instructions that an SM partition caches (beyond them every pass costs 2 - 3 clocks per instruction more, measured).
+// The last row block computes a tile past the end on stale data and drops it.  `part`: this warp's K share of the row sums,
+// [row][m].
+template <int FMT, int T, int MODE, bool BF16>
+__device__ __forceinline__ void stream_loop(const Ctx& c, const StreamSeg& sg, Producer<FMT, T>& prod, float* part) {
+    using F = Fmt<FMT>;
+    constexpr int NB = ModeOf<MODE>::NB;
+    constexpr bool kInt = MODE == kI8 && FMT != kDense16;
+    const int M = c.M, depth = sg.depth, nrb = c.nrb, mp = sg.mp, gshift = sg.gshift;
+    const uint32_t row_u32 = c.ring + (uint32_t)(c.g * kSlotRowBytes);
+    constexpr uint32_t BATCH = T * kSlotBytes;
+    const uint32_t sc_lane = T * kTileBytes + c.g * 16 - c.g * kSlotRowBytes;               // from the lane's row of a batch to its scales
+    uint32_t co[F::NG];
+    code_offsets<FMT>(c.t, c.sw, co);
+    // this lane's activation row / digit column
+    uint32_t xrow[NB];
+    const int col = M == 1 ? (c.g & 3) : c.g;                    // digit column (integer path)
+    if constexpr (kInt) xrow[0] = c.x + (uint32_t)col * 128;
+    else {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) xrow[b] = c.x + (uint32_t)min(b * 8 + c.g, M - 1) * (uint32_t)sg.xpitch;
+    }
+    const uint32_t up_u32 = c.up + (uint32_t)min(c.t >> 1, M - 1) * 4;                     // integer path
+    float zf[4]; int zi[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { asm volatile("mov.b32 %0, 0;" : "=f"(zf[e])); asm volatile("mov.b32 %0, 0;" : "=r"(zi[e])); }
+    const int sc_mask = prod.sc_mask;
+    const uint32_t end = row_u32 + prod.end;
+    uint32_t slot = row_u32;                          // the lane's row in the current batch
+    for (int rb = 0; rb < nrb; ++rb) {
+        float y[T][NB][4];
+#pragma unroll
+        for (int ti = 0; ti < T; ++ti)
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[ti][b][e] = 0.0f;
+
+        for (int s = c.s0; s < c.s1; ++s) {
+            cp_async_wait_depth(depth);
+            __syncwarp();
+            if constexpr (F::kPacked) {
+                const int b0 = (s - c.sbase) * F::KB;                                      // the slot's first block in the CTA's slice
+                uint32_t xa[NB], ua = kInt ? up_u32 + (uint32_t)(b0 * M) * 4 : c.up + (uint32_t)(b0 * M) * 4;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) xa[b] = xrow[b] + (uint32_t)b0 * (kInt ? (uint32_t)M * 512 : 256u);
+                float2* tab = reinterpret_cast<float2*>(c.sx) + (size_t)(s - c.s0) * (F::KB * F::NG * NB * 4) + c.t;
+                uint32_t sa = slot + sc_lane;
+                const int e0 = F::NG > 1 ? 0 : ((s * F::KB) >> gshift) & sc_mask;
+#pragma unroll 1
+                for (int kk = 0; kk < F::KB; ++kk) {
+                    const uint32_t sc0 = F::NG > 1 || gshift == 0 ? sa : slot + sc_lane + (uint32_t)((((s * F::KB + kk) >> gshift) - e0) * 2);
+                    auto tile_operands = [&](int ti, uint32_t (&w0)[F::W], uint32_t (&w1)[F::W], float (&s0)[F::NG], float (&s1)[F::NG]) {
+                        load_codes<FMT>(slot + ti * kTileBytes, co, (uint32_t)(kk * (F::W * 16)), w0, w1);
+#pragma unroll
+                        for (int j = 0; j < F::NG; ++j) {
+                            s0[j] = lds_half(sc0 + ti * (kStreamTileRows * 16) + j * 2);
+                            s1[j] = lds_half(sc0 + (ti * kStreamTileRows + 8) * 16 + j * 2);
+                        }
+                    };
+                    if constexpr (kInt) {
+                        uint32_t fr[8];
+                        int ci[F::NG][4];
+                        load_digits<FMT>(xa[0], col, c.t, fr);
+                        const float up = __uint_as_float(lds32(ua));
+                        digit_offsets<FMT>(fr, zi, ci);
+#pragma unroll
+                        for (int ti = 0; ti < T; ++ti) {
+                            uint32_t w0[F::W], w1[F::W];
+                            float s0[F::NG], s1[F::NG];
+                            tile_operands(ti, w0, w1, s0, s1);
+                            tile_block_s8<FMT>(w0, w1, fr, zi, ci, s0, s1, up, y[ti][0]);
+                        }
+                    } else {
+                        uint32_t fr[NB][16];
+                        float2 sx[NB][F::NG], up[NB];
+#pragma unroll
+                        for (int b = 0; b < NB; ++b) {
+                            load_frags<FMT>(xa[b], c.t, fr[b]);
+                            if (rb == 0) {
+                                group_sums<FMT>(fr[b], zf, sx[b]);
+                                if (nrb > 1 && c.g == 0) {
+#pragma unroll
+                                    for (int j = 0; j < F::NG; ++j) tab[(b * F::NG + j) * 4] = sx[b][j];
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < F::NG; ++j) sx[b][j] = tab[(b * F::NG + j) * 4];
+                            }
+                            up[b] = make_float2(1.0f, 1.0f);
+                            if constexpr (BF16) {
+                                up[b].x = __uint_as_float(lds32(ua + (uint32_t)min(b * 8 + 2 * c.t, M - 1) * 4));
+                                up[b].y = __uint_as_float(lds32(ua + (uint32_t)min(b * 8 + 2 * c.t + 1, M - 1) * 4));
+                            }
+                        }
+#pragma unroll
+                        for (int ti = 0; ti < T; ++ti) {
+                            uint32_t w0[F::W], w1[F::W];
+                            float s0[F::NG], s1[F::NG];
+                            tile_operands(ti, w0, w1, s0, s1);
+#pragma unroll
+                            for (int b = 0; b < NB; ++b) tile_block<FMT, BF16>(w0, w1, fr[b], zf, sx[b], s0, s1, up[b], y[ti][b]);
+                        }
+                        tab += F::NG * NB * 4;
+                    }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) xa[b] += kInt ? (uint32_t)M * 512 : 256u;
+                    ua += (uint32_t)M * 4;
+                    sa += F::NG * 2;
+                }
+            } else {                                  // 16-bit weights: 64 columns per slot
+#pragma unroll 1
+              for (int kk = 0; kk < 2; ++kk) {
+                uint4 xv[NB];
+#pragma unroll
+                for (int b = 0; b < NB; ++b) xv[b] = lds128(xrow[b] + (uint32_t)x_swizzle((s - c.sbase) * 8 + kk * 4 + c.t) * 16);
+                const uint32_t o = (uint32_t)(((kk * 4 + c.t) ^ c.sw) << 4);
+#pragma unroll
+                for (int ti = 0; ti < T; ++ti) {
+                    const uint4 a = lds128(slot + ti * kTileBytes + o), d = lds128(slot + ti * kTileBytes + 8 * kSlotRowBytes + o);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        if constexpr (BF16) {
+                            mma_bf16(y[ti][b], a.x, d.x, a.y, d.y, xv[b].x, xv[b].y);
+                            mma_bf16(y[ti][b], a.z, d.z, a.w, d.w, xv[b].z, xv[b].w);
+                        } else {
+                            mma_f16(y[ti][b], a.x, d.x, a.y, d.y, xv[b].x, xv[b].y);
+                            mma_f16(y[ti][b], a.z, d.z, a.w, d.w, xv[b].z, xv[b].w);
+                        }
+                    }
+                }
+              }
+            }
+            __syncwarp();                             // every lane has read the batch before its slots are refilled
+            prod.issue(sg);
+            slot = slot + BATCH == end ? row_u32 : slot + BATCH;
+        }
+        // park this row block's sums of the warp's K share
+#pragma unroll
+        for (int ti = 0; ti < T; ++ti) {
+            if (rb * T + ti < c.tiles) {              // uniform
+                float* dst = part + (size_t)(c.row0 + (rb * T + ti) * kStreamTileRows + c.g) * mp;
+                if constexpr (kInt) {                 // the quad's digits meet: lanes 0, 1 hold row 0's, lanes 2, 3 row 1's
+                    const float wgt = (c.t & 1) ? 65536.0f : 1.0f;
+                    float v0 = fmaf(y[ti][0][1], 256.0f, y[ti][0][0]) * wgt, v1 = fmaf(y[ti][0][3], 256.0f, y[ti][0][2]) * wgt;
+                    v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
+                    v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
+                    if (!(c.t & 1) && (c.t >> 1) < M) { dst[c.t >> 1] = v0; dst[8 * mp + (c.t >> 1)] = v1; }
+                } else {
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        const int m = b * 8 + 2 * c.t;
+                        if (m < M) {
+                            *reinterpret_cast<float2*>(dst + m) = make_float2(y[ti][b][0], y[ti][b][1]);
+                            *reinterpret_cast<float2*>(dst + 8 * mp + m) = make_float2(y[ti][b][2], y[ti][b][3]);
+                        }
+                    }
+                }
+            }
+        }
+    }
+    cp_async_wait_n<0>();
+}
+
+// Runs f with the segment's weight format and tiles per row block as compile-time constants.
+template <typename F>
+__device__ __forceinline__ void with_shape(int fmt, int T, F f) {
+    auto tiles = [&](auto fmt_c) {
+        if (T == 1) f(fmt_c, std::integral_constant<int, 1>{});
+        else f(fmt_c, std::integral_constant<int, 2>{});
+    };
+    switch (fmt) {
+        case kInt2G128: tiles(std::integral_constant<int, kInt2G128>{}); break;
+        case kInt2G64: tiles(std::integral_constant<int, kInt2G64>{}); break;
+        case kInt4G128: tiles(std::integral_constant<int, kInt4G128>{}); break;
+        case kInt4G64: tiles(std::integral_constant<int, kInt4G64>{}); break;
+        case kInt4G32: tiles(std::integral_constant<int, kInt4G32>{}); break;
+        default: tiles(std::integral_constant<int, kDense16>{}); break;
+    }
+}
+
+// Eight activations of row m from column k, zero past the last column.
+template <bool BF16>
+__device__ __forceinline__ uint4 load_x8(const StreamArgs& p, int m, int k) {
+    using XT = typename Act16<BF16>::T;
+    const XT* src = static_cast<const XT*>(p.x) + (size_t)m * p.ldx + k;
+    if (p.xaligned && k + 8 <= p.korig) return *reinterpret_cast<const uint4*>(src);
+    uint32_t e[4] = {0u, 0u, 0u, 0u};
+    if (k < p.korig) {
+        const unsigned short* s16 = reinterpret_cast<const unsigned short*>(src);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t lo = k + 2 * q < p.korig ? s16[2 * q] : 0, hi = k + 2 * q + 1 < p.korig ? s16[2 * q + 1] : 0;
+            e[q] = lo | (hi << 16);
+        }
+    }
+    return make_uint4(e[0], e[1], e[2], e[3]);
+}
+template <bool BF16>
+__device__ __forceinline__ void widen8(const uint4& v, float* f) {
+    using XT = typename Act16<BF16>::T;
+    const XT* e = reinterpret_cast<const XT*>(&v);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) f[q] = Act16<BF16>::to_float(e[q]);
+}
+// Exponent of a block's largest magnitude (given as float bits), limited to where 2^(30 - e) and 2^(e - 29) are normal.
+__device__ __forceinline__ int block_exponent(uint32_t bits) { return max(-96, (int)(bits >> 23) - 127); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+constexpr uint32_t kInfBits = 0x7f800000u;
+
+// x of the CTA's K slice to shared memory, in the form the segment's main loop reads.
+template <int MODE, bool BF16>
+__device__ __forceinline__ void stage_x(const StreamArgs& p, const StreamSeg& sg, unsigned char* smem, int slice_k0, int tid, int nthr) {
+    const int M = p.m, nu = sg.np / 2, total = M * nu;          // units of 16 columns
+    const bool dense = sg.fmt == kDense16, two = sg.fmt <= kInt2G64;
+    for (int base = 0; base < total; base += 2 * nthr) {
+        uint4 v[2][2];
+        int mm[2], uu[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int i = base + r * nthr + tid;
+            mm[r] = -1; uu[r] = 0;
+            v[r][0] = v[r][1] = make_uint4(0u, 0u, 0u, 0u);
+            if (i < total) {
+                mm[r] = (int)__umulhi((unsigned)i, (unsigned)sg.nu_magic);
+                uu[r] = i - mm[r] * nu;
+                v[r][0] = load_x8<BF16>(p, mm[r], slice_k0 + uu[r] * 16);
+                v[r][1] = load_x8<BF16>(p, mm[r], slice_k0 + uu[r] * 16 + 8);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (base + r * nthr >= total) continue;             // uniform
+            const int m = mm[r], u = uu[r];
+            if (!dense && (MODE == kI8 || BF16)) {
+                float f[16];
+                widen8<BF16>(v[r][0], f);
+                widen8<BF16>(v[r][1], f + 8);
+                uint32_t big = 0;
+#pragma unroll
+                for (int q = 0; q < 16; ++q) big = max(big, __float_as_uint(f[q]) & 0x7fffffffu);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));     // 8 lanes hold one block
+                const int e = block_exponent(big);
+                float* up = reinterpret_cast<float*>(smem + sg.off_up) + (size_t)(u >> 3) * M + m;
+                const bool first = m >= 0 && (u & 7) == 0;
+                if constexpr (MODE == kI8) {
+                    if (first) *up = big >= kInfBits ? __int_as_float(0x7fffffff)
+                                                     : pow2f(e - 29) * (two ? 1.0f / 6.0f : sg.fmt == kInt4G32 ? 1.0f : 1.0f / 16.0f);
+                    uint4 plane[4];
+                    const float down = pow2f(29 - e);
+                    if (two) digit_planes<2>(f, down, plane); else if (sg.fmt == kInt4G32) digit_planes<32>(f, down, plane); else digit_planes<4>(f, down, plane);
+                    if (m >= 0) {
+#pragma unroll
+                        for (int d = 0; d < 4; ++d)
+                            *reinterpret_cast<uint4*>(smem + ((size_t)((u >> 3) * M + m) * 4 + d) * 128 + digit_unit_pos(u & 7, m * 4 + d)) = plane[d];
+                    }
+                    continue;
+                } else {
+                    if (first) *up = big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
+                    const float down = pow2f(13 - e);
+                    uint32_t h[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const __half2 hh = __floats2half2_rn(f[2 * q] * down, f[2 * q + 1] * down);
+                        h[q] = *reinterpret_cast<const uint32_t*>(&hh);
+                    }
+                    v[r][0] = make_uint4(h[0], h[1], h[2], h[3]);
+                    v[r][1] = make_uint4(h[4], h[5], h[6], h[7]);
+                }
+            }
+            if (!dense) { if (two) to_frag_order<2>(v[r][0], v[r][1]); else to_frag_order<4>(v[r][0], v[r][1]); }
+            if (m >= 0) {
+                unsigned char* row = smem + (size_t)m * sg.xpitch;
+                *reinterpret_cast<uint4*>(row + x_swizzle(2 * u) * 16) = v[r][0];
+                *reinterpret_cast<uint4*>(row + x_swizzle(2 * u + 1) * 16) = v[r][1];
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The kernel: p.nw warps stream, one more (the last) gathers outlier activations and deals with the residual projections.
+// ---------------------------------------------------------------------------------------------
+template <int MODE, bool BF16>
+__global__ void __launch_bounds__(MODE == kF16x2 ? 288 : 544, 1) qgemv_stream_kernel(const __grid_constant__ StreamArgs p) {
+    using XT = typename Act16<BF16>::T;
+    constexpr int NB = ModeOf<MODE>::NB;
+    extern __shared__ __align__(128) unsigned char smem[];
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, M = p.m;
+    int si = 0;
+    while (si + 1 < p.nseg && (int)blockIdx.x >= p.seg[si + 1].cta0) ++si;
+    const StreamSeg& sg = p.seg[si];
+    const int cta = (int)blockIdx.x - sg.cta0;
+    const int split = cta / sg.groups, grp = cta - split * sg.groups;      // consecutive CTAs: row groups of one K split
+    const int rowbase = grp * sg.rows_per, rows = min(sg.rows_per, sg.n - rowbase);
+    const bool aux = warp == p.nw;
+
+    Ctx c;
+    c.M = M;
+    c.lane = lane; c.g = lane >> 2; c.t = lane & 3; c.sw = row_swizzle(c.g);
+    const int wk = aux ? sg.wk : warp / sg.wr, wrow = warp - wk * sg.wr;
+    c.sbase = split * sg.ns_split;
+    const int ns = min(sg.ns_split, sg.ns - c.sbase);                      // weight slots of this CTA's K slice, cut into wk runs
+    c.s0 = c.sbase + (wk < sg.wk ? wk * ns / sg.wk : ns);
+    c.s1 = c.sbase + (wk < sg.wk ? (wk + 1) * ns / sg.wk : ns);
+    const int tiles = (rows + kStreamTileRows - 1) / kStreamTileRows;
+    const int t0 = wrow * sg.tiles_w;
+    c.tiles = max(0, min(sg.tiles_w, tiles - t0));
+    c.row0 = t0 * kStreamTileRows;
+    c.rows = max(0, min(rows - c.row0, c.tiles * kStreamTileRows));
+    c.rowbase = rowbase;
+    c.x = smem_u32(smem);
+    c.up = smem_u32(smem + sg.off_up);
+    c.sx = smem + sg.off_sx + (size_t)warp * sg.sx_bytes;
+    c.ring = smem_u32(smem + sg.off_ring + (size_t)warp * sg.depth * sg.T * kSlotBytes);
+    c.nrb = c.s1 > c.s0 ? (c.tiles + sg.T - 1) / sg.T : 0;
+    const int slot_cols = sg.fmt == kDense16 ? 64 : sg.fmt <= kInt2G64 ? 512 : 256;
+    const int slice_k0 = c.sbase * slot_cols;
+    const bool has_o = sg.noc > 0 && split == sg.ksplit - 1;
+    const bool finisher = sg.ksplit == 1;               // else: decided by arrival
+    const int oc_pad = sg.noc * 32, rank8 = sg.upitch / 2;
+    float* part = reinterpret_cast<float*>(smem + sg.off_part);
+    float* tt = reinterpret_cast<float*>(smem + sg.off_tt);                 // residual projections [r][mp], rank padded to 8
+    unsigned t_tag = 0;
+
+    // residual projections of all K parts: {value, tag} words, added in part order (one warp)
+    auto collect_t = [&]() {
+        const int limit = (p.debug & QGEMV_DEBUG_DROP_PROJECTIONS) ? (1 << 7) : (1 << 20);
+        const int per = sg.rank * M;
+        for (int i = lane; i < rank8 * sg.mp; i += 32) tt[i] = 0.0f;
+        __syncwarp();
+        for (int i = lane; i < per; i += 32) {
+            float v = 0.0f;
+            for (int q0 = 0; q0 < sg.t_parts; q0 += 8) {
+                unsigned long long w[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) w[q] = q0 + q < sg.t_parts ? ld_relaxed_u64(sg.tparts + (size_t)(q0 + q) * per + i) : (unsigned long long)t_tag << 32;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    int spins = 0;
+                    while ((unsigned)(w[q] >> 32) != t_tag) {
+                        if (++spins > limit) { atomicExch(p.status, 1); break; }
+                        __nanosleep(32);
+                        w[q] = ld_relaxed_u64(sg.tparts + (size_t)(q0 + q) * per + i);
+                    }
+                    v += __uint_as_float((unsigned)w[q]);
+                }
+            }
+            const int r = i / M;
+            tt[r * sg.mp + i - r * M] = v;
+        }
+    };
+
+    if (!aux) {
+        with_shape(sg.fmt, sg.T, [&](auto fmt_c, auto t_c) {
+            Producer<fmt_c.value, t_c.value> prod(c, sg);
+            for (int st = 0; st < sg.depth; ++st) prod.issue(sg);      // before the dependency wait: weights are final
+            pdl_wait();
+            stage_x<MODE, BF16>(p, sg, smem, slice_k0, tid, p.nw * 32);
+            named_barrier(1, p.nw * 32);
+            if (c.nrb > 0)
+                stream_loop<fmt_c.value, t_c.value, MODE, BF16>(c, sg, prod, part + (size_t)wk * sg.rows_pad * sg.mp);
+        });
+        if (c.nrb == 0 && wk < sg.wk) {                 // no slots for this warp: its share of the sums is zero
+            float* mine = part + ((size_t)wk * sg.rows_pad + c.row0) * sg.mp;
+            for (int i = lane; i < c.tiles * kStreamTileRows * sg.mp; i += 32) mine[i] = 0.0f;
+        }
+    } else {
+        // ---- before the dependency wait: outlier and residual rows, bias ------------------------------------
+        if (has_o) {                                   // outlier rows, in blocks of 64 columns laid out like ring slots
+            const int blocks = (sg.noc + 1) >> 1;
+            for (int i = lane; i < rows * blocks * 8; i += 32) {
+                const int pc = i & 7, rr = i >> 3, blk = rr / rows, r = rr - blk * rows;
+                const int col = blk * 64 + pc * 8, left = min(8, sg.oc - col);
+                unsigned char* d = smem + sg.off_ow + ((size_t)blk * sg.rows_pad + r) * kSlotRowBytes + ((pc ^ row_swizzle(r)) << 4);
+                const __half* src = sg.ow + (size_t)(rowbase + r) * sg.ldow + col;
+                if (sg.flags & kSegOutlierAligned) {
+                    cp_async16z(smem_u32(d), left > 0 ? src : sg.ow, left > 0 ? 16 : 0);
+                } else {
+                    for (int q = 0; q < 8; ++q) reinterpret_cast<__half*>(d)[q] = q < left ? __ldg(src + q) : __half(0.0f);
+                }
+            }
+        }
+        if (sg.rank > 0) {                             // rows of U for the epilogue, zero-padded to 8 columns
+            const int pieces = sg.upitch / 16;
+            for (int i = lane; i < rows * pieces; i += 32) {
+                const int r = i / pieces, q = i - r * pieces;
+                const __half* src = sg.ru + (size_t)(rowbase + r) * sg.ldu + q * 8;
+                unsigned char* d = smem + sg.off_u + (size_t)r * sg.upitch + q * 16;
+                if (sg.flags & kSegUAligned) {
+                    cp_async16z(smem_u32(d), src, 16);
+                } else {
+                    for (int k = 0; k < 8; ++k) reinterpret_cast<__half*>(d)[k] = q * 8 + k < sg.rank ? __ldg(src + k) : __half(0.0f);
+                }
+            }
+        }
+        if (sg.bias)
+            for (int i = lane; i < rows; i += 32) *reinterpret_cast<__half*>(smem + sg.off_bias + i * 2) = __ldg(sg.bias + rowbase + i);
+        const int rtiles = (sg.rank + kStreamTileRows - 1) / kStreamTileRows, jobs = rtiles * sg.t_parts_split;
+        const int kend = min(p.korig, slice_k0 + ns * slot_cols);
+        for (int job = grp; job < jobs; job += sg.groups) {                 // rows of V this CTA projects: to L2 while waiting
+            const int rt = job / sg.t_parts_split, k0 = slice_k0 + (job - rt * sg.t_parts_split) * sg.t_rounds * kProjectionK;
+            const int r = rt * kStreamTileRows + (lane & 15);
+            if (r < sg.rank)
+                for (int k = k0 + (lane >> 4) * 64; k < min(kend, k0 + sg.t_rounds * kProjectionK); k += 128) prefetch_l2(sg.rv + (size_t)r * sg.ldv + k);
+        }
+        constexpr int XO = 8;                          // outlier activations a lane keeps in flight
+        const int n_xo = has_o ? oc_pad * M : 0;
+        int xcol[XO];
+#pragma unroll
+        for (int u = 0; u < XO; ++u) {
+            const int i = u * 32 + lane, j = i % max(oc_pad, 1);
+            xcol[u] = i < n_xo && j < sg.oc ? __ldg(sg.oidx + j) : -1;
+        }
+        pdl_wait();
+        if (sg.rank > 0) t_tag = (unsigned)(ld_relaxed_u64(p.epoch) >> 8) + 1u;
+        XT xval[XO];
+#pragma unroll
+        for (int u = 0; u < XO; ++u) {
+            const int m = (u * 32 + lane) / max(oc_pad, 1);
+            xval[u] = xcol[u] >= 0 && xcol[u] < p.korig ? static_cast<const XT*>(p.x)[(size_t)m * p.ldx + xcol[u]] : XT(0.0f);
+        }
+        // ---- residual projections: t[r][m] = sum_k V[r,k] x[m,k] over a K part -----------------------------------
+        for (int job = grp; job < jobs; job += sg.groups) {
+            const int rt = job / sg.t_parts_split, kp = job - rt * sg.t_parts_split;
+            float acc[NB][4];
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[b][e] = 0.0f;
+#pragma unroll 1
+            for (int round = 0; round < sg.t_rounds * 2; ++round) {         // 128 columns a time
+                const int k0 = slice_k0 + kp * sg.t_rounds * kProjectionK + round * 128 + c.t * 8;
+                if (k0 - c.t * 8 >= kend) break;
+                uint4 va[4], vb[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int r = rt * kStreamTileRows + h * 8 + c.g, k = k0 + q * 32;
+                        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                        if (r < sg.rank && k < kend) {
+                            const __half* src = sg.rv + (size_t)r * sg.ldv + k;
+                            if ((sg.flags & kSegVAligned) && k + 8 <= kend) {
+                                v = __ldg(reinterpret_cast<const uint4*>(src));
+                            } else {
+                                __align__(16) __half e[8];
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) e[i] = k + i < kend ? __ldg(src + i) : __half(0.0f);
+                                v = *reinterpret_cast<const uint4*>(e);
+                            }
+                        }
+                        if (h == 0) va[q] = v; else vb[q] = v;
+                    }
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    uint4 xv[4];
+                    const int m = b * 8 + c.g;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) xv[q] = m < M ? load_x8<BF16>(p, m, k0 + q * 32) : make_uint4(0u, 0u, 0u, 0u);
+                    float2 up = make_float2(1.0f, 1.0f);
+                    if constexpr (BF16) {
+                        uint32_t big = 0;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            float f[8];
+                            widen8<BF16>(xv[q], f);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) big = max(big, __float_as_uint(f[i]) & 0x7fffffffu);
+                        }
+                        big = max(big, __shfl_xor_sync(0xffffffffu, big, 1));
+                        big = max(big, __shfl_xor_sync(0xffffffffu, big, 2));
+                        const int e = block_exponent(big);
+                        const float mine = big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
+                        up.x = __shfl_sync(0xffffffffu, mine, (2 * c.t) * 4);
+                        up.y = __shfl_sync(0xffffffffu, mine, (2 * c.t + 1) * 4);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            float f[8];
+                            widen8<BF16>(xv[q], f);
+                            uint32_t h[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const __half2 hh = __floats2half2_rn(f[2 * i] * pow2f(13 - e), f[2 * i + 1] * pow2f(13 - e));
+                                h[i] = *reinterpret_cast<const uint32_t*>(&hh);
+                            }
+                            xv[q] = make_uint4(h[0], h[1], h[2], h[3]);
+                        }
+                    }
+                    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        mma_f16(a, va[q].x, vb[q].x, va[q].y, vb[q].y, xv[q].x, xv[q].y);
+                        mma_f16(a, va[q].z, vb[q].z, va[q].w, vb[q].w, xv[q].z, xv[q].w);
+                    }
+                    acc[b][0] = fmaf(a[0], up.x, acc[b][0]); acc[b][1] = fmaf(a[1], up.y, acc[b][1]);
+                    acc[b][2] = fmaf(a[2], up.x, acc[b][2]); acc[b][3] = fmaf(a[3], up.y, acc[b][3]);
+                }
+            }
+            if (!(p.debug & QGEMV_DEBUG_DROP_PROJECTIONS)) {
+                const int kpart = split * sg.t_parts_split + kp;
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int r = rt * kStreamTileRows + c.g + (e >> 1) * 8, m = b * 8 + 2 * c.t + (e & 1);
+                        if (r < sg.rank && m < M)
+                            st_relaxed_u64(sg.tparts + ((size_t)kpart * sg.rank + r) * M + m,
+                                           ((unsigned long long)t_tag << 32) | __float_as_uint(acc[b][e]));
+                    }
+            }
+        }
+        auto put_xo = [&](int i, float f) {            // activations of the outlier columns as fp16, [m][oc_pad]
+            const int m = i / oc_pad, j = i - m * oc_pad;
+            if constexpr (BF16) {                      // a power of two per 32 columns keeps fp16 exact
+                uint32_t big = __float_as_uint(f) & 0x7fffffffu;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+                const int e = block_exponent(big);
+                f *= pow2f(13 - e);
+                if (lane == 0)
+                    reinterpret_cast<float*>(smem + sg.off_upo)[(j >> 5) * M + m] = big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
+            }
+            *reinterpret_cast<__half*>(smem + sg.off_xo + (size_t)m * (sg.noc * 64 + 16) + j * 2) = __float2half_rn(f);
+        };
+#pragma unroll
+        for (int u = 0; u < XO; ++u)
+            if (u * 32 < n_xo) put_xo(u * 32 + lane, Act16<BF16>::to_float(xval[u]));
+        for (int i = XO * 32 + lane; i < n_xo; i += 32) {
+            const int j = i % oc_pad, col = j < sg.oc ? __ldg(sg.oidx + j) : -1;
+            put_xo(i, col >= 0 && col < p.korig ? Act16<BF16>::to_float(static_cast<const XT*>(p.x)[(size_t)(i / oc_pad) * p.ldx + col]) : 0.0f);
+        }
+        if (finisher && sg.rank > 0) collect_t();
+    }
+    cp_async_wait_n<0>();
+    __syncthreads();
+    // From here on a warp finishes whole tiles in the mma layout: lane (g, t) holds rows g and g + 8, activation rows
+    // 2t and 2t + 1 of each block of eight.
+    auto tile_sums = [&](int tile, float (&v)[NB][4]) {
+        const int r = tile * kStreamTileRows + c.g;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const int m = b * 8 + 2 * c.t;
+            v[b][0] = v[b][1] = v[b][2] = v[b][3] = 0.0f;
+            if (m < M)
+                for (int k = 0; k < sg.wk; ++k) {
+                    const float* src = part + ((size_t)k * sg.rows_pad + r) * sg.mp + m;
+                    const float2 a = *reinterpret_cast<const float2*>(src), d = *reinterpret_cast<const float2*>(src + 8 * sg.mp);
+                    v[b][0] += a.x; v[b][1] += a.y; v[b][2] += d.x; v[b][3] += d.y;
+                }
+        }
+        if (has_o) {                                            // outlier columns: 32 per two mma
+            for (int blk = 0; blk < sg.noc; ++blk) {
+                const uint32_t w = smem_u32(smem + sg.off_ow + ((size_t)(blk >> 1) * sg.rows_pad + r) * kSlotRowBytes) +
+                                   ((((blk & 1) * 4 + c.t) ^ c.sw) << 4);
+                const uint4 a = lds128(w), d = lds128(w + 8 * kSlotRowBytes);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const uint4 xv = lds128(smem_u32(smem + sg.off_xo) + (uint32_t)min(b * 8 + c.g, M - 1) * (sg.noc * 64 + 16) + blk * 64 + c.t * 16);
+                    if constexpr (BF16) {
+                        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_f16(acc, a.x, d.x, a.y, d.y, xv.x, xv.y);
+                        mma_f16(acc, a.z, d.z, a.w, d.w, xv.z, xv.w);
+                        const float* upo = reinterpret_cast<const float*>(smem + sg.off_upo) + blk * M;
+                        const float ua = upo[min(b * 8 + 2 * c.t, M - 1)], ub = upo[min(b * 8 + 2 * c.t + 1, M - 1)];
+                        v[b][0] = fmaf(acc[0], ua, v[b][0]); v[b][1] = fmaf(acc[1], ub, v[b][1]);
+                        v[b][2] = fmaf(acc[2], ua, v[b][2]); v[b][3] = fmaf(acc[3], ub, v[b][3]);
+                    } else {
+                        mma_f16(v[b], a.x, d.x, a.y, d.y, xv.x, xv.y);
+                        mma_f16(v[b], a.z, d.z, a.w, d.w, xv.z, xv.w);
+                    }
+                }
+            }
+        }
+    };
+    if (!finisher) {
+        int* flag = reinterpret_cast<int*>(smem + sg.off_ring);      // the rings are idle by now
+        float* mine = sg.partial + ((size_t)split * sg.n + rowbase) * sg.mp;
+        for (int tile = warp; tile < tiles; tile += p.nw + 1) {
+            float v[NB][4];
+            tile_sums(tile, v);
+            const int r = tile * kStreamTileRows + c.g;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int m = b * 8 + 2 * c.t;
+                if (m < M) {
+                    if (r < rows) *reinterpret_cast<float2*>(mine + (size_t)r * sg.mp + m) = make_float2(v[b][0], v[b][1]);
+                    if (r + 8 < rows) *reinterpret_cast<float2*>(mine + (size_t)(r + 8) * sg.mp + m) = make_float2(v[b][2], v[b][3]);
+                }
+            }
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            const int old = atomicAdd(sg.counters + grp, 1);
+            *flag = old == sg.ksplit - 1;
+            if (old == sg.ksplit - 1) sg.counters[grp] = 0;
+        }
+        __syncthreads();
+        if (*flag == 0) {
+            if (p.epoch && tid == 0) atomicAdd(p.epoch, blockIdx.x == 0 ? 257ull - gridDim.x : 1ull);
+            return;
+        }
+        __threadfence();
+        if (sg.rank > 0) {
+            if (aux) collect_t();
+            __syncthreads();
+        }
+    }
+
+    // ---- epilogue: residual, bias, activation, store ----------------------------------------------------------
+    XT* out = static_cast<XT*>(sg.y);
+    auto r16 = [](float v) { return Act16<BF16>::to_float(Act16<BF16>::from_float(v)); };
+    for (int tile = warp; tile < tiles; tile += p.nw + 1) {
+        float v[NB][4];
+        const int r = tile * kStreamTileRows + c.g;
+        if (finisher) {
+            tile_sums(tile, v);
+        } else {                                                // the K splits, in order
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int m = b * 8 + 2 * c.t;
+                v[b][0] = v[b][1] = v[b][2] = v[b][3] = 0.0f;
+                if (m < M)
+                    for (int k = 0; k < sg.ksplit; ++k) {
+                        const float* src = sg.partial + ((size_t)k * sg.n + rowbase + r) * sg.mp + m;
+                        if (r < rows) { const float2 a = __ldcg(reinterpret_cast<const float2*>(src)); v[b][0] += a.x; v[b][1] += a.y; }
+                        if (r + 8 < rows) { const float2 a = __ldcg(reinterpret_cast<const float2*>(src + 8 * sg.mp)); v[b][2] += a.x; v[b][3] += a.y; }
+                    }
+            }
+        }
+        for (int q = 0; q < rank8; q += 8) {
+            const uint4 u0 = lds128(smem_u32(smem + sg.off_u) + (uint32_t)(r * sg.upitch + q * 2));
+            const uint4 u1 = lds128(smem_u32(smem + sg.off_u) + (uint32_t)((r + 8) * sg.upitch + q * 2));
+            float f0[8], f1[8];
+            widen8<false>(u0, f0);
+            widen8<false>(u1, f1);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int m = min(b * 8 + 2 * c.t, sg.mp - 2);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 t2 = *reinterpret_cast<const float2*>(tt + (q + i) * sg.mp + m);
+                    v[b][0] = fmaf(f0[i], t2.x, v[b][0]); v[b][1] = fmaf(f0[i], t2.y, v[b][1]);
+                    v[b][2] = fmaf(f1[i], t2.x, v[b][2]); v[b][3] = fmaf(f1[i], t2.y, v[b][3]);
+                }
+            }
+        }
+        float b0 = 0.0f, b1 = 0.0f;
+        if (sg.bias) {
+            const __half* bp = reinterpret_cast<const __half*>(smem + sg.off_bias) + r;
+            b0 = __half2float(bp[0]); b1 = __half2float(bp[8]);
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int m = b * 8 + 2 * c.t + h;
+                if (m >= M) continue;
+                if (sg.act == QGEMV_ACT_SILU_MUL) {
+                    // rows g and g + 8 are a (gate, up) pair: one output, rounded where separate 16-bit operators would round
+                    const float gate = r16(v[b][h] + b0), upv = r16(v[b][2 + h] + b1);
+                    const float s = r16(gate / (1.0f + __expf(-gate)));
+                    out[(size_t)m * sg.ldy + (rowbase + tile * kStreamTileRows) / 2 + c.g] = Act16<BF16>::from_float(s * upv);
+                } else {
+                    XT* o = out + (size_t)m * sg.ldy + rowbase + r;
+                    if (r < rows) o[0] = Act16<BF16>::from_float(apply_act(v[b][h] + b0, sg.act));
+                    if (r + 8 < rows) o[8] = Act16<BF16>::from_float(apply_act(v[b][2 + h] + b1, sg.act));
+                }
+            }
+    }
+    // The launch count that tags the residual projections: every CTA adds one, the first one what is missing to 256, so
+    // count / 256 does not change while a CTA of this launch may still read it.
+    if (p.epoch && tid == 0) atomicAdd(p.epoch, blockIdx.x == 0 ? 257ull - gridDim.x : 1ull);
+}
+
+template <int MODE, bool BF16>
+int launch_one(const StreamArgs& a, bool dependent, int grid, int threads, int smem, cudaStream_t s) {
+    auto kern = qgemv_stream_kernel<MODE, BF16>;
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!configured[dev]) {
+        // the carve-out is the same for every kernel of a decode step: a launch that needs another split of L1 and shared
+        // memory would wait for the SM to drain
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamMaxSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
+            return check_launch("cudaFuncSetAttribute(qgemv_stream_kernel)");
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kern, a) != cudaSuccess) return check_launch("qgemv_stream_kernel");
+    return QGEMV_OK;
+}
+
+}  // namespace
+
+// One translation unit per path and activation type keeps the build parallel.
+#if !defined(QGEMV_STREAM_MODE) || !defined(QGEMV_STREAM_BF16)
+#error "compile with -DQGEMV_STREAM_MODE=0..2 and -DQGEMV_STREAM_BF16=0|1"
+#endif
+template <int MODE, bool BF16> int launch_stream_mode(const StreamArgs& a, bool dependent, int grid, int threads, int smem, cudaStream_t s) {
+    return launch_one<MODE, BF16>(a, dependent, grid, threads, smem, s);
+}
+template int launch_stream_mode<QGEMV_STREAM_MODE, QGEMV_STREAM_BF16>(const StreamArgs&, bool, int, int, int, cudaStream_t);
+
+}  // namespace qgemv

@@ -19,7 +19,7 @@
 extern "C" {
 #endif
 
-#define QGEMV_ABI_VERSION 4
+#define QGEMV_ABI_VERSION 5
 
 enum qgemv_status {
     QGEMV_OK = 0,
@@ -54,7 +54,8 @@ enum qgemv_dtype { QGEMV_F16 = 0, QGEMV_BF16 = 1, QGEMV_F32 = 2 };
  * shape does not allow returns QGEMV_ERR_SHAPE. */
 enum qgemv_kernel { QGEMV_KERNEL_AUTO = 0, QGEMV_KERNEL_SIMT = 1, QGEMV_KERNEL_MMA = 2, QGEMV_KERNEL_MMA_PIPE = 3 };
 
-#define QGEMV_MAX_M 4
+#define QGEMV_MAX_M 4          /* qgemv_run, qgemv_run_static */
+#define QGEMV_MAX_BATCH 16     /* qgemv_prepare */
 
 /* qgemv_problem.debug bits.  DROP_PROJECTIONS makes the CTAs that compute the residual
  * projections of a launch keep them to themselves and shortens the readers' wait to a few
@@ -95,7 +96,7 @@ enum qgemv_kernel { QGEMV_KERNEL_AUTO = 0, QGEMV_KERNEL_SIMT = 1, QGEMV_KERNEL_M
  *              different streams without ordering need a workspace each).  The kernels leave it
  *              ready for the next call, so no memset is needed between calls: every arrival
  *              counter is back at zero, while three bookkeeping words near the end of the counter
- *              area keep their values on purpose -- the number of launches completed so far (the
+ *              area keep their values on purpose -- the numbers of launches completed so far (the
  *              tag of the residual projections that CTAs of one launch pass to each other), the
  *              count of CTAs that have finished the current launch (zero between calls) and the
  *              sticky status word that qgemv_workspace_status() reads.
@@ -167,6 +168,17 @@ int qgemv_run_static(const qgemv_problem* p, void* stream);
  * built-in scratch of qgemv_run_static on the current device.  Not capturable in a CUDA graph.
  * It has no counterpart in the reference project (its kernels never wait on each other). */
 int qgemv_workspace_status(const void* workspace, void* stream, int32_t* host_out);
+
+/* The same GEMV for loops that issue it again and again, and for up to QGEMV_MAX_BATCH rows: qgemv_prepare validates and plans
+ * once, into a caller-owned host buffer of qgemv_prepared_bytes() bytes; qgemv_launch_prepared only launches.  x and y may
+ * change from call to call (same shape, strides and alignment), and so may the workspace.  x needs only k_original columns
+ * (ldx >= k_original) except for the CUDA-core kernel, which qgemv_prepare reports with QGEMV_ERR_ALIGN (pad x, and pass
+ * k_original = k_padded with res_v padded likewise, or use qgemv_run).  `ordered` != 0: the
+ * preceding kernel of the stream may still be writing the weights, so the launch does not overlap it.  One buffer must not be
+ * launched from two threads at a time. */
+size_t qgemv_prepared_bytes(void);
+int qgemv_prepare(const qgemv_problem* p, void* prepared);
+int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspace, int ordered, void* stream);
 
 /* Bytes of workspace qgemv_run needs for a problem of this shape (never 0; at most a few MB). */
 size_t qgemv_workspace_bytes(int bits, int m, int n, int k_padded, int group, int rank);
