@@ -9,11 +9,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libqgemv_b200.so"
+NATIVE = PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX"))      # host side of eager calls, links the library above
 # (source, extra defines, object name).  The tensor-core-assisted kernels are compiled in parts (per bit width; per
 # path and activation type) so that the objects build in parallel.
 UNITS = [
@@ -52,12 +54,31 @@ def _stale(target: Path = LIB, patterns=("*.cu", "*.cuh")) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def build_native(force: bool = False) -> Path:
+    """The CPython extension with the host side of eager calls (csrc/qtorch.cpp); needs the library to link against."""
+    if not force and not _stale(NATIVE, ("qtorch.cpp",)):
+        return NATIVE
+    import torch
+    from torch.utils import cpp_extension
+    libdir = Path(torch.__file__).parent / "lib"
+    cuda_inc = Path(_nvcc()).resolve().parent.parent / "include"
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{p}" for p in cpp_extension.include_paths()], f"-I{cuda_inc}", f"-I{sysconfig.get_paths()['include']}",
+           str(CSRC / "qtorch.cpp"), "-o", str(NATIVE), f"-L{PKG}", "-l:" + LIB.name, f"-L{libdir}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"building {NATIVE.name} failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+    return NATIVE
+
+
 def build(force: bool = False, verbose: bool = False, extra_flags: tuple = (), lib: Path = LIB) -> Path:
     """Compile the library if it is missing or older than its sources; return its path.
 
     ``extra_flags`` (e.g. ``("-DQGEMV_TRACE",)``) and ``lib`` let a measurement build sit beside the
     product build; objects of such a build go to their own directory."""
     if not force and not extra_flags and lib == LIB and not _stale():
+        build_native()
         return lib
     nvcc = _nvcc()
     objdir = OBJDIR if not extra_flags else OBJDIR.with_name("build_" + "".join(c for c in "".join(extra_flags) if c.isalnum()))
@@ -83,6 +104,8 @@ def build(force: bool = False, verbose: bool = False, extra_flags: tuple = (), l
     res = subprocess.run(link, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+    if lib == LIB:
+        build_native(force)
     return lib
 
 

@@ -1,0 +1,291 @@
+// Host side of an eager packed-Linear call, in C++: what a module's forward does per call is an output allocation, the
+// current stream, a workspace look-up and one launch.  In Python that took 13 - 17 us, longer than the kernels.
+//
+// Two things live here: `Linear`, the prepared launches of one module (one per row count, up to 16 rows), and
+// `functional`, the prepared-problem cache of the decode_int*_linear functions.  The C ABI (include/qgemv_b200.h) does the
+// work; nothing here knows about kernels.
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <unordered_map>
+#include <vector>
+
+#include "../../include/qgemv_b200.h"
+
+namespace {
+
+using Opt = std::optional<at::Tensor>;
+
+PyObject* g_workspace_fn = nullptr;                   // ops.ensure_workspace: (device index) -> tensor for the current stream
+std::mutex g_mutex;
+std::unordered_map<uint64_t, void*> g_workspace;      // (device, stream) -> workspace; the buffers live as long as the process
+
+struct PyError {};                                    // a Python exception is set
+
+PyObject* g_error_class = nullptr;                    // _cabi.QgemvError(code, message)
+
+void check(int rc) {
+    if (rc == QGEMV_OK) return;
+    PyObject* e = PyObject_CallFunction(g_error_class, "is", rc, qgemv_error_string());
+    if (e) { PyErr_SetObject(g_error_class, e); Py_DECREF(e); }
+    throw PyError{};
+}
+
+// Called with the GIL held.
+void* workspace(int device, cudaStream_t stream, size_t* bytes) {
+    *bytes = qgemv_workspace_bytes(4, QGEMV_MAX_M, 1, 256, 128, 64);
+    const uint64_t key = (reinterpret_cast<uint64_t>(stream) << 6) ^ (uint64_t)device;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        auto it = g_workspace.find(key);
+        if (it != g_workspace.end()) return it->second;
+    }
+    PyObject* t = PyObject_CallFunction(g_workspace_fn, "i", device);
+    if (!t) throw PyError{};
+    void* p = THPVariable_Unpack(t).data_ptr();
+    Py_DECREF(t);
+    std::lock_guard<std::mutex> lock(g_mutex);
+    g_workspace[key] = p;
+    return p;
+}
+
+Opt optional_tensor(PyObject* o) {
+    if (!o || o == Py_None) return std::nullopt;
+    return THPVariable_Unpack(o);
+}
+
+void fill(qgemv_problem& p, int bits, int64_t k_original, int group, int act, int kernel, const at::Tensor& packed, const at::Tensor& scales,
+          const Opt& bias, const Opt& oidx, const Opt& ow, const Opt& ru, const Opt& rv) {
+    p = qgemv_problem{};
+    p.bits = bits; p.n = (int)packed.size(0); p.k_padded = (int)(packed.size(1) * (8 / bits)); p.k_original = (int)k_original;
+    p.group = group; p.act = act; p.kernel = kernel & 0xff; p.debug = kernel >> 8;
+    p.packed = packed.data_ptr<uint8_t>(); p.ldp = packed.stride(0);
+    p.scales = scales.data_ptr(); p.lds = scales.stride(0);
+    if (bias) p.bias = bias->data_ptr();
+    if (oidx && oidx->numel()) {
+        p.outliers = (int)oidx->numel();
+        p.outlier_idx = oidx->data_ptr<int32_t>(); p.outlier_w = ow->data_ptr(); p.ldow = ow->stride(0);
+    }
+    if (ru && ru->numel()) {
+        p.rank = (int)ru->size(1);
+        p.res_u = ru->data_ptr(); p.ldu = ru->stride(0); p.res_v = rv->data_ptr(); p.ldv = rv->stride(0);
+    }
+}
+
+// ---- Linear ---------------------------------------------------------------------------------------------
+
+struct Linear {
+    std::vector<at::Tensor> keep;                     // every weight-side tensor: alive, and watched for in-place changes
+    qgemv_problem base;
+    int device;
+    int64_t in_features, out_features, max_rows;
+    uint64_t version = ~0ull;
+    struct Slot { std::vector<char> blob; bool usable = false; };
+    std::unordered_map<int, Slot> slots;              // rows * 2 + bf16
+};
+
+// Sum of the version counters: changes when a weight was written in place (then its writer may still be running, and the
+// launch must not start reading weights early).
+uint64_t versions(const Linear& l) {
+    uint64_t v = 0;
+    for (const auto& t : l.keep) v += t.is_inference() ? 0 : t._version();
+    return v;
+}
+
+struct LinearObject { PyObject_HEAD Linear* self; };
+
+void linear_dealloc(LinearObject* o) { delete o->self; Py_TYPE(o)->tp_free(reinterpret_cast<PyObject*>(o)); }
+
+// Linear(bits, k_original, group, act, kernel, in_features, out_features, max_rows, packed, scales, bias, oidx, ow, ru, rv)
+PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    int bits, group, act, kernel;
+    long long korig, in, out, max_rows;
+    PyObject *packed, *scales, *bias, *oidx, *ow, *ru, *rv;
+    if (!PyArg_ParseTuple(args, "iLiiiLLLOOOOOOO", &bits, &korig, &group, &act, &kernel, &in, &out, &max_rows, &packed, &scales, &bias, &oidx, &ow, &ru, &rv))
+        return nullptr;
+    auto l = std::make_unique<Linear>();
+    try {
+        const at::Tensor pk = THPVariable_Unpack(packed), sc = THPVariable_Unpack(scales);
+        const Opt b = optional_tensor(bias), oi = optional_tensor(oidx), w = optional_tensor(ow), u = optional_tensor(ru), v = optional_tensor(rv);
+        fill(l->base, bits, korig, group, act, kernel, pk, sc, b, oi, w, u, v);
+        l->keep = {pk, sc};
+        for (const Opt* t : {&b, &oi, &w, &u, &v}) if (*t) l->keep.push_back(**t);
+        l->device = pk.get_device();
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    l->in_features = in; l->out_features = out; l->max_rows = max_rows;
+    auto* o = reinterpret_cast<LinearObject*>(type->tp_alloc(type, 0));
+    if (o) o->self = l.release();
+    return reinterpret_cast<PyObject*>(o);
+}
+
+// call(x): the result, or None where the caller has to take its general route (shape, type, device, layout).
+PyObject* linear_call(LinearObject* o, PyObject* arg) {
+    Linear& l = *o->self;
+    if (!THPVariable_CheckExact(arg)) Py_RETURN_NONE;
+    try {
+        const at::Tensor& x = THPVariable_Unpack(arg);
+        const int64_t dims = x.dim();
+        const auto dtype = x.scalar_type();
+        if (dims < 1 || !x.is_cuda() || x.get_device() != l.device || x.size(-1) != l.in_features || !x.is_contiguous() ||
+            (dtype != at::kHalf && dtype != at::kBFloat16) || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16)
+            Py_RETURN_NONE;
+        const int64_t rows = x.numel() / l.in_features;
+        if (rows < 1 || rows > l.max_rows) Py_RETURN_NONE;
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != l.device) guard.set_index(l.device);
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(l.device).stream();
+        size_t ws_bytes = 0;
+        void* ws = workspace(l.device, stream, &ws_bytes);
+        const bool bf16 = dtype == at::kBFloat16;
+        Linear::Slot& slot = l.slots[(int)rows * 2 + bf16];
+        if (slot.blob.empty()) {
+            slot.blob.resize(qgemv_prepared_bytes());
+            qgemv_problem p = l.base;
+            p.m = (int)rows; p.x_dtype = bf16 ? QGEMV_BF16 : QGEMV_F16;
+            p.x = x.data_ptr(); p.ldx = l.in_features;
+            p.y = x.data_ptr(); p.ldy = l.out_features;       // a valid address for the plan; the launch names the real one
+            p.workspace = ws; p.workspace_bytes = ws_bytes;
+            const int rc = qgemv_prepare(&p, slot.blob.data());
+            slot.usable = rc == QGEMV_OK;
+            if (rc != QGEMV_OK && rc != QGEMV_ERR_ALIGN) check(rc);
+        }
+        if (!slot.usable) Py_RETURN_NONE;
+        const uint64_t v = versions(l);
+        const bool fresh = v != l.version;
+        at::Tensor y;
+        if (dims == 2) {
+            y = at::empty({rows, l.out_features}, x.options());
+        } else {
+            std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+            shape.back() = l.out_features;
+            y = at::empty(shape, x.options());
+        }
+        check(qgemv_launch_prepared(slot.blob.data(), x.data_ptr(), y.data_ptr(), ws, fresh, stream));
+        l.version = v;
+        return THPVariable_Wrap(std::move(y));
+    } catch (const PyError&) { return nullptr; }
+    catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
+PyObject* linear_tp_call(PyObject* self, PyObject* args, PyObject* kw) {
+    if (PyTuple_GET_SIZE(args) != 1 || (kw && PyDict_GET_SIZE(kw))) { PyErr_SetString(PyExc_TypeError, "one activation tensor expected"); return nullptr; }
+    return linear_call(reinterpret_cast<LinearObject*>(self), PyTuple_GET_ITEM(args, 0));
+}
+
+PyMethodDef linear_methods[] = {{"call", reinterpret_cast<PyCFunction>(linear_call), METH_O, "call(x) -> y, or None for the caller's general route"}, {nullptr, nullptr, 0, nullptr}};
+PyTypeObject LinearType = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+// ---- functional -----------------------------------------------------------------------------------------
+
+// A problem is reused when addresses AND shapes of the operands of this call are the ones it was built from; the cache
+// holds no tensor alive.
+struct Key {
+    uint64_t w[20];
+    bool operator==(const Key& o) const { return std::equal(w, w + 20, o.w); }
+};
+struct KeyHash {
+    size_t operator()(const Key& k) const {
+        uint64_t h = 1469598103934665603ull;
+        for (uint64_t v : k.w) { h ^= v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2); }
+        return (size_t)h;
+    }
+};
+constexpr size_t kMaxProblems = 256;
+std::unordered_map<Key, qgemv_problem, KeyHash> g_problems;      // guarded by the GIL
+
+// functional(bits, group, k_original, act, kernel, x, packed, scales, bias, oidx, ow, ru, rv) -> y, or None for the general route
+PyObject* functional(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 13) { PyErr_SetString(PyExc_TypeError, "functional takes 13 arguments"); return nullptr; }
+    long v[5];
+    for (int i = 0; i < 5; ++i) { v[i] = PyLong_AsLong(a[i]); if (v[i] == -1 && PyErr_Occurred()) return nullptr; }
+    for (int i = 5; i < 13; ++i) {
+        if (a[i] == Py_None && i > 7) continue;
+        if (!THPVariable_CheckExact(a[i])) Py_RETURN_NONE;
+    }
+    try {
+        const at::Tensor &x = THPVariable_Unpack(a[5]), &packed = THPVariable_Unpack(a[6]), &scales = THPVariable_Unpack(a[7]);
+        const auto dtype = x.scalar_type();
+        const int cpb = 8 / (int)v[0];
+        if (!x.is_cuda() || x.dim() != 2 || x.size(0) < 1 || x.size(0) > QGEMV_MAX_M || x.stride(1) != 1 || (dtype != at::kHalf && dtype != at::kBFloat16) ||
+            packed.dim() != 2 || packed.scalar_type() != at::kByte || packed.stride(1) != 1 || packed.size(1) * cpb != x.size(1) ||
+            scales.dim() != 2 || scales.scalar_type() != at::kHalf || scales.stride(1) != 1)
+            Py_RETURN_NONE;
+        const int dev = x.get_device();
+        Key key{};
+        uint64_t* w = key.w;
+        *w++ = (uint64_t)v[0] | (uint64_t)v[1] << 8 | (uint64_t)v[3] << 40 | (uint64_t)dev << 48 | (uint64_t)(dtype == at::kHalf) << 56;
+        *w++ = (uint64_t)v[2] | (uint64_t)v[4] << 32;
+        *w++ = (uint64_t)x.size(0) | (uint64_t)x.stride(0) << 8;
+        *w++ = (uint64_t)packed.data_ptr(); *w++ = (uint64_t)packed.size(0) | (uint64_t)packed.size(1) << 32; *w++ = packed.stride(0);
+        *w++ = (uint64_t)scales.data_ptr(); *w++ = scales.stride(0);
+        for (int i = 8; i < 13; ++i) {
+            if (a[i] == Py_None) { *w++ = 0; *w++ = 0; continue; }
+            const at::Tensor& t = THPVariable_Unpack(a[i]);
+            if (!t.is_cuda() || t.get_device() != dev || t.scalar_type() != (i == 9 ? at::kInt : at::kHalf) || (t.dim() && t.numel() && t.stride(-1) != 1)) Py_RETURN_NONE;
+            *w++ = (uint64_t)t.data_ptr();
+            *w++ = t.dim() == 2 ? (uint64_t)t.size(0) << 40 ^ (uint64_t)t.size(1) << 20 ^ (uint64_t)t.stride(0) : (uint64_t)t.numel();
+        }
+        auto it = g_problems.find(key);
+        if (it == g_problems.end()) {
+            if (packed.get_device() != dev || scales.get_device() != dev || scales.size(0) != packed.size(0) || scales.size(1) * v[1] != x.size(1)) Py_RETURN_NONE;
+            qgemv_problem p;
+            const Opt oi = optional_tensor(a[9]), ow = optional_tensor(a[10]), ru = optional_tensor(a[11]), rv = optional_tensor(a[12]);
+            if ((oi && oi->numel() && (!ow || ow->dim() != 2)) || (ru && ru->numel() && (ru->dim() != 2 || !rv || rv->dim() != 2))) Py_RETURN_NONE;
+            fill(p, (int)v[0], v[2], (int)v[1], (int)v[3], (int)v[4], packed, scales, optional_tensor(a[8]), oi, ow, ru, rv);
+            p.m = (int)x.size(0); p.x_dtype = dtype == at::kHalf ? QGEMV_F16 : QGEMV_BF16;
+            p.ldx = x.stride(0); p.ldy = p.n;
+            if (g_problems.size() >= kMaxProblems) g_problems.clear();
+            it = g_problems.emplace(key, p).first;
+        }
+        qgemv_problem& p = it->second;
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != dev) guard.set_index(dev);
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+        size_t ws_bytes = 0;
+        void* ws = workspace(dev, stream, &ws_bytes);
+        at::Tensor y = at::empty({x.size(0), p.n}, x.options());
+        p.x = x.data_ptr(); p.y = y.data_ptr(); p.workspace = ws; p.workspace_bytes = ws_bytes;
+        check(qgemv_run(&p, stream));
+        return THPVariable_Wrap(std::move(y));
+    } catch (const PyError&) { return nullptr; }
+    catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
+// setup(ensure_workspace, error_class)
+PyObject* setup(PyObject*, PyObject* args) {
+    PyObject *fn, *err;
+    if (!PyArg_ParseTuple(args, "OO", &fn, &err)) return nullptr;
+    Py_INCREF(fn); Py_INCREF(err);
+    g_workspace_fn = fn; g_error_class = err;
+    Py_RETURN_NONE;
+}
+
+PyMethodDef module_methods[] = {
+    {"setup", setup, METH_VARARGS, "setup(ensure_workspace, error_class)"},
+    {"functional", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(functional)), METH_FASTCALL, "prepared-problem call of the decode_int*_linear functions"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", "Host side of eager packed-Linear calls", -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) {
+    LinearType.tp_name = "ai_accel_studio_b200._native.Linear";
+    LinearType.tp_basicsize = sizeof(LinearObject);
+    LinearType.tp_dealloc = reinterpret_cast<destructor>(linear_dealloc);
+    LinearType.tp_flags = Py_TPFLAGS_DEFAULT;
+    LinearType.tp_new = linear_new;
+    LinearType.tp_call = linear_tp_call;
+    LinearType.tp_methods = linear_methods;
+    LinearType.tp_doc = "Prepared launches of one packed Linear module, one per row count";
+    if (PyType_Ready(&LinearType) < 0) return nullptr;
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m) return nullptr;
+    Py_INCREF(&LinearType);
+    PyModule_AddObject(m, "Linear", reinterpret_cast<PyObject*>(&LinearType));
+    return m;
+}

@@ -28,6 +28,16 @@ def _as_half(t, device):
 
 def _fused(bits, x, pw, bias, outlier_idx, outlier_weight, res_u, res_v, activation, kernel):
     from .. import ops
+    if not torch.compiler.is_compiling() and activation in _cabi.ACT and kernel in _cabi.KERNEL:
+        # operands already in the kernel's types: validated and launched natively; None = anything else
+        if outlier_weight is None:
+            outlier_idx = None
+        if res_v is None:
+            res_u = None
+        y = ops.native().functional(bits, pw.group_size, pw.original_k, _cabi.ACT[activation], _cabi.KERNEL[kernel], x, pw.packed,
+                                    pw.scales, bias, outlier_idx, outlier_weight, res_u, res_v)
+        if y is not None:
+            return y
     if not x.is_cuda:
         raise RuntimeError("CUDA is required: the packed decode path has no CPU implementation")
     if x.dtype not in (torch.float16, torch.bfloat16):

@@ -91,6 +91,20 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
         raise RuntimeError(f"{name} must be a CUDA tensor: this build has no CPU path")
 
 
+_NATIVE = None
+
+
+def native():
+    """The extension module with the host side of eager calls (``csrc/qtorch.cpp``), loaded and set up once."""
+    global _NATIVE
+    if _NATIVE is None:
+        _cabi.lib()                        # the extension links the library; a missing build is reported there
+        from . import _native
+        _native.setup(lambda idx: ensure_workspace(torch.device("cuda", idx)), _cabi.QgemvError)
+        _NATIVE = _native
+    return _NATIVE
+
+
 ACT_SILU_MUL = 3      # qgemv_act: rows are (8 gate, 8 up) blocks, the output is silu(gate) * up of width N / 2
 
 

@@ -43,9 +43,8 @@ def select_outliers(module: nn.Module, w: torch.Tensor, activation_rms, outlier_
 
 
 class HybridPackedLinear(nn.Module):
-    """Common forward: M <= 4 -> one fused GEMV launch; up to ``chunked_max_rows`` rows -> one fused launch per
-    four rows; larger M -> CUDA dequantisation into the activation dtype + library GEMMs for the base, outlier
-    and residual terms."""
+    """Common forward: up to ``chunked_max_rows`` rows -> one fused launch (a few shapes: one per four rows); larger M ->
+    CUDA dequantisation into the activation dtype + library GEMMs for the base, outlier and residual terms."""
 
     bits: int = 0
     residual_rank: int = 0
@@ -56,7 +55,7 @@ class HybridPackedLinear(nn.Module):
     # Optional hint for the decode path: a static tensor (normally the packed codes of the module that
     # runs next) announced to L2 while this module's GEMV runs; see model_tools.chain_weight_prefetch.
     prefetch_next = None
-    # Largest row count served by repeated fused GEMVs (groups of four rows) instead of the dequantise + GEMM route.
+    # Largest row count (at most 16) served by the fused GEMV instead of the dequantise + GEMM route.
     chunked_max_rows: int = 16
     # Set by siblings.merge_gate_up: the rows are (8 gate, 8 up) blocks of a feed-forward block's two
     # input projections and forward returns silu(gate(x)) * up(x), of width out_features = rows / 2.
@@ -146,20 +145,30 @@ class HybridPackedLinear(nn.Module):
                 del self.__dict__[name]     # plain None placeholders make way for buffers
             if name in self._buffers:
                 del self._buffers[name]
-        self.__dict__.pop("_call", None)
+        self._drop_prepared()
         self.register_buffer("res_u", res_u.detach().to(dev, torch.float16).contiguous())
         self.register_buffer("res_v", res_v.detach().to(dev, torch.float16).contiguous())
         self.residual_rank = int(res_u.shape[1])
 
-    _LAUNCH_OPERANDS = frozenset(("packed", "scales", "bias", "outlier_idx", "outlier_weight", "res_u", "res_v", "residual_rank"))
+    _LAUNCH_OPERANDS = frozenset(("packed", "scales", "bias", "outlier_idx", "outlier_weight", "res_u", "res_v", "residual_rank",
+                                  "kernel", "debug", "prefetch_next", "gated_pairs", "chunked_max_rows", "out_features"))
+
+    def _drop_prepared(self) -> None:
+        """Forget the prepared launches: they hold the operands' addresses and the settings they were built from."""
+        self.__dict__.pop("_call", None)
+        self.__dict__.pop("_native_call", None)
 
     def __setattr__(self, name, value):
         if name in HybridPackedLinear._LAUNCH_OPERANDS:
-            self.__dict__.pop("_call", None)          # the prepared launch holds the old tensor's address
+            self._drop_prepared()
         super().__setattr__(name, value)
 
+    def __delattr__(self, name):
+        self._drop_prepared()
+        super().__delattr__(name)
+
     def _apply(self, fn, *args, **kwargs):
-        self.__dict__.pop("_call", None)
+        self._drop_prepared()
         out = super()._apply(fn, *args, **kwargs)
         if self.packed.is_cuda:
             from .. import ops
@@ -189,6 +198,22 @@ class HybridPackedLinear(nn.Module):
                         self.outlier_weight if self.outlier_idx.numel() else None,
                         self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None,
                         self.bits, self.group_size, self.original_k, 3 if self.gated_pairs else 0, self._kernel_code(), self.prefetch_next)
+
+    def _prepare_native(self):
+        """The module's prepared launches (``csrc/qtorch.cpp``), one per row count, or None where forward has to take its
+        general route (buffers on the CPU, an L2 hint).  Dropped whenever an operand or a setting changes."""
+        d = self.__dict__
+        packed = d["_buffers"]["packed"]
+        call = None
+        if packed.is_cuda and self.prefetch_next is None and self.bits in (2, 4):
+            from .. import ops
+            has_o = self.outlier_idx.numel() > 0
+            call = ops.native().Linear(self.bits, self.original_k, self.group_size, 3 if self.gated_pairs else 0, self._kernel_code(),
+                                       self.in_features, self.out_features, min(self.chunked_max_rows, 16), packed, self.scales, self.bias,
+                                       self.outlier_idx if has_o else None, self.outlier_weight if has_o else None,
+                                       self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None)
+        d["_native_call"], d["_native_packed"] = call, packed
+        return call
 
     def _kernel_code(self) -> int:
         from .. import _cabi
@@ -227,6 +252,17 @@ class HybridPackedLinear(nn.Module):
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if not torch.compiler.is_compiling():
+            d = self.__dict__
+            call = d["_native_call"] if "_native_call" in d and d["_native_packed"] is d["_buffers"]["packed"] else self._prepare_native()
+            if call is not None and not HybridPackedLinear.skip_gemv:
+                y = call(x)
+                if y is not None:
+                    return y
+        return self._forward_general(x)
+
+    def _forward_general(self, x: torch.Tensor) -> torch.Tensor:
+        """Any input: tracing, layouts the prepared launches do not take, more rows, wrong arguments."""
         if not x.is_cuda:
             raise RuntimeError(f"{type(self).__name__} computes on CUDA only (no CPU fallback); got a {x.device} tensor")
         if x.dtype not in (torch.float16, torch.bfloat16):
@@ -251,7 +287,7 @@ class HybridPackedLinear(nn.Module):
         return y.reshape(*shape[:-1], self.out_features)
 
     def _fused_chunks(self, xflat: torch.Tensor) -> torch.Tensor:
-        """5 .. ``chunked_max_rows`` rows (a decode batch beyond the kernel's four): the fused GEMV over groups of
+        """5 .. ``chunked_max_rows`` rows where the prepared launches do not apply: the fused GEMV over groups of
         four rows, written into one result.  The packed weights of one Linear stay in L2 between the launches,
         where dequantising the whole matrix for every token (the M > 4 route of the reference,
         ``ai_accel_lab/optimize/hybrid_int4.py:36-37``) would write and re-read 2 bytes per weight."""
