@@ -41,12 +41,14 @@ constexpr int kGroupsPerBlock[6] = {1, 2, 1, 2, 4, 1};
 constexpr int kTileCost[2][6] = {{220, 260, 110, 130, 170, 34}, {320, 400, 170, 210, 300, 34}};
 constexpr int kSlotCost[2][6] = {{180, 180, 110, 110, 110, 60}, {220, 240, 130, 140, 150, 60}};
 
+constexpr int kMaxJobs = 32;                          // CTAs of a split that compute residual projections
+
 // Lays out one matrix for `ctas` CTAs of `nw` warps and `cap` bytes of shared memory; false if it does not fit.
 // What is chosen: K splits between CTAs (S), warps along K (wk; the others along the rows), tiles per row block (T), ring
 // depth.  Estimated clocks of a CTA: the larger of its stream (HBM gives an SM 23 bytes a clock, less when the ring keeps
 // under 40 KB in flight) and its instructions (four schedulers, measured 0.55 per clock), a third of the smaller, and 2500
 // for a hand-over between splits.
-bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, int ctas, int cap, size_t partial_floats, StreamSeg& out, int& smem_out) {
+bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, int ctas, int cap, size_t split_floats, size_t word_floats, StreamSeg& out, int& smem_out) {
     const int fmt = out.fmt, cps = kCodesPerSlot[fmt], nb = mode == 2 ? 2 : 1;
     const bool digits = mode == 0 && fmt != kDense16;
     const int tiles = cdiv(p.n, kStreamTileRows), rtiles = cdiv(p.rank, kStreamTileRows);
@@ -79,10 +81,11 @@ bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, in
                 s.t_parts_split = cdiv(slice, kProjectionK * s.t_rounds);
                 s.t_parts = s.t_parts_split * S;
                 words = (size_t)s.t_parts * p.rank * m;
-                if ((words <= 1024 && rtiles * s.t_parts_split <= s.groups) || s.t_parts_split == 1) break;
+                // in the first CTAs of a split: those are resident whenever a CTA that waits for them is
+                if ((words <= 1024 && rtiles * s.t_parts_split <= (s.groups < kMaxJobs ? s.groups : kMaxJobs)) || s.t_parts_split == 1) break;
             }
         }
-        if (words * 2 + (S > 1 ? (size_t)S * p.n * s.mp : 0) > partial_floats) continue;
+        if (words * 2 + 2 > word_floats || (S > 1 && (size_t)S * p.n * s.mp > split_floats)) continue;
         int off = digits ? s.np / 16 * m * 512 : m * s.xpitch;
         s.off_up = off;   off = up_to(off + (digits || bf16 ? s.np / 16 * m * 4 : 0), 16);
         s.off_xo = off;   off += s.noc ? m * (s.noc * 64 + 16) : 0;
@@ -174,8 +177,12 @@ bool plan_stream(const qgemv_problem* const* probs, int count, size_t partial_fl
         const bool whole = order[t] != 0;
         const int nw = mode == 2 || !whole ? 8 : 16, cap = whole ? kStreamMaxSmem : kHalfSmem;
         int cta = 0, smem = 0, counters = 0;
-        size_t tail = partial_floats;              // words from the end, split sums from the start of the scratch
-        size_t head = 0;
+        // Split sums from the start of the scratch; words of residual projections in a region of their own at its end, below
+        // the one of the other kernels: a word is recognised by its launch tag, and no other data, nor tags of another count,
+        // may ever be taken for one.
+        if (partial_floats < kTPartFloats + kStreamWordFloats) return false;
+        const size_t floor = partial_floats - kTPartFloats - kStreamWordFloats;
+        size_t tail = partial_floats - kTPartFloats, head = 0;
         bool ok = true, epoch = false;
         for (int i = 0; i < count && ok; ++i) {
             const qgemv_problem& p = *probs[i];
@@ -184,7 +191,7 @@ bool plan_stream(const qgemv_problem* const* probs, int count, size_t partial_fl
             if (share < 1) share = 1;
             if (i == count - 1 && cta + share > sms && sms - cta >= 1) share = sms - cta;
             int need = 0;
-            ok = plan_segment(p, m, mode, bf16, nw, share, cap, tail - head, s, need);
+            ok = plan_segment(p, m, mode, bf16, nw, share, cap, floor - head, tail - floor, s, need);
             if (!ok) break;
             s.cta0 = cta;
             cta += s.groups * s.ksplit;
@@ -195,7 +202,6 @@ bool plan_stream(const qgemv_problem* const* probs, int count, size_t partial_fl
             out->part_off[i] = kWsPartialOff + head * sizeof(float);
             out->cnt_off[i] = kWsCounterOff + counters * sizeof(int);
             if (s.ksplit > 1) { head += (size_t)s.ksplit * s.n * s.mp; counters += s.groups; }
-            if (head > tail) ok = false;
             epoch = epoch || s.rank > 0;
         }
         if (!ok || cta > 256) continue;

@@ -15,6 +15,7 @@ constexpr int kMaxTiles = 2;           // tiles a warp keeps accumulators for (o
 constexpr int kMaxSegments = 4;        // weight matrices one launch can serve
 constexpr int kMaxDepth = 4;           // ring depth in batches (one batch = one slot per tile of a row block)
 constexpr int kHalfSmem = 115712;      // 113 KB: two CTAs per SM, so that the next launch is resident while this one runs
+constexpr size_t kStreamWordFloats = size_t(1) << 17;     // scratch kept for {value, launch tag} words, in 32-bit units
 constexpr int kProjectionK = 256;      // K columns of one round of an in-kernel residual projection
 
 // Weight formats: packed codes by the scale groups per 128-column block, or plain 16-bit rows.

@@ -73,3 +73,24 @@ def test_weights_written_in_place_are_seen():
         assert torch.equal(a(x), want_b)
         a.load_state_dict(host)
         assert torch.equal(a(x), want_a)
+
+
+def test_kernels_of_one_workspace_keep_their_projections_apart():
+    """One to four rows and five to sixteen rows run different kernels, each with a launch count of its own as the tag of the
+    residual projections: alternating them on one stream (equal counts) must not let one take the other's words."""
+    torch.manual_seed(1)
+    mod = HybridInt4Linear(torch.nn.Linear(4096, 2048, bias=False), 128)
+    mod.set_residual(torch.randn(2048, 8), torch.randn(8, 4096))
+    mod = mod.cuda()
+    s = torch.cuda.Stream()                                          # a fresh workspace: both counts start at zero
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        for _ in range(30):
+            x1, x8 = torch.randn(4, 4096).half().cuda(), torch.randn(16, 4096).half().cuda()
+            y1, y8 = mod(x1), mod(x8)
+            w = mod.effective_weight()
+            for x, y in ((x1, y1), (x8, y8)):
+                want = x.float() @ w.t()
+                assert float((y.float() - want).norm() / want.norm()) < 2e-3
+    s.synchronize()
+    assert ops.workspace_status("cuda", s) == 0
