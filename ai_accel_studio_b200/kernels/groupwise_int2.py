@@ -58,6 +58,22 @@ def _activation_weights(activation_rms: torch.Tensor, original_k: int, kp: int, 
     return ar.view(1, ng, group_size).square().clamp_min(1e-8)
 
 
+def _pack_on_device(weight, bits, group_size, activation_rms, first, last, steps):
+    """(packed, scales, padded K) from the CUDA quantiser, or None where it does not apply (CPU tensors, other types or groups)."""
+    from .. import ops
+    if not weight.is_cuda or weight.ndim != 2 or weight.dtype not in ops._DT or group_size not in ops.PACK_GROUPS or \
+            weight.numel() == 0 or not 1 <= steps <= 1024:
+        return None
+    w, rms = weight.detach(), None
+    if activation_rms is not None:
+        rms = activation_rms.detach().to(w.device).float().flatten()
+        if rms.numel() < w.shape[1]:
+            raise ValueError("activation_rms is shorter than K")
+        rms = rms.contiguous()
+    packed, scales = ops.pack(w, bits, group_size, rms, first, last, steps)
+    return packed, scales, scales.shape[1] * group_size
+
+
 def _levels(ref: torch.Tensor) -> torch.Tensor:
     return torch.tensor(INT2_LEVELS, device=ref.device, dtype=ref.dtype)
 
@@ -75,8 +91,12 @@ def pack_groupwise_int2(weight: torch.Tensor, group_size: int = 128,
     Without ``activation_rms`` the scale of a group is its largest magnitude.  With it, 13
     shrink/grow factors in [0.55, 1.15] are tried per group and the one with the smallest
     activation-energy-weighted squared error wins.  Rows are independent, so they are
-    processed in chunks; the result does not depend on the chunking.
+    processed in chunks; the result does not depend on the chunking.  CUDA weights are quantised by one
+    kernel (``qgemv_pack``) with the same result.
     """
+    dev = _pack_on_device(weight, 2, group_size, activation_rms, 0.55, 1.15, refine_steps)
+    if dev is not None:
+        return GroupwiseInt2Weight(dev[0], dev[1], int(weight.shape[1]), dev[2], group_size, activation_rms is not None)
     w, original_k, kp = _padded_float(weight, group_size, 4)
     n = w.shape[0]
     ng = kp // group_size

@@ -12,7 +12,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
-from .groupwise_int2 import _activation_weights, _dtype_name, _padded_float, _ROW_CHUNK_ELEMS
+from .groupwise_int2 import _activation_weights, _dtype_name, _pack_on_device, _padded_float, _ROW_CHUNK_ELEMS
 
 
 @dataclass
@@ -37,7 +37,11 @@ def pack_groupwise_int4(weight: torch.Tensor, group_size: int = 128, activation_
                         refine_steps: int = 11) -> GroupwiseInt4Weight:
     """Symmetric round-to-nearest-even INT4 with scale ``max|w| / 7`` per group; with
     ``activation_rms`` the scale is picked among 11 factors in [0.72, 1.18] by the smallest
-    activation-energy-weighted squared error.  Row-chunked; chunking does not change the result."""
+    activation-energy-weighted squared error.  Row-chunked; chunking does not change the result.  CUDA weights are
+    quantised by one kernel (``qgemv_pack``) with the same result."""
+    dev = _pack_on_device(weight, 4, group_size, activation_rms, 0.72, 1.18, refine_steps)
+    if dev is not None:
+        return GroupwiseInt4Weight(dev[0], dev[1], int(weight.shape[1]), dev[2], group_size, activation_rms is not None)
     w, original_k, kp = _padded_float(weight, group_size, 2)
     n = w.shape[0]
     ng = kp // group_size

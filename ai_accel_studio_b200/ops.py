@@ -327,6 +327,34 @@ def _(packed, bits):
     return packed.new_empty((packed.shape[0], packed.shape[1] * (8 // bits)))
 
 
+PACK_GROUPS = (16, 32, 64, 128, 256, 512)
+_FACTORS: dict = {}          # (device, first, last, steps) -> candidate factors of the scale search
+
+
+def pack(weight: torch.Tensor, bits: int, group: int, activation_rms, first: float, last: float, steps: int):
+    """Packed codes and fp16 scales of a CUDA matrix (``qgemv_pack``): bit-identical to the torch expression of the quantisers.
+    ``activation_rms``: float32 [>= K] or None; the candidate scales are ``steps`` multiples from ``first`` to ``last``."""
+    w = weight if weight.stride(1) == 1 else weight.contiguous()
+    n, k = w.shape
+    ng = -(-k // group)
+    packed = torch.empty((n, ng * group * bits // 8), dtype=torch.uint8, device=w.device)
+    scales = torch.empty((n, ng), dtype=torch.float16, device=w.device)
+    factors = None
+    if activation_rms is not None:
+        key = (w.device, first, last, steps)
+        factors = _FACTORS.get(key)
+        if factors is None:
+            factors = torch.linspace(first, last, steps, device=w.device)
+            if len(_FACTORS) < 64:
+                _FACTORS[key] = factors
+    with torch.cuda.device(w.device):
+        _cabi.check(_cabi.lib().qgemv_pack(bits, w.data_ptr(), w.stride(0), _DT[w.dtype], n, k, group,
+                                           None if activation_rms is None else activation_rms.data_ptr(),
+                                           None if factors is None else factors.data_ptr(), steps, packed.data_ptr(), scales.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream))
+    return packed, scales
+
+
 def plan_name(x, packed, scales, bits, group, k_original, outliers=0, rank=0, kernel="auto"):
     """Name of the kernel variant a call of this shape would launch (no launch happens)."""
     ws = ensure_workspace(x.device)

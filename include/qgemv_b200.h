@@ -223,6 +223,15 @@ int qdequant(int bits, const uint8_t* packed, int64_t ldp, const void* scales, i
              int n, int k_padded, int k_original, int group,
              void* out, int64_t ld_out, int out_dtype, void* stream);
 
+/* Quantise a dense matrix w [n, k] (fp16 / bf16 / fp32, rows of ldw elements) to packed codes [n, ceil(k / group) * group *
+ * bits / 8] and fp16 scales [n, ceil(k / group)], both contiguous.  Without `rms` a group's scale follows from its largest
+ * magnitude; with rms [k] (fp32) the `steps` multiples factors[i] of it are tried and the one with the smallest squared
+ * error weighted by rms^2 wins, the first of equal ones.  Groups of 16, 32, 64, 128, 256 and 512 (QGEMV_ERR_SHAPE otherwise).
+ * Replaces: pack_groupwise_int2  ai_accel_lab/kernels/groupwise_int2.py:66-119,
+ *           pack_groupwise_int4  ai_accel_lab/kernels/groupwise_int4.py:40-60. */
+int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, const float* factors,
+               int steps, uint8_t* packed, void* scales, void* stream);
+
 /* Expand packed bytes to one uint8 code per weight, [N, Kpad].
  * Replaces the code extraction of ai_accel_lab/kernels/groupwise_int2.py:123-124 and
  * ai_accel_lab/kernels/groupwise_int4.py:64-65. */
