@@ -20,7 +20,7 @@ MAX_BATCH = 16
 ABI_VERSION = 5
 
 EXPORTS = ("qgemv_run", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_describe", "qgemv_workspace_status", "qgemv_workspace_bytes", "qgemv_plan_name", "qdequant", "qunpack_codes", "qgemv_pack",
-           "qgemv_prepared_bytes", "qgemv_prepare", "qgemv_launch_prepared", "qgemv_error_string", "qgemv_abi_version", "qgemv_sizeof_problem",
+           "qgemv_prepared_bytes", "qgemv_prepare", "qgemv_launch_prepared", "qgemv_batch_scratch_bytes", "qgemv_run_batch", "qgemv_error_string", "qgemv_abi_version", "qgemv_sizeof_problem",
            "qcomm_slot_bytes", "qcomm_flag_bytes", "qcomm_state_bytes", "qcomm_allreduce", "qcomm_allreduce_rmsnorm", "qcomm_status", "qcomm_alloc", "qcomm_free",
            "qcomm_ipc_export", "qcomm_ipc_open", "qcomm_ipc_close",
            "qdec_rmsnorm", "qdec_rope_append", "qdec_attention_workspace_bytes", "qdec_attention", "qdec_silu_mul")

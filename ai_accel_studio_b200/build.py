@@ -23,6 +23,7 @@ UNITS = [
     ("qgemv_simt.cu", [], "qgemv_simt.o"),
     ("qdequant.cu", [], "qdequant.o"),
     ("qpack.cu", [], "qpack.o"),
+    ("qgemm.cu", [], "qgemm.o"),
     ("qcomm.cu", [], "qcomm.o"),
     ("qdecode.cu", [], "qdecode.o"),
     ("qgemv_mma.cu", ["-DQGEMV_INST_BITS=2"], "qgemv_mma_int2.o"),

@@ -1,0 +1,968 @@
+// Fused dequantise + GEMM for packed groupwise INT2 / INT4 weights and many activation rows (prompts), sm_100a.
+//
+//     y[m, n] = act( x . dequant(W)^T + outlier term + low-rank residual + bias )
+//
+// The dense matrix is never written: a persistent CTA per SM turns packed codes into 16-bit weights in registers and puts
+// them straight into tensor memory, where tcgen05.mma takes them as its A operand (128 weight rows; lane = row, a 32-bit
+// column = two K neighbours).  B is a tile of up to 256 activation rows, brought into shared memory by TMA (128-byte
+// swizzle); the accumulator (128 x 256 fp32) takes the other half of tensor memory.
+//
+//   bound      tensor pipe: 128 x 256 x 128 MACs take 1024 clocks per SM; making 128 x 128 weights takes 8 warps about 260
+//              issue slots per scheduler of those (INT4 1.6, INT2 1.3 instructions per weight, from a byte permute of the
+//              four scaled levels), reading B takes 64 of shared memory's 128 bytes a clock.
+//   A in TMEM  keeps the converted weights out of shared memory, whose bandwidth B and the TMA writes need.
+//   extra K    outlier columns and the residual are further K columns: [ W | W_outlier | U ] . [ x | x_outlier | V x ]^T, so
+//              they cost no passes over y.  With bf16 activations U and V x go in as high and low halves (three products).
+//   split      units of 128 K columns are dealt out evenly over the SMs when whole tiles would leave more than that idle; the
+//              contributions of a tile then meet in scratch memory and whichever CTA comes last adds them in CTA order.
+//
+// A first small kernel lays x out for this: K columns permuted the way the codes leave a word, padded with zeros to
+// whole units, gathered outlier activations and the projections V x behind them.
+//
+// Weights are rounded exactly as qdequant rounds them; sums are fp32 and are rounded to the activation type once.
+// Replaces, for these shapes, dequantisation to a dense matrix + library GEMMs for base, outlier and residual term.
+#include <cuda.h>
+
+#include "qgemv_common.cuh"
+
+namespace qgemv {
+namespace {
+
+constexpr int kRows = 128;                 // weight rows of a tile (lanes of tensor memory)
+constexpr int kUnit = 128;                 // K columns of one stage (A: 64 columns of tensor memory, B: two chunks)
+constexpr int kChunk = 64;                 // K columns of one TMA box: 128 bytes of a 16-bit row
+constexpr int kMaxStages = 6;
+constexpr int kMaxWidth = 256;             // activation rows of a tile
+constexpr int kGroups = 4;                 // warpgroups that dequantise (every fourth unit each) and finish tiles
+constexpr int kGemmThreads = kGroups * 128 + 64;     // and one warp that issues TMA, one that issues the mma
+constexpr int kTmaWarp = kGroups * 4, kMmaWarp = kTmaWarp + 1;
+constexpr int kSmemCtl = 512;              // barriers, at the end of shared memory
+
+struct GemmArgs {
+    const uint8_t* packed;    long long ldp;
+    const __half* scales;     long long lds;
+    const __half* bias;
+    const __half* ow;         long long ldow;
+    const __half* ru;         long long ldu;
+    void* y;                  long long ldy;
+    float* partial;           // contributions of split tiles: [cta * 2 + piece][column][row]
+    int* counters;            // arrivals per tile (zero between launches)
+    int* status;
+    int m, n, group, ng, pieces, act;         // pieces: 16-byte pieces of a packed row
+    int oc, oc8, rank, rank8, xcopies;        // padded to 8; xcopies: 1, or 3 with bf16 (high / low halves)
+    int ow_vec, ru_vec;                       // rows readable in 16-byte pieces
+    int wunits, units, chunks;                // weight units, all units and 64-column chunks of K
+    int width, mtiles, ntiles;
+    int sc_odd;                               // 1: the scales start on an odd 2-byte boundary
+    int stages, ring;                         // stages of A and B (one barrier for both: a wait costs the mma warp 200 clocks); units of codes the ring holds (power of two)
+    int ctl_off;                              // barriers in shared memory
+    int groups;                               // warpgroups that dequantise: at most `stages`, see the wait for a stage
+    int split;                                // 1: units dealt out evenly, 0: whole tiles
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits for a phase; false after about two seconds, or when another role has given up.
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* gave_up, int* status) {
+    const long long t0 = clock64();
+    for (;;) {
+        if (mbar_try(bar, parity)) return true;
+        if (*gave_up) return false;
+        if (clock64() - t0 > 4000000000ll) { *gave_up = 1; atomicExch(status, 2); return false; }
+    }
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* gave_up, int* status) {
+    for (int i = 0; i < 64; ++i) if (mbar_try(bar, parity)) return true;
+    return mbar_wait_slow(bar, parity, gave_up, status);
+}
+// One lane of a converged warp.  The roles that issue TMA and mma run as whole warps and pick a lane only for the instruction:
+// their operands are then uniform registers; a loop run by one lane alone spent some 400 clocks on a chunk's four mma.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
+}
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// D[128 x N] (+)= A (tensor memory, 128 x 16) . B (shared memory, N x 16)^T
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t add) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                 ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(add) : "memory");
+}
+__device__ __forceinline__ void tc_st32(uint32_t at, const uint32_t (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+                 "%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(at), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+                 "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+__device__ __forceinline__ void tc_ld16(uint32_t at, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(at) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
+// Codes to 16-bit weights.  Order of the K columns as they leave a word (x is permuted alike):
+//   INT4, 8 columns:  0 4 1 5 2 6 3 7        INT2, 16 columns: 0 2 4 6 8 10 12 14 1 3 5 7 9 11 13 15
+// ---------------------------------------------------------------------------------------------
+// What a scale becomes: INT4 the scale twice in the activation type; INT2 the four levels times the scale, low and high bytes.
+template <int BITS, bool BF16>
+__device__ __forceinline__ uint2 scale_table(__half s) {
+    if constexpr (BITS == 4) {
+        if constexpr (BF16) { const __nv_bfloat162 b = __bfloat162bfloat162(__float2bfloat16_rn(__half2float(s))); return make_uint2(*reinterpret_cast<const uint32_t*>(&b), 0u); }
+        else { const __half2 h = __half2half2(s); return make_uint2(*reinterpret_cast<const uint32_t*>(&h), 0u); }
+    } else {
+        uint32_t one, third;                            // 1 and 1/3 (rounded to the type) times the scale
+        if constexpr (BF16) {
+            const float sb = __bfloat162float(__float2bfloat16_rn(__half2float(s)));
+            one = __bfloat16_as_ushort(__float2bfloat16_rn(sb));
+            third = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(0x3EAB0000u), sb)));
+        } else {
+            one = __half_as_ushort(s);
+            third = __half_as_ushort(__float2half_rn(__fmul_rn(__half2float(__ushort_as_half(0x3555u)), __half2float(s))));
+        }
+        const uint32_t none = one ^ 0x8000u, nthird = third ^ 0x8000u;          // levels -1, -1/3, 1/3, 1
+        const uint32_t lo = (none & 0xff) | (nthird & 0xff) << 8 | (third & 0xff) << 16 | (one & 0xff) << 24;
+        const uint32_t hi = none >> 8 | (nthird >> 8) << 8 | (third >> 8) << 16 | (one >> 8) << 24;
+        return make_uint2(lo, hi);
+    }
+}
+template <bool BF16> __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (BF16) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// One word of codes: 16 (INT2) or 8 (INT4) columns into 8 or 4 registers.
+template <int BITS, bool BF16>
+__device__ __forceinline__ void expand(uint32_t w, uint2 tab, uint32_t* out) {
+    if constexpr (BITS == 2) {
+        const uint32_t s0 = w & 0x33333333u, s1 = (w >> 2) & 0x33333333u;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t sel = (h & 2 ? s1 : s0) >> (h & 1 ? 16 : 0);
+            const uint32_t lo = __byte_perm(tab.x, 0u, sel), hi = __byte_perm(tab.y, 0u, sel);      // nibbles 0 .. 3 of sel
+            out[2 * h] = __byte_perm(lo, hi, 0x5140);
+            out[2 * h + 1] = __byte_perm(lo, hi, 0x7362);
+        }
+    } else if constexpr (BF16) {
+        // 128 + c is exact in bf16 (units of 1), and so is c - 8
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t v = ((w >> (4 * q)) & 0x000f000fu) | 0x43004300u;
+            asm("sub.rn.bf16x2 %0, %0, %1;" : "+r"(v) : "r"(0x43084308u));
+            out[q] = mul2<true>(v, tab.x);
+        }
+    } else {
+        // 1024 + c, and 1024 + 16 c for the upper nibble: both exact, as is c - 8
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t src = q & 2 ? w >> 8 : w;
+            uint32_t v;
+            if (q & 1) {
+                v = (src & 0x00f000f0u) | 0x64006400u;
+                asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(v) : "r"(0x2c002c00u), "r"(0xd480d480u));      // / 16 - 72
+            } else {
+                v = (src & 0x000f000fu) | 0x64006400u;
+                asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(v) : "r"(0x64086408u));
+            }
+            out[q] = mul2<false>(v, tab.x);
+        }
+    }
+}
+
+// 128 columns of one row: 32 or 64 bytes of codes, and the scales.
+template <int BITS> struct Raw { uint4 w[BITS]; __half s[4]; };
+
+// Codes and scales travel through a ring of shared memory, filled by cp.async many units ahead (HBM's latency is several
+// units of a narrow tile).  A warp copies the 32 rows it will read itself: coalesced pieces of 16 bytes, stored [piece][row].
+template <int BITS, int NG> struct RawSlot {
+    static constexpr int WORDS = NG == 1 ? 1 : NG / 2 + 1;             // aligned 4-byte words that cover NG scales
+    static constexpr int CODES = BITS * kRows * 16;
+    static constexpr int BYTES = CODES + WORDS * kRows * 4;
+};
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, int valid) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void cp4(uint32_t dst, const void* src, int valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+// slot: shared address; row0: first weight row of the warp (its rows are row0 .. row0 + 31, clamped to the matrix).
+template <int BITS, int NG>
+__device__ __forceinline__ void request_raw(const GemmArgs& p, uint32_t slot, int quarter, int lane, int row0, int unit) {
+    using S = RawSlot<BITS, NG>;
+    constexpr int RPI = 32 / BITS;                                     // rows of one warp-wide copy
+    const int piece = lane % BITS, r = lane / BITS;
+    const int ok = unit * BITS + piece < p.pieces ? 16 : 0;
+    const uint8_t* src = p.packed + (ok ? (size_t)unit * (16 * BITS) + piece * 16 : 0);
+    const uint32_t dst = slot + piece * (kRows * 16) + (quarter * 32 + r) * 16;
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) cp16(dst + i * (RPI * 16), src + (size_t)min(row0 + i * RPI + r, p.n - 1) * p.ldp, ok);
+    const long long e = (long long)min(row0 + lane, p.n - 1) * p.lds, end = (long long)(p.n - 1) * p.lds + p.ng;      // halves
+    const int g0 = NG > 1 ? unit * NG : unit * kUnit / p.group;
+    const long long first = (p.sc_odd + e + g0) & ~1ll;                // in halves from the aligned base
+#pragma unroll
+    for (int w = 0; w < S::WORDS; ++w) {
+        const long long at = first + 2 * w - p.sc_odd;
+        const int left = (int)min((long long)4, max(0ll, (end - at) * 2));
+        cp4(slot + S::CODES + (w * kRows + quarter * 32 + lane) * 4, left > 0 ? (const void*)(p.scales + at) : (const void*)(p.scales - p.sc_odd), left);
+    }
+}
+template <int BITS, int NG>
+__device__ __forceinline__ void read_raw(const GemmArgs& p, uint32_t slot, int trow, int row, int unit, Raw<BITS>& r) {
+    using S = RawSlot<BITS, NG>;
+#pragma unroll
+    for (int i = 0; i < BITS; ++i)
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w[i].x), "=r"(r.w[i].y), "=r"(r.w[i].z), "=r"(r.w[i].w) : "r"(slot + (i * kRows + trow) * 16) : "memory");
+    const int g0 = NG > 1 ? unit * NG : unit * kUnit / p.group;
+    const int odd = (p.sc_odd + (int)((row * p.lds + g0) & 1)) & 1;
+    uint32_t w[S::WORDS];
+#pragma unroll
+    for (int i = 0; i < S::WORDS; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(slot + S::CODES + (i * kRows + trow) * 4) : "memory");
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+        const int h = j + odd;
+        uint32_t word = w[0];
+#pragma unroll
+        for (int i = 1; i < S::WORDS; ++i) if ((h >> 1) == i) word = w[i];
+        r.s[j] = g0 + j < p.ng ? __ushort_as_half((unsigned short)(h & 1 ? word >> 16 : word)) : __half(0.0f);      // columns past K: weight 0
+    }
+}
+
+// Half h (64 columns) of a unit into 32 registers.
+template <int BITS, int NG, bool BF16>
+__device__ __forceinline__ void expand_half(const Raw<BITS>& r, int h, uint32_t (&out)[32]) {
+    constexpr int WORDS = BITS * 2;                                    // words of 64 columns
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(r.w) + h * WORDS;
+    constexpr int PER = WORDS / (NG > 1 ? NG / 2 : 1);                 // words per scale
+    uint2 tab;
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        if (i % PER == 0) tab = scale_table<BITS, BF16>(r.s[NG > 1 ? h * (NG / 2) + i / PER : 0]);
+        expand<BITS, BF16>(w[i], tab, out + i * (32 / WORDS));
+    }
+}
+
+// This CTA's share: units [u0, u1) of the sequence tile-major, unit-minor.
+__device__ __forceinline__ int first_unit(const GemmArgs& p, int cta, int grid) {
+    const long long tiles = (long long)p.mtiles * p.ntiles;
+    return (int)(p.split ? cta * (tiles * p.units) / grid : cta * tiles / grid * p.units);
+}
+
+// Extra columns from k0 into an A stage: outlier weights, then U (with bf16 activations high, low and high halves), each
+// padded to 8 columns.  All loads of 64 columns are issued before the first is used.
+template <bool BF16>
+__device__ __noinline__ void extra_unit(const GemmArgs& p, int row, int k0, uint32_t at) {
+    const unsigned short* ow = reinterpret_cast<const unsigned short*>(p.ow) + (size_t)row * p.ldow;
+    const unsigned short* ru = reinterpret_cast<const unsigned short*>(p.ru) + (size_t)row * p.ldu;
+    for (int h = 0; h < 2; ++h) {
+        uint32_t out[32];
+        auto load8 = [&](const unsigned short* src, int left, bool vec, uint32_t* o) {
+            if (vec) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+                o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+            } else {
+                unsigned short v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = i < left ? __ldg(src + i) : (unsigned short)0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[i] = v[2 * i] | (uint32_t)v[2 * i + 1] << 16;
+            }
+        };
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int j = k0 + h * kChunk + 8 * q, r = j - p.oc8;
+            out[4 * q] = out[4 * q + 1] = out[4 * q + 2] = out[4 * q + 3] = 0u;
+            if (j < p.oc) load8(ow + j, p.oc - j, p.ow_vec, out + 4 * q);
+            else if (p.rank > 0 && r >= 0 && r < p.rank8 * p.xcopies) load8(ru + r % p.rank8, p.rank - r % p.rank8, p.ru_vec, out + 4 * q);
+        }
+        if constexpr (BF16) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r = k0 + h * kChunk + 8 * q - p.oc8;
+                const bool low = r >= p.rank8 && r < 2 * p.rank8;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&out[4 * q + i]));
+                    __nv_bfloat162 v = __floats2bfloat162_rn(f.x, f.y);
+                    if (low) v = __floats2bfloat162_rn(f.x - __low2float(v), f.y - __high2float(v));
+                    out[4 * q + i] = *reinterpret_cast<const uint32_t*>(&v);
+                }
+            }
+        }
+        tc_st32(at + h * 32, out);
+    }
+}
+
+struct Ends {                                          // what a warp needs to finish tiles
+    uint32_t tmem, accfull, accempty, meeting, accph, meetph;
+    int wg, quarter, lane, u0, grid, cta;
+    volatile int* gave_up;
+    volatile int* last_flag;
+};
+// Values of 16 activation rows from m0 of this lane's weight row: bias, activation, store.  Everything by value: a field read
+// through a reference would be loaded again after every store.
+template <bool BF16>
+__device__ __forceinline__ void put(typename Act16<BF16>::T* y, long long ldy, int m, int n, int act, int row, int m0, int lane, float b, const float (&v)[16]) {
+    using XT = typename Act16<BF16>::T;
+    auto r16 = [](float f) { return Act16<BF16>::to_float(Act16<BF16>::from_float(f)); };
+    const int count = min(16, m - m0);
+    if (act == QGEMV_ACT_SILU_MUL) {                   // rows come in blocks of 8 gate and 8 up rows
+        XT* o = y + (size_t)m0 * ldy + (row >> 4) * 8 + (row & 7);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const float mine = r16(v[q] + b), up = __shfl_down_sync(0xffffffffu, mine, 8);
+            const float s = r16(mine / (1.0f + __expf(-mine)));
+            if (!(lane & 8) && row < n && q < count) *o = Act16<BF16>::from_float(s * up);
+            o += ldy;
+        }
+        return;
+    }
+    if (row >= n) return;
+    XT* o = y + (size_t)m0 * ldy + row;
+    XT w[16];
+    if (act == QGEMV_ACT_NONE) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) w[q] = Act16<BF16>::from_float(v[q] + b);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) w[q] = Act16<BF16>::from_float(apply_act(v[q] + b, act));
+    }
+    if (count == 16) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) { *o = w[q]; o += ldy; }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) { if (q < count) *o = w[q]; o += ldy; }
+    }
+}
+// The accumulator is complete: a whole tile is stored; a piece of a tile is parked, and the last CTA to park one adds them in
+// CTA order.  Out of line: the loop that makes weights has to stay inside the instruction cache.
+template <bool BF16>
+__device__ __noinline__ bool finish_tile(const GemmArgs& args, Ends& e, int tile, int unit) {
+    using XT = typename Act16<BF16>::T;
+    const GemmArgs p = args;
+    XT* const y = static_cast<XT*>(p.y);
+    const int lane = threadIdx.x & 31;
+    bool ok = __all_sync(0xffffffffu, mbar_wait(e.accfull, e.accph, e.gave_up, p.status));
+    if (!ok) return false;
+    e.accph ^= 1;
+    tc_fence_after();
+    const int nt = tile / p.mtiles, mt = tile - nt * p.mtiles, trow = e.quarter * 32 + e.lane, row = nt * kRows + trow;
+    const float b = p.bias ? __half2float(__ldg(p.bias + min(row, p.n - 1))) : 0.0f;
+    const int c0 = e.wg * (p.width / 16) / kGroups * 16, c1 = (e.wg + 1) * (p.width / 16) / kGroups * 16;      // this warpgroup's columns
+    const bool whole = unit + 1 == p.units && tile * p.units >= e.u0;
+    // a CTA has at most two pieces of split tiles: the one at its first unit, and one at its last
+    const size_t piece = (size_t)p.width * kRows;
+    float* mine = p.partial + (size_t)(e.cta * 2 + (tile * p.units < e.u0 ? 0 : 1)) * piece;
+    for (int col = c0; col < c1; col += 16) {
+        uint32_t r[16];
+        tc_ld16(e.tmem + ((uint32_t)(e.quarter * 32) << 16) + col, r);
+        if (whole) {
+            float v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
+            put<BF16>(y, p.ldy, p.m, p.n, p.act, row, mt * p.width + col, lane, b, v);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) mine[(size_t)(col + q) * kRows + trow] = __uint_as_float(r[q]);
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (e.lane == 0) mbar_arrive(e.accempty);
+    if (whole) return true;
+    const int total = p.mtiles * p.ntiles * p.units, first = tile * p.units, last = first + p.units - 1;
+    auto owner = [&](int u) {
+        int c = (int)((long long)u * e.grid / total);
+        while (first_unit(p, c + 1, e.grid) <= u) ++c;
+        while (first_unit(p, c, e.grid) > u) --c;
+        return c;
+    };
+    const int cf = owner(first), cl = owner(last);     // contributors: the CTAs whose ranges meet this tile
+    __threadfence();
+    auto meet = [&]() {                                // all warps that are here, with a limit as everywhere
+        __syncwarp();
+        if (e.lane == 0) mbar_arrive(e.meeting);
+        ok = __all_sync(0xffffffffu, mbar_wait(e.meeting, e.meetph, e.gave_up, p.status));
+        e.meetph ^= 1;
+        return ok;
+    };
+    if (!meet()) return false;
+    if (threadIdx.x == 0) {
+        const int old = atomicAdd(p.counters + tile, 1);
+        if (old == cl - cf) p.counters[tile] = 0;
+        *e.last_flag = old == cl - cf;
+    }
+    if (!meet()) return false;
+    if (*e.last_flag == 0) return true;                // (rewritten only after the next meeting of the warps)
+    __threadfence();
+    for (int col = c0; col < c1; col += 16) {
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+#pragma unroll 2
+        for (int c = cf; c <= cl; ++c) {
+            const float* src = p.partial + (size_t)(c * 2 + (first < first_unit(p, c, e.grid) ? 0 : 1)) * piece;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] += __ldcg(src + (size_t)(col + q) * kRows + trow);
+        }
+        put<BF16>(y, p.ldy, p.m, p.n, p.act, row, mt * p.width + col, lane, b, v);
+    }
+    return true;
+}
+
+template <int BITS, int NG, bool BF16>
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ GemmArgs p, const __grid_constant__ CUtensorMap xmap) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + p.ctl_off;        // B stages first: their 128-byte swizzle wants 1024-byte alignment
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t ctl = smem_u32(smem);
+    const uint32_t full = ctl, empty = ctl + 64, accfull = ctl + 192, accempty = ctl + 200, meeting = ctl + 208;
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smem + 256);
+    volatile int* last_flag = reinterpret_cast<volatile int*>(smem + 260);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 264);
+    const uint32_t bbase = smem_u32(smem_raw), bbytes = (uint32_t)p.width * 128;      // one chunk
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid == 0) {
+        for (int i = 0; i < kMaxStages; ++i) {
+            mbar_init(full + 8 * i, 5);                // four warps' weights and the TMA
+            mbar_init(empty + 8 * i, 1);
+        }
+        mbar_init(accfull, 1); mbar_init(accempty, kGroups * 4); mbar_init(meeting, kGroups * 4);
+        *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(ctl + 264) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // All of tensor memory is this CTA's: the accumulator from column 0, the A stages at the end.
+    constexpr uint32_t tmem = 0;
+    const uint32_t a_base = 512 - p.stages * 64;
+    const int grid = gridDim.x, cta = blockIdx.x;
+    const int u0 = first_unit(p, cta, grid), u1 = first_unit(p, cta + 1, grid);
+
+    if (warp == kTmaWarp) {                            // ---- TMA: activation chunks in order -----------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("fence.proxy.async;" ::: "memory");
+        int stage = 0, tile = u0 / p.units, unit = u0 - tile * p.units;
+        uint32_t phase = 1;
+        for (int u = u0; u < u1; ++u) {
+            if (!__all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase, gave_up, p.status))) break;
+            if (elect_one()) {
+                const int y = tile % p.mtiles * p.width;
+                const uint32_t dst = bbase + stage * 2 * bbytes;
+                const bool two = unit * 2 + 1 < p.chunks;
+                mbar_expect(full + 8 * stage, two ? 2 * bbytes : bbytes);
+                tma_load(dst, &xmap, unit * kUnit, y, full + 8 * stage);
+                if (two) tma_load(dst + bbytes, &xmap, unit * kUnit + kChunk, y, full + 8 * stage);
+            }
+            __syncwarp();
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
+            if (++unit == p.units) { unit = 0; ++tile; }
+        }
+    } else if (warp == kMmaWarp) {                     // ---- mma issue --------------------------------------------------
+        const uint32_t idesc = (1u << 4) | (BF16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(p.width >> 3) << 17) | ((kRows >> 4) << 24);
+        // K-major, 128-byte swizzle: 8 rows x 128 bytes per 1024-byte atom
+        const uint64_t desc0 = (uint64_t)((bbase & 0x3ffff) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+        const uint64_t step = 2 * (bbytes >> 4);
+        int stage = 0, unit = u0 % p.units;
+        uint32_t phase = 0, accph = 1, add = 0, a = a_base;
+        uint64_t desc = desc0;
+        for (int u = u0; u < u1; ++u) {
+            if (!add) {                                // a new accumulation: the previous one has been read
+                if (!__all_sync(0xffffffffu, mbar_wait(accempty, accph, gave_up, p.status))) break;
+                accph ^= 1;
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * stage, phase, gave_up, p.status))) break;
+            tc_fence_after();
+            const bool two = unit * 2 + 1 < p.chunks, end = unit + 1 == p.units || u + 1 == u1;
+            if (elect_one()) {
+                tc_mma(0, a, desc, idesc, add);
+                tc_mma(0, a + 8, desc + 2, idesc, 1);
+                tc_mma(0, a + 16, desc + 4, idesc, 1);
+                tc_mma(0, a + 24, desc + 6, idesc, 1);
+                if (two) {
+                    const uint64_t d2 = desc + (bbytes >> 4);
+                    tc_mma(0, a + 32, d2, idesc, 1);
+                    tc_mma(0, a + 40, d2 + 2, idesc, 1);
+                    tc_mma(0, a + 48, d2 + 4, idesc, 1);
+                    tc_mma(0, a + 56, d2 + 6, idesc, 1);
+                }
+                tc_commit(empty + 8 * stage);
+                if (end) tc_commit(accfull);
+            }
+            __syncwarp();
+            add = !end;
+            a += 64; desc += step;
+            if (++stage == p.stages) { stage = 0; phase ^= 1; a = a_base; desc = desc0; }
+            if (++unit == p.units) unit = 0;
+        }
+    } else {                                           // ---- weights, and the tiles' ends ------------------------------
+        const int wg = warp >> 2, quarter = warp & 3, count = u1 - u0;
+        const uint32_t a_lane = a_base + ((uint32_t)(quarter * 32) << 16);
+        Ends e;
+        e.tmem = tmem; e.wg = wg; e.quarter = quarter; e.lane = lane; e.u0 = u0; e.grid = grid; e.cta = cta;
+        e.accfull = accfull; e.accempty = accempty; e.meeting = meeting; e.accph = 0; e.meetph = 0;
+        e.gave_up = gave_up; e.last_flag = last_flag;
+        const int lrow = quarter * 32 + lane;
+        int tile = u0 / p.units, unit = u0 - tile * p.units;
+        // requests of this warpgroup's units (every p.groups-th one), `ahead` of them; the slots are the warpgroup's own
+        const int G = p.groups;
+        int ftile = tile, funit = unit + wg, fi = wg < G ? wg : count, fq = 0;
+        while (funit >= p.units) { funit -= p.units; ++ftile; }
+        const int ahead = p.ring / kGroups;                // 1, 2 or 4
+        const uint32_t ring = bbase + p.stages * 2 * bbytes + wg * ahead * RawSlot<BITS, NG>::BYTES;
+        auto request = [&]() {
+            if (fi < count && funit < p.wunits)
+                request_raw<BITS, NG>(p, ring + (fq & (ahead - 1)) * RawSlot<BITS, NG>::BYTES, quarter, lane, (ftile / p.mtiles) * kRows + quarter * 32, funit);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            ++fq;
+            fi += G;
+            funit += G;
+            while (funit >= p.units) { funit -= p.units; ++ftile; }
+        };
+        for (int i = 0; i < ahead; ++i) request();
+        auto landed = [&]() {                          // the oldest request is complete
+            if (ahead == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            else if (ahead == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 3;" ::: "memory");
+            __syncwarp();
+        };
+        bool ok = true;
+        uint32_t phase = 1;                            // parity of the stage's last release (passes at once the first time)
+        int stage = wg, done = tile;                   // done: first tile of this CTA not finished yet
+        int q = 0;
+        unit += wg;
+        while (unit >= p.units) { unit -= p.units; ++tile; }
+#pragma unroll 1
+        for (int i = wg < G ? wg : count; i < count; i += G, ++q) {
+            for (; done < tile && ok; ++done) ok = finish_tile<BF16>(p, e, done, p.units - 1);      // tiles that ended with others' units
+            if (!ok) break;
+            landed();
+            // A parity cannot tell a release from the one two before it.  This warpgroup's last unit was G <= stages ago and waited
+            // for a release no older than that, so the one before the awaited release has happened.
+            auto stage_free = [&]() {
+                ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase, gave_up, p.status));
+                tc_fence_after();
+                return ok;
+            };
+            if (unit < p.wunits) {
+                Raw<BITS> cur;
+                read_raw<BITS, NG>(p, ring + (q & (ahead - 1)) * RawSlot<BITS, NG>::BYTES, lrow, min((tile / p.mtiles) * kRows + lrow, p.n - 1), unit, cur);
+                __syncwarp();
+                request();
+                uint32_t lo[32], hi[32];               // converted before the stage is free: it is held for the store only
+                expand_half<BITS, NG, BF16>(cur, 0, lo);
+                expand_half<BITS, NG, BF16>(cur, 1, hi);
+                if (!stage_free()) break;
+                tc_st32(a_lane + stage * 64, lo);
+                tc_st32(a_lane + stage * 64 + 32, hi);
+            } else {
+                request();
+                if (!stage_free()) break;
+                extra_unit<BF16>(p, min((tile / p.mtiles) * kRows + lrow, p.n - 1), (unit - p.wunits) * kUnit, a_lane + stage * 64);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * stage);
+            stage += G;
+            if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
+            unit += G;
+            while (unit >= p.units) { unit -= p.units; ++tile; }
+        }
+        const int last = (u1 - 1) / p.units;
+        for (; done < last && ok; ++done) ok = finish_tile<BF16>(p, e, done, p.units - 1);
+        if (ok && count > 0) finish_tile<BF16>(p, e, last, u1 - 1 - last * p.units);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*gave_up) {                                    // let copies and mma in flight end before the CTA's memory goes
+        const long long t0 = clock64();
+        while (clock64() - t0 < 20000000ll) __nanosleep(1000);
+    }
+    if (warp == kMmaWarp) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*tmem_slot) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// x in the order the mma meets it: [M, chunks * 64], see the head of the file.  A CTA takes 8 activation rows and a share of
+// K; a warp 64 columns at a time: lane (g, t) 16 columns of row g, which it permutes and stores, and which are its B
+// fragments for the projections (V rows as A; any order of K does, as long as both sides use it).  The last CTA of a row
+// group adds the K shares in order and writes the extra columns.  Bound by its traffic (x once in, once out); a version
+// with fp32 FMAs took 26 us for 1000 x 8192 and rank 8, all of it latency.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+struct PrepArgs {
+    const unsigned short* x;  long long ldx;
+    const int32_t* oidx;
+    const __half* rv;         long long ldv;
+    unsigned short* out;
+    float* tparts;            // [share][row][rank]
+    int* counters;            // per row group
+    int m, k, oc, oc8, rank, kw, ke, vec, vvec;
+};
+constexpr int kPrepWarps = 8;
+
+template <int BITS, bool BF16>
+__global__ void __launch_bounds__(kPrepWarps * 32) prepare_kernel(const __grid_constant__ PrepArgs p) {
+    using XT = typename Act16<BF16>::T;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float red[kPrepWarps][64][8];
+    __shared__ float ts[8][64];
+    __shared__ int last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int m0 = blockIdx.x * 8, share = blockIdx.y, shares = gridDim.y, row = min(m0 + g, p.m - 1);
+    const int rtiles = (p.rank + 15) >> 4, blocks = p.kw / 64;
+    const unsigned short* xr = p.x + (size_t)row * p.ldx;
+    float acc[4][4];                                   // up to 64 ranks
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[i][q] = 0.0f;
+    auto load8 = [&](const unsigned short* src, int c, bool v16) {
+        if (v16 && c + 8 <= p.k) return __ldg(reinterpret_cast<const uint4*>(src + c));
+        uint32_t e[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t lo = c + 2 * q < p.k ? src[c + 2 * q] : 0, hi = c + 2 * q + 1 < p.k ? src[c + 2 * q + 1] : 0;
+            e[q] = lo | hi << 16;
+        }
+        return make_uint4(e[0], e[1], e[2], e[3]);
+    };
+#pragma unroll 2
+    for (int blk = share * kPrepWarps + warp; blk < blocks; blk += shares * kPrepWarps) {
+        const int c = blk * 64 + t * 16;
+        uint4 a = load8(xr, c, p.vec), b = load8(xr, c + 8, p.vec);
+        uint4 o0, o1;
+        if constexpr (BITS == 4) {                     // (0 1) (2 3) (4 5) (6 7) -> (0 4) (1 5) (2 6) (3 7)
+            o0 = make_uint4(__byte_perm(a.x, a.z, 0x5410), __byte_perm(a.x, a.z, 0x7632), __byte_perm(a.y, a.w, 0x5410), __byte_perm(a.y, a.w, 0x7632));
+            o1 = make_uint4(__byte_perm(b.x, b.z, 0x5410), __byte_perm(b.x, b.z, 0x7632), __byte_perm(b.y, b.w, 0x5410), __byte_perm(b.y, b.w, 0x7632));
+        } else {                                       // evens, then odds
+            o0 = make_uint4(__byte_perm(a.x, a.y, 0x5410), __byte_perm(a.z, a.w, 0x5410), __byte_perm(b.x, b.y, 0x5410), __byte_perm(b.z, b.w, 0x5410));
+            o1 = make_uint4(__byte_perm(a.x, a.y, 0x7632), __byte_perm(a.z, a.w, 0x7632), __byte_perm(b.x, b.y, 0x7632), __byte_perm(b.z, b.w, 0x7632));
+        }
+        if (m0 + g < p.m) {
+            uint4* d = reinterpret_cast<uint4*>(p.out + (size_t)row * p.ke + c);
+            d[0] = o0;
+            d[1] = o1;
+        }
+        if (rtiles == 0) continue;
+        float2 up = make_float2(1.0f, 1.0f);
+        if constexpr (BF16) {                          // as fp16, with a power of two per row and 64 columns (exact)
+            float f[16];
+            const XT* ea = reinterpret_cast<const XT*>(&a);
+            const XT* eb = reinterpret_cast<const XT*>(&b);
+            uint32_t big = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) { f[q] = Act16<BF16>::to_float(ea[q]); f[8 + q] = Act16<BF16>::to_float(eb[q]); }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) big = max(big, __float_as_uint(f[q]) & 0x7fffffffu);
+            big = max(big, __shfl_xor_sync(0xffffffffu, big, 1));
+            big = max(big, __shfl_xor_sync(0xffffffffu, big, 2));
+            const int e = max(-96, (int)(big >> 23) - 127);
+            const float down = __int_as_float((127 + 13 - e) << 23);
+            const float mine = big >= 0x7f800000u ? __int_as_float(0x7fffffff) : __int_as_float((127 - 13 + e) << 23);
+            up.x = __shfl_sync(0xffffffffu, mine, 8 * t);
+            up.y = __shfl_sync(0xffffffffu, mine, 8 * t + 4);
+            __half2 h[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) h[q] = __floats2half2_rn(f[2 * q] * down, f[2 * q + 1] * down);
+            const uint32_t* hw = reinterpret_cast<const uint32_t*>(h);
+            a = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            b = make_uint4(hw[4], hw[5], hw[6], hw[7]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i >= rtiles) break;
+            const int r0 = i * 16 + g, r1 = r0 + 8;
+            const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+            const unsigned short* v0 = reinterpret_cast<const unsigned short*>(p.rv) + (size_t)r0 * p.ldv;
+            const unsigned short* v1 = v0 + 8 * p.ldv;
+            const uint4 va0 = r0 < p.rank ? load8(v0, c, p.vvec) : z, vb0 = r0 < p.rank ? load8(v0, c + 8, p.vvec) : z;
+            const uint4 va1 = r1 < p.rank ? load8(v1, c, p.vvec) : z, vb1 = r1 < p.rank ? load8(v1, c + 8, p.vvec) : z;
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            mma16816(s, va0.x, va1.x, va0.y, va1.y, a.x, a.y);
+            mma16816(s, va0.z, va1.z, va0.w, va1.w, a.z, a.w);
+            mma16816(s, vb0.x, vb1.x, vb0.y, vb1.y, b.x, b.y);
+            mma16816(s, vb0.z, vb1.z, vb0.w, vb1.w, b.z, b.w);
+            acc[i][0] = fmaf(s[0], up.x, acc[i][0]); acc[i][1] = fmaf(s[1], up.y, acc[i][1]);
+            acc[i][2] = fmaf(s[2], up.x, acc[i][2]); acc[i][3] = fmaf(s[3], up.y, acc[i][3]);
+        }
+    }
+    const int per = p.rank * 8;
+    if (rtiles > 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) red[warp][i * 16 + g + (q >> 1) * 8][2 * t + (q & 1)] = acc[i][q];
+        __syncthreads();
+        for (int i = tid; i < per; i += kPrepWarps * 32) {
+            const int r = i >> 3, m = i & 7;
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kPrepWarps; ++w) v += red[w][r][m];
+            ts[m][r] = v;
+            if (shares > 1) p.tparts[((size_t)share * gridDim.x + blockIdx.x) * per + i] = v;
+        }
+        if (shares > 1) {
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) {
+                const int old = atomicAdd(p.counters + blockIdx.x, 1);
+                last = old == shares - 1;
+                if (last) p.counters[blockIdx.x] = 0;
+            }
+            __syncthreads();
+            if (!last) return;
+            __threadfence();
+            for (int i = tid; i < per; i += kPrepWarps * 32) {
+                float v = 0.0f;
+                for (int q = 0; q < shares; ++q) v += __ldcg(p.tparts + ((size_t)q * gridDim.x + blockIdx.x) * per + i);
+                ts[i & 7][i >> 3] = v;
+            }
+        }
+        __syncthreads();
+    } else if (share != 0) {
+        return;
+    }
+    // the extra columns: outlier activations, projections (fp16; bf16: high, high, low), zeros
+    const int xc = BF16 ? 3 : 1, extra = p.ke - p.kw, rank8 = max(8, (p.rank + 7) & ~7);
+    for (int i = tid; i < 8 * extra; i += kPrepWarps * 32) {
+        const int r = i / extra, j = i - r * extra;
+        if (m0 + r >= p.m) break;
+        unsigned short v = 0;
+        if (j < p.oc) {
+            const int col = __ldg(p.oidx + j);
+            if (col >= 0 && col < p.k) v = p.x[(size_t)(m0 + r) * p.ldx + col];
+        } else if (j >= p.oc8 && j < p.oc8 + rank8 * xc && (j - p.oc8) % rank8 < p.rank) {
+            const int q = j - p.oc8, copy = q / rank8;
+            const float tv = ts[r][q - copy * rank8];
+            if constexpr (BF16) {
+                const __nv_bfloat16 hi = __float2bfloat16_rn(tv);
+                v = __bfloat16_as_ushort(copy == 2 ? __float2bfloat16_rn(tv - __bfloat162float(hi)) : hi);
+            } else {
+                v = __half_as_ushort(__float2half_rn(tv));
+            }
+        }
+        p.out[(size_t)(m0 + r) * p.ke + p.kw + j] = v;
+    }
+}
+
+struct GemmPlan { GemmArgs a; int grid, smem, kw, ke, groups, shares; size_t x_bytes, t_bytes, scratch; };
+
+int sms() {
+    static int cached[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return 148; }
+    if (!cached[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = 148; }
+        cached[dev] = n;
+    }
+    return cached[dev];
+}
+
+// Arrival counters of the workspace: tiles first, then the row groups of the layout kernel.
+constexpr int kTileCounters = 8192, kRowCounters = kWsMaxCounters - 16 - kTileCounters;
+
+// Geometry; false where the shape is not for this kernel (the caller dequantises and uses a library GEMM).
+bool plan_gemm(const qgemv_problem& p, GemmPlan& g) {
+    auto al = [](const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; };
+    const int per = p.group >= 128 ? (p.group % 128 ? 0 : 1) : p.group == 64 ? 2 : p.group == 32 && p.bits == 4 ? 4 : 0;
+    if (!per || p.m < 1 || !al(p.packed, 16) || !al(p.scales, 2) || p.ldp % 16 || (long long)p.k_padded * p.bits / 8 % 16 || p.rank > kMaxRank || p.outliers > 4096) return false;
+    GemmArgs& a = g.a;
+    a = GemmArgs{};
+    const bool bf16 = p.x_dtype == QGEMV_BF16;
+    a.packed = p.packed; a.ldp = p.ldp;
+    a.scales = static_cast<const __half*>(p.scales); a.lds = p.lds;
+    a.bias = static_cast<const __half*>(p.bias);
+    a.ow = static_cast<const __half*>(p.outlier_w); a.ldow = p.ldow;
+    a.ru = static_cast<const __half*>(p.res_u); a.ldu = p.ldu;
+    a.y = p.y; a.ldy = p.ldy;
+    a.m = p.m; a.n = p.n; a.group = p.group; a.ng = p.k_padded / p.group; a.act = p.act;
+    a.pieces = (int)((long long)p.k_padded * p.bits / 8 / 16);
+    a.oc = p.outliers; a.oc8 = (p.outliers + 7) / 8 * 8; a.rank = p.rank; a.xcopies = bf16 ? 3 : 1;
+    a.rank8 = (p.rank + 7) / 8 * 8;
+    a.ow_vec = p.outliers % 8 == 0 && al(p.outlier_w, 16) && p.ldow % 8 == 0;
+    a.ru_vec = p.rank % 8 == 0 && al(p.res_u, 16) && p.ldu % 8 == 0;
+    const int extra = (a.rank ? a.oc8 + a.rank8 * a.xcopies : a.oc);
+    a.wunits = (p.k_padded + kUnit - 1) / kUnit;
+    a.chunks = a.wunits * 2 + (extra + kChunk - 1) / kChunk;
+    a.units = (a.chunks + 1) / 2;
+    g.kw = a.wunits * kUnit; g.ke = a.chunks * kChunk;
+    a.mtiles = (p.m + kMaxWidth - 1) / kMaxWidth;
+    a.width = ((p.m + a.mtiles - 1) / a.mtiles + 15) / 16 * 16;
+    a.ntiles = (p.n + kRows - 1) / kRows;
+    const long long tiles = (long long)a.mtiles * a.ntiles;
+    g.groups = (p.m + 7) / 8;
+    if (tiles > kTileCounters || g.groups > kRowCounters || tiles * a.units > 0x3fffffff) return false;
+    const int s = sms();
+    // Whole tiles, or units dealt out evenly over `grid` CTAs: clocks of the busiest one.  A unit takes about 5 x width, at
+    // least 600 (the chain of barriers); storing a tile 1500 + 24 x width; handing pieces over some 3000, and the last CTA of a
+    // tile reads its contributions one after the other, 1500 each.
+    const long long unit_clk = 5 * a.width > 600 ? 5 * a.width : 600, end_clk = 1500 + 24 * a.width, all = tiles * a.units;
+    long long best = (tiles + s - 1) / s * (a.units * unit_clk + end_clk);
+    a.split = 0;
+    g.grid = (int)(tiles < s ? tiles : s);
+    for (int parts = 1; parts <= 32; parts += parts < 4 ? 1 : parts / 4) {
+        const long long want = tiles * parts < s ? tiles * parts : s, share = (all + want - 1) / want;
+        if (want > all) break;
+        const long long cost = share * unit_clk + (share / a.units + 1) * end_clk + 3000 + 1500 * (a.units / share + 1);
+        if (cost < best) { best = cost; a.split = 1; g.grid = (int)want; }
+        if (want == s) break;
+    }
+    g.x_bytes = ((size_t)p.m * g.ke * 2 + 255) / 256 * 256;
+    // enough CTAs of the layout kernel for two per SM, each warp with at least two blocks of 64 columns
+    g.shares = 2 * s / g.groups;
+    const int most = g.kw / 64 / (2 * kPrepWarps);
+    g.shares = g.shares > most ? most : g.shares;
+    g.shares = g.shares < 1 ? 1 : g.shares > 32 ? 32 : g.shares;
+    g.t_bytes = ((size_t)(g.shares > 1 ? g.shares : 0) * g.groups * a.rank * 8 * sizeof(float) + 255) / 256 * 256;
+    g.scratch = g.x_bytes + g.t_bytes + (a.split ? (size_t)g.grid * 2 * a.width * kRows * sizeof(float) : 0);
+    a.sc_odd = (int)(reinterpret_cast<uintptr_t>(p.scales) >> 1 & 1);
+    // the ring of codes and the stages of x share what shared memory there is: a deep ring where tiles are narrow (a unit is
+    // then short against HBM's latency), as many stages of x as fit beside a short one where they are wide
+    const int words = per == 1 ? 1 : per / 2 + 1, slot = p.bits * kRows * 16 + words * kRows * 4, room = 232448 - kSmemCtl;
+    const int stage = a.width * 256, by_tmem = (512 - (a.width + 31) / 32 * 32) / 64;
+    for (a.ring = 16; a.ring > kGroups && room - a.ring * slot < 4 * stage; a.ring /= 2) {}
+    a.stages = (room - a.ring * slot) / stage;
+    a.stages = a.stages > by_tmem ? by_tmem : a.stages;
+    a.stages = a.stages > kMaxStages ? kMaxStages : a.stages;
+    a.groups = a.stages < kGroups ? a.stages : kGroups;
+    a.ctl_off = a.stages * stage + (a.ring * slot + 1023) / 1024 * 1024;
+    if (a.ctl_off + kSmemCtl > 232448) a.ctl_off = a.stages * stage + (a.ring * slot + 127) / 128 * 128;
+    g.smem = a.ctl_off + kSmemCtl;
+    if (g.smem < 120 * 1024) g.smem = 120 * 1024;      // one CTA per SM: it takes all of tensor memory
+    return true;
+}
+
+using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn encoder() {
+    static EncodeFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<EncodeFn>(p);
+    }();
+    return fn;
+}
+
+template <int BITS, int NG, bool BF16>
+int launch_gemm(const GemmPlan& g, const CUtensorMap& map, cudaStream_t s) {
+    auto kern = gemm_kernel<BITS, NG, BF16>;
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448) != cudaSuccess) return check_launch("cudaFuncSetAttribute(gemm_kernel)");
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g.grid);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, g.a, map);
+    return check_launch("gemm_kernel");
+}
+
+template <int BITS, bool BF16>
+int launch_prepare(const qgemv_problem& p, const GemmPlan& g, void* scratch, cudaStream_t s) {
+    auto al = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+    PrepArgs a{};
+    a.x = static_cast<const unsigned short*>(p.x); a.ldx = p.ldx;
+    a.oidx = p.outlier_idx;
+    a.rv = static_cast<const __half*>(p.res_v); a.ldv = p.ldv;
+    a.out = static_cast<unsigned short*>(scratch);
+    a.tparts = reinterpret_cast<float*>(static_cast<char*>(scratch) + g.x_bytes);
+    a.counters = g.a.counters + kTileCounters;
+    a.m = p.m; a.k = p.k_original; a.oc = p.outliers; a.oc8 = g.a.oc8; a.rank = p.rank; a.kw = g.kw; a.ke = g.ke;
+    a.vec = al(p.x) && p.ldx % 8 == 0;
+    a.vvec = p.rank > 0 && al(p.res_v) && p.ldv % 8 == 0;
+    prepare_kernel<BITS, BF16><<<dim3(g.groups, g.shares), kPrepWarps * 32, 0, s>>>(a);
+    return check_launch("prepare_kernel");
+}
+
+}  // namespace
+
+// `p` is validated (shapes, types) by the caller, except for M.
+size_t gemm_scratch_bytes(const qgemv_problem& p) {
+    GemmPlan g;
+    return plan_gemm(p, g) ? g.scratch : 0;
+}
+
+int run_gemm(const qgemv_problem& p, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+    GemmPlan g;
+    if (!plan_gemm(p, g)) { set_error("qgemm_run: this shape is not built (see qgemm_scratch_bytes)"); return QGEMV_ERR_SHAPE; }
+    if (!scratch || scratch_bytes < g.scratch || reinterpret_cast<uintptr_t>(scratch) % 256) {
+        set_error("qgemm_run: scratch of %zu bytes (256-byte aligned) required", g.scratch);
+        return QGEMV_ERR_WORKSPACE;
+    }
+    const bool bf16 = p.x_dtype == QGEMV_BF16;
+    EncodeFn enc = encoder();
+    if (!enc) { set_error("qgemm_run: the driver has no cuTensorMapEncodeTiled"); return QGEMV_ERR_LAUNCH; }
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)g.ke, (cuuint64_t)p.m}, strides[1] = {(cuuint64_t)g.ke * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)kChunk, (cuuint32_t)g.a.width}, ones[2] = {1, 1};
+    if (enc(&map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scratch, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        set_error("qgemm_run: cuTensorMapEncodeTiled failed");
+        return QGEMV_ERR_LAUNCH;
+    }
+    char* ws = static_cast<char*>(p.workspace);
+    int* cnt = reinterpret_cast<int*>(ws + kWsCounterOff);
+    g.a.counters = cnt;
+    g.a.status = cnt + kWsStatusIdx;
+    g.a.partial = reinterpret_cast<float*>(static_cast<char*>(scratch) + g.x_bytes + g.t_bytes);
+    int r = p.bits == 2 ? (bf16 ? launch_prepare<2, true>(p, g, scratch, s) : launch_prepare<2, false>(p, g, scratch, s))
+                        : (bf16 ? launch_prepare<4, true>(p, g, scratch, s) : launch_prepare<4, false>(p, g, scratch, s));
+    if (r != QGEMV_OK) return r;
+    const int ng = p.group >= 128 ? 1 : p.group == 64 ? 2 : 4;
+#define QG(B, G) (bf16 ? launch_gemm<B, G, true>(g, map, s) : launch_gemm<B, G, false>(g, map, s))
+    if (p.bits == 2) return ng == 1 ? QG(2, 1) : QG(2, 2);
+    return ng == 1 ? QG(4, 1) : ng == 2 ? QG(4, 2) : QG(4, 4);
+#undef QG
+}
+
+}  // namespace qgemv

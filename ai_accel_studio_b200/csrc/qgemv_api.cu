@@ -364,3 +364,16 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
     }
     return QGEMV_OK;
 }
+
+// ---- any number of rows ----------------------------------------------------------------------------------
+
+extern "C" size_t qgemv_batch_scratch_bytes(const qgemv_problem* p) {
+    if (validate(p, 0, 0x7fffffff) != QGEMV_OK) return 0;
+    return gemm_scratch_bytes(*p);
+}
+
+extern "C" int qgemv_run_batch(const qgemv_problem* p, void* scratch, size_t scratch_bytes, void* stream) {
+    const int v = validate(p, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), 0x7fffffff);
+    if (v != QGEMV_OK) return v;
+    return run_gemm(*p, scratch, scratch_bytes, static_cast<cudaStream_t>(stream));
+}

@@ -73,6 +73,8 @@ void set_error(const char* fmt, ...);
 int  check_launch(const char* what);
 
 // Launchers implemented in the kernel translation units.
+size_t gemm_scratch_bytes(const qgemv_problem& p);
+int run_gemm(const qgemv_problem& p, void* scratch, size_t scratch_bytes, cudaStream_t s);
 int launch_residual_t(const Args& a, bool bf16, cudaStream_t s);
 int launch_simt(const Args& a, int bits, bool bf16, int unit_bytes, cudaStream_t s);
 const char* simt_name(int bits, int m, int unit_bytes);

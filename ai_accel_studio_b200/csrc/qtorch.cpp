@@ -132,16 +132,37 @@ PyObject* linear_call(LinearObject* o, PyObject* arg) {
         const int64_t dims = x.dim();
         const auto dtype = x.scalar_type();
         if (dims < 1 || !x.is_cuda() || x.get_device() != l.device || x.size(-1) != l.in_features || !x.is_contiguous() ||
-            (dtype != at::kHalf && dtype != at::kBFloat16) || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16)
+            (dtype != at::kHalf && dtype != at::kBFloat16))
             Py_RETURN_NONE;
         const int64_t rows = x.numel() / l.in_features;
-        if (rows < 1 || rows > l.max_rows) Py_RETURN_NONE;
+        const bool batch = rows > l.max_rows;
+        if (rows < 1 || rows > (1 << 24) || (!batch && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16)) Py_RETURN_NONE;
         c10::cuda::OptionalCUDAGuard guard;
         if (c10::cuda::current_device() != l.device) guard.set_index(l.device);
         const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(l.device).stream();
         size_t ws_bytes = 0;
         void* ws = workspace(l.device, stream, &ws_bytes);
         const bool bf16 = dtype == at::kBFloat16;
+        auto result = [&]() {
+            if (dims == 2) return at::empty({rows, l.out_features}, x.options());
+            std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+            shape.back() = l.out_features;
+            return at::empty(shape, x.options());
+        };
+        if (batch) {                                  // weights are read after the layout kernel, which starts in stream order
+            qgemv_problem p = l.base;
+            if ((p.kernel & 0xff) == QGEMV_KERNEL_SIMT) Py_RETURN_NONE;
+            p.m = (int)rows; p.x_dtype = bf16 ? QGEMV_BF16 : QGEMV_F16;
+            p.x = x.data_ptr(); p.ldx = l.in_features;
+            p.y = x.data_ptr(); p.ldy = l.out_features;
+            p.workspace = ws; p.workspace_bytes = ws_bytes;
+            const size_t bytes = qgemv_batch_scratch_bytes(&p);
+            if (!bytes) Py_RETURN_NONE;
+            at::Tensor y = result(), scratch = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
+            p.y = y.data_ptr();
+            check(qgemv_run_batch(&p, scratch.data_ptr(), bytes, stream));
+            return THPVariable_Wrap(std::move(y));
+        }
         Linear::Slot& slot = l.slots[(int)rows * 2 + bf16];
         if (slot.blob.empty()) {
             slot.blob.resize(qgemv_prepared_bytes());
@@ -157,14 +178,7 @@ PyObject* linear_call(LinearObject* o, PyObject* arg) {
         if (!slot.usable) Py_RETURN_NONE;
         const uint64_t v = versions(l);
         const bool fresh = v != l.version;
-        at::Tensor y;
-        if (dims == 2) {
-            y = at::empty({rows, l.out_features}, x.options());
-        } else {
-            std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
-            shape.back() = l.out_features;
-            y = at::empty(shape, x.options());
-        }
+        at::Tensor y = result();
         check(qgemv_launch_prepared(slot.blob.data(), x.data_ptr(), y.data_ptr(), ws, fresh, stream));
         l.version = v;
         return THPVariable_Wrap(std::move(y));

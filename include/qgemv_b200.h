@@ -180,6 +180,15 @@ size_t qgemv_prepared_bytes(void);
 int qgemv_prepare(const qgemv_problem* p, void* prepared);
 int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspace, int ordered, void* stream);
 
+/* The same computation for any number of rows (prompts): one kernel lays x out, one dequantises the codes into tensor memory
+ * and multiplies there; the dense matrix is never written.  Weights are rounded as qdequant rounds them to the activation
+ * type, sums are fp32.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
+ * private to the call until it completes (0: this shape is not built -- groups other than 32 (INT4), 64 and multiples of
+ * 128, unaligned packed rows -- dequantise and use a library GEMM).  x needs only k_original columns.
+ * Replaces the M > 4 route of ai_accel_lab/optimize/hybrid_int4.py:36-37 and hybrid_int2.py:102-106. */
+size_t qgemv_batch_scratch_bytes(const qgemv_problem* p);
+int qgemv_run_batch(const qgemv_problem* p, void* scratch, size_t scratch_bytes, void* stream);
+
 /* Bytes of workspace qgemv_run needs for a problem of this shape (never 0; at most a few MB). */
 size_t qgemv_workspace_bytes(int bits, int m, int n, int k_padded, int group, int rank);
 

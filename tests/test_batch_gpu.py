@@ -1,0 +1,70 @@
+"""The fused dequantise + GEMM route of the modules (more than 16 rows) against float64 products of the module's own
+matrix.  Sizes at the edges of its tiles: 128 weight rows, 128 K columns per unit, 16 - 256 activation rows, units dealt out
+over CTAs (few tiles) and whole tiles."""
+import pytest
+import torch
+
+from ai_accel_studio_b200 import ops
+from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2
+from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4
+from ai_accel_studio_b200.optimize import HybridInt2Linear, HybridInt4Linear
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # bits, rows, n, k, group, outliers, rank, bias
+    (4, 17, 128, 128, 128, 0, 0, False),         # one tile, one unit
+    (4, 64, 129, 130, 32, 3, 1, True),           # one weight row and two columns more; odd outlier count and rank
+    (2, 100, 1000, 896, 64, 8, 8, True),
+    (2, 256, 300, 1000, 128, 33, 9, False),      # full tile of rows; padded K; x rows off 16-byte alignment
+    (4, 257, 640, 4096, 64, 40, 0, True),        # a second tile of rows
+    (2, 33, 4999, 512, 256, 0, 64, True),        # largest rank
+    (4, 40, 256, 28672, 128, 64, 8, False),      # few tiles, long K: every tile split over many CTAs
+    (4, 700, 6400, 1024, 128, 16, 8, True),      # 150 tiles of 240 rows
+    (2, 20, 14336, 4096, 128, 40, 8, False),
+]
+
+
+def _module(bits, n, k, group, oc, rank, has_bias, gen):
+    pw = (pack_groupwise_int2 if bits == 2 else pack_groupwise_int4)(torch.randn(n, k, generator=gen) * 0.05, group)
+    cu = lambda t: None if t is None else t.cuda()
+    rnd = lambda *s: (torch.randn(*s, generator=gen) * 0.05).half()
+    cls = HybridInt2Linear if bits == 2 else HybridInt4Linear
+    return cls.from_buffers(pw.packed.cuda(), pw.scales.cuda(), k, group,
+                            torch.randperm(k, generator=gen)[:oc].to(torch.int32).cuda() if oc else None, cu(rnd(n, oc)) if oc else None,
+                            cu(rnd(n)) if has_bias else None, cu(rnd(n, rank)) if rank else None, cu(rnd(rank, k)) if rank else None)
+
+
+@pytest.mark.parametrize("bits,rows,n,k,group,oc,rank,has_bias", CASES)
+def test_batch_against_float64(bits, rows, n, k, group, oc, rank, has_bias):
+    gen = torch.Generator().manual_seed(n + k + rows)
+    mod = _module(bits, n, k, group, oc, rank, has_bias, gen)
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(rows, k, generator=gen).to(dtype).cuda()
+        y = mod(x)
+        again = mod(x)
+        want = x.double() @ mod.effective_weight().double().t()
+        if has_bias:
+            want = want + mod.bias.double()
+        assert y.shape == want.shape and y.dtype == dtype
+        # weights rounded to the activation type (relative u each, random), the result once more: 2 u in the 2-norm
+        u = 2.0 ** (-11 if dtype == torch.float16 else -8)
+        err = (y.double() - want).norm() / want.norm()
+        assert float(err) <= 2 * u, float(err)
+        assert float((y.double() - want).abs().max()) <= 16 * u * float(want.pow(2).mean().sqrt()) + 2 * u * float(want.abs().max())
+        assert torch.equal(y, again)                       # contributions of split tiles are added in a fixed order
+    assert ops.workspace_status("cuda") == 0
+
+
+def test_batch_of_gated_pairs_and_three_dimensions():
+    from ai_accel_studio_b200.optimize.siblings import merge_gate_up
+    torch.manual_seed(3)
+    gate, up = (HybridInt4Linear(torch.nn.Linear(1024, 1016), 128, None, 8) for _ in range(2))
+    up.set_residual(torch.randn(1016, 8) * 0.02, torch.randn(8, 1024) * 0.02)
+    fused = merge_gate_up(gate, up).cuda()
+    gate, up = gate.cuda(), up.cuda()
+    x = torch.randn(3, 50, 1024).half().cuda()
+    y = fused(x)
+    sep = torch.nn.functional.silu(gate(x)) * up(x)
+    assert y.shape == (3, 50, 1016)
+    assert float((y.float() - sep.float()).abs().max()) <= 2e-3 * float(sep.float().abs().max()) + 1e-3
