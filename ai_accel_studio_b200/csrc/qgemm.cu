@@ -418,7 +418,6 @@ __device__ __noinline__ bool finish_tile(const GemmArgs& args, Ends& e, int tile
         float v[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q) v[q] = 0.0f;
-#pragma unroll 2
         for (int c = cf; c <= cl; ++c) {
             const float* src = p.partial + (size_t)(c * 2 + (first < first_unit(p, c, e.grid) ? 0 : 1)) * piece;
 #pragma unroll
