@@ -23,7 +23,7 @@ EXPORTS = ("qgemv_run", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_d
            "qgemv_prepared_bytes", "qgemv_prepare", "qgemv_launch_prepared", "qgemv_batch_scratch_bytes", "qgemv_run_batch", "qgemv_error_string", "qgemv_abi_version", "qgemv_sizeof_problem",
            "qcomm_slot_bytes", "qcomm_flag_bytes", "qcomm_state_bytes", "qcomm_allreduce", "qcomm_allreduce_rmsnorm", "qcomm_status", "qcomm_alloc", "qcomm_free",
            "qcomm_ipc_export", "qcomm_ipc_open", "qcomm_ipc_close",
-           "qdec_rmsnorm", "qdec_rope_append", "qdec_attention_workspace_bytes", "qdec_attention", "qdec_silu_mul")
+           "qdec_rmsnorm", "qdec_rope_append", "qdec_attention_workspace_bytes", "qdec_attention", "qdec_rope_attention", "qdec_silu_mul")
 COMM_MAX_RANKS, COMM_MAX_BLOCKS, COMM_IPC_HANDLE_BYTES = 8, 64, 64
 
 
@@ -127,6 +127,8 @@ def lib():
     l.qdec_attention_workspace_bytes.restype = C.c_size_t
     l.qdec_attention.argtypes = [vp, i64, vp, vp, vp, vp, i64, ci, ci, ci, ci, ci, C.c_float, vp, C.c_size_t, ci, vp]
     l.qdec_attention.restype = ci
+    l.qdec_rope_attention.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, ci, vp, vp, vp, vp, i64, ci, ci, ci, ci, ci, C.c_float, vp, C.c_size_t, vp, ci, vp]
+    l.qdec_rope_attention.restype = ci
     l.qdec_silu_mul.argtypes = [vp, i64, vp, i64, vp, i64, ci, ci, ci, vp]
     l.qdec_silu_mul.restype = ci
     l.qdequant.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_int,

@@ -142,140 +142,280 @@ __global__ void __launch_bounds__(128) rope_append_kernel(void* q_, long long ld
 }
 
 // ---------------------------------------------------------------------------------------------
-// attention of one query token per sequence: grid (slice, kv head, sequence), 8 warps per CTA
+// attention of one query token per sequence: grid (slice, kv head, sequence), 8 warps per CTA, 16 positions per warp and turn
 // ---------------------------------------------------------------------------------------------
 constexpr int kAttWarps = 8;
 constexpr int kAttMaxSlices = 16;
-constexpr int kAttMinSlice = 16;                 // positions: shorter slices are not worth a CTA
+constexpr int kAttBlock = 16;                    // positions of a warp's turn
+constexpr int kAttSlice = kAttWarps * kAttBlock; // one turn of a CTA
+constexpr int kAttMaxHeads = 8;                  // query heads per kv head
 
-// Slices the sequence axis is cut into: enough CTAs to cover the SMs, at most kAttMaxSlices.
+// Slices the sequence axis is cut into: as many CTAs as fit the SMs one each, each with a turn's positions at least.  Meeting
+// again (fence, counter, reading the parts back) costs 2.5 us, a turn well under 1: shorter slices only pay the former, and a
+// second wave (9 slices for 32 (sequence, kv head) pairs) measured slower than more turns.
 inline int attention_slices(int batch, int kv_heads, int max_len) {
-    const int ctas = batch * kv_heads;
-    int s = (148 + ctas - 1) / ctas;
-    s = s < 1 ? 1 : s > kAttMaxSlices ? kAttMaxSlices : s;
-    const int by_len = max_len / kAttMinSlice;
-    if (s > by_len) s = by_len < 1 ? 1 : by_len;
-    return s;
+    const int ctas = batch * kv_heads, by_len = max_len / kAttSlice;
+    int s = 148 / ctas;
+    s = s > kAttMaxSlices ? kAttMaxSlices : s;
+    s = s > by_len ? by_len : s;
+    return s < 1 ? 1 : s;
 }
 
-// One slice's result per (query head of the group): running maximum, sum of exponentials, weighted values.
-template <int D> struct alignas(8) Partial { float m, l, o[D]; };
+__device__ __forceinline__ uint32_t transpose8(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
 
-template <int D, int G, bool BF16>
-__global__ void __launch_bounds__(kAttWarps * 32) attention_kernel(const void* q_, long long ldq, const void* kc_, const void* vc_,
-                                                                   const long long* pos_, void* out_, long long ldo, int hq, int hkv,
-                                                                   int max_len, float scale, float* parts, int* counters) {
+// c += A (16 x 16, row) B (16 x 8, col), both of the activation type.
+template <bool BF16>
+__device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    const typename Act16<BF16>::T a = Act16<BF16>::from_float(lo), b = Act16<BF16>::from_float(hi);
+    return (uint32_t)*reinterpret_cast<const unsigned short*>(&a) | (uint32_t)*reinterpret_cast<const unsigned short*>(&b) << 16;
+}
+
+// Lane t of a quad holds, of a row of D elements, the eight from 32 c + 8 t in word c of v: so the partner of every element
+// under the rotation (D / 2 away) is the same lane's, D / 64 words further on.
+template <int D, bool BF16>
+__device__ __forceinline__ void rotate_row(uint4 (&v)[D / 32], const void* cos_, const void* sin_, int t) {
     using T = typename Act16<BF16>::T;
-    constexpr int E = D / 32;                     // elements per lane
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int slice = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, slices = gridDim.x;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    long long len = *pos_ + 1;
-    len = len < 0 ? 0 : len > max_len ? max_len : len;
-    const int per = (int)((len + slices - 1) / slices);
-    const int s0 = slice * per, s1 = (int)min((long long)(s0 + per), len);
-
-    float qv[G][E];
+    constexpr int H = D / 64;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const T* q = static_cast<const T*>(q_) + (size_t)b * ldq + (size_t)(kvh * G + g) * D + lane * E;
+    for (int c = 0; c < H; ++c) {
+        T* lo = reinterpret_cast<T*>(&v[c]);
+        T* hi = reinterpret_cast<T*>(&v[c + H]);
+        const T* cs = static_cast<const T*>(cos_) + c * 32 + t * 8;
+        const T* sn = static_cast<const T*>(sin_) + c * 32 + t * 8;
 #pragma unroll
-        for (int e = 0; e < E; ++e) qv[g][e] = Act16<BF16>::to_float(q[e]) * scale;
-    }
-    const T* kbase = static_cast<const T*>(kc_) + ((size_t)b * hkv + kvh) * (size_t)max_len * D + lane * E;
-    const T* vbase = static_cast<const T*>(vc_) + ((size_t)b * hkv + kvh) * (size_t)max_len * D + lane * E;
-
-    float m[G], l[G], o[G][E];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        m[g] = -1.0e30f; l[g] = 0.0f;
-#pragma unroll
-        for (int e = 0; e < E; ++e) o[g][e] = 0.0f;
-    }
-    // Raw 4 / 8-byte pieces of a cache row; converted only when their turn comes, so that the loads of the
-    // next pair of positions stay in flight while this pair is processed (a warp issues in order: the
-    // first instruction that needs a pending load stalls everything behind it).
-    using Raw = typename std::conditional<E == 4, uint2, uint32_t>::type;
-    auto widen = [&](const Raw& raw, float (&dst)[E]) {
-        const T* el = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int e = 0; e < E; ++e) dst[e] = Act16<BF16>::to_float(el[e]);
-    };
-    constexpr int STEP = kAttWarps * 2;           // two positions per warp and iteration: independent reductions overlap
-    int p0 = s0 + warp * 2;
-    Raw rk0 = {}, rv0 = {}, rk1 = {}, rv1 = {};
-    auto fetch = [&](int p, Raw& a, Raw& b, Raw& c, Raw& d) {
-        const size_t pa = (size_t)min(p, s1 - 1) * D, pb = (size_t)min(p + 1, s1 - 1) * D;
-        a = *reinterpret_cast<const Raw*>(kbase + pa);
-        b = *reinterpret_cast<const Raw*>(vbase + pa);
-        c = *reinterpret_cast<const Raw*>(kbase + pb);
-        d = *reinterpret_cast<const Raw*>(vbase + pb);
-    };
-    if (p0 < s1) fetch(p0, rk0, rv0, rk1, rv1);
-    for (; p0 < s1; p0 += STEP) {
-        Raw nk0, nv0, nk1, nv1;
-        fetch(p0 + STEP, nk0, nv0, nk1, nv1);       // clamped to the slice: the last iteration re-reads its final row
-        const bool two = p0 + 1 < s1;
-        float k0[E], k1[E], v0[E], v1[E];
-        widen(rk0, k0); widen(rv0, v0); widen(rk1, k1); widen(rv1, v1);
-        float sc0[G], sc1[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float a = 0.0f, c = 0.0f;
-#pragma unroll
-            for (int e = 0; e < E; ++e) { a = fmaf(qv[g][e], k0[e], a); c = fmaf(qv[g][e], k1[e], c); }
-            sc0[g] = a; sc1[g] = c;
+        for (int q = 0; q < 8; ++q) {
+            const float a = Act16<BF16>::to_float(lo[q]), b = Act16<BF16>::to_float(hi[q]);
+            lo[q] = Act16<BF16>::from_float(r16<BF16>(a * Act16<BF16>::to_float(cs[q])) + r16<BF16>(-b * Act16<BF16>::to_float(sn[q])));
+            hi[q] = Act16<BF16>::from_float(r16<BF16>(b * Act16<BF16>::to_float(cs[q + D / 2])) + r16<BF16>(a * Act16<BF16>::to_float(sn[q + D / 2])));
         }
+    }
+}
+
+// What the fused form adds: the new token's key and value rows, the rotary tables.
+struct NewToken {
+    const void* k; long long ldk;
+    const void* v; long long ldv;
+    const void* cos; const void* sin;
+    int table_rows; int* status;
+};
+
+// With the lanes of a warp along D this kernel spent its time in shuffles (five per position and query head: 36 us for 4
+// sequences x 8 kv heads x 8 query heads over 1088 positions, 17 MB).  Here a warp takes 16 positions of a kv head for all
+// its query heads: scores are mma m16n8k16 of 16 keys with up to 8 queries, and the values' turn is a second one, their
+// transposition done in registers (movmatrix).  Keys and values go from global memory straight to fragments, 16 bytes a lane.
+// The weights of the softmax enter the second product as a sum of two fp16 (three bf16) numbers, 22 (24) bits, so that no
+// precision is lost against fp32 weights.  With it and the announcement to L2, fp16, in a chain of launches over caches that
+// come from DRAM, rope and append included: 34.3 -> 12.1 us at the size above, 11.6 -> 7.6 us for 8 kv heads x 4 over 577
+// positions, 7.1 -> 5.1 us for 2 x 7 of 64 elements over 162.  What is left is the chain position -> rows -> products ->
+// softmax -> meeting, and the launch.  One CTA per SM: with registers for two (128) the rotation spilled, 18.4 us above.
+// ROPE: the queries are rotated on their way to fragments; the warp whose turn holds the new position takes that row from the
+// projections instead of the cache, rotates the key, and writes both to the cache.
+template <int D, bool BF16, bool ROPE>
+__global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void* q_, long long ldq, void* kc_, void* vc_,
+                                                                   const long long* pos_, void* out_, long long ldo, int heads, int hkv,
+                                                                   int max_len, float scale, float* parts, int* counters, bool wide,
+                                                                   const NewToken nt) {
+    using T = typename Act16<BF16>::T;
+    constexpr int C = D / 32;                     // 16-byte words of a row per lane
+    constexpr int SPLIT = BF16 ? 3 : 2;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int slice = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, slices = gridDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    T* kbase = static_cast<T*>(kc_) + ((size_t)b * hkv + kvh) * (size_t)max_len * D + t * 8;
+    T* vbase = static_cast<T*>(vc_) + ((size_t)b * hkv + kvh) * (size_t)max_len * D + t * 8;
+    int s0, s1;
+    auto cut = [&](long long pos) {
+        const long long len = pos < 0 ? 0 : pos >= max_len ? max_len : pos + 1;
+        const int per = (int)((len + slices - 1) / slices + kAttBlock - 1) / kAttBlock * kAttBlock;
+        s0 = min(slice * per, (int)len);
+        s1 = min(s0 + per, (int)len);
+    };
+    // The cache rows go to L2 while the projections still run: only an announcement, so neither a position nor rows that
+    // are not final yet can do harm.
+    cut(*static_cast<const volatile long long*>(pos_));
+    for (int p = s0 + warp * kAttBlock + (lane & 15); p < s1; p += kAttWarps * kAttBlock) {
+        const T* row = (lane < 16 ? kbase : vbase) + (size_t)p * D - t * 8;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
+        for (int c = 0; c < D; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long pos = *static_cast<const volatile long long*>(pos_);
+    cut(pos);
+    bool append = false;
+    if constexpr (ROPE) {
+        append = pos >= 0 && pos < max_len && pos < nt.table_rows;
+        if (!append && nt.status && tid == 0) atomicExch(nt.status, 1);
+    }
+    const T* cs = nullptr;
+    const T* sn = nullptr;
+    if (append) { cs = static_cast<const T*>(nt.cos) + (size_t)pos * D; sn = static_cast<const T*>(nt.sin) + (size_t)pos * D; }
+
+    auto load_row = [&](const T* row, uint4 (&v)[C]) {      // row points at the lane's first element
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                sc0[g] += __shfl_xor_sync(0xffffffffu, sc0[g], off);
-                sc1[g] += __shfl_xor_sync(0xffffffffu, sc1[g], off);
+        for (int c = 0; c < C; ++c) {
+            if (wide) {
+                v[c] = *reinterpret_cast<const uint4*>(row + c * 32);
+            } else {
+                const uint2 x = *reinterpret_cast<const uint2*>(row + c * 32), y = *reinterpret_cast<const uint2*>(row + c * 32 + 4);
+                v[c] = make_uint4(x.x, x.y, y.x, y.y);
             }
         }
+    };
+    auto store_row = [&](T* row, const uint4 (&v)[C]) {
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float second = two ? sc1[g] : -1.0e30f;
-            const float mn = fmaxf(m[g], fmaxf(sc0[g], second));
-            const float alpha = __expf(m[g] - mn), p0w = __expf(sc0[g] - mn), p1w = two ? __expf(second - mn) : 0.0f;
-            m[g] = mn;
-            l[g] = l[g] * alpha + p0w + p1w;
-#pragma unroll
-            for (int e = 0; e < E; ++e) o[g][e] = fmaf(p1w, v1[e], fmaf(p0w, v0[e], o[g][e] * alpha));
+        for (int c = 0; c < C; ++c) {
+            if (wide) {
+                *reinterpret_cast<uint4*>(row + c * 32) = v[c];
+            } else {
+                *reinterpret_cast<uint2*>(row + c * 32) = make_uint2(v[c].x, v[c].y);
+                *reinterpret_cast<uint2*>(row + c * 32 + 4) = make_uint2(v[c].z, v[c].w);
+            }
         }
-        rk0 = nk0; rv0 = nv0; rk1 = nk1; rv1 = nv1;
+    };
+    auto clear = [&](uint4 (&v)[C]) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = make_uint4(0u, 0u, 0u, 0u);
+    };
+
+    uint4 ka[C], kb[C], va[C], vb[C];             // positions p + g and p + g + 8 of the turn
+    auto fetch = [&](int p) {
+        const int pa = p + g, pb = p + g + 8;
+        clear(ka); clear(kb); clear(va); clear(vb);
+        const bool na = append && pa == (int)pos, nb = append && pb == (int)pos;
+        if (pa < s1 && !na) { load_row(kbase + (size_t)pa * D, ka); load_row(vbase + (size_t)pa * D, va); }
+        if (pb < s1 && !nb) { load_row(kbase + (size_t)pb * D, kb); load_row(vbase + (size_t)pb * D, vb); }
+        if constexpr (ROPE) {
+            auto fresh = [&](uint4 (&k)[C], uint4 (&v)[C]) {
+                load_row(static_cast<const T*>(nt.k) + (size_t)b * nt.ldk + (size_t)kvh * D + t * 8, k);
+                load_row(static_cast<const T*>(nt.v) + (size_t)b * nt.ldv + (size_t)kvh * D + t * 8, v);
+                rotate_row<D, BF16>(k, cs, sn, t);
+                store_row(kbase + (size_t)pos * D, k);
+                store_row(vbase + (size_t)pos * D, v);
+            };
+            if (na && pa < s1) fresh(ka, va);
+            if (nb && pb < s1) fresh(kb, vb);
+        }
+        __syncwarp();
+    };
+    int p = s0 + warp * kAttBlock;
+    uint4 qf[C];                                  // head g of the group
+    clear(qf);
+    if (g < heads) {
+        load_row(static_cast<const T*>(q_) + (size_t)b * ldq + (size_t)(kvh * heads + g) * D + t * 8, qf);
+    }
+    if (p < s1) fetch(p);                         // before anything waits for the queries
+    if (append) rotate_row<D, BF16>(qf, cs, sn, t);
+    float m0 = -1.0e30f, m1 = -1.0e30f, l0 = 0.0f, l1 = 0.0f;      // heads 2t, 2t + 1; the sums of this lane's positions
+    float o[D / 16][4];                           // rows: elements, see below; columns: heads 2t, 2t + 1
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
+
+    while (p < s1) {
+        const bool ia = p + g < s1, ib = p + g + 8 < s1;
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};    // positions p + g (0, 1), p + g + 8 (2, 3); heads 2t, 2t + 1
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            mma16<BF16>(s, ka[c].x, kb[c].x, ka[c].y, kb[c].y, qf[c].x, qf[c].y);
+            mma16<BF16>(s, ka[c].z, kb[c].z, ka[c].w, kb[c].w, qf[c].z, qf[c].w);
+        }
+        s[0] = ia ? s[0] * scale : -1.0e30f; s[1] = ia ? s[1] * scale : -1.0e30f;
+        s[2] = ib ? s[2] * scale : -1.0e30f; s[3] = ib ? s[3] * scale : -1.0e30f;
+        float x0 = fmaxf(s[0], s[2]), x1 = fmaxf(s[1], s[3]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
+        }
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        const float f0 = __expf(m0 - n0), f1 = __expf(m1 - n1);
+        m0 = n0; m1 = n1;
+        float w[4] = {ia ? __expf(s[0] - n0) : 0.0f, ia ? __expf(s[1] - n1) : 0.0f, ib ? __expf(s[2] - n0) : 0.0f, ib ? __expf(s[3] - n1) : 0.0f};
+        l0 = fmaf(l0, f0, w[0] + w[2]);
+        l1 = fmaf(l1, f1, w[1] + w[3]);
+        uint32_t pw[SPLIT][2];                    // [part][positions 0 - 7, 8 - 15], transposed: head g, positions 2t, 2t + 1
+#pragma unroll
+        for (int i = 0; i < SPLIT; ++i) {
+            pw[i][0] = transpose8(pack2<BF16>(w[0], w[1]));
+            pw[i][1] = transpose8(pack2<BF16>(w[2], w[3]));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] -= r16<BF16>(w[e]);
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const uint32_t wa[4] = {va[c].x, va[c].y, va[c].z, va[c].w}, wb[4] = {vb[c].x, vb[c].y, vb[c].z, vb[c].w};
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {         // word w of a lane's eight elements: row r of the transposed block is element 32 c + 8 (r / 2) + 2 w + r % 2
+                float (&acc)[4] = o[c * 2 + j];
+                acc[0] *= f0; acc[1] *= f1; acc[2] *= f0; acc[3] *= f1;
+                const uint32_t a0 = transpose8(wa[2 * j]), a1 = transpose8(wa[2 * j + 1]), a2 = transpose8(wb[2 * j]), a3 = transpose8(wb[2 * j + 1]);
+#pragma unroll
+                for (int i = 0; i < SPLIT; ++i) mma16<BF16>(acc, a0, a1, a2, a3, pw[i][0], pw[i][1]);
+            }
+        }
+        p += kAttWarps * kAttBlock;
+        if (p < s1) fetch(p);
+    }
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+        l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, off);
     }
 
     // the CTA's warps meet in shared memory
-    __shared__ float sm_m[kAttWarps][G], sm_l[kAttWarps][G];
-    __shared__ float sm_o[kAttWarps][G][D];
+    __shared__ float sm_m[kAttWarps][kAttMaxHeads], sm_l[kAttWarps][kAttMaxHeads];
+    __shared__ float sm_o[kAttWarps][kAttMaxHeads][D];
     __shared__ int is_last;
+    const int active = max(1, min(kAttWarps, (s1 - s0 + kAttBlock - 1) / kAttBlock));      // warps that had a turn
+    if (warp < active) {
+        if (g == 0) {
+            sm_m[warp][2 * t] = m0; sm_m[warp][2 * t + 1] = m1;
+            sm_l[warp][2 * t] = l0; sm_l[warp][2 * t + 1] = l1;
+        }
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        if (lane == 0) { sm_m[warp][g] = m[g]; sm_l[warp][g] = l[g]; }
-#pragma unroll
-        for (int e = 0; e < E; ++e) sm_o[warp][g][lane * E + e] = o[g][e];
+        for (int i = 0; i < D / 16; ++i) {
+            const int d = (i >> 1) * 32 + (g >> 1) * 8 + (i & 1) * 4 + (g & 1);
+            if (2 * t < heads) { sm_o[warp][2 * t][d] = o[i][0]; sm_o[warp][2 * t][d + 2] = o[i][2]; }
+            if (2 * t + 1 < heads) { sm_o[warp][2 * t + 1][d] = o[i][1]; sm_o[warp][2 * t + 1][d + 2] = o[i][3]; }
+        }
     }
     __syncthreads();
     constexpr int STRIDE = D + 4;                 // floats per (slice, head): m, l, two unused, o[D] (16-byte aligned)
-    float* mine = parts + ((((size_t)b * hkv + kvh) * slices + slice) * G) * STRIDE;
-    for (int i = tid; i < G * D; i += kAttWarps * 32) {
-        const int g = i / D, dd = i - g * D;
-        float mm = sm_m[0][g];
-#pragma unroll
-        for (int w = 1; w < kAttWarps; ++w) mm = fmaxf(mm, sm_m[w][g]);
+    T* out = static_cast<T*>(out_) + (size_t)b * ldo + (size_t)kvh * heads * D;
+    float* mine = parts + ((((size_t)b * hkv + kvh) * slices + slice) * heads) * STRIDE;
+    for (int i = tid; i < heads * D; i += kAttWarps * 32) {
+        const int h = i / D, dd = i - h * D;
+        float mm = sm_m[0][h];
+        for (int w = 1; w < active; ++w) mm = fmaxf(mm, sm_m[w][h]);
         float acc = 0.0f, ll = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kAttWarps; ++w) {
-            const float f = __expf(sm_m[w][g] - mm);
-            acc = fmaf(sm_o[w][g][dd], f, acc);
-            ll = fmaf(sm_l[w][g], f, ll);
+        for (int w = 0; w < active; ++w) {
+            const float f = __expf(sm_m[w][h] - mm);
+            acc = fmaf(sm_o[w][h][dd], f, acc);
+            ll = fmaf(sm_l[w][h], f, ll);
         }
-        mine[g * STRIDE + 4 + dd] = acc;
-        if (dd == 0) { mine[g * STRIDE] = mm; mine[g * STRIDE + 1] = ll; }
+        if (slices == 1) {
+            out[i] = Act16<BF16>::from_float(ll > 0.0f ? acc * (1.0f / ll) : 0.0f);
+        } else {
+            mine[h * STRIDE + 4 + dd] = acc;
+            if (dd == 0) { mine[h * STRIDE] = mm; mine[h * STRIDE + 1] = ll; }
+        }
     }
+    if (slices == 1) return;
     // arrival: the last CTA of this (sequence, kv head) merges the slices; nobody waits
     __threadfence();
     __syncthreads();
@@ -288,17 +428,16 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_kernel(const void* q
     __threadfence();
     // Every load of the merge is independent of the others and issued before the first use: one
     // trip to L2 per head instead of one per slice.  A warp takes a head; a lane takes 4 output elements.
-    const float* all = parts + (((size_t)b * hkv + kvh) * slices) * G * STRIDE;
-    T* out = static_cast<T*>(out_) + (size_t)b * ldo + (size_t)kvh * G * D;
+    const float* all = parts + (((size_t)b * hkv + kvh) * slices) * heads * STRIDE;
     const bool has_o = lane * 4 < D;
-    for (int g = warp; g < G; g += kAttWarps) {
+    for (int h = warp; h < heads; h += kAttWarps) {
         float mv[kAttMaxSlices], lv[kAttMaxSlices];
         float4 ov[kAttMaxSlices];
 #pragma unroll
         for (int s = 0; s < kAttMaxSlices; ++s) {
             mv[s] = -1.0e30f; lv[s] = 0.0f; ov[s] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (s < slices) {
-                const float* pp = all + ((size_t)s * G + g) * STRIDE;
+                const float* pp = all + ((size_t)s * heads + h) * STRIDE;
                 const float2 ml = __ldcg(reinterpret_cast<const float2*>(pp));
                 mv[s] = ml.x; lv[s] = ml.y;
                 if (has_o) ov[s] = __ldcg(reinterpret_cast<const float4*>(pp + 4) + lane);
@@ -322,7 +461,7 @@ __global__ void __launch_bounds__(kAttWarps * 32) attention_kernel(const void* q
             T* pe = reinterpret_cast<T*>(&packed);
             pe[0] = Act16<BF16>::from_float(acc.x * inv); pe[1] = Act16<BF16>::from_float(acc.y * inv);
             pe[2] = Act16<BF16>::from_float(acc.z * inv); pe[3] = Act16<BF16>::from_float(acc.w * inv);
-            *reinterpret_cast<uint2*>(out + g * D + lane * 4) = packed;
+            *reinterpret_cast<uint2*>(out + h * D + lane * 4) = packed;
         }
     }
     if (tid == 0) counters[b * hkv + kvh] = 0;       // ready for the next launch (stream order makes it visible)
@@ -380,21 +519,16 @@ int launch_pdl(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, 
     return check_launch(what);
 }
 
-template <int D, bool BF16>
-int launch_attention(int group, dim3 grid, cudaStream_t s, const void* q, long long ldq, const void* kc, const void* vc,
-                     const long long* pos, void* out, long long ldo, int hq, int hkv, int max_len, float scale, float* parts,
-                     int* counters) {
+template <bool ROPE>
+int launch_attention(bool bf16, int head_dim, dim3 grid, cudaStream_t s, const void* q, long long ldq, void* kc, void* vc, const long long* pos,
+                     void* out, long long ldo, int heads, int hkv, int max_len, float scale, float* parts, int* counters, bool wide,
+                     const NewToken& nt) {
     const dim3 block(kAttWarps * 32);
-#define QDEC_ATT(GG)                                                                                                    \
-    case GG: return launch_pdl("attention_kernel", attention_kernel<D, GG, BF16>, grid, block, s, q, ldq, kc, vc, pos, out, ldo, \
-                               hq, hkv, max_len, scale, parts, counters)
-    switch (group) {
-        QDEC_ATT(1); QDEC_ATT(2); QDEC_ATT(3); QDEC_ATT(4); QDEC_ATT(5); QDEC_ATT(6); QDEC_ATT(7); QDEC_ATT(8);
-        default: break;
-    }
+#define QDEC_ATT(D, B) launch_pdl("attention_kernel", attention_kernel<D, B, ROPE>, grid, block, s, q, ldq, kc, vc, pos, out, ldo, heads, hkv, \
+                                  max_len, scale, parts, counters, wide, nt)
+    if (head_dim == 64) return bf16 ? QDEC_ATT(64, true) : QDEC_ATT(64, false);
+    return bf16 ? QDEC_ATT(128, true) : QDEC_ATT(128, false);
 #undef QDEC_ATT
-    set_error("qdec_attention: %d query heads per kv head (1..8 supported)", group);
-    return QGEMV_ERR_SHAPE;
 }
 
 size_t attention_parts_floats(int batch, int q_heads, int kv_heads, int head_dim, int max_len) {
@@ -449,35 +583,52 @@ extern "C" size_t qdec_attention_workspace_bytes(int batch, int q_heads, int kv_
     return counters + (parts + 255) / 256 * 256;
 }
 
-extern "C" int qdec_attention(const void* q, int64_t ldq, const void* kcache, const void* vcache, const int64_t* pos,
-                              void* out, int64_t ldo, int batch, int q_heads, int kv_heads, int head_dim, int max_len,
-                              float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream) {
-    if (!q || !kcache || !vcache || !pos || !out || !workspace) { set_error("qdec_attention: null pointer"); return QGEMV_ERR_BAD_ARG; }
-    if (batch < 1 || q_heads < 1 || kv_heads < 1 || max_len < 1) { set_error("qdec_attention: non-positive size"); return QGEMV_ERR_BAD_ARG; }
-    if (dtype != QGEMV_F16 && dtype != QGEMV_BF16) { set_error("qdec_attention: dtype must be fp16 or bf16"); return QGEMV_ERR_BAD_ARG; }
-    if (head_dim != 64 && head_dim != 128) { set_error("qdec_attention: head_dim=%d (64 and 128 are built)", head_dim); return QGEMV_ERR_SHAPE; }
-    if (q_heads % kv_heads || q_heads / kv_heads > 8) { set_error("qdec_attention: %d query heads over %d kv heads (a group of 1..8 is built)", q_heads, kv_heads); return QGEMV_ERR_SHAPE; }
-    if (ldq < (int64_t)q_heads * head_dim || ldo < (int64_t)q_heads * head_dim) { set_error("qdec_attention: a leading dimension is smaller than its row"); return QGEMV_ERR_SHAPE; }
-    if (batch > 65535 || kv_heads > 65535) { set_error("qdec_attention: batch and kv_heads are grid dimensions (at most 65535)"); return QGEMV_ERR_TOO_LARGE; }
+namespace {
+// Argument checks and launch shared by the two forms; `nt.k` == NULL: attention alone.
+int run_attention(const char* name, const void* q, int64_t ldq, void* kcache, void* vcache, const int64_t* pos, void* out, int64_t ldo, int batch,
+                  int q_heads, int kv_heads, int head_dim, int max_len, float scale, void* workspace, size_t workspace_bytes, int dtype,
+                  const NewToken& nt, void* stream) {
+    if (!q || !kcache || !vcache || !pos || !out || !workspace) { set_error("%s: null pointer", name); return QGEMV_ERR_BAD_ARG; }
+    if (batch < 1 || q_heads < 1 || kv_heads < 1 || max_len < 1) { set_error("%s: non-positive size", name); return QGEMV_ERR_BAD_ARG; }
+    if (dtype != QGEMV_F16 && dtype != QGEMV_BF16) { set_error("%s: dtype must be fp16 or bf16", name); return QGEMV_ERR_BAD_ARG; }
+    if (head_dim != 64 && head_dim != 128) { set_error("%s: head_dim=%d (64 and 128 are built)", name, head_dim); return QGEMV_ERR_SHAPE; }
+    if (q_heads % kv_heads || q_heads / kv_heads > kAttMaxHeads) { set_error("%s: %d query heads over %d kv heads (a group of 1..8 is built)", name, q_heads, kv_heads); return QGEMV_ERR_SHAPE; }
+    if (ldq < (int64_t)q_heads * head_dim || ldo < (int64_t)q_heads * head_dim) { set_error("%s: a leading dimension is smaller than its row", name); return QGEMV_ERR_SHAPE; }
+    if (batch > 65535 || kv_heads > 65535) { set_error("%s: batch and kv_heads are grid dimensions (at most 65535)", name); return QGEMV_ERR_TOO_LARGE; }
     const size_t need = qdec_attention_workspace_bytes(batch, q_heads, kv_heads, head_dim, max_len);
-    if (workspace_bytes < need) { set_error("qdec_attention: workspace of %zu bytes required (got %zu)", need, workspace_bytes); return QGEMV_ERR_WORKSPACE; }
-    if (reinterpret_cast<uintptr_t>(workspace) % 256 || reinterpret_cast<uintptr_t>(q) % 8 || reinterpret_cast<uintptr_t>(kcache) % 8 ||
-        reinterpret_cast<uintptr_t>(vcache) % 8 || (ldq * 2) % 8 || reinterpret_cast<uintptr_t>(out) % 8 || (ldo * 2) % 8) {
-        set_error("qdec_attention: workspace must be 256-byte aligned, q, out and the caches 8-byte aligned");
+    if (workspace_bytes < need) { set_error("%s: workspace of %zu bytes required (got %zu)", name, need, workspace_bytes); return QGEMV_ERR_WORKSPACE; }
+    auto rows = [](const void* p, int64_t ld, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0 && ld * 2 % (int64_t)a == 0; };
+    auto all = [&](size_t a) {
+        return rows(q, ldq, a) && rows(kcache, 0, a) && rows(vcache, 0, a) && (!nt.k || (rows(nt.k, nt.ldk, a) && rows(nt.v, nt.ldv, a)));
+    };
+    if (reinterpret_cast<uintptr_t>(workspace) % 256 || !all(8) || !rows(out, ldo, 8)) {
+        set_error("%s: workspace must be 256-byte aligned, q, out, new rows and the caches 8-byte aligned", name);
         return QGEMV_ERR_ALIGN;
     }
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     int* counters = static_cast<int*>(workspace);
     float* parts = reinterpret_cast<float*>(static_cast<char*>(workspace) + ((size_t)batch * kv_heads * sizeof(int) + 255) / 256 * 256);
     const dim3 grid(attention_slices(batch, kv_heads, max_len), kv_heads, batch);
-    const int group = q_heads / kv_heads;
-    const long long* p = reinterpret_cast<const long long*>(pos);
-    const bool bf16 = dtype == QGEMV_BF16;
-    if (head_dim == 64)
-        return bf16 ? launch_attention<64, true>(group, grid, s, q, ldq, kcache, vcache, p, out, ldo, q_heads, kv_heads, max_len, scale, parts, counters)
-                    : launch_attention<64, false>(group, grid, s, q, ldq, kcache, vcache, p, out, ldo, q_heads, kv_heads, max_len, scale, parts, counters);
-    return bf16 ? launch_attention<128, true>(group, grid, s, q, ldq, kcache, vcache, p, out, ldo, q_heads, kv_heads, max_len, scale, parts, counters)
-                : launch_attention<128, false>(group, grid, s, q, ldq, kcache, vcache, p, out, ldo, q_heads, kv_heads, max_len, scale, parts, counters);
+    return (nt.k ? launch_attention<true> : launch_attention<false>)(dtype == QGEMV_BF16, head_dim, grid, static_cast<cudaStream_t>(stream), q, ldq, kcache,
+        vcache, reinterpret_cast<const long long*>(pos), out, ldo, q_heads / kv_heads, kv_heads, max_len, scale, parts, counters, all(16), nt);
+}
+}  // namespace
+
+extern "C" int qdec_attention(const void* q, int64_t ldq, const void* kcache, const void* vcache, const int64_t* pos,
+                              void* out, int64_t ldo, int batch, int q_heads, int kv_heads, int head_dim, int max_len,
+                              float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream) {
+    return run_attention("qdec_attention", q, ldq, const_cast<void*>(kcache), const_cast<void*>(vcache), pos, out, ldo, batch, q_heads, kv_heads,
+                         head_dim, max_len, scale, workspace, workspace_bytes, dtype, NewToken{}, stream);
+}
+
+extern "C" int qdec_rope_attention(const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv,
+                                   const void* cos_table, const void* sin_table, int table_rows, const int64_t* pos,
+                                   void* kcache, void* vcache, void* out, int64_t ldo, int batch, int q_heads, int kv_heads,
+                                   int head_dim, int max_len, float scale, void* workspace, size_t workspace_bytes,
+                                   int32_t* status, int dtype, void* stream) {
+    if (!k || !v || !cos_table || !sin_table || table_rows < 1) { set_error("qdec_rope_attention: null pointer or empty table"); return QGEMV_ERR_BAD_ARG; }
+    if (ldk < (int64_t)kv_heads * head_dim || ldv < (int64_t)kv_heads * head_dim) { set_error("qdec_rope_attention: a leading dimension is smaller than its row"); return QGEMV_ERR_SHAPE; }
+    return run_attention("qdec_rope_attention", q, ldq, kcache, vcache, pos, out, ldo, batch, q_heads, kv_heads, head_dim, max_len, scale, workspace,
+                         workspace_bytes, dtype, NewToken{k, ldk, v, ldv, cos_table, sin_table, table_rows, status}, stream);
 }
 
 extern "C" int qdec_silu_mul(const void* gate, int64_t ldg, const void* up, int64_t ldu, void* y, int64_t ldy,

@@ -6,9 +6,9 @@ SwiGLU product and residual additions between its packed GEMVs are whatever the 
 Run eagerly those are some fifty small kernels per layer, and on a B200 they cost about twice what the
 packed GEMVs cost.  ``NativeDecodeStep`` walks the same modules (the Linear layers are called as they
 are: packed modules, fp16 ``nn.Linear``, tensor-parallel shards with their all-reduce, fused siblings)
-and replaces everything in between by four kernels of ``include/qdecode_b200.h``:
+and replaces everything in between by three kernels of ``include/qdecode_b200.h``:
 
-    rmsnorm (+ residual update) -> q, k, v -> rope + cache append -> attention -> o
+    rmsnorm (+ residual update) -> q, k, v -> rope + cache append + attention -> o
     rmsnorm (+ residual update) -> gate / up (+ silu * mul, fused into the GEMV where possible) -> down
 
 It reads and writes the ``StaticCache`` tensors of the Hugging Face model in place, so the prompt can
@@ -93,6 +93,20 @@ def attention(q, kcache, vcache, pos, scale: float, workspace: torch.Tensor, out
         _cabi.check(_cabi.lib().qdec_attention(_ptr(q), q.stride(0), _ptr(kcache), _ptr(vcache), _ptr(pos), _ptr(o), o.stride(0),
                                                b, hq, hkv, d, max_len, float(scale), C.c_void_p(workspace.data_ptr() + off),
                                                workspace.numel() - off, _DT[q.dtype], _stream()))
+    return o
+
+
+def rope_attention(q, k, v, cos, sin, pos, kcache, vcache, scale: float, workspace: torch.Tensor, status=None) -> torch.Tensor:
+    """``rope_append`` and ``attention`` in one launch, ``q`` left as it is; returns ``[B, Hq * D]``."""
+    b, hkv, max_len, d = kcache.shape
+    hq = q.shape[1] // d
+    o = torch.empty((b, hq * d), dtype=q.dtype, device=q.device)
+    off = (-workspace.data_ptr()) % 256
+    with torch.cuda.device(q.device):
+        _cabi.check(_cabi.lib().qdec_rope_attention(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(cos), _ptr(sin),
+                                                    cos.shape[0], _ptr(pos), _ptr(kcache), _ptr(vcache), _ptr(o), o.stride(0), b, hq, hkv, d, max_len,
+                                                    float(scale), C.c_void_p(workspace.data_ptr() + off), workspace.numel() - off, _ptr(status),
+                                                    _DT[q.dtype], _stream()))
     return o
 
 
@@ -255,8 +269,12 @@ class NativeDecodeStep:
             x = self._norm(h, delta, comm, layer.input_layernorm)
             q, k, v = self._qkv(attn, x)
             kc, vc = self.kv[i]
-            rope_append(q, k, v, self.cos, self.sin, pos, kc, vc, d, self.status)
-            a = attention(q, kc, vc, pos, float(getattr(attn, "scaling", d ** -0.5)), self.att_ws)
+            scale = float(getattr(attn, "scaling", d ** -0.5))
+            if all(t.data_ptr() % 8 == 0 and t.stride(0) % 4 == 0 and t.stride(1) == 1 for t in (q, k, v)):
+                a = rope_attention(q, k, v, self.cos, self.sin, pos, kc, vc, scale, self.att_ws, self.status)
+            else:                                                # outputs of foreign modules may sit anywhere
+                rope_append(q, k, v, self.cos, self.sin, pos, kc, vc, d, self.status)
+                a = attention(q.contiguous(), kc, vc, pos, scale, self.att_ws)
             delta, comm = self._project(attn.o_proj, a)
             x = self._norm(h, delta, comm, layer.post_attention_layernorm)
             if type(mlp).__name__ == "GatedFeedForward":

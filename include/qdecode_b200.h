@@ -64,6 +64,16 @@ int qdec_attention(const void* q, int64_t ldq, const void* kcache, const void* v
                    void* out, int64_t ldo, int batch, int q_heads, int kv_heads, int head_dim, int max_len,
                    float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream);
 
+/* qdec_rope_append and qdec_attention in one launch: the queries are rotated on their way in (q itself is
+ * left as it is), the new token's key and value are written to the caches at position *pos and take part
+ * in the attention.  k, v and the caches 8-byte aligned like q.  A position outside
+ * [0, min(max_len, table_rows)) appends nothing and raises *status. */
+int qdec_rope_attention(const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv,
+                        const void* cos_table, const void* sin_table, int table_rows, const int64_t* pos,
+                        void* kcache, void* vcache, void* out, int64_t ldo, int batch, int q_heads, int kv_heads,
+                        int head_dim, int max_len, float scale, void* workspace, size_t workspace_bytes,
+                        int32_t* status, int dtype, void* stream);
+
 /* y[i] = r(r(silu(gate[i])) * up[i]) for [rows, width] tensors (leading dimensions in elements). */
 int qdec_silu_mul(const void* gate, int64_t ldg, const void* up, int64_t ldu, void* y, int64_t ldy,
                   int rows, int width, int dtype, void* stream);

@@ -118,6 +118,48 @@ def test_attention_over_the_cache(dtype, batch, hq, hkv, d, max_len, p):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shift", [0, 4])                                        # rows 16-byte aligned, or 8-byte only
+@pytest.mark.parametrize("batch,hq,hkv,d,max_len,p", [(1, 1, 1, 64, 8, 0), (2, 14, 2, 64, 300, 15), (1, 16, 2, 128, 300, 16), (2, 8, 1, 128, 256, 255),
+                                                       (1, 10, 2, 64, 700, 256), (3, 6, 2, 128, 700, 128), (1, 8, 8, 64, 5000, 4999)])
+def test_rope_append_and_attention_in_one_launch(dtype, shift, batch, hq, hkv, d, max_len, p):
+    """Edges of a warp's 16 positions, a CTA's turn and the slices: against the two launches it stands for (caches and outputs
+    equal) and against float64."""
+    torch.manual_seed(hq * d + p)
+
+    def rows(width):
+        return torch.randn(batch, width + 8).to(dtype).cuda()[:, shift:shift + width] if shift else torch.randn(batch, width).to(dtype).cuda()
+    q, k, v = rows(hq * d), rows(hkv * d), rows(hkv * d)
+    ang = torch.rand(max_len, d, device="cuda") * 6
+    cos, sin = ang.cos().to(dtype), ang.sin().to(dtype)
+    kc, vc = (torch.randn(batch, hkv, max_len, d).to(dtype).cuda() for _ in range(2))
+    kc[:, :, p:] = float("nan")                                                  # the new position comes from k and v, later ones are not read
+    vc[:, :, p:] = float("nan")
+    kc2, vc2, q2 = kc.clone(), vc.clone(), q.clone()
+    pos = torch.tensor([p], dtype=torch.int64, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws, scale = ds.attention_workspace(batch, hq, hkv, d, max_len, "cuda"), d ** -0.5
+    got = ds.rope_attention(q, k, v, cos, sin, pos, kc, vc, scale, ws, status)
+    ds.rope_append(q2, k, v, cos, sin, pos, kc2, vc2, d, status)
+    assert torch.equal(kc[:, :, :p + 1], kc2[:, :, :p + 1]) and torch.equal(vc[:, :, :p + 1], vc2[:, :, :p + 1])
+    assert torch.equal(got, ds.attention(q2, kc2, vc2, pos, scale, ws)) and int(status.item()) == 0
+    g, n = hq // hkv, p + 1
+    kf, vf = (c[:, :, :n].double().repeat_interleave(g, dim=1) for c in (kc, vc))
+    qd = q2.double().reshape(batch, hq, d)
+    score = torch.einsum("bhd,bhjd->bhj", qd, kf) * scale
+    ref = torch.einsum("bhj,bhjd->bhd", torch.softmax(score, -1), vf)
+    # fp32 dot products of d terms move an exponent by at most d 2^-24 sum |q k| scale, the exponential by a few 2^-22 of
+    # its argument; a relative change of every weight by e changes the result by at most 2 e max |v|; then one rounding
+    size = torch.einsum("bhd,bhjd->bhj", qd.abs(), kf.abs()).amax(-1) * scale
+    e = d * 2.0 ** -24 * size + 2.0 ** -20 * (1 + score.abs().amax(-1)) + n * 2.0 ** -24
+    tol = 2 * e[..., None] * vf.abs().amax(2) .amax(-1)[..., None] + 2.0 ** (-11 if dtype == torch.float16 else -8) * ref.abs() * 1.01 + 2.0 ** -24
+    assert bool(((got.double().reshape(batch, hq, d) - ref).abs() <= tol).all())
+    pos.fill_(max_len)                                                           # past the cache: nothing written, status raised
+    before = kc.clone()
+    ds.rope_attention(q, k, v, cos, sin, pos, kc, vc, scale, ws, status)
+    assert int(status.item()) == 1 and torch.equal(kc.nan_to_num(9.0), before.nan_to_num(9.0))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_silu_mul(dtype):
     torch.manual_seed(1)
     for rows, width in ((1, 14336), (4, 4864), (3, 50)):
