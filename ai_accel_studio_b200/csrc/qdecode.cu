@@ -23,74 +23,75 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// residual update + RMS normalisation: one CTA per row
+// residual update + RMS normalisation: one CTA per row, a thread for every 8 elements up to 1024 of them.  A chain of
+// latencies (h and delta from L2, two reductions, the store), so the norm's weight, which comes from DRAM, is fetched before
+// the preceding kernel has finished, and one barrier is all that the threads meet at.
 // ---------------------------------------------------------------------------------------------
-constexpr int kNormThreads = 256;
-constexpr int kNormMaxVec = 8;                    // 8-element vectors per thread: hidden <= 256 * 8 * 8
+constexpr int kNormMaxThreads = 1024;
+constexpr int kNormMaxVec = 2;                    // 8-element vectors per thread: hidden <= 1024 * 2 * 8
 
 template <bool BF16>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(void* h_, long long ldh, const void* delta_, long long ldd,
-                                                               const void* w_, void* y_, long long ldy, int hidden, float eps) {
+__global__ void __launch_bounds__(kNormMaxThreads) rmsnorm_kernel(void* h_, long long ldh, const void* delta_, long long ldd,
+                                                                  const void* w_, void* y_, long long ldy, int hidden, float eps) {
     using T = typename Act16<BF16>::T;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int row = blockIdx.x, tid = threadIdx.x, nvec = hidden >> 3;
+    const int row = blockIdx.x, tid = threadIdx.x, threads = blockDim.x, nvec = hidden >> 3;
     T* h = static_cast<T*>(h_) + (size_t)row * ldh;
     const T* delta = delta_ ? static_cast<const T*>(delta_) + (size_t)row * ldd : nullptr;
     const T* w = static_cast<const T*>(w_);
     T* y = static_cast<T*>(y_) + (size_t)row * ldy;
-    __shared__ float red[kNormThreads / 32];
-    __shared__ float total;
+    __shared__ float red[32];
 
-    float f[kNormMaxVec][8];
+    uint4 wv[kNormMaxVec];
+#pragma unroll
+    for (int i = 0; i < kNormMaxVec; ++i)
+        if (tid + i * threads < nvec) wv[i] = __ldg(reinterpret_cast<const uint4*>(w) + tid + i * threads);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    uint4 hv[kNormMaxVec], dv[kNormMaxVec];
+#pragma unroll
+    for (int i = 0; i < kNormMaxVec; ++i) {
+        const int v = tid + i * threads;
+        if (v < nvec) {
+            hv[i] = *reinterpret_cast<const uint4*>(h + v * 8);
+            if (delta) dv[i] = *reinterpret_cast<const uint4*>(delta + v * 8);
+        }
+    }
     float sq = 0.0f;
 #pragma unroll
     for (int i = 0; i < kNormMaxVec; ++i) {
-        const int v = tid + i * kNormThreads;
+        const int v = tid + i * threads;
         if (v < nvec) {
-            uint4 hv = *reinterpret_cast<const uint4*>(h + v * 8);
-            const T* he = reinterpret_cast<const T*>(&hv);
+            T* he = reinterpret_cast<T*>(&hv[i]);
             if (delta) {
-                const uint4 dv = *reinterpret_cast<const uint4*>(delta + v * 8);
-                const T* de = reinterpret_cast<const T*>(&dv);
-                uint4 ov;
-                T* oe = reinterpret_cast<T*>(&ov);
+                const T* de = reinterpret_cast<const T*>(&dv[i]);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    oe[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(he[q]) + Act16<BF16>::to_float(de[q]));
-                    f[i][q] = Act16<BF16>::to_float(oe[q]);
-                }
-                *reinterpret_cast<uint4*>(h + v * 8) = ov;
-            } else {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) f[i][q] = Act16<BF16>::to_float(he[q]);
+                for (int q = 0; q < 8; ++q) he[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(he[q]) + Act16<BF16>::to_float(de[q]));
+                *reinterpret_cast<uint4*>(h + v * 8) = hv[i];
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q) sq = fmaf(f[i][q], f[i][q], sq);
+            for (int q = 0; q < 8; ++q) {
+                const float f = Act16<BF16>::to_float(he[q]);
+                sq = fmaf(f, f, sq);
+            }
         }
     }
     sq = warp_sum(sq);
     if ((tid & 31) == 0) red[tid >> 5] = sq;
     __syncthreads();
-    if (tid == 0) {
-        float t = 0.0f;
-#pragma unroll
-        for (int i = 0; i < kNormThreads / 32; ++i) t += red[i];
-        total = rsqrtf(t / (float)hidden + eps);
-    }
-    __syncthreads();
-    const float inv = total;
+    const int lane = tid & 31;
+    const float inv = rsqrtf(warp_sum(lane < threads >> 5 ? red[lane] : 0.0f) / (float)hidden + eps);
 #pragma unroll
     for (int i = 0; i < kNormMaxVec; ++i) {
-        const int v = tid + i * kNormThreads;
+        const int v = tid + i * threads;
         if (v < nvec) {
-            const uint4 wv = *reinterpret_cast<const uint4*>(w + v * 8);
-            const T* we = reinterpret_cast<const T*>(&wv);
+            const T* he = reinterpret_cast<const T*>(&hv[i]);
+            const T* we = reinterpret_cast<const T*>(&wv[i]);
             uint4 ov;
             T* oe = reinterpret_cast<T*>(&ov);
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-                oe[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(we[q]) * r16<BF16>(f[i][q] * inv));
+                oe[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(we[q]) * r16<BF16>(Act16<BF16>::to_float(he[q]) * inv));
             *reinterpret_cast<uint4*>(y + v * 8) = ov;
         }
     }
@@ -545,16 +546,17 @@ extern "C" int qdec_rmsnorm(void* h, int64_t ldh, const void* delta, int64_t ldd
                             int rows, int hidden, float eps, int dtype, void* stream) {
     if (!h || !weight || !y || rows < 1 || hidden < 8) { set_error("qdec_rmsnorm: null pointer or non-positive size"); return QGEMV_ERR_BAD_ARG; }
     if (dtype != QGEMV_F16 && dtype != QGEMV_BF16) { set_error("qdec_rmsnorm: dtype must be fp16 or bf16"); return QGEMV_ERR_BAD_ARG; }
-    if (hidden % 8 || hidden > kNormThreads * kNormMaxVec * 8) { set_error("qdec_rmsnorm: hidden=%d must be a multiple of 8, at most %d", hidden, kNormThreads * kNormMaxVec * 8); return QGEMV_ERR_SHAPE; }
+    if (hidden % 8 || hidden > kNormMaxThreads * kNormMaxVec * 8) { set_error("qdec_rmsnorm: hidden=%d must be a multiple of 8, at most %d", hidden, kNormMaxThreads * kNormMaxVec * 8); return QGEMV_ERR_SHAPE; }
     if (ldh < hidden || ldy < hidden || (delta && ldd < hidden)) { set_error("qdec_rmsnorm: a leading dimension is smaller than hidden"); return QGEMV_ERR_SHAPE; }
     if (!aligned16(h) || !aligned16(y) || !aligned16(weight) || (delta && !aligned16(delta)) || ldh % 8 || ldy % 8 || (delta && ldd % 8)) {
         set_error("qdec_rmsnorm: rows must be 16-byte aligned");
         return QGEMV_ERR_ALIGN;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int vecs = hidden / 8, threads = vecs >= kNormMaxThreads ? kNormMaxThreads : (vecs + 31) / 32 * 32;
     if (dtype == QGEMV_BF16)
-        return launch_pdl("rmsnorm_kernel", rmsnorm_kernel<true>, dim3(rows), dim3(kNormThreads), s, h, (long long)ldh, delta, (long long)ldd, weight, y, (long long)ldy, hidden, eps);
-    return launch_pdl("rmsnorm_kernel", rmsnorm_kernel<false>, dim3(rows), dim3(kNormThreads), s, h, (long long)ldh, delta, (long long)ldd, weight, y, (long long)ldy, hidden, eps);
+        return launch_pdl("rmsnorm_kernel", rmsnorm_kernel<true>, dim3(rows), dim3(threads), s, h, (long long)ldh, delta, (long long)ldd, weight, y, (long long)ldy, hidden, eps);
+    return launch_pdl("rmsnorm_kernel", rmsnorm_kernel<false>, dim3(rows), dim3(threads), s, h, (long long)ldh, delta, (long long)ldd, weight, y, (long long)ldy, hidden, eps);
 }
 
 extern "C" int qdec_rope_append(void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv,

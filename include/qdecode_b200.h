@@ -31,7 +31,8 @@ extern "C" {
 /* h[m, :] = r(h[m, :] + delta[m, :]) in place when delta != NULL, then
  * y[m, :] = r(weight[:] * r(h[m, :] * rsqrt(mean(h[m, :]^2) + eps))).
  * hidden: a multiple of 8, at most 16384; h, delta, y: [rows, hidden] with leading dimensions ldh,
- * ldd, ldy (elements) and 16-byte aligned rows; weight: [hidden] of the activation type. */
+ * ldd, ldy (elements) and 16-byte aligned rows; weight: [hidden] of the activation type, final when the
+ * call is issued (it is read before the preceding kernel of the stream has finished). */
 int qdec_rmsnorm(void* h, int64_t ldh, const void* delta, int64_t ldd, const void* weight, void* y, int64_t ldy,
                  int rows, int hidden, float eps, int dtype, void* stream);
 
