@@ -43,8 +43,9 @@ def select_outliers(module: nn.Module, w: torch.Tensor, activation_rms, outlier_
 
 
 class HybridPackedLinear(nn.Module):
-    """Common forward: up to ``chunked_max_rows`` rows -> one fused launch (a few shapes: one per four rows); larger M ->
-    CUDA dequantisation into the activation dtype + library GEMMs for the base, outlier and residual terms."""
+    """Common forward: up to ``chunked_max_rows`` rows -> one fused launch; larger M -> a GEMM that dequantises on its way to
+    tensor memory.  Where neither applies (group sizes, layouts): launches per four rows, and CUDA dequantisation into the
+    activation dtype + library GEMMs for the base, outlier and residual terms."""
 
     bits: int = 0
     residual_rank: int = 0
@@ -55,7 +56,7 @@ class HybridPackedLinear(nn.Module):
     # Optional hint for the decode path: a static tensor (normally the packed codes of the module that
     # runs next) announced to L2 while this module's GEMV runs; see model_tools.chain_weight_prefetch.
     prefetch_next = None
-    # Largest row count (at most 16) served by the fused GEMV instead of the dequantise + GEMM route.
+    # Largest row count (at most 16) served by the fused GEMV instead of the GEMM route.
     chunked_max_rows: int = 16
     # Set by siblings.merge_gate_up: the rows are (8 gate, 8 up) blocks of a feed-forward block's two
     # input projections and forward returns silu(gate(x)) * up(x), of width out_features = rows / 2.

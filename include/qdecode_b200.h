@@ -9,6 +9,7 @@
  *   qdec_rmsnorm       residual update + RMS normalisation            (2 per layer + 1 final)
  *   qdec_rope_append   rotary embedding of q and k, k / v appended to the cache
  *   qdec_attention     one query token per sequence over the cache (grouped-query, split over the sequence)
+ *   qdec_rope_attention  the two above in one launch: what the decode step uses
  *   qdec_silu_mul      silu(gate) * up, where the two projections could not be fused into one GEMV
  *
  * Arithmetic follows what a 16-bit framework computes operator by operator: values are rounded to
