@@ -313,8 +313,10 @@ extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
 // padded to k_padded columns or not 16-byte aligned -- and leaves one to four aligned rows to the kernels above: those
 // launches last about as long as their code takes to arrive in the instruction caches (some 3.5 clocks per instruction on
 // a first pass), and the streaming kernel has more of it (4096 x 4096 INT4, M = 1: 10.8 against 7.1 us).  The exception are
-// rows so long that their activations leave the phased kernel at most half of its 16 warps, or do not fit beside it at all
-// (M = 4, K = 28672; the CUDA-core kernel took those): the streaming kernel cuts K between CTAs instead.
+// rows so long that their activations leave the phased kernel few of its 16 warps, or do not fit beside it at all (M = 4,
+// K = 28672; the CUDA-core kernel took those): the streaming kernel cuts K between CTAs instead.  With 4 warps left it wins
+// (14336 x 14336 INT4, M = 4: 44 against 65 us), with 8 it loses (4096 x 14336 INT4, M = 4: 24 against 18 us) unless there are
+// at most two rows, which it multiplies as integers (8192 x 28672 INT2, M = 2: 37 against 44 us).
 extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     const size_t need = qgemv_workspace_bytes(0, 0, 0, 0, 0, 0);
     const int v = validate(p, need, QGEMV_MAX_BATCH);
@@ -329,7 +331,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && padded) {
         bool none = false;
         const MmaPlan plan = choose(*p, kMaxPartialFloats, &none);
-        starved = !plan.ok || (plan.variant == 1 && plan.nw <= 8);
+        starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 ? 8 : 4));
     }
     if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8 || starved) &&
         plan_stream(&one, 1, kMaxPartialFloats, &q->plan))
