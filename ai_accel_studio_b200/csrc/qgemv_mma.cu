@@ -113,7 +113,9 @@ __device__ __forceinline__ void stage_activations(const MmaArgs& p, unsigned cha
     // What does not depend on x goes first.  Where the preceding launch is a small one (a norm, the attention), this CTA is
     // resident beside it, and its V row, column indices and ring of weights arrive while that launch still runs.  (x used to
     // be loaded first, lest its loads queue behind the weights'; a launch alone gained from the change as well: 896 x 128
-    // INT4, M = 1, 5.8 -> 5.3 us a call, 4096 x 11008, M = 4, 10.2 -> 9.9; a 24-layer decode step at 0.5B 1225 -> 1139.)
+    // INT4, M = 1, 5.8 -> 5.3 us a call, 4096 x 11008, M = 4, 10.2 -> 9.7; a 24-layer decode step at 0.5B 1225 -> 1139.)
+    // Half the ring, though: behind all of it x arrives late where whole-SM launches follow each other (the latter shape in
+    // a chain of itself: 10.84 us, with half 10.20; the 8B step of 16 layers 1313 against 1303).
     start_weights();
     QTRACE(10);
     wait_for_x();
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qgemv_mma_kernel(const __gr
     stage_activations<BITS, GB, M, BF16, EX>(p, smem,
         [&]() {
             first_prefetch();
-            for (int s = 1; s < GE::STAGES; ++s) issue_next(s);
+            for (int s = 1; s < GE::STAGES / 2; ++s) issue_next(s);
             QTRACE(1);
         },
         [&]() {
@@ -502,6 +504,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qgemv_mma_kernel(const __gr
             QTRACE(9);
             if (t_inline && (warp == 0 || t_reader)) t_tag = ld_relaxed_u32(a.counters + kWsEpochIdx) + 1u;
         });
+    for (int s = GE::STAGES / 2; s < GE::STAGES; ++s) issue_next(s);
     __syncthreads();                                  // staged activations visible to every warp
     QTRACE(2);
     if (has_job && warp == 0 && !(p.debug & QGEMV_DEBUG_DROP_PROJECTIONS)) {
