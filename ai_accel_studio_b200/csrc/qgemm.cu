@@ -11,17 +11,21 @@
 //              issue slots per scheduler of those (INT4 1.6, INT2 1.3 instructions per weight, from a byte permute of the
 //              four scaled levels), reading B takes 64 of shared memory's 128 bytes a clock.
 //   A in TMEM  keeps the converted weights out of shared memory, whose bandwidth B and the TMA writes need.
-//   extra K    outlier columns and the residual are further K columns: [ W | W_outlier | U ] . [ x | x_outlier | V x ]^T, so
-//              they cost no passes over y.  With bf16 activations U and V x go in as high and low halves (three products).
+//   terms      base, outlier columns and residual are three products, and the framework's expression rounds each of them to the
+//              activation type before it adds them.  So do the results here: this kernel stores the rounded base, and a third
+//              one (terms_kernel) adds the two small products to it.  As further K columns of one sum they cost next to nothing,
+//              but that is another number (512 rows, bf16: 3.4e-3 apart), and a decoder's layers make 1e-2 of it.
 //   split      units of 128 K columns are dealt out evenly over the SMs when whole tiles would leave more than that idle; the
 //              contributions of a tile then meet in scratch memory and whichever CTA comes last adds them in CTA order.
 //
 // A first small kernel lays x out for this: K columns permuted the way the codes leave a word, padded with zeros to
 // whole units, gathered outlier activations and the projections V x behind them.
 //
-// Weights are rounded exactly as qdequant rounds them; sums are fp32 and are rounded to the activation type once.
+// Weights are rounded exactly as qdequant rounds them; the sum of each term is fp32 and rounded to the activation type.
 // Replaces, for these shapes, dequantisation to a dense matrix + library GEMMs for base, outlier and residual term.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "qgemv_common.cuh"
 
@@ -42,16 +46,12 @@ struct GemmArgs {
     const uint8_t* packed;    long long ldp;
     const __half* scales;     long long lds;
     const __half* bias;
-    const __half* ow;         long long ldow;
-    const __half* ru;         long long ldu;
     void* y;                  long long ldy;
     float* partial;           // contributions of split tiles: [cta * 2 + piece][column][row]
     int* counters;            // arrivals per tile (zero between launches)
     int* status;
     int m, n, group, ng, pieces, act;         // pieces: 16-byte pieces of a packed row
-    int oc, oc8, rank, rank8, xcopies;        // padded to 8; xcopies: 1, or 3 with bf16 (high / low halves)
-    int ow_vec, ru_vec;                       // rows readable in 16-byte pieces
-    int wunits, units, chunks;                // weight units, all units and 64-column chunks of K
+    int units;                                // of 128 K columns
     int width, mtiles, ntiles;
     int sc_odd;                               // 1: the scales start on an odd 2-byte boundary
     int stages, ring;                         // stages of A and B (one barrier for both: a wait costs the mma warp 200 clocks); units of codes the ring holds (power of two)
@@ -266,51 +266,6 @@ __device__ __forceinline__ int first_unit(const GemmArgs& p, int cta, int grid) 
     return (int)(p.split ? cta * (tiles * p.units) / grid : cta * tiles / grid * p.units);
 }
 
-// Extra columns from k0 into an A stage: outlier weights, then U (with bf16 activations high, low and high halves), each
-// padded to 8 columns.  All loads of 64 columns are issued before the first is used.
-template <bool BF16>
-__device__ __noinline__ void extra_unit(const GemmArgs& p, int row, int k0, uint32_t at) {
-    const unsigned short* ow = reinterpret_cast<const unsigned short*>(p.ow) + (size_t)row * p.ldow;
-    const unsigned short* ru = reinterpret_cast<const unsigned short*>(p.ru) + (size_t)row * p.ldu;
-    for (int h = 0; h < 2; ++h) {
-        uint32_t out[32];
-        auto load8 = [&](const unsigned short* src, int left, bool vec, uint32_t* o) {
-            if (vec) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-                o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-            } else {
-                unsigned short v[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = i < left ? __ldg(src + i) : (unsigned short)0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) o[i] = v[2 * i] | (uint32_t)v[2 * i + 1] << 16;
-            }
-        };
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int j = k0 + h * kChunk + 8 * q, r = j - p.oc8;
-            out[4 * q] = out[4 * q + 1] = out[4 * q + 2] = out[4 * q + 3] = 0u;
-            if (j < p.oc) load8(ow + j, p.oc - j, p.ow_vec, out + 4 * q);
-            else if (p.rank > 0 && r >= 0 && r < p.rank8 * p.xcopies) load8(ru + r % p.rank8, p.rank - r % p.rank8, p.ru_vec, out + 4 * q);
-        }
-        if constexpr (BF16) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int r = k0 + h * kChunk + 8 * q - p.oc8;
-                const bool low = r >= p.rank8 && r < 2 * p.rank8;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&out[4 * q + i]));
-                    __nv_bfloat162 v = __floats2bfloat162_rn(f.x, f.y);
-                    if (low) v = __floats2bfloat162_rn(f.x - __low2float(v), f.y - __high2float(v));
-                    out[4 * q + i] = *reinterpret_cast<const uint32_t*>(&v);
-                }
-            }
-        }
-        tc_st32(at + h * 32, out);
-    }
-}
-
 struct Ends {                                          // what a warp needs to finish tiles
     uint32_t tmem, accfull, accempty, meeting, accph, meetph;
     int wg, quarter, lane, u0, grid, cta;
@@ -366,7 +321,7 @@ __device__ __noinline__ bool finish_tile(const GemmArgs& args, Ends& e, int tile
     e.accph ^= 1;
     tc_fence_after();
     const int nt = tile / p.mtiles, mt = tile - nt * p.mtiles, trow = e.quarter * 32 + e.lane, row = nt * kRows + trow;
-    const float b = p.bias ? __half2float(__ldg(p.bias + min(row, p.n - 1))) : 0.0f;
+    const float b = p.bias ? Act16<BF16>::to_float(Act16<BF16>::from_float(__half2float(__ldg(p.bias + min(row, p.n - 1))))) : 0.0f;
     const int c0 = e.wg * (p.width / 16) / kGroups * 16, c1 = (e.wg + 1) * (p.width / 16) / kGroups * 16;      // this warpgroup's columns
     const bool whole = unit + 1 == p.units && tile * p.units >= e.u0;
     // a CTA has at most two pieces of split tiles: the one at its first unit, and one at its last
@@ -473,10 +428,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             if (elect_one()) {
                 const int y = tile % p.mtiles * p.width;
                 const uint32_t dst = bbase + stage * 2 * bbytes;
-                const bool two = unit * 2 + 1 < p.chunks;
-                mbar_expect(full + 8 * stage, two ? 2 * bbytes : bbytes);
+                mbar_expect(full + 8 * stage, 2 * bbytes);
                 tma_load(dst, &xmap, unit * kUnit, y, full + 8 * stage);
-                if (two) tma_load(dst + bbytes, &xmap, unit * kUnit + kChunk, y, full + 8 * stage);
+                tma_load(dst + bbytes, &xmap, unit * kUnit + kChunk, y, full + 8 * stage);
             }
             __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -497,19 +451,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             }
             if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * stage, phase, gave_up, p.status))) break;
             tc_fence_after();
-            const bool two = unit * 2 + 1 < p.chunks, end = unit + 1 == p.units || u + 1 == u1;
+            const bool end = unit + 1 == p.units || u + 1 == u1;
             if (elect_one()) {
                 tc_mma(0, a, desc, idesc, add);
                 tc_mma(0, a + 8, desc + 2, idesc, 1);
                 tc_mma(0, a + 16, desc + 4, idesc, 1);
                 tc_mma(0, a + 24, desc + 6, idesc, 1);
-                if (two) {
-                    const uint64_t d2 = desc + (bbytes >> 4);
-                    tc_mma(0, a + 32, d2, idesc, 1);
-                    tc_mma(0, a + 40, d2 + 2, idesc, 1);
-                    tc_mma(0, a + 48, d2 + 4, idesc, 1);
-                    tc_mma(0, a + 56, d2 + 6, idesc, 1);
-                }
+                const uint64_t d2 = desc + (bbytes >> 4);
+                tc_mma(0, a + 32, d2, idesc, 1);
+                tc_mma(0, a + 40, d2 + 2, idesc, 1);
+                tc_mma(0, a + 48, d2 + 4, idesc, 1);
+                tc_mma(0, a + 56, d2 + 6, idesc, 1);
                 tc_commit(empty + 8 * stage);
                 if (end) tc_commit(accfull);
             }
@@ -535,7 +487,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
         const int ahead = p.ring / kGroups;                // 1, 2 or 4
         const uint32_t ring = bbase + p.stages * 2 * bbytes + wg * ahead * RawSlot<BITS, NG>::BYTES;
         auto request = [&]() {
-            if (fi < count && funit < p.wunits)
+            if (fi < count)
                 request_raw<BITS, NG>(p, ring + (fq & (ahead - 1)) * RawSlot<BITS, NG>::BYTES, quarter, lane, (ftile / p.mtiles) * kRows + quarter * 32, funit);
             asm volatile("cp.async.commit_group;" ::: "memory");
             ++fq;
@@ -563,27 +515,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             landed();
             // A parity cannot tell a release from the one two before it.  This warpgroup's last unit was G <= stages ago and waited
             // for a release no older than that, so the one before the awaited release has happened.
-            auto stage_free = [&]() {
-                ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase, gave_up, p.status));
-                tc_fence_after();
-                return ok;
-            };
-            if (unit < p.wunits) {
-                Raw<BITS> cur;
-                read_raw<BITS, NG>(p, ring + (q & (ahead - 1)) * RawSlot<BITS, NG>::BYTES, lrow, min((tile / p.mtiles) * kRows + lrow, p.n - 1), unit, cur);
-                __syncwarp();
-                request();
-                uint32_t lo[32], hi[32];               // converted before the stage is free: it is held for the store only
-                expand_half<BITS, NG, BF16>(cur, 0, lo);
-                expand_half<BITS, NG, BF16>(cur, 1, hi);
-                if (!stage_free()) break;
-                tc_st32(a_lane + stage * 64, lo);
-                tc_st32(a_lane + stage * 64 + 32, hi);
-            } else {
-                request();
-                if (!stage_free()) break;
-                extra_unit<BF16>(p, min((tile / p.mtiles) * kRows + lrow, p.n - 1), (unit - p.wunits) * kUnit, a_lane + stage * 64);
-            }
+            Raw<BITS> cur;
+            read_raw<BITS, NG>(p, ring + (q & (ahead - 1)) * RawSlot<BITS, NG>::BYTES, lrow, min((tile / p.mtiles) * kRows + lrow, p.n - 1), unit, cur);
+            __syncwarp();
+            request();
+            uint32_t lo[32], hi[32];                   // converted before the stage is free: it is held for the store only
+            expand_half<BITS, NG, BF16>(cur, 0, lo);
+            expand_half<BITS, NG, BF16>(cur, 1, hi);
+            ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * stage, phase, gave_up, p.status));
+            if (!ok) break;
+            tc_fence_after();
+            tc_st32(a_lane + stage * 64, lo);
+            tc_st32(a_lane + stage * 64 + 32, hi);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -612,7 +555,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------
-// x in the order the mma meets it: [M, chunks * 64], see the head of the file.  A CTA takes 8 activation rows and a share of
+// x in the order the mma meets it: [M, units * 128 + extra columns], see the head of the file.  A CTA takes 8 activation rows and a share of
 // K; a warp 64 columns at a time: lane (g, t) 16 columns of row g, which it permutes and stores, and which are its B
 // fragments for the projections (V rows as A; any order of K does, as long as both sides use it).  The last CTA of a row
 // group adds the K shares in order and writes the extra columns.  Bound by its traffic (x once in, once out); a version
@@ -629,7 +572,7 @@ struct PrepArgs {
     unsigned short* out;
     float* tparts;            // [share][row][rank]
     int* counters;            // per row group
-    int m, k, oc, oc8, rank, kw, ke, vec, vvec;
+    int m, k, oc, oc32, rank, kw, ke, vec, vvec;      // oc32: outlier columns padded to what terms_kernel takes at a time
 };
 constexpr int kPrepWarps = 8;
 
@@ -755,8 +698,8 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prepare_kernel(const __grid_c
     } else if (share != 0) {
         return;
     }
-    // the extra columns: outlier activations, projections (fp16; bf16: high, high, low), zeros
-    const int xc = BF16 ? 3 : 1, extra = p.ke - p.kw, rank8 = max(8, (p.rank + 7) & ~7);
+    // the extra columns: outlier activations and, in fp16 for either activation type, projections; zeros up to blocks of 32
+    const int extra = p.ke - p.kw;
     for (int i = tid; i < 8 * extra; i += kPrepWarps * 32) {
         const int r = i / extra, j = i - r * extra;
         if (m0 + r >= p.m) break;
@@ -764,21 +707,189 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prepare_kernel(const __grid_c
         if (j < p.oc) {
             const int col = __ldg(p.oidx + j);
             if (col >= 0 && col < p.k) v = p.x[(size_t)(m0 + r) * p.ldx + col];
-        } else if (j >= p.oc8 && j < p.oc8 + rank8 * xc && (j - p.oc8) % rank8 < p.rank) {
-            const int q = j - p.oc8, copy = q / rank8;
-            const float tv = ts[r][q - copy * rank8];
-            if constexpr (BF16) {
-                const __nv_bfloat16 hi = __float2bfloat16_rn(tv);
-                v = __bfloat16_as_ushort(copy == 2 ? __float2bfloat16_rn(tv - __bfloat162float(hi)) : hi);
-            } else {
-                v = __half_as_ushort(__float2half_rn(tv));
-            }
+        } else if (j >= p.oc32 && j < p.oc32 + p.rank) {
+            v = __half_as_ushort(__float2half_rn(ts[r][j - p.oc32]));
         }
         p.out[(size_t)(m0 + r) * p.ke + p.kw + j] = v;
     }
 }
 
-struct GemmPlan { GemmArgs a; int grid, smem, kw, ke, groups, shares; size_t x_bytes, t_bytes, scratch; };
+// ---------------------------------------------------------------------------------------------
+// y = act( r( r( base + r(x_o . W_o^T) ) + r(t . U^T) ) ), r: rounding to the activation type; base as gemm_kernel left it.  A warp
+// takes 16 activation rows x 32 weight rows, four mma.m16n8k16 side by side whose columns are dealt so that a lane of a quad holds
+// eight neighbours of y: 16-byte accesses, 64 bytes a row.  K comes 32 columns at a time, eight neighbours a lane (any order of K does,
+// as long as both operands use it), straight from memory.  Bound by latency and instructions around its traffic, y in and out.
+// Two terms take 28 of 117 us at 512 x 14336 (K 4096, bf16), 80 of 470 at 1000 x 28672 (K 8192, fp16), the projections V x included;
+// with 32 activation rows a warp (128 registers, two CTAs an SM) the same within 5 %, and 4 us more on 32 x 4096.
+// ---------------------------------------------------------------------------------------------
+struct TermArgs {
+    const unsigned short* x;                           // extra columns of the laid out x: [m][ke], outliers, then projections
+    const __half* ow;         long long ldow;
+    const __half* ru;         long long ldu;
+    const void* base;         long long ldb;           // y itself, or (gated pairs) a matrix in scratch
+    void* y;                  long long ldy;
+    int m, n, ke, oc, oc32, rank, act;
+    int ow_vec, ru_vec, vec;                           // rows accessible in 16-byte pieces
+};
+constexpr int kTermWarps = 8, kTermRows = 16, kTermTile = 32;
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    uint32_t r;
+    if constexpr (BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// A sum of two 16-bit values in 16-bit arithmetic: rounded once, as the sum in fp32 and its rounding are.
+template <bool BF16>
+__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (BF16) asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+template <bool BF16>
+__global__ void __launch_bounds__(kTermWarps * 32, 3) terms_kernel(const __grid_constant__ TermArgs p) {
+    using XT = typename Act16<BF16>::T;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int n0 = (blockIdx.x * kTermWarps + warp) * kTermTile;
+    if (n0 >= p.n) return;
+    const int nl = n0 + t * 8;                                                               // the lane's eight weight rows
+    int m0 = 0;
+    auto arow = [&](int i) { return m0 + i * 8 + g; };                                       // ... and its two activation rows
+    // acc[j]: columns c of mma j are weight rows n0 + (c / 2) * 8 + 2 j + c % 2
+    auto product = [&](const unsigned short* x, const __half* w, long long ldw, int cols, bool wide, auto type, float (&acc)[4][4]) {
+        constexpr bool kBf16 = decltype(type)::value;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
+        for (int k = t * 8; k - t * 8 < cols; k += 32) {
+            uint4 a[2], b[4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                a[i] = k < cols ? __ldg(reinterpret_cast<const uint4*>(x + (size_t)min(arow(i), p.m - 1) * p.ke + k)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int row = n0 + (g >> 1) * 8 + 2 * j + (g & 1);
+                const unsigned short* src = reinterpret_cast<const unsigned short*>(w) + (size_t)min(row, p.n - 1) * ldw + k;
+                if (k >= cols) {
+                    b[j] = make_uint4(0u, 0u, 0u, 0u);
+                } else if (wide && k + 8 <= cols) {
+                    b[j] = __ldg(reinterpret_cast<const uint4*>(src));
+                } else {
+                    uint32_t e[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t lo = k + 2 * q < cols ? __ldg(src + 2 * q) : 0, hi = k + 2 * q + 1 < cols ? __ldg(src + 2 * q + 1) : 0;
+                        e[q] = lo | hi << 16;
+                    }
+                    b[j] = make_uint4(e[0], e[1], e[2], e[3]);
+                }
+                if constexpr (kBf16) {
+                    uint32_t* e = reinterpret_cast<uint32_t*>(&b[j]);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(e + q));
+                        e[q] = pack2<true>(f.x, f.y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if constexpr (kBf16) {
+                    mma_bf16(acc[j], a[0].x, a[1].x, a[0].y, a[1].y, b[j].x, b[j].y);
+                    mma_bf16(acc[j], a[0].z, a[1].z, a[0].w, a[1].w, b[j].z, b[j].w);
+                } else {
+                    mma16816(acc[j], a[0].x, a[1].x, a[0].y, a[1].y, b[j].x, b[j].y);
+                    mma16816(acc[j], a[0].z, a[1].z, a[0].w, a[1].w, b[j].z, b[j].w);
+                }
+            }
+        }
+    };
+    for (int tile = blockIdx.y; tile * kTermRows < p.m; tile += gridDim.y) {
+        m0 = tile * kTermRows;
+        uint4 raw[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            raw[i] = make_uint4(0u, 0u, 0u, 0u);
+            const XT* src = static_cast<const XT*>(p.base) + (size_t)arow(i) * p.ldb + nl;
+            XT* e = reinterpret_cast<XT*>(&raw[i]);
+            if (arow(i) < p.m) {
+                if (p.vec && nl + 8 <= p.n) {
+                    raw[i] = *reinterpret_cast<const uint4*>(src);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) if (nl + q < p.n) e[q] = src[q];
+                }
+            }
+        }
+        float acc[4][4];
+        if (p.oc > 0) {
+            product(p.x, p.ow, p.ldow, p.oc, p.ow_vec, std::integral_constant<bool, BF16>{}, acc);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t& w = reinterpret_cast<uint32_t*>(&raw[i])[j];
+                    w = add2<BF16>(w, pack2<BF16>(acc[j][i * 2], acc[j][i * 2 + 1]));
+                }
+        }
+        if (p.rank > 0) {                              // an fp16 product for either activation type
+            product(p.x + p.oc32, p.ru, p.ldu, p.rank, p.ru_vec, std::false_type{}, acc);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t& w = reinterpret_cast<uint32_t*>(&raw[i])[j];
+                    uint32_t term = pack2<false>(acc[j][i * 2], acc[j][i * 2 + 1]);
+                    if constexpr (BF16) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&term));
+                        term = pack2<true>(f.x, f.y);
+                    }
+                    w = add2<BF16>(w, term);
+                }
+        }
+        XT* y = static_cast<XT*>(p.y);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint4 w = raw[i];
+            XT* e = reinterpret_cast<XT*>(&w);
+            int col = nl;
+            bool mine = arow(i) < p.m;
+            if (p.act == QGEMV_ACT_SILU_MUL) {         // lanes of even t hold eight gate rows, their neighbours the eight up rows
+                col = nl / 16 * 8;
+                mine = mine && !(t & 1) && nl < p.n;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float gate = Act16<BF16>::to_float(e[q]), up = __shfl_down_sync(0xffffffffu, gate, 1);
+                    e[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(Act16<BF16>::from_float(gate / (1.0f + __expf(-gate)))) * up);
+                }
+            } else if (p.act != QGEMV_ACT_NONE) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) e[q] = Act16<BF16>::from_float(apply_act(Act16<BF16>::to_float(e[q]), p.act));
+            }
+            if (!mine) continue;
+            XT* dst = y + (size_t)arow(i) * p.ldy + col;
+            const int left = p.act == QGEMV_ACT_SILU_MUL ? 8 : p.n - nl;
+            if (p.vec && left >= 8) {
+                *reinterpret_cast<uint4*>(dst) = w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) if (q < left) dst[q] = e[q];
+            }
+        }
+    }
+}
+
+struct GemmPlan { GemmArgs a; int grid, smem, kw, ke, oc32, groups, shares; bool terms; size_t x_bytes, t_bytes, b_bytes, scratch; };
 
 int sms() {
     static int cached[64] = {0};
@@ -802,24 +913,16 @@ bool plan_gemm(const qgemv_problem& p, GemmPlan& g) {
     if (!per || p.m < 1 || !al(p.packed, 16) || !al(p.scales, 2) || p.ldp % 16 || (long long)p.k_padded * p.bits / 8 % 16 || p.rank > kMaxRank || p.outliers > 4096) return false;
     GemmArgs& a = g.a;
     a = GemmArgs{};
-    const bool bf16 = p.x_dtype == QGEMV_BF16;
     a.packed = p.packed; a.ldp = p.ldp;
     a.scales = static_cast<const __half*>(p.scales); a.lds = p.lds;
     a.bias = static_cast<const __half*>(p.bias);
-    a.ow = static_cast<const __half*>(p.outlier_w); a.ldow = p.ldow;
-    a.ru = static_cast<const __half*>(p.res_u); a.ldu = p.ldu;
     a.y = p.y; a.ldy = p.ldy;
-    a.m = p.m; a.n = p.n; a.group = p.group; a.ng = p.k_padded / p.group; a.act = p.act;
+    g.terms = p.outliers > 0 || p.rank > 0;            // the base has the bias; the activation is left to whoever comes last
+    a.m = p.m; a.n = p.n; a.group = p.group; a.ng = p.k_padded / p.group; a.act = g.terms ? QGEMV_ACT_NONE : p.act;
     a.pieces = (int)((long long)p.k_padded * p.bits / 8 / 16);
-    a.oc = p.outliers; a.oc8 = (p.outliers + 7) / 8 * 8; a.rank = p.rank; a.xcopies = bf16 ? 3 : 1;
-    a.rank8 = (p.rank + 7) / 8 * 8;
-    a.ow_vec = p.outliers % 8 == 0 && al(p.outlier_w, 16) && p.ldow % 8 == 0;
-    a.ru_vec = p.rank % 8 == 0 && al(p.res_u, 16) && p.ldu % 8 == 0;
-    const int extra = (a.rank ? a.oc8 + a.rank8 * a.xcopies : a.oc);
-    a.wunits = (p.k_padded + kUnit - 1) / kUnit;
-    a.chunks = a.wunits * 2 + (extra + kChunk - 1) / kChunk;
-    a.units = (a.chunks + 1) / 2;
-    g.kw = a.wunits * kUnit; g.ke = a.chunks * kChunk;
+    a.units = (p.k_padded + kUnit - 1) / kUnit;
+    g.oc32 = (p.outliers + 31) / 32 * 32;
+    g.kw = a.units * kUnit; g.ke = g.kw + g.oc32 + (p.rank + 31) / 32 * 32;
     a.mtiles = (p.m + kMaxWidth - 1) / kMaxWidth;
     a.width = ((p.m + a.mtiles - 1) / a.mtiles + 15) / 16 * 16;
     a.ntiles = (p.n + kRows - 1) / kRows;
@@ -847,8 +950,10 @@ bool plan_gemm(const qgemv_problem& p, GemmPlan& g) {
     const int most = g.kw / 64 / (2 * kPrepWarps);
     g.shares = g.shares > most ? most : g.shares;
     g.shares = g.shares < 1 ? 1 : g.shares > 32 ? 32 : g.shares;
-    g.t_bytes = ((size_t)(g.shares > 1 ? g.shares : 0) * g.groups * a.rank * 8 * sizeof(float) + 255) / 256 * 256;
-    g.scratch = g.x_bytes + g.t_bytes + (a.split ? (size_t)g.grid * 2 * a.width * kRows * sizeof(float) : 0);
+    g.t_bytes = ((size_t)(g.shares > 1 ? g.shares : 0) * g.groups * p.rank * 8 * sizeof(float) + 255) / 256 * 256;
+    // gated pairs: y has half the base's width, which then needs a place of its own
+    g.b_bytes = g.terms && p.act == QGEMV_ACT_SILU_MUL ? ((size_t)p.m * p.n * 2 + 255) / 256 * 256 : 0;
+    g.scratch = g.x_bytes + g.t_bytes + g.b_bytes + (a.split ? (size_t)g.grid * 2 * a.width * kRows * sizeof(float) : 0);
     a.sc_odd = (int)(reinterpret_cast<uintptr_t>(p.scales) >> 1 & 1);
     // the ring of codes and the stages of x share what shared memory there is: a deep ring where tiles are narrow (a unit is
     // then short against HBM's latency), as many stages of x as fit beside a short one where they are wide
@@ -906,6 +1011,34 @@ int launch_gemm(const GemmPlan& g, const CUtensorMap& map, cudaStream_t s) {
     return check_launch("gemm_kernel");
 }
 
+template <bool BF16>
+int launch_terms(const qgemv_problem& p, const GemmPlan& g, const void* scratch, cudaStream_t s) {
+    auto al = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+    TermArgs a{};
+    a.x = static_cast<const unsigned short*>(scratch) + g.kw; a.ke = g.ke;
+    a.ow = static_cast<const __half*>(p.outlier_w); a.ldow = p.ldow;
+    a.ru = static_cast<const __half*>(p.res_u); a.ldu = p.ldu;
+    a.base = g.a.y; a.ldb = g.a.ldy;
+    a.y = p.y; a.ldy = p.ldy;
+    a.m = p.m; a.n = p.n; a.oc = p.outliers; a.oc32 = g.oc32; a.rank = p.rank; a.act = p.act;
+    a.ow_vec = p.outliers > 0 && al(p.outlier_w) && p.ldow % 8 == 0;
+    a.ru_vec = p.rank > 0 && al(p.res_u) && p.ldu % 8 == 0;
+    a.vec = al(a.base) && a.ldb % 8 == 0 && al(p.y) && p.ldy % 8 == 0;
+    // three CTAs fit an SM; up to two rounds of them, so that a CTA's weights serve several tiles of activation rows
+    const int cols = (p.n + kTermWarps * kTermTile - 1) / (kTermWarps * kTermTile), tiles = (p.m + kTermRows - 1) / kTermRows, fit = 6 * sms() / cols;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cols, fit < 1 ? 1 : fit < tiles ? fit : tiles);
+    cfg.blockDim = dim3(kTermWarps * 32);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, terms_kernel<BF16>, a);
+    return check_launch("terms_kernel");
+}
+
 template <int BITS, bool BF16>
 int launch_prepare(const qgemv_problem& p, const GemmPlan& g, void* scratch, cudaStream_t s) {
     auto al = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
@@ -916,7 +1049,7 @@ int launch_prepare(const qgemv_problem& p, const GemmPlan& g, void* scratch, cud
     a.out = static_cast<unsigned short*>(scratch);
     a.tparts = reinterpret_cast<float*>(static_cast<char*>(scratch) + g.x_bytes);
     a.counters = g.a.counters + kTileCounters;
-    a.m = p.m; a.k = p.k_original; a.oc = p.outliers; a.oc8 = g.a.oc8; a.rank = p.rank; a.kw = g.kw; a.ke = g.ke;
+    a.m = p.m; a.k = p.k_original; a.oc = p.outliers; a.oc32 = g.oc32; a.rank = p.rank; a.kw = g.kw; a.ke = g.ke;
     a.vec = al(p.x) && p.ldx % 8 == 0;
     a.vvec = p.rank > 0 && al(p.res_v) && p.ldv % 8 == 0;
     prepare_kernel<BITS, BF16><<<dim3(g.groups, g.shares), kPrepWarps * 32, 0, s>>>(a);
@@ -942,7 +1075,7 @@ int run_gemm(const qgemv_problem& p, void* scratch, size_t scratch_bytes, cudaSt
     EncodeFn enc = encoder();
     if (!enc) { set_error("qgemm_run: the driver has no cuTensorMapEncodeTiled"); return QGEMV_ERR_LAUNCH; }
     CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)g.ke, (cuuint64_t)p.m}, strides[1] = {(cuuint64_t)g.ke * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)g.kw, (cuuint64_t)p.m}, strides[1] = {(cuuint64_t)g.ke * 2};
     const cuuint32_t box[2] = {(cuuint32_t)kChunk, (cuuint32_t)g.a.width}, ones[2] = {1, 1};
     if (enc(&map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scratch, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
@@ -953,14 +1086,18 @@ int run_gemm(const qgemv_problem& p, void* scratch, size_t scratch_bytes, cudaSt
     int* cnt = reinterpret_cast<int*>(ws + kWsCounterOff);
     g.a.counters = cnt;
     g.a.status = cnt + kWsStatusIdx;
-    g.a.partial = reinterpret_cast<float*>(static_cast<char*>(scratch) + g.x_bytes + g.t_bytes);
+    char* const behind_x = static_cast<char*>(scratch) + g.x_bytes + g.t_bytes;
+    if (g.b_bytes) { g.a.y = behind_x; g.a.ldy = p.n; }
+    g.a.partial = reinterpret_cast<float*>(behind_x + g.b_bytes);
     int r = p.bits == 2 ? (bf16 ? launch_prepare<2, true>(p, g, scratch, s) : launch_prepare<2, false>(p, g, scratch, s))
                         : (bf16 ? launch_prepare<4, true>(p, g, scratch, s) : launch_prepare<4, false>(p, g, scratch, s));
     if (r != QGEMV_OK) return r;
     const int ng = p.group >= 128 ? 1 : p.group == 64 ? 2 : 4;
 #define QG(B, G) (bf16 ? launch_gemm<B, G, true>(g, map, s) : launch_gemm<B, G, false>(g, map, s))
-    if (p.bits == 2) return ng == 1 ? QG(2, 1) : QG(2, 2);
-    return ng == 1 ? QG(4, 1) : ng == 2 ? QG(4, 2) : QG(4, 4);
+    if (p.bits == 2) r = ng == 1 ? QG(2, 1) : QG(2, 2);
+    else r = ng == 1 ? QG(4, 1) : ng == 2 ? QG(4, 2) : QG(4, 4);
+    if (r != QGEMV_OK || !g.terms) return r;
+    return bf16 ? launch_terms<true>(p, g, scratch, s) : launch_terms<false>(p, g, scratch, s);
 #undef QG
 }
 

@@ -182,7 +182,8 @@ int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspac
 
 /* The same computation for any number of rows (prompts): one kernel lays x out, one dequantises the codes into tensor memory
  * and multiplies there; the dense matrix is never written.  Weights are rounded as qdequant rounds them to the activation
- * type, sums are fp32.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
+ * type; base (with the bias), outlier term and residual are fp32 sums, each rounded to the activation type (the residual, whose V x
+ * is rounded to fp16, to fp16 first) before they are added in this order, as the expression over a dense matrix does.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
  * private to the call until it completes (0: this shape is not built -- groups other than 32 (INT4), 64 and multiples of
  * 128, unaligned packed rows -- dequantise and use a library GEMM).  x needs only k_original columns.
  * Replaces the M > 4 route of ai_accel_lab/optimize/hybrid_int4.py:36-37 and hybrid_int2.py:102-106. */

@@ -56,6 +56,55 @@ def test_batch_against_float64(bits, rows, n, k, group, oc, rank, has_bias):
     assert ops.workspace_status("cuda") == 0
 
 
+ROUNDING_CASES = [
+    # bits, rows, n, k, group, outliers, rank, bias: every term alone and together, one block of columns and many
+    (4, 64, 256, 1024, 128, 0, 0, True),
+    (4, 130, 384, 1024, 128, 40, 0, False),
+    (2, 300, 300, 1000, 128, 0, 8, True),        # rows of y off 16-byte alignment, ragged last tile of weight rows
+    (2, 96, 1016, 2048, 64, 33, 9, True),        # outlier columns and ranks that fill no block
+    (4, 257, 640, 4096, 64, 130, 64, False),     # five blocks of outlier columns, largest rank
+    (4, 40, 256, 28672, 128, 1100, 8, True),     # tiles split over many CTAs, many outlier columns
+    (4, 512, 14336, 4096, 128, 40, 8, False),
+    (2, 700, 19200, 1024, 128, 16, 8, True),     # whole tiles, several per CTA
+]
+
+
+@pytest.mark.parametrize("bits,rows,n,k,group,oc,rank,has_bias", ROUNDING_CASES)
+def test_batch_rounds_as_the_expression_does(monkeypatch, bits, rows, n, k, group, oc, rank, has_bias):
+    """Base, outlier term and residual are rounded to the activation type one by one, then added, as in the expression over the
+    dequantised matrix (library GEMMs): what is left are sums of the same products in another order, which land on the other
+    side of a rounding boundary now and then."""
+    mod = _module(bits, n, k, group, oc, rank, has_bias, torch.Generator().manual_seed(n + k + rows))
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    for name in ("fp16", "bf16"):                # or the library adds pieces of K in 16 bits where it splits a product
+        monkeypatch.setattr(torch.backends.cuda.matmul, f"allow_{name}_reduced_precision_reduction", False)
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(rows, k, generator=gen, device="cuda").to(dtype)
+        y, want = mod(x), mod._dense(x)
+        # 32-bit sums in two orders are some 2^-20 of the result's size apart and the spacing of fp16 (bf16) is 2^-11 (2^-8) of
+        # it, so a rounding differs once in a few hundred (thousand); up to five roundings, and a result near zero is the small
+        # difference of larger ones, whose spacing is wider.  One rounding instead of one per term differs in a third of them.
+        moved = (y != want).float().mean()
+        assert float(moved) < 0.04, float(moved)
+        u = 2.0 ** (-11 if dtype == torch.float16 else -8)
+        assert float((y.double() - want.double()).norm() / want.double().norm()) < 0.3 * u
+    assert ops.workspace_status("cuda") == 0
+
+
+def test_batch_of_gated_pairs_round_as_the_expression_does(monkeypatch):
+    from ai_accel_studio_b200.optimize.siblings import merge_gate_up
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_fp16_reduced_precision_reduction", False)
+    torch.manual_seed(4)
+    gate, up = (HybridInt4Linear(torch.nn.Linear(1024, 1016), 128, None, 8) for _ in range(2))
+    for lin in (gate, up):
+        lin.set_residual(torch.randn(1016, 8) * 0.02, torch.randn(8, 1024) * 0.02)
+    fused = merge_gate_up(gate, up).cuda()
+    x = torch.randn(150, 1024).half().cuda()
+    y, want = fused(x), fused._dense(x)
+    assert float((y != want).float().mean()) < 0.04            # as above; the activation's own rounding is shared
+    assert float((y.double() - want.double()).norm() / want.double().norm()) < 0.5 * 2.0 ** -11
+
+
 def test_batch_of_gated_pairs_and_three_dimensions():
     from ai_accel_studio_b200.optimize.siblings import merge_gate_up
     torch.manual_seed(3)
