@@ -17,9 +17,9 @@ KERNEL = {"auto": 0, "simt": 1, "mma": 2, "mma_pipe": 3}
 DEBUG_DROP_PROJECTIONS, DEBUG_NO_L2_HINT = 1, 2
 MAX_M = 4
 MAX_BATCH = 16
-ABI_VERSION = 5
+ABI_VERSION = 6
 
-EXPORTS = ("qgemv_run", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_describe", "qgemv_workspace_status", "qgemv_workspace_bytes", "qgemv_plan_name", "qdequant", "qunpack_codes", "qgemv_pack",
+EXPORTS = ("qgemv_run", "qgemv_run_ordered", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_describe", "qgemv_workspace_status", "qgemv_workspace_bytes", "qgemv_plan_name", "qdequant", "qunpack_codes", "qgemv_pack",
            "qgemv_prepared_bytes", "qgemv_prepare", "qgemv_launch_prepared", "qgemv_batch_scratch_bytes", "qgemv_run_batch", "qgemv_error_string", "qgemv_abi_version", "qgemv_sizeof_problem",
            "qcomm_slot_bytes", "qcomm_flag_bytes", "qcomm_state_bytes", "qcomm_allreduce", "qcomm_allreduce_rmsnorm", "qcomm_status", "qcomm_alloc", "qcomm_free",
            "qcomm_ipc_export", "qcomm_ipc_open", "qcomm_ipc_close",
@@ -83,6 +83,8 @@ def lib():
     l = C.CDLL(str(LIB_PATH))
     l.qgemv_run.argtypes = [C.POINTER(Problem), C.c_void_p]
     l.qgemv_run.restype = C.c_int
+    l.qgemv_run_ordered.argtypes = [C.POINTER(Problem), C.c_void_p]
+    l.qgemv_run_ordered.restype = C.c_int
     l.qgemv_run_static.argtypes = [C.POINTER(Problem), C.c_void_p]
     l.qgemv_run_static.restype = C.c_int
     l.qgemv_workspace_bytes.argtypes = [C.c_int] * 6
@@ -165,8 +167,10 @@ def workspace_bytes(bits: int, m: int, n: int, k_padded: int, group: int, rank: 
     return int(lib().qgemv_workspace_bytes(bits, m, n, k_padded, group, rank))
 
 
-def run(problem: Problem, stream: int) -> None:
-    check(lib().qgemv_run(C.byref(problem), C.c_void_p(stream)))
+def run(problem: Problem, stream: int, ordered: bool) -> None:
+    """One launch; ``ordered``: work issued earlier on the stream may still be writing the weights."""
+    l = lib()
+    check((l.qgemv_run_ordered if ordered else l.qgemv_run)(C.byref(problem), C.c_void_p(stream)))
 
 
 def plan_launches(problem: Problem) -> int:

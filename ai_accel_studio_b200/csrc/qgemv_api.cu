@@ -153,8 +153,8 @@ extern "C" const char* qgemv_plan_name(const qgemv_problem* p) {
 namespace {
 
 // Validate, pick a kernel, launch.  `partial_floats` is the capacity of the partial-sum area of
-// the workspace the problem points at.
-int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t partial_floats) {
+// the workspace the problem points at; `ordered`: the launch must not overlap the work issued before it.
+int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t partial_floats, bool ordered) {
     const int v = validate(p, need_bytes);
     if (v != QGEMV_OK) return v;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -162,7 +162,8 @@ int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t 
     const bool bf16 = p->x_dtype == QGEMV_BF16;
 
     bool missing = false;
-    const MmaPlan plan = choose(*p, partial_floats, &missing);
+    MmaPlan plan = choose(*p, partial_floats, &missing);
+    plan.ordered = ordered;
     const bool use_mma = plan.ok;
     {
         if (missing) {
@@ -232,7 +233,7 @@ extern "C" int qgemv_run_static(const qgemv_problem* p, void* stream) {
     qgemv_problem q = *p;
     q.workspace = g_static_scratch_addr[dev];
     q.workspace_bytes = kStaticScratchBytes;
-    return run_checked(&q, stream, kStaticScratchBytes, kStaticPartialFloats);
+    return run_checked(&q, stream, kStaticScratchBytes, kStaticPartialFloats, false);
 }
 
 extern "C" int qgemv_plan_describe(const qgemv_problem* p, qgemv_plan_info* out) {
@@ -295,7 +296,11 @@ extern "C" int qgemv_workspace_status(const void* workspace, void* stream, int32
 }
 
 extern "C" int qgemv_run(const qgemv_problem* p, void* stream) {
-    return run_checked(p, stream, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), kMaxPartialFloats);
+    return run_checked(p, stream, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), kMaxPartialFloats, false);
+}
+
+extern "C" int qgemv_run_ordered(const qgemv_problem* p, void* stream) {
+    return run_checked(p, stream, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), kMaxPartialFloats, true);
 }
 
 // ---- prepared launches, up to 16 rows ------------------------------------------------------------------
@@ -361,7 +366,7 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
         p.m = q->problem.m - lo < QGEMV_MAX_M ? q->problem.m - lo : QGEMV_MAX_M;
         p.x = static_cast<const char*>(x) + (size_t)lo * p.ldx * 2;
         p.y = static_cast<char*>(y) + (size_t)lo * p.ldy * 2;
-        const int r = run_checked(&p, stream, 0, kMaxPartialFloats);
+        const int r = run_checked(&p, stream, 0, kMaxPartialFloats, ordered != 0);
         if (r != QGEMV_OK) return r;
     }
     return QGEMV_OK;

@@ -80,6 +80,7 @@ int launch_simt(const Args& a, int bits, bool bf16, int unit_bytes, cudaStream_t
 const char* simt_name(int bits, int m, int unit_bytes);
 
 struct MmaPlan {
+    bool ordered;           // the launch must not overlap the preceding kernel of the stream, which may be writing the weights
     bool ok;
     int gb;                 // packed bytes per group per row (16, 32 or 64)
     int nw, stages;         // warps per CTA, ring depth per warp

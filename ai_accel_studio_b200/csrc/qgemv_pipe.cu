@@ -760,7 +760,7 @@ int pipe_launch_ex(const MmaArgs& p, int grid, int smem_bytes, cudaStream_t s) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.wait_for_x == 2 ? 0 : 1;         // 2: weights, read before the wait, may not be final
     if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return check_launch("qgemv_pipe_kernel");
     return check_launch("qgemv_pipe_kernel");
 }
@@ -943,7 +943,7 @@ int launch_pipe(const Args& a, int bits, bool bf16, const MmaPlan& pl, int debug
     p.t_inline = pl.t_inline; p.t_parts = pl.t_parts; p.t_pv = pl.t_pv;
     p.l2_chunks = pl.l2_chunks;
     p.debug = debug;
-    p.wait_for_x = (a.rank > 0 && !pl.t_inline) ? 0 : 1;
+    p.wait_for_x = (a.rank > 0 && !pl.t_inline) ? 0 : pl.ordered ? 2 : 1;
     p.tile_aligned = 1;
     return bits == 2 ? launch_pipe_int2(p, pl.gb, pl.chunk, bf16, pl.grid, pl.smem_bytes, s)
                      : launch_pipe_int4(p, pl.gb, pl.chunk, bf16, pl.grid, pl.smem_bytes, s);

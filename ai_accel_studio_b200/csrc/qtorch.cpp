@@ -1,14 +1,17 @@
 // Host side of an eager packed-Linear call, in C++: what a module's forward does per call is an output allocation, the
 // current stream, a workspace look-up and one launch.  In Python that took 13 - 17 us, longer than the kernels.
 //
-// Two things live here: `Linear`, the prepared launches of one module (one per row count, up to 16 rows), and
-// `functional`, the prepared-problem cache of the decode_int*_linear functions.  The C ABI (include/qgemv_b200.h) does the
-// work; nothing here knows about kernels.
+// Three things live here: `Linear`, the prepared launches of one module (one per row count, up to 16 rows), `functional`,
+// the prepared-problem cache of the decode_int*_linear functions, and `settled`, the record of weights that launches have
+// already waited for.  The C ABI (include/qgemv_b200.h) does the work; nothing here knows about kernels.
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
+#include <iterator>
 #include <memory>
 #include <mutex>
 #include <optional>
@@ -77,24 +80,96 @@ void fill(qgemv_problem& p, int bits, int64_t k_original, int group, int act, in
     }
 }
 
+// ---- settled weights ------------------------------------------------------------------------------------
+
+// A launch may read weights before the preceding kernel of its stream has finished, unless that kernel may be what writes them.
+// Weights are settled once a launch that waited for everything before it has seen them: from then on the version counter that
+// their views share changes with every write that goes through the framework (a write through `.data` or a raw pointer leaves no
+// trace on the host).  Inference tensors have no counter and are never settled.
+// While a graph is captured nothing runs: what is recorded settles weights for launches recorded later (when the graph runs, all
+// that was issued before it has finished), not for eager ones.
+uint64_t g_failures = 0;                              // launches that were to wait and were not issued: nothing is settled any more
+struct Settled {
+    uint64_t version = ~0ull, failures = 0;
+    bool eager = false;
+    // Whether a launch has waited for this version; one has from now on (the caller's, which waits if this says no).
+    template <typename Capturing> bool pass(uint64_t now, Capturing capturing) {
+        const bool same = version == now && failures == g_failures;
+        if (same && eager) return true;
+        const bool cap = capturing(), was = same && cap;
+        version = now;
+        failures = g_failures;
+        eager = !cap;
+        return was;
+    }
+};
+bool capturing_now() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }      // current device's current stream
+
+// By storage.  The weak reference keeps the address of a freed storage from being given to another one, so a match of addresses
+// is the same storage.
+struct Seen {
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage{c10::intrusive_ptr<c10::StorageImpl>()};
+    Settled state;
+};
+std::unordered_map<const void*, Seen> g_seen;         // guarded by the GIL
+constexpr size_t kMaxSeen = 8192;
+size_t g_seen_sweep = 256;                            // entries of freed storages are dropped when this many are held
+
+bool settle(const at::Tensor& t) {
+    if (t.is_inference()) return false;
+    const c10::Storage& storage = t.storage();
+    const void* key = storage.unsafeGetStorageImpl();
+    auto it = g_seen.find(key);
+    if (it != g_seen.end()) return it->second.state.pass(t._version(), capturing_now);
+    if (g_seen.size() >= g_seen_sweep) {
+        for (auto i = g_seen.begin(); i != g_seen.end();) i = i->second.storage.expired() ? g_seen.erase(i) : std::next(i);
+        if (g_seen.size() >= kMaxSeen) g_seen.clear();
+        g_seen_sweep = std::min(kMaxSeen, std::max<size_t>(256, 2 * g_seen.size()));
+    }
+    return g_seen.emplace(key, Seen{storage.getWeakStorageImpl(), {}}).first->second.state.pass(t._version(), capturing_now);
+}
+
+// settled(tensor or None, ...): whether launches have waited for all of them; they count as settled from this call on
+PyObject* settled(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    bool all = true;
+    c10::cuda::OptionalCUDAGuard guard;
+    try {
+        for (Py_ssize_t i = 0; i < n; ++i) {
+            if (a[i] == Py_None) continue;
+            if (!THPVariable_Check(a[i])) { PyErr_SetString(PyExc_TypeError, "settled takes tensors"); return nullptr; }
+            const at::Tensor& t = THPVariable_Unpack(a[i]);
+            if (t.is_cuda() && c10::cuda::current_device() != t.get_device()) guard.set_index(t.get_device());
+            all = settle(t) && all;
+        }
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+    return PyBool_FromLong(all);
+}
+
+// forget(): a launch that was to wait was not issued
+PyObject* forget(PyObject*, PyObject*) { ++g_failures; Py_RETURN_NONE; }
+void check_launched(int rc) {
+    if (rc != QGEMV_OK) ++g_failures;
+    check(rc);
+}
+
 // ---- Linear ---------------------------------------------------------------------------------------------
 
 struct Linear {
-    std::vector<at::Tensor> keep;                     // every weight-side tensor: alive, and watched for in-place changes
+    std::vector<at::Tensor> keep;                     // every weight-side tensor
+    bool counted = true;                              // all of them have version counters
+    Settled settled;                                  // by the sum of the counters
     qgemv_problem base;
     int device;
     int64_t in_features, out_features, max_rows;
-    uint64_t version = ~0ull;
     struct Slot { std::vector<char> blob; bool usable = false; };
     std::unordered_map<int, Slot> slots;              // rows * 2 + bf16
 };
 
-// Sum of the version counters: changes when a weight was written in place (then its writer may still be running, and the
-// launch must not start reading weights early).
-uint64_t versions(const Linear& l) {
+bool settle(Linear& l) {
+    if (!l.counted) return false;
     uint64_t v = 0;
-    for (const auto& t : l.keep) v += t.is_inference() ? 0 : t._version();
-    return v;
+    for (const at::Tensor& t : l.keep) v += t._version();
+    return l.settled.pass(v, capturing_now);
 }
 
 struct LinearObject { PyObject_HEAD Linear* self; };
@@ -115,6 +190,7 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*) {
         fill(l->base, bits, korig, group, act, kernel, pk, sc, b, oi, w, u, v);
         l->keep = {pk, sc};
         for (const Opt* t : {&b, &oi, &w, &u, &v}) if (*t) l->keep.push_back(**t);
+        for (const at::Tensor& t : l->keep) l->counted = l->counted && !t.is_inference();
         l->device = pk.get_device();
     } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
     l->in_features = in; l->out_features = out; l->max_rows = max_rows;
@@ -176,11 +252,8 @@ PyObject* linear_call(LinearObject* o, PyObject* arg) {
             if (rc != QGEMV_OK && rc != QGEMV_ERR_ALIGN) check(rc);
         }
         if (!slot.usable) Py_RETURN_NONE;
-        const uint64_t v = versions(l);
-        const bool fresh = v != l.version;
         at::Tensor y = result();
-        check(qgemv_launch_prepared(slot.blob.data(), x.data_ptr(), y.data_ptr(), ws, fresh, stream));
-        l.version = v;
+        check_launched(qgemv_launch_prepared(slot.blob.data(), x.data_ptr(), y.data_ptr(), ws, !settle(l), stream));
         return THPVariable_Wrap(std::move(y));
     } catch (const PyError&) { return nullptr; }
     catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
@@ -191,13 +264,24 @@ PyObject* linear_tp_call(PyObject* self, PyObject* args, PyObject* kw) {
     return linear_call(reinterpret_cast<LinearObject*>(self), PyTuple_GET_ITEM(args, 0));
 }
 
-PyMethodDef linear_methods[] = {{"call", reinterpret_cast<PyCFunction>(linear_call), METH_O, "call(x) -> y, or None for the caller's general route"}, {nullptr, nullptr, 0, nullptr}};
+// settled(): as the function of this name, for the module's operands (a launch made without this object)
+PyObject* linear_settled(LinearObject* o, PyObject*) {
+    Linear& l = *o->self;
+    try {
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != l.device) guard.set_index(l.device);
+        return PyBool_FromLong(settle(l));
+    } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
+PyMethodDef linear_methods[] = {{"settled", reinterpret_cast<PyCFunction>(linear_settled), METH_NOARGS, "whether launches have waited for the operands as they are"},
+                                {"call", reinterpret_cast<PyCFunction>(linear_call), METH_O, "call(x) -> y, or None for the caller's general route"}, {nullptr, nullptr, 0, nullptr}};
 PyTypeObject LinearType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 // ---- functional -----------------------------------------------------------------------------------------
 
 // A problem is reused when addresses AND shapes of the operands of this call are the ones it was built from; the cache
-// holds no tensor alive.
+// holds no tensor alive.  Whether the operands are settled is asked apart from that: by their storages and versions.
 struct Key {
     uint64_t w[20];
     bool operator==(const Key& o) const { return std::equal(w, w + 20, o.w); }
@@ -210,7 +294,23 @@ struct KeyHash {
     }
 };
 constexpr size_t kMaxProblems = 256;
-std::unordered_map<Key, qgemv_problem, KeyHash> g_problems;      // guarded by the GIL
+struct Problem {
+    qgemv_problem p;
+    Seen seen[7];                                     // packed, scales, bias, oidx, ow, ru, rv
+    bool settle(PyObject* const* a) {
+        bool all = true;
+        for (int i = 0; i < 7; ++i) {
+            if (a[6 + i] == Py_None) continue;
+            const at::Tensor& t = THPVariable_Unpack(a[6 + i]);
+            if (t.is_inference()) { all = false; continue; }
+            const c10::Storage& storage = t.storage();
+            if (seen[i].storage._unsafe_get_target() != storage.unsafeGetStorageImpl()) seen[i] = Seen{storage.getWeakStorageImpl(), {}};
+            all = seen[i].state.pass(t._version(), capturing_now) && all;
+        }
+        return all;
+    }
+};
+std::unordered_map<Key, Problem, KeyHash> g_problems;      // guarded by the GIL
 
 // functional(bits, group, k_original, act, kernel, x, packed, scales, bias, oidx, ow, ru, rv) -> y, or None for the general route
 PyObject* functional(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -247,16 +347,17 @@ PyObject* functional(PyObject*, PyObject* const* a, Py_ssize_t n) {
         auto it = g_problems.find(key);
         if (it == g_problems.end()) {
             if (packed.get_device() != dev || scales.get_device() != dev || scales.size(0) != packed.size(0) || scales.size(1) * v[1] != x.size(1)) Py_RETURN_NONE;
-            qgemv_problem p;
+            Problem entry;
+            qgemv_problem& p = entry.p;
             const Opt oi = optional_tensor(a[9]), ow = optional_tensor(a[10]), ru = optional_tensor(a[11]), rv = optional_tensor(a[12]);
             if ((oi && oi->numel() && (!ow || ow->dim() != 2)) || (ru && ru->numel() && (ru->dim() != 2 || !rv || rv->dim() != 2))) Py_RETURN_NONE;
             fill(p, (int)v[0], v[2], (int)v[1], (int)v[3], (int)v[4], packed, scales, optional_tensor(a[8]), oi, ow, ru, rv);
             p.m = (int)x.size(0); p.x_dtype = dtype == at::kHalf ? QGEMV_F16 : QGEMV_BF16;
             p.ldx = x.stride(0); p.ldy = p.n;
             if (g_problems.size() >= kMaxProblems) g_problems.clear();
-            it = g_problems.emplace(key, p).first;
+            it = g_problems.emplace(key, std::move(entry)).first;
         }
-        qgemv_problem& p = it->second;
+        qgemv_problem& p = it->second.p;
         c10::cuda::OptionalCUDAGuard guard;
         if (c10::cuda::current_device() != dev) guard.set_index(dev);
         const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
@@ -264,7 +365,7 @@ PyObject* functional(PyObject*, PyObject* const* a, Py_ssize_t n) {
         void* ws = workspace(dev, stream, &ws_bytes);
         at::Tensor y = at::empty({x.size(0), p.n}, x.options());
         p.x = x.data_ptr(); p.y = y.data_ptr(); p.workspace = ws; p.workspace_bytes = ws_bytes;
-        check(qgemv_run(&p, stream));
+        check_launched((it->second.settle(a) ? qgemv_run : qgemv_run_ordered)(&p, stream));
         return THPVariable_Wrap(std::move(y));
     } catch (const PyError&) { return nullptr; }
     catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
@@ -281,6 +382,8 @@ PyObject* setup(PyObject*, PyObject* args) {
 
 PyMethodDef module_methods[] = {
     {"setup", setup, METH_VARARGS, "setup(ensure_workspace, error_class)"},
+    {"forget", forget, METH_NOARGS, "no weights are settled any more"},
+    {"settled", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(settled)), METH_FASTCALL, "whether launches have waited for these weights"},
     {"functional", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(functional)), METH_FASTCALL, "prepared-problem call of the decode_int*_linear functions"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", "Host side of eager packed-Linear calls", -1, module_methods, nullptr, nullptr, nullptr, nullptr};

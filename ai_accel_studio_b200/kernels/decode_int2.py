@@ -82,7 +82,7 @@ def _fused(bits, x, pw, bias, outlier_idx, outlier_weight, res_u, res_v, activat
             _CALLS.clear()
         call = _CALLS[key] = ops.prepare_call(x, pw.packed, pw.scales, b16, oi, ow, ru, rv, bits, pw.group_size,
                                               pw.original_k, act, _cabi.KERNEL[kernel], None, key)
-    return call.run(x)
+    return call.run(x, not ops.settled(pw.packed, pw.scales, b16, oi, ow, ru, rv))
 
 
 def decode_int2_linear(x: torch.Tensor, pw: GroupwiseInt2Weight, bias: torch.Tensor | None = None,

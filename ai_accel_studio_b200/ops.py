@@ -105,6 +105,22 @@ def native():
     return _NATIVE
 
 
+def settled(*weights) -> bool:
+    """Whether earlier launches have waited for these weights (tensors or None) as they are now.  If not, the launch that reads
+    them next must not overlap the work before it; they count as settled from this call on."""
+    return native().settled(*weights)
+
+
+def _launch(prob, weights) -> None:
+    """Issue the problem on the current stream, after everything before it where its weights are not settled; ``weights``: the
+    tensors, or the answer itself."""
+    try:
+        _cabi.run(prob, torch.cuda.current_stream().cuda_stream, not (weights if isinstance(weights, bool) else settled(*weights)))
+    except _cabi.QgemvError:
+        native().forget()
+        raise
+
+
 ACT_SILU_MUL = 3      # qgemv_act: rows are (8 gate, 8 up) blocks, the output is silu(gate) * up of width N / 2
 
 
@@ -190,7 +206,7 @@ def gemv_eager(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias
     prob = _problem(x, packed, scales, bias, outlier_idx, outlier_weight, res_u, res_v, y, ws,
                     bits, group, k_original, act, kernel, prefetch)
     with torch.cuda.device(x.device):
-        _cabi.run(prob, torch.cuda.current_stream().cuda_stream)
+        _launch(prob, (packed, scales, bias, outlier_idx, outlier_weight, res_u, res_v))
     return y
 
 
@@ -211,7 +227,8 @@ class CachedCall:
         self.key, self.problem, self.out_width, self.device_index = key, problem, out_width, device_index
         self.keep = None                      # tensors the struct points at, when the caller does not hold them itself
 
-    def run(self, x: torch.Tensor) -> torch.Tensor:
+    def run(self, x: torch.Tensor, ordered: bool) -> torch.Tensor:
+        """``ordered``: the weights may still be being written by work issued before (see ``settled``)."""
         import ctypes
         idx = self.device_index
         y = torch.empty((x.shape[0], self.out_width), dtype=x.dtype, device=x.device)
@@ -222,12 +239,14 @@ class CachedCall:
             ws = ensure_workspace(x.device, stream)
         p = self.problem
         p.x, p.y, p.workspace = x.data_ptr(), y.data_ptr(), ws.data_ptr()
+        launch = _cabi.lib().qgemv_run_ordered if ordered else _cabi.lib().qgemv_run
         if torch.cuda.current_device() == idx:
-            rc = _cabi.lib().qgemv_run(ctypes.byref(p), handle)
+            rc = launch(ctypes.byref(p), handle)
         else:
             with torch.cuda.device(idx):
-                rc = _cabi.lib().qgemv_run(ctypes.byref(p), handle)
+                rc = launch(ctypes.byref(p), handle)
         if rc != 0:
+            native().forget()
             _cabi.check(rc)
         return y
 
@@ -257,13 +276,13 @@ def gemv_into(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias:
               outlier_idx: Optional[torch.Tensor], outlier_weight: Optional[torch.Tensor],
               res_u: Optional[torch.Tensor], res_v: Optional[torch.Tensor],
               bits: int, group: int, k_original: int, act: int, kernel: int, out: torch.Tensor,
-              prefetch: Optional[torch.Tensor] = None) -> torch.Tensor:
+              prefetch: Optional[torch.Tensor] = None, weights_settled: Optional[bool] = None) -> torch.Tensor:
     """Same computation as ``gemv`` written into ``out`` ([M, N], x.dtype, unit inner stride).
 
     ``out`` is a CUDA tensor on x's device or a *pinned* host tensor: pinned memory is addressable by
     the device, so the kernel's stores then go straight to host memory and no separate device-to-host
     copy is needed (worth it for results this small; the host must still wait for the stream before it
-    reads them).  A plain function, not a registered op: it mutates its argument and is meant for
+    reads them).  ``weights_settled``: the caller's answer to ``settled`` where it has one.  A plain function, not a registered op: it mutates its argument and is meant for
     serving loops, eager or captured in a CUDA graph."""
     _check_gemv_inputs(x, packed, scales, bias, outlier_idx, outlier_weight, res_u, res_v, bits)
     if out.dtype != x.dtype or out.ndim != 2 or tuple(out.shape) != (x.shape[0], _out_width(packed, act)) or out.stride(1) != 1:
@@ -281,7 +300,7 @@ def gemv_into(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias:
     prob = _problem(x, packed, scales, bias, outlier_idx, outlier_weight, res_u, res_v, out, ws,
                     bits, group, k_original, act, kernel, prefetch)
     with torch.cuda.device(x.device):
-        _cabi.run(prob, torch.cuda.current_stream().cuda_stream)
+        _launch(prob, (packed, scales, bias, outlier_idx, outlier_weight, res_u, res_v) if weights_settled is None else weights_settled)
     return out
 
 

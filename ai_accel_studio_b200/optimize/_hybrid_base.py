@@ -158,6 +158,7 @@ class HybridPackedLinear(nn.Module):
         """Forget the prepared launches: they hold the operands' addresses and the settings they were built from."""
         self.__dict__.pop("_call", None)
         self.__dict__.pop("_native_call", None)
+        self.__dict__.pop("_native_state", None)
 
     def __setattr__(self, name, value):
         if name in HybridPackedLinear._LAUNCH_OPERANDS:
@@ -194,7 +195,7 @@ class HybridPackedLinear(nn.Module):
                                         self._kernel_code(), pre, sig)
                 call.keep = (self.packed, self.scales, self.bias, self.outlier_idx, self.outlier_weight, self.res_u, self.res_v, pre)
                 d["_call"] = call
-            return call.run(xp)
+            return call.run(xp, not self._weights_settled())
         return ops.gemv(xp, self.packed, self.scales, self.bias, self.outlier_idx if self.outlier_idx.numel() else None,
                         self.outlier_weight if self.outlier_idx.numel() else None,
                         self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None,
@@ -205,16 +206,23 @@ class HybridPackedLinear(nn.Module):
         general route (buffers on the CPU, an L2 hint).  Dropped whenever an operand or a setting changes."""
         d = self.__dict__
         packed = d["_buffers"]["packed"]
-        call = None
-        if packed.is_cuda and self.prefetch_next is None and self.bits in (2, 4):
+        state = None
+        if packed.is_cuda and self.bits in (2, 4):
             from .. import ops
             has_o = self.outlier_idx.numel() > 0
-            call = ops.native().Linear(self.bits, self.original_k, self.group_size, 3 if self.gated_pairs else 0, self._kernel_code(),
+            state = ops.native().Linear(self.bits, self.original_k, self.group_size, 3 if self.gated_pairs else 0, self._kernel_code(),
                                        self.in_features, self.out_features, min(self.chunked_max_rows, 16), packed, self.scales, self.bias,
                                        self.outlier_idx if has_o else None, self.outlier_weight if has_o else None,
                                        self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None)
-        d["_native_call"], d["_native_packed"] = call, packed
-        return call
+        d["_native_call"], d["_native_state"], d["_native_packed"] = state if self.prefetch_next is None else None, state, packed
+        return d["_native_call"]
+
+    def _weights_settled(self) -> bool:
+        """``ops.settled`` for this module's operands."""
+        d = self.__dict__
+        if d.get("_native_state") is None or d["_native_packed"] is not d["_buffers"]["packed"]:
+            self._prepare_native()
+        return d["_native_state"].settled()
 
     def _kernel_code(self) -> int:
         from .. import _cabi
@@ -236,7 +244,7 @@ class HybridPackedLinear(nn.Module):
         return ops.gemv_into(xp, self.packed, self.scales, self.bias, self.outlier_idx if has_o else None,
                              self.outlier_weight if has_o else None,
                              self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None,
-                             self.bits, self.group_size, self.original_k, 3 if self.gated_pairs else 0, self._kernel_code(), out, self.prefetch_next)
+                             self.bits, self.group_size, self.original_k, 3 if self.gated_pairs else 0, self._kernel_code(), out, self.prefetch_next, self._weights_settled())
 
     def _dense(self, xflat: torch.Tensor) -> torch.Tensor:
         from .. import ops
@@ -303,5 +311,5 @@ class HybridPackedLinear(nn.Module):
             ops.gemv_into(xp[lo:lo + 4], self.packed, self.scales, self.bias, self.outlier_idx if has_o else None,
                           self.outlier_weight if has_o else None,
                           self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None,
-                          self.bits, self.group_size, self.original_k, act, self._kernel_code(), y[lo:lo + 4], self.prefetch_next)
+                          self.bits, self.group_size, self.original_k, act, self._kernel_code(), y[lo:lo + 4], self.prefetch_next, self._weights_settled())
         return y

@@ -19,7 +19,7 @@
 extern "C" {
 #endif
 
-#define QGEMV_ABI_VERSION 5
+#define QGEMV_ABI_VERSION 6
 
 enum qgemv_status {
     QGEMV_OK = 0,
@@ -90,7 +90,8 @@ enum qgemv_kernel { QGEMV_KERNEL_AUTO = 0, QGEMV_KERNEL_SIMT = 1, QGEMV_KERNEL_M
  *   y          fp16 or bf16 (same type as x) [M, N]
  *   The weight-side tensors (packed, scales, bias, outlier_*, res_*) must already be final when
  *   the call is issued: the kernel may start reading them before the preceding kernel of the
- *   stream has finished (it waits for that kernel only before it reads x).
+ *   stream has finished (it waits for that kernel only before it reads x).  Where work issued earlier
+ *   on the stream may still be writing them, call qgemv_run_ordered.
  *   workspace  zero-initialised ONCE by the caller, at least qgemv_workspace_bytes() bytes,
  *              256-byte aligned, private to calls that may overlap on the device (calls on
  *              different streams without ordering need a workspace each).  The kernels leave it
@@ -138,6 +139,10 @@ typedef struct qgemv_problem {
  *           (packed_dense_kernel<0>, csrc/packed_kernels_cuda.cu:27-83). */
 int qgemv_run(const qgemv_problem* p, void* stream);
 
+/* The same launch, started only when everything issued earlier on the stream has finished: for weight-side tensors that
+ * this work may still be writing. */
+int qgemv_run_ordered(const qgemv_problem* p, void* stream);
+
 /* The same fused GEMV for callers that may not allocate device memory (code running under a
  * memory budget fixed at start-up, inside somebody else's allocator-free plugin hook, or in a
  * process whose only device buffers are the ones handed to it): p->workspace and
@@ -174,7 +179,8 @@ int qgemv_workspace_status(const void* workspace, void* stream, int32_t* host_ou
  * change from call to call (same shape, strides and alignment), and so may the workspace.  x needs only k_original columns
  * (ldx >= k_original) except for the CUDA-core kernel, which qgemv_prepare reports with QGEMV_ERR_ALIGN (pad x, and pass
  * k_original = k_padded with res_v padded likewise, or use qgemv_run).  `ordered` != 0: the
- * preceding kernel of the stream may still be writing the weights, so the launch does not overlap it.  One buffer must not be
+ * preceding kernel of the stream may still be writing the weights, so the launch does not overlap it, whichever kernel was
+ * planned.  One buffer must not be
  * launched from two threads at a time. */
 size_t qgemv_prepared_bytes(void);
 int qgemv_prepare(const qgemv_problem* p, void* prepared);

@@ -94,3 +94,71 @@ def test_kernels_of_one_workspace_keep_their_projections_apart():
                 assert float((y.float() - want).norm() / want.norm()) < 2e-3
     s.synchronize()
     assert ops.workspace_status("cuda", s) == 0
+
+
+def _overlapping_launches(call):
+    """Edges of a graph captured from ``call`` that let a kernel start before its predecessor has finished."""
+    import ctypes
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    rt, raw, n = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert rt.cudaGraphGetEdges_v2(raw, None, None, None, ctypes.byref(n)) == 0
+    ends, data = ((ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)()), (ctypes.c_uint8 * (8 * n.value))()
+    assert rt.cudaGraphGetEdges_v2(raw, ends[0], ends[1], data, ctypes.byref(n)) == 0
+    return sum(data[8 * i + 2] == 1 for i in range(n.value))           # cudaGraphEdgeData.type: cudaGraphDependencyTypeProgrammatic
+
+
+@pytest.mark.parametrize("rows", [1, 4, 8])
+def test_launches_overlap_their_predecessor_only_over_settled_weights(rows):
+    """What may still be being written must not be read ahead of the dependency wait: the first launch over weights that are
+    new, or were written in place, starts after its predecessor; the next one may overlap it."""
+    torch.manual_seed(5)
+    mod = HybridInt4Linear(torch.nn.Linear(1024, 512), 128, None, 8).cuda()
+    x = torch.randn(rows, 1024).half().cuda()
+    out = torch.empty(rows, 512, dtype=torch.float16, device="cuda")
+    into = rows <= 4
+
+    def calls(write):
+        x.mul_(1)                                                      # the predecessor of the first launch
+        if write:
+            mod.scales.mul_(1)
+        mod(x)
+        mod(x)
+
+    mod(x)
+    assert _overlapping_launches(lambda: calls(False)) == 2
+    assert _overlapping_launches(lambda: calls(True)) == 1
+    if into:
+        def calls_into():
+            mod.scales.mul_(1)
+            mod.forward_into(x, out)
+            mod.forward_into(x, out)
+        assert _overlapping_launches(calls_into) == 1
+    # a batch beyond 16 rows: its layout kernel starts in stream order, the two behind it overlap only their predecessors
+    xl = torch.randn(64, 1024).half().cuda()
+
+    def batch():
+        mod.scales.mul_(1)
+        mod(xl)
+    assert _overlapping_launches(batch) == 2
+
+
+def test_functional_launch_right_after_packing_does_not_overlap_it():
+    from ai_accel_studio_b200.kernels.decode_int2 import decode_int2_linear
+    w = torch.randn(512, 1024, device="cuda").half()
+    x = torch.randn(2, 1024, device="cuda").half()
+    keep = []
+
+    def pack_and_call(again):
+        pw = pack_groupwise_int2(w, 128)
+        keep.append(pw)
+        for _ in range(1 + again):
+            decode_int2_linear(x, pw)
+
+    pack_and_call(0)
+    torch.cuda.synchronize()
+    keep.clear()                                                       # the next tensors may get the same addresses
+    assert _overlapping_launches(lambda: pack_and_call(0)) == 0
+    assert _overlapping_launches(lambda: pack_and_call(1)) == 1
