@@ -154,21 +154,72 @@ void check_launched(int rc) {
 
 // ---- Linear ---------------------------------------------------------------------------------------------
 
+enum Operand { kPacked, kScales, kBias, kOutlierIdx, kOutlierW, kResU, kResV, kOperands };
+
 struct Linear {
-    std::vector<at::Tensor> keep;                     // every weight-side tensor
+    Opt operand[kOperands];                           // kept alive
+    const void* address[kOperands] = {};              // where they were when `base` was filled
+    bool valid = false;                               // `base` is filled: types, strides, shapes and devices are the kernels'
     bool counted = true;                              // all of them have version counters
     Settled settled;                                  // by the sum of the counters
     qgemv_problem base;
-    int device;
-    int64_t in_features, out_features, max_rows;
+    int bits, group, act, kernel, device = -1;
+    int64_t k_original, in_features, out_features, max_rows;
     struct Slot { std::vector<char> blob; bool usable = false; };
     std::unordered_map<int, Slot> slots;              // rows * 2 + bf16
 };
 
+// The kernels read raw memory: a module whose buffers were cast (`module.to(torch.bfloat16)`), or that was put together from
+// something else, must not get here.  Its calls take the general route, which says what is wrong.
+bool fits(const Linear& l) {
+    const Opt* o = l.operand;
+    auto matrix = [&](const Opt& t, at::ScalarType type, int64_t rows, int64_t cols) {
+        return t && t->dim() == 2 && t->scalar_type() == type && t->is_cuda() && t->get_device() == o[kPacked]->get_device() && t->size(0) == rows &&
+               t->size(1) >= cols && (t->size(1) == 1 || t->stride(1) == 1);
+    };
+    auto vector = [&](const Opt& t, at::ScalarType type, int64_t n) {
+        return t && t->dim() == 1 && t->scalar_type() == type && t->is_cuda() && t->get_device() == o[kPacked]->get_device() && t->size(0) == n && (n < 2 || t->stride(0) == 1);
+    };
+    if (!o[kPacked] || !o[kPacked]->is_cuda() || o[kPacked]->dim() != 2 || l.group < 1) return false;
+    const int64_t n = o[kPacked]->size(0), kpad = o[kPacked]->size(1) * (8 / l.bits);
+    if (!matrix(o[kPacked], at::kByte, n, 1) || !matrix(o[kScales], at::kHalf, n, (kpad + l.group - 1) / l.group)) return false;
+    if (o[kBias] && !vector(o[kBias], at::kHalf, n)) return false;
+    if (o[kOutlierIdx]) {
+        const int64_t oc = o[kOutlierIdx]->numel();
+        if (!vector(o[kOutlierIdx], at::kInt, oc) || !matrix(o[kOutlierW], at::kHalf, n, oc)) return false;
+    }
+    if (o[kResU] || o[kResV])
+        return o[kResU] && o[kResV] && o[kResU]->dim() == 2 && matrix(o[kResU], at::kHalf, n, 1) && matrix(o[kResV], at::kHalf, o[kResU]->size(1), l.k_original);
+    return true;
+}
+
+// Fills `base` from the operands as they are now; what was prepared from earlier addresses goes.
+void bind(Linear& l) {
+    l.slots.clear();
+    l.settled = {};
+    l.counted = true;
+    for (int i = 0; i < kOperands; ++i) {
+        l.address[i] = l.operand[i] ? l.operand[i]->const_data_ptr() : nullptr;
+        l.counted = l.counted && !(l.operand[i] && l.operand[i]->is_inference());
+    }
+    l.valid = fits(l);
+    if (!l.valid) return;
+    l.device = l.operand[kPacked]->get_device();
+    fill(l.base, l.bits, l.k_original, l.group, l.act, l.kernel, *l.operand[kPacked], *l.operand[kScales], l.operand[kBias], l.operand[kOutlierIdx], l.operand[kOutlierW],
+         l.operand[kResU], l.operand[kResV]);
+}
+
+// Whether `base` may be used; operands that were given other memory (`module.scales.data = ...`) are taken up.
+bool bound(Linear& l) {
+    for (int i = 0; i < kOperands; ++i)
+        if (l.operand[i] && l.operand[i]->const_data_ptr() != l.address[i]) { bind(l); break; }
+    return l.valid;
+}
+
 bool settle(Linear& l) {
     if (!l.counted) return false;
     uint64_t v = 0;
-    for (const at::Tensor& t : l.keep) v += t._version();
+    for (const Opt& t : l.operand) if (t) v += t->_version();
     return l.settled.pass(v, capturing_now);
 }
 
@@ -183,15 +234,13 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*) {
     PyObject *packed, *scales, *bias, *oidx, *ow, *ru, *rv;
     if (!PyArg_ParseTuple(args, "iLiiiLLLOOOOOOO", &bits, &korig, &group, &act, &kernel, &in, &out, &max_rows, &packed, &scales, &bias, &oidx, &ow, &ru, &rv))
         return nullptr;
+    if (bits != 2 && bits != 4) { PyErr_SetString(PyExc_ValueError, "bits must be 2 or 4"); return nullptr; }
     auto l = std::make_unique<Linear>();
+    l->bits = bits; l->k_original = korig; l->group = group; l->act = act; l->kernel = kernel;
     try {
-        const at::Tensor pk = THPVariable_Unpack(packed), sc = THPVariable_Unpack(scales);
-        const Opt b = optional_tensor(bias), oi = optional_tensor(oidx), w = optional_tensor(ow), u = optional_tensor(ru), v = optional_tensor(rv);
-        fill(l->base, bits, korig, group, act, kernel, pk, sc, b, oi, w, u, v);
-        l->keep = {pk, sc};
-        for (const Opt* t : {&b, &oi, &w, &u, &v}) if (*t) l->keep.push_back(**t);
-        for (const at::Tensor& t : l->keep) l->counted = l->counted && !t.is_inference();
-        l->device = pk.get_device();
+        PyObject* const given[kOperands] = {packed, scales, bias, oidx, ow, ru, rv};
+        for (int i = 0; i < kOperands; ++i) l->operand[i] = optional_tensor(given[i]);
+        bind(*l);
     } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
     l->in_features = in; l->out_features = out; l->max_rows = max_rows;
     auto* o = reinterpret_cast<LinearObject*>(type->tp_alloc(type, 0));
@@ -199,12 +248,14 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*) {
     return reinterpret_cast<PyObject*>(o);
 }
 
-// call(x): the result, or None where the caller has to take its general route (shape, type, device, layout).
+// call(x): the result, or None where the caller has to take its general route (shape, type, device, layout; operands that are
+// not the kernels').
 PyObject* linear_call(LinearObject* o, PyObject* arg) {
     Linear& l = *o->self;
     if (!THPVariable_CheckExact(arg)) Py_RETURN_NONE;
     try {
         const at::Tensor& x = THPVariable_Unpack(arg);
+        if (!bound(l)) Py_RETURN_NONE;
         const int64_t dims = x.dim();
         const auto dtype = x.scalar_type();
         if (dims < 1 || !x.is_cuda() || x.get_device() != l.device || x.size(-1) != l.in_features || !x.is_contiguous() ||
@@ -269,6 +320,7 @@ PyObject* linear_settled(LinearObject* o, PyObject*) {
     Linear& l = *o->self;
     try {
         c10::cuda::OptionalCUDAGuard guard;
+        if (!bound(l)) Py_RETURN_FALSE;
         if (c10::cuda::current_device() != l.device) guard.set_index(l.device);
         return PyBool_FromLong(settle(l));
     } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }

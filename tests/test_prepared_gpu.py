@@ -162,3 +162,38 @@ def test_functional_launch_right_after_packing_does_not_overlap_it():
     keep.clear()                                                       # the next tensors may get the same addresses
     assert _overlapping_launches(lambda: pack_and_call(0)) == 0
     assert _overlapping_launches(lambda: pack_and_call(1)) == 1
+
+
+@pytest.mark.parametrize("rows", [1, 4, 8, 64])
+def test_operands_of_other_types_are_refused(rows):
+    """A cast of the whole model reaches the buffers of packed modules; their bits must not be read as fp16."""
+    for cast in (lambda m: m.to(torch.bfloat16), lambda m: m.float()):
+        mod = HybridInt4Linear(torch.nn.Linear(512, 256), 128, None, 8).cuda()
+        x = torch.randn(rows, 512).half().cuda()
+        want = mod(x)
+        cast(mod)
+        with pytest.raises(RuntimeError, match="float16"):
+            mod(x)
+        if rows <= 4:
+            with pytest.raises(RuntimeError, match="float16"):
+                mod.forward_into(x, torch.empty(rows, 256, dtype=torch.float16, device="cuda"))
+        mod.half()
+        assert mod(x).shape == want.shape
+    bias = HybridInt4Linear(torch.nn.Linear(512, 256), 128).cuda()
+    bias.bias = bias.bias.float()                                       # one operand: refused by the fused kernels, cast by the expression
+    if rows <= 16:
+        with pytest.raises(RuntimeError, match="bias"):
+            bias(x)
+    else:
+        assert bias(x).dtype == torch.float16
+
+
+@pytest.mark.parametrize("rows", [1, 8, 64])
+def test_operands_given_other_memory_are_taken_up(rows):
+    torch.manual_seed(6)
+    mod = HybridInt4Linear(torch.nn.Linear(512, 256, bias=False), 128).cuda()
+    x = torch.randn(rows, 512).half().cuda()
+    want = mod(x)
+    mod.scales.data = mod.scales.data * 2
+    # a power of two is exact but for results among fp16's subnormals, which are 2^-24 apart
+    assert float((mod(x).float() - 2 * want.float()).abs().max()) <= 2.0 ** -23
