@@ -6,9 +6,11 @@
 // already waited for.  The C ABI (include/qgemv_b200.h) does the work; nothing here knows about kernels.
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 
 #include <algorithm>
 #include <iterator>
@@ -248,6 +250,23 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*) {
     return reinterpret_cast<PyObject*>(o);
 }
 
+// Whether something other than the plain forward pass wants to see the operators of this call: a transform (vmap, jvp, grad), a
+// tracer, a dispatch mode, a batched or functional wrapper of x.
+bool observed(const at::Tensor& x) {
+    constexpr c10::DispatchKeySet watching({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::PythonDispatcher, c10::DispatchKey::Functionalize,
+                                            c10::DispatchKey::Tracer, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::FuncTorchVmapMode,
+                                            c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchDynamicLayerBackMode});
+    return !((x.key_set() | c10::impl::tls_local_dispatch_key_set().included_) & watching).empty();
+}
+
+// Beyond the rows of the fused GEMV a module is an expression of differentiable operators; the fused GEMM stands for it only where
+// nobody asks for derivatives, or through autocast for other types (the residual's products are fp16 ones).
+bool plain_forward(const Linear& l, const at::Tensor& x) {
+    if ((at::GradMode::is_enabled() && x.requires_grad()) || x._fw_grad(/*level=*/0).defined()) return false;
+    return !at::autocast::is_autocast_enabled(at::kCUDA) ||
+           (at::autocast::get_autocast_dtype(at::kCUDA) == x.scalar_type() && (x.scalar_type() == at::kHalf || !l.operand[kResU]));
+}
+
 // call(x): the result, or None where the caller has to take its general route (shape, type, device, layout; operands that are
 // not the kernels').
 PyObject* linear_call(LinearObject* o, PyObject* arg) {
@@ -255,7 +274,7 @@ PyObject* linear_call(LinearObject* o, PyObject* arg) {
     if (!THPVariable_CheckExact(arg)) Py_RETURN_NONE;
     try {
         const at::Tensor& x = THPVariable_Unpack(arg);
-        if (!bound(l)) Py_RETURN_NONE;
+        if (observed(x) || !bound(l)) Py_RETURN_NONE;
         const int64_t dims = x.dim();
         const auto dtype = x.scalar_type();
         if (dims < 1 || !x.is_cuda() || x.get_device() != l.device || x.size(-1) != l.in_features || !x.is_contiguous() ||
@@ -263,6 +282,7 @@ PyObject* linear_call(LinearObject* o, PyObject* arg) {
             Py_RETURN_NONE;
         const int64_t rows = x.numel() / l.in_features;
         const bool batch = rows > l.max_rows;
+        if (batch && !plain_forward(l, x)) Py_RETURN_NONE;
         if (rows < 1 || rows > (1 << 24) || (!batch && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16)) Py_RETURN_NONE;
         c10::cuda::OptionalCUDAGuard guard;
         if (c10::cuda::current_device() != l.device) guard.set_index(l.device);

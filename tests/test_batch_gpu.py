@@ -117,3 +117,36 @@ def test_batch_of_gated_pairs_and_three_dimensions():
     sep = torch.nn.functional.silu(gate(x)) * up(x)
     assert y.shape == (3, 50, 1016)
     assert float((y.float() - sep.float()).abs().max()) <= 2e-3 * float(sep.float().abs().max()) + 1e-3
+
+
+@pytest.mark.parametrize("bits,oc,rank", [(4, 0, 0), (2, 16, 8)])
+def test_prompts_are_differentiable_and_transformable_in_x(bits, oc, rank):
+    """Beyond the rows of the fused GEMV a module is an expression of framework operators in x: gradients, forward-mode
+    derivatives, vmap and autocast see it as one."""
+    mod = _module(bits, 256, 512, 128, oc, rank, True, torch.Generator().manual_seed(11))
+    w = mod.effective_weight().double()
+    x = torch.randn(32, 512, device="cuda").half()
+    tangent = torch.randn(32, 512, device="cuda").half()
+    u = 2.0 ** -11
+
+    def near(got, want, at):                                   # weights, and each of up to five operators' results, rounded
+        return float((got.double() - want).norm() / want.norm()) <= at * u
+
+    leaf = x.clone().requires_grad_()
+    y = mod(leaf)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    assert near(leaf.grad, dy.double() @ w, 4)
+    with torch.no_grad():
+        assert not mod(leaf).requires_grad
+    _, jvp = torch.func.jvp(mod, (x,), (tangent,))
+    assert near(jvp, tangent.double() @ w.t(), 4)
+    stacked = torch.stack([x, tangent])
+    got = torch.func.vmap(mod)(stacked)
+    assert got.shape == (2, 32, 256) and near(got, stacked.double() @ w.t() + mod.bias.double(), 4)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert mod(x).dtype == torch.nn.functional.linear(x, w.half()).dtype == torch.bfloat16
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert torch.equal(mod(x), got[0]) or near(mod(x), got[0].double(), 4)
+    traced = torch.jit.trace(mod, x, check_trace=False)
+    assert near(traced(tangent), tangent.double() @ w.t() + mod.bias.double(), 4)
