@@ -347,7 +347,6 @@ def _(packed, bits):
 
 
 PACK_GROUPS = (16, 32, 64, 128, 256, 512)
-_FACTORS: dict = {}          # (device, first, last, steps) -> candidate factors of the scale search
 
 
 def pack(weight: torch.Tensor, bits: int, group: int, activation_rms, first: float, last: float, steps: int):
@@ -358,14 +357,9 @@ def pack(weight: torch.Tensor, bits: int, group: int, activation_rms, first: flo
     ng = -(-k // group)
     packed = torch.empty((n, ng * group * bits // 8), dtype=torch.uint8, device=w.device)
     scales = torch.empty((n, ng), dtype=torch.float16, device=w.device)
-    factors = None
-    if activation_rms is not None:
-        key = (w.device, first, last, steps)
-        factors = _FACTORS.get(key)
-        if factors is None:
-            factors = torch.linspace(first, last, steps, device=w.device)
-            if len(_FACTORS) < 64:
-                _FACTORS[key] = factors
+    # made on the stream that reads them: a copy kept between calls may not be written yet for another stream, or for the eager
+    # call after a captured one
+    factors = None if activation_rms is None else torch.linspace(first, last, steps, device=w.device)
     with torch.cuda.device(w.device):
         _cabi.check(_cabi.lib().qgemv_pack(bits, w.data_ptr(), w.stride(0), _DT[w.dtype], n, k, group,
                                            None if activation_rms is None else activation_rms.data_ptr(),

@@ -32,3 +32,22 @@ def test_pack_equals_the_torch_expression(monkeypatch, bits, n, k, group):
             assert int(differ.sum()) <= differ.numel() // 1000 * (arms is not None), (dtype, int(differ.sum()))
             same = ~differ.repeat_interleave(group * bits // 8, dim=1)
             assert torch.equal(got.packed[same], want.packed[same])
+
+
+def test_pack_first_captured_then_eager(monkeypatch):
+    """The candidate factors of a captured call are written when the graph runs: an eager call in between has its own."""
+    w = torch.empty((64, 512), device="cuda").normal_(0, 0.02, generator=torch.Generator(device="cuda").manual_seed(1))
+    rms = torch.ones(512, device="cuda")
+    steps = 7                                                      # a count that nothing else uses
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = groupwise_int4.pack_groupwise_int4(w, 128, rms, steps)
+    got = groupwise_int4.pack_groupwise_int4(w, 128, rms, steps)
+    graph.replay()
+    with monkeypatch.context() as m:
+        m.setattr(groupwise_int4, "_pack_on_device", lambda *a: None)
+        want = groupwise_int4.pack_groupwise_int4(w, 128, rms, steps)
+    for other in (got, captured):
+        assert torch.equal(other.packed, want.packed) and torch.equal(other.scales, want.scales)
+
+
