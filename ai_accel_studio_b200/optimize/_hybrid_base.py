@@ -154,11 +154,16 @@ class HybridPackedLinear(nn.Module):
     _LAUNCH_OPERANDS = frozenset(("packed", "scales", "bias", "outlier_idx", "outlier_weight", "res_u", "res_v", "residual_rank",
                                   "kernel", "debug", "prefetch_next", "gated_pairs", "chunked_max_rows", "out_features"))
 
+    _PREPARED = ("_call", "_native_call", "_native_state", "_native_packed")
+
     def _drop_prepared(self) -> None:
-        """Forget the prepared launches: they hold the operands' addresses and the settings they were built from."""
-        self.__dict__.pop("_call", None)
-        self.__dict__.pop("_native_call", None)
-        self.__dict__.pop("_native_state", None)
+        """Forget the prepared launches: they hold the operands, their addresses and the settings they were built from."""
+        for name in HybridPackedLinear._PREPARED:
+            self.__dict__.pop(name, None)
+
+    def __getstate__(self):
+        """What copies and pickles carry: not the prepared launches."""
+        return {k: v for k, v in self.__dict__.items() if k not in HybridPackedLinear._PREPARED}
 
     def __setattr__(self, name, value):
         if name in HybridPackedLinear._LAUNCH_OPERANDS:

@@ -295,3 +295,19 @@ def test_prepared_launch_follows_the_module():
     assert (a(x).float() - y_res.float()).abs().max() < 2e-3                 # another kernel, same answer to rounding
     moved = a.cpu().cuda()
     assert (moved(x).float() - y_res.float()).abs().max() < 2e-3
+
+
+@pytest.mark.parametrize("rows", [2, 8, 40])
+def test_a_used_module_copies_pickles_and_leaves_the_gpu(rows):
+    import copy
+    import pickle
+    mod = HybridInt4Linear(torch.nn.Linear(2048, 1024), 128, None, 8).cuda()
+    x = torch.randn(rows, 2048).half().cuda()
+    want = mod(x)
+    for twin in (copy.deepcopy(mod), pickle.loads(pickle.dumps(mod))):
+        assert torch.equal(twin(x), want)
+        assert twin.packed.data_ptr() != mod.packed.data_ptr()
+    nbytes = mod.packed.nbytes + mod.scales.nbytes
+    before = torch.cuda.memory_allocated()
+    mod.cpu()                                                          # a planner or an offloading loop
+    assert before - torch.cuda.memory_allocated() >= nbytes
