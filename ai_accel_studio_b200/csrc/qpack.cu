@@ -63,6 +63,9 @@ __device__ __forceinline__ float magnitude(float a, float w, float cand, float c
 }
 constexpr float kMargin = 1e-5f;
 
+// max(x, 1e-8) that leaves NaN as it is, as the framework's clamp does.
+__device__ __forceinline__ float at_least_tiny(float x) { return x < 1e-8f ? 1e-8f : x; }
+
 template <int DT> __device__ __forceinline__ float load_w(const void* w, size_t i) {
     if constexpr (DT == QGEMV_F16) return __half2float(static_cast<const __half*>(w)[i]);
     else if constexpr (DT == QGEMV_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(w)[i]);
@@ -82,7 +85,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const void* __restrict__ w, l
     for (long long trip = blockIdx.x; trip < trips; trip += gridDim.x) {
         const long long gi = min(trip * per_block + sub, groups - 1);       // the last block repeats a group: shuffles stay converged
         const int row = (int)(gi / ng), grp = (int)(gi - (long long)row * ng);
-        float f[V][16], aw[V][16], peak = 0.0f, tiny = 3.0e38f;             // tiny: smallest magnitude that is not zero
+        float f[V][16], aw[V][16], tiny = 3.0e38f;                          // tiny: smallest magnitude that is not zero
+        uint32_t peak_bits = 0;                                             // largest magnitude; by its bits, above which NaN's are
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             const int k0 = grp * group + v * 128 + l * 16;
@@ -106,7 +110,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const void* __restrict__ w, l
             }
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-                peak = fmaxf(peak, fabsf(f[v][e]));
+                peak_bits = max(peak_bits, __float_as_uint(fabsf(f[v][e])));
                 tiny = f[v][e] != 0.0f ? fminf(tiny, fabsf(f[v][e])) : tiny;
             }
             if (rms) {
@@ -117,13 +121,13 @@ __global__ void __launch_bounds__(256) pack_kernel(const void* __restrict__ w, l
                     const int c = k0 + q * 4;
                     if (whole) a = __ldg(reinterpret_cast<const float4*>(rms + c));
                     else { if (c < k) a.x = rms[c]; if (c + 1 < k) a.y = rms[c + 1]; if (c + 2 < k) a.z = rms[c + 2]; if (c + 3 < k) a.w = rms[c + 3]; }
-                    aw[v][q * 4] = fmaxf(__fmul_rn(a.x, a.x), 1e-8f); aw[v][q * 4 + 1] = fmaxf(__fmul_rn(a.y, a.y), 1e-8f);
-                    aw[v][q * 4 + 2] = fmaxf(__fmul_rn(a.z, a.z), 1e-8f); aw[v][q * 4 + 3] = fmaxf(__fmul_rn(a.w, a.w), 1e-8f);
+                    aw[v][q * 4] = at_least_tiny(__fmul_rn(a.x, a.x)); aw[v][q * 4 + 1] = at_least_tiny(__fmul_rn(a.y, a.y));
+                    aw[v][q * 4 + 2] = at_least_tiny(__fmul_rn(a.z, a.z)); aw[v][q * 4 + 3] = at_least_tiny(__fmul_rn(a.w, a.w));
                 }
             }
         }
-        for (int o = 1; o < lg; o <<= 1) peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, o));
-        const float base = BITS == 2 ? fmaxf(peak, 1e-8f) : fmaxf(__fmul_rn(peak, 1.0f / 7.0f), 1e-8f);
+        for (int o = 1; o < lg; o <<= 1) peak_bits = max(peak_bits, __shfl_xor_sync(0xffffffffu, peak_bits, o));
+        const float peak = __uint_as_float(peak_bits), base = at_least_tiny(BITS == 2 ? peak : __fmul_rn(peak, 1.0f / 7.0f));
         float chosen = base;
         if (rms) {
             float best = 0.0f;

@@ -51,3 +51,26 @@ def test_pack_first_captured_then_eager(monkeypatch):
         assert torch.equal(other.packed, want.packed) and torch.equal(other.scales, want.scales)
 
 
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+def test_pack_of_values_that_are_not_finite(monkeypatch, bits):
+    """NaN makes its group's scale NaN and infinity makes it infinite, with or without the search, and a NaN among the statistics
+    leaves its group the first candidate, as in the torch expression; other groups are as they would be."""
+    mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
+    w = torch.empty((8, 256), device="cuda").normal_(0, 0.02, generator=torch.Generator(device="cuda").manual_seed(2))
+    w[1, 3] = float("nan")
+    w[2, 200] = float("inf")
+    w[3, 100] = -float("inf")
+    w[4, 10], w[4, 11] = float("nan"), float("inf")
+    rms = torch.ones(256, device="cuda")
+    odd = rms.clone()
+    odd[130] = float("nan")
+    for arms in (None, rms, odd):
+        got = fn(w, 64, arms)
+        with monkeypatch.context() as m:
+            m.setattr(mod, "_pack_on_device", lambda *a: None)
+            want = fn(w, 64, arms)
+        assert torch.equal(got.scales.isnan(), want.scales.isnan()) and torch.equal(got.scales.nan_to_num(), want.scales.nan_to_num())
+        finite = want.scales.isfinite().repeat_interleave(64 * bits // 8, dim=1)      # NaN has no code
+        assert torch.equal(got.packed[finite], want.packed[finite])
