@@ -321,7 +321,9 @@ extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
 // rows so long that their activations leave the phased kernel few of its 16 warps, or do not fit beside it at all (M = 4,
 // K = 28672; the CUDA-core kernel took those): the streaming kernel cuts K between CTAs instead.  With 4 warps left it wins
 // (14336 x 14336 INT4, M = 4: 44 against 65 us), with 8 it loses (4096 x 14336 INT4, M = 4: 24 against 18 us) unless there are
-// at most two rows, which it multiplies as integers (8192 x 28672 INT2, M = 2: 37 against 44 us).
+// at most two rows, which it multiplies as integers (K = 28672, M = 2, N = 2048 and 8192: INT4 24 against 33 and 48 against 51 us,
+// INT2 21 against 16 and 36 against 43 us).  INT2 matrices of no more than one tile of 16 rows per SM, which the phased kernel reads
+// in a single round, stay with it (N = 512 to 2048: 16 us, streaming 17 to 21).
 extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     const size_t need = qgemv_workspace_bytes(0, 0, 0, 0, 0, 0);
     const int v = validate(p, need, QGEMV_MAX_BATCH);
@@ -336,7 +338,8 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && padded) {
         bool none = false;
         const MmaPlan plan = choose(*p, kMaxPartialFloats, &none);
-        starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 ? 8 : 4));
+        const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
+        starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
     }
     if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8 || starved) &&
         plan_stream(&one, 1, kMaxPartialFloats, &q->plan))

@@ -191,7 +191,8 @@ int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspac
  * type; base (with the bias), outlier term and residual are fp32 sums, each rounded to the activation type (the residual, whose V x
  * is rounded to fp16, to fp16 first) before they are added in this order, as the expression over a dense matrix does.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
  * private to the call until it completes (0: this shape is not built -- groups other than 32 (INT4), 64 and multiples of
- * 128, unaligned packed rows -- dequantise and use a library GEMM).  x needs only k_original columns.
+ * 128, unaligned packed rows, more than 8192 tiles of 128 weight rows x 256 rows of x, more than 4096 outlier columns --
+ * dequantise and use a library GEMM).  x needs only k_original columns.
  * Replaces the M > 4 route of ai_accel_lab/optimize/hybrid_int4.py:36-37 and hybrid_int2.py:102-106. */
 size_t qgemv_batch_scratch_bytes(const qgemv_problem* p);
 int qgemv_run_batch(const qgemv_problem* p, void* scratch, size_t scratch_bytes, void* stream);

@@ -150,3 +150,23 @@ def test_prompts_are_differentiable_and_transformable_in_x(bits, oc, rank):
         assert torch.equal(mod(x), got[0]) or near(mod(x), got[0].double(), 4)
     traced = torch.jit.trace(mod, x, check_trace=False)
     assert near(traced(tangent), tangent.double() @ w.t() + mod.bias.double(), 4)
+
+
+def test_many_rows_over_long_k_take_the_expression():
+    mod = _module(2, 64, 28672, 128, 8, 8, True, torch.Generator().manual_seed(12))
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    for rows in (1090, 1100):                                        # either side of 30 Mi elements of x
+        x = torch.randn(rows, 28672, generator=gen, device="cuda").half()
+        y, want = mod(x), mod._dense(x)
+        assert torch.equal(y, want) or rows * 28672 <= 30 << 20
+        assert float((y.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -11
+
+
+@pytest.mark.parametrize("bits,n", [(2, 300), (2, 2368), (2, 2400), (4, 300)])
+def test_two_rows_of_long_k_on_either_side_of_the_route(bits, n):
+    """K = 28672: INT2 matrices of one round of tiles stay with the phased kernel, the others go to the streaming one."""
+    mod = _module(bits, n, 28672, 128, 8, 8, True, torch.Generator().manual_seed(n))
+    x = torch.randn(2, 28672, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda").half()
+    want = x.double() @ mod.effective_weight().double().t() + mod.bias.double()
+    assert float((mod(x).double() - want).norm() / want.norm()) <= 2.0 ** -11      # one rounding of a 32-bit sum, and its own error
+    assert ops.workspace_status("cuda") == 0
