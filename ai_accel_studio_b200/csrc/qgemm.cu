@@ -930,19 +930,24 @@ bool plan_gemm(const qgemv_problem& p, GemmPlan& g) {
     g.groups = (p.m + 7) / 8;
     if (tiles > kTileCounters || g.groups > kRowCounters || tiles * a.units > 0x3fffffff) return false;
     const int s = sms();
-    // Whole tiles, or units dealt out evenly over `grid` CTAs: clocks of the busiest one.  A unit takes about 5 x width, at
-    // least 600 (the chain of barriers); storing a tile 1500 + 24 x width; handing pieces over some 3000, and the last CTA of a
-    // tile reads its contributions one after the other, 1500 each.
-    const long long unit_clk = 5 * a.width > 600 ? 5 * a.width : 600, end_clk = 1500 + 24 * a.width, all = tiles * a.units;
+    // Whole tiles, each tile cut into `parts` CTAs, or all units dealt out evenly over the SMs: clocks of the busiest CTA.  Fitted to
+    // a sweep of 35 shapes (N and K from 896 to 28672, 17 - 2048 rows; the choice is within 5 % of the best one for all
+    // but two): a unit takes 1070 whatever the width, its weights being what it waits for; storing a tile 1000 + 110 x width;
+    // handing a piece over 3800 + 45 x width, the pieces' traffic through L2 0.93 x width for each in the whole grid, and the last CTA
+    // of a tile reads its pieces one after the other.  Dealt out evenly a CTA has two pieces, and tiles are cut anywhere: 4096 x 4096, 256 rows
+    // took 53 us on 148 CTAs, 37 as 32 whole tiles; 4096 x 14336 takes 51 us in four parts a tile against 79.
+    const long long unit_clk = 1070, end_clk = 1000 + 110 * a.width, all = tiles * a.units;
     long long best = (tiles + s - 1) / s * (a.units * unit_clk + end_clk);
     a.split = 0;
     g.grid = (int)(tiles < s ? tiles : s);
-    for (int parts = 1; parts <= 32; parts += parts < 4 ? 1 : parts / 4) {
-        const long long want = tiles * parts < s ? tiles * parts : s, share = (all + want - 1) / want;
+    for (int parts = 2; parts <= 32; parts += parts < 4 ? 1 : parts / 4) {
+        const bool even = tiles * parts <= s;
+        const long long want = even ? tiles * parts : s, share = (all + want - 1) / want;
         if (want > all) break;
-        const long long cost = share * unit_clk + (share / a.units + 1) * end_clk + 3000 + 1500 * (a.units / share + 1);
+        const long long ends = even ? end_clk / 2 : share / a.units * end_clk, per_tile = even ? parts : a.units / share + 1;
+        const long long cost = share * unit_clk + ends + 3800 + a.width * (93 * (even ? want : 2 * want) + 74 * per_tile * per_tile + (even ? 4500 : 9000)) / 100;
         if (cost < best) { best = cost; a.split = 1; g.grid = (int)want; }
-        if (want == s) break;
+        if (!even) break;
     }
     g.x_bytes = ((size_t)p.m * g.ke * 2 + 255) / 256 * 256;
     // enough CTAs of the layout kernel for two per SM, each warp with at least two blocks of 64 columns
