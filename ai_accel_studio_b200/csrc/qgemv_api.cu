@@ -332,8 +332,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     Prepared* q = static_cast<Prepared*>(prepared);
     q->problem = *p;
     q->plan = StreamPlan{};
-    const bool padded = p->ldx >= p->k_padded && (p->k_padded == p->k_original || p->m > QGEMV_MAX_BATCH);
-    const qgemv_problem* one = p;
+    const bool padded = p->ldx >= p->k_padded && p->k_padded == p->k_original;
     bool starved = false;
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && padded) {
         bool none = false;
@@ -342,7 +341,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
     }
     if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8 || starved) &&
-        plan_stream(&one, 1, kMaxPartialFloats, &q->plan))
+        plan_stream(*p, kMaxPartialFloats, &q->plan))
         return QGEMV_OK;
     q->plan = StreamPlan{};
     if (p->ldx < p->k_padded || p->k_padded != p->k_original) { set_error("qgemv_prepare: this shape needs x padded to k_padded columns"); return QGEMV_ERR_ALIGN; }
@@ -360,7 +359,7 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
     if (q->plan.ok) {
         if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
         q->plan.args.x = x;
-        q->plan.args.seg[0].y = y;
+        q->plan.args.seg.y = y;
         return launch_stream(q->plan, q->problem.x_dtype == QGEMV_BF16, !ordered, workspace, static_cast<cudaStream_t>(stream));
     }
     qgemv_problem p = q->problem;

@@ -7,7 +7,6 @@ namespace {
 bool al(const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; }
 int up_to(int v, int a) { return (v + a - 1) / a * a; }
 int cdiv(int a, int b) { return (a + b - 1) / b; }
-int pow2_at_least(int v) { int p = 1; while (p < v) p *= 2; return p; }
 
 int sm_count() {
     static int cached[64] = {0};
@@ -24,7 +23,6 @@ int sm_count() {
 int log2_exact(int v) { int s = 0; while ((1 << s) < v) ++s; return (1 << s) == v ? s : -1; }
 
 int stream_format(int bits, int group) {
-    if (bits == 16) return kDense16;
     if (bits == 2 && group == 64) return kInt2G64;
     if (bits == 4 && group == 32) return kInt4G32;
     if (bits == 4 && group == 64) return kInt4G64;
@@ -32,14 +30,14 @@ int stream_format(int bits, int group) {
     return bits == 2 ? kInt2G128 : kInt4G128;
 }
 
-constexpr int kCodesPerSlot[6] = {512, 512, 256, 256, 256, 64};
-constexpr int kBlocksPerSlot[6] = {4, 4, 2, 2, 2, 0};            // 128-column blocks
-constexpr int kGroupsPerBlock[6] = {1, 2, 1, 2, 4, 1};
+constexpr int kCodesPerSlot[5] = {512, 512, 256, 256, 256};
+constexpr int kBlocksPerSlot[5] = {4, 4, 2, 2, 2};               // 128-column blocks
+constexpr int kGroupsPerBlock[5] = {1, 2, 1, 2, 4};
 
 // Instructions of a warp per tile and slot, and per slot and row block (fetching activations), by path and format: counted
 // from the main loop (ncu agrees within 10 %).  Only their ratios to each other and to the bytes matter here.
-constexpr int kTileCost[2][6] = {{220, 260, 110, 130, 170, 34}, {320, 400, 170, 210, 300, 34}};
-constexpr int kSlotCost[2][6] = {{180, 180, 110, 110, 110, 60}, {220, 240, 130, 140, 150, 60}};
+constexpr int kTileCost[2][5] = {{220, 260, 110, 130, 170}, {320, 400, 170, 210, 300}};
+constexpr int kSlotCost[2][5] = {{180, 180, 110, 110, 110}, {220, 240, 130, 140, 150}};
 
 constexpr int kMaxJobs = 32;                          // CTAs of a split that compute residual projections
 
@@ -50,7 +48,7 @@ constexpr int kMaxJobs = 32;                          // CTAs of a split that co
 // for a hand-over between splits.
 bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, int ctas, int cap, size_t split_floats, size_t word_floats, StreamSeg& out, int& smem_out) {
     const int fmt = out.fmt, cps = kCodesPerSlot[fmt], nb = mode == 2 ? 2 : 1;
-    const bool digits = mode == 0 && fmt != kDense16;
+    const bool digits = mode == 0;
     const int tiles = cdiv(p.n, kStreamTileRows), rtiles = cdiv(p.rank, kStreamTileRows);
     out.ns = cdiv(out.row_bytes, kSlotRowBytes);
     out.mp = up_to(m, 2);
@@ -101,7 +99,7 @@ bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, in
             const int q = cdiv(s.ns_split, s.wk);
             for (s.T = 1; s.T <= kMaxTiles && s.T <= s.tiles_w; ++s.T) {
                 s.nrb = cdiv(s.tiles_w, s.T);
-                s.sx_bytes = mode != 0 && s.nrb > 1 && fmt != kDense16 ? q * kBlocksPerSlot[fmt] * kGroupsPerBlock[fmt] * nb * 32 : 0;
+                s.sx_bytes = mode != 0 && s.nrb > 1 ? q * kBlocksPerSlot[fmt] * kGroupsPerBlock[fmt] * nb * 32 : 0;
                 s.off_sx = fixed;
                 s.off_part = fixed + nw * s.sx_bytes;
                 s.off_ring = up_to(s.off_part + s.wk * s.rows_pad * s.mp * 4, 128);
@@ -127,89 +125,59 @@ bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, in
 
 }  // namespace
 
-bool plan_stream(const qgemv_problem* const* probs, int count, size_t partial_floats, StreamPlan* out) {
+bool plan_stream(const qgemv_problem& p, size_t partial_floats, StreamPlan* out) {
     *out = StreamPlan{};
     StreamArgs& a = out->args;
-    if (count < 1 || count > kMaxSegments) return false;
-    const qgemv_problem& p0 = *probs[0];
-    const int m = p0.m;
-    if (m < 1 || m > 16 || !al(p0.x, 16)) return false;
+    StreamSeg& s = a.seg;
+    const int m = p.m;
+    if (m < 1 || m > 16 || !al(p.x, 16)) return false;
     const int mode = m > 8 ? 2 : m > 2 ? 1 : 0, sms = sm_count();
-    const bool bf16 = p0.x_dtype == QGEMV_BF16;
-    size_t total_bytes = 0, bytes[kMaxSegments];
-    for (int i = 0; i < count; ++i) {
-        const qgemv_problem& p = *probs[i];
-        StreamSeg& s = a.seg[i];
-        s.fmt = stream_format(p.bits, p.group);
-        if (s.fmt < 0 || !al(p.packed, 16) || p.ldp % 16 || p.outliers > kStreamMaxOutliers || p.rank > kMaxRank) return false;
-        if (p.bits != 16 && !al(p.scales, 2)) return false;
-        if (p.x != p0.x || p.ldx != p0.ldx || p.m != m || p.k_original != p0.k_original) return false;
-        s.w = p.packed; s.ldw = p.ldp;
-        s.sc = static_cast<const __half*>(p.scales); s.lds = p.lds;
-        s.bias = static_cast<const __half*>(p.bias);
-        s.oidx = p.outlier_idx; s.ow = static_cast<const __half*>(p.outlier_w); s.ldow = p.ldow;
-        s.ru = static_cast<const __half*>(p.res_u); s.ldu = p.ldu;
-        s.rv = static_cast<const __half*>(p.res_v); s.ldv = p.ldv;
-        s.y = p.y; s.ldy = p.ldy;
-        s.n = p.n; s.act = p.act;
-        s.row_bytes = (int)((long long)p.k_padded * p.bits / 8);
-        s.ng = p.bits == 16 ? 0 : p.k_padded / p.group;
-        s.gshift = p.bits != 16 && p.group >= 128 ? log2_exact(p.group / 128) : 0;
-        s.oc = p.outliers; s.noc = cdiv(p.outliers, 32);
-        s.rank = p.rank;
-        if (p.bits != 16) {                            // a slot's scales of a row as one aligned copy of 4, 8 or 16 bytes
-            const int count = kBlocksPerSlot[s.fmt] * kGroupsPerBlock[s.fmt] >> s.gshift, halves = count < 2 ? 2 : count;
-            if (al(p.scales, halves * 2) && p.lds % halves == 0) s.flags |= kSegScaleAligned;
-        }
-        if (p.outliers && al(p.outlier_w, 16) && p.ldow % 8 == 0 && p.outliers % 8 == 0) s.flags |= kSegOutlierAligned;
-        if (p.rank && al(p.res_v, 16) && p.ldv % 8 == 0) s.flags |= kSegVAligned;
-        if (p.rank && al(p.res_u, 16) && p.ldu % 8 == 0 && p.rank % 8 == 0) s.flags |= kSegUAligned;
-        bytes[i] = (size_t)p.n * s.row_bytes;
-        total_bytes += bytes[i];
-    }
+    const bool bf16 = p.x_dtype == QGEMV_BF16;
+    s.fmt = stream_format(p.bits, p.group);
+    if (s.fmt < 0 || !al(p.packed, 16) || p.ldp % 16 || p.outliers > kStreamMaxOutliers || p.rank > kMaxRank || !al(p.scales, 2)) return false;
+    s.w = p.packed; s.ldw = p.ldp;
+    s.sc = static_cast<const __half*>(p.scales); s.lds = p.lds;
+    s.bias = static_cast<const __half*>(p.bias);
+    s.oidx = p.outlier_idx; s.ow = static_cast<const __half*>(p.outlier_w); s.ldow = p.ldow;
+    s.ru = static_cast<const __half*>(p.res_u); s.ldu = p.ldu;
+    s.rv = static_cast<const __half*>(p.res_v); s.ldv = p.ldv;
+    s.y = p.y; s.ldy = p.ldy;
+    s.n = p.n; s.act = p.act;
+    s.row_bytes = (int)((long long)p.k_padded * p.bits / 8);
+    s.ng = p.k_padded / p.group;
+    s.gshift = p.group >= 128 ? log2_exact(p.group / 128) : 0;
+    s.oc = p.outliers; s.noc = cdiv(p.outliers, 32);
+    s.rank = p.rank;
+    // a slot's scales of a row as one aligned copy of 4, 8 or 16 bytes
+    const int count = kBlocksPerSlot[s.fmt] * kGroupsPerBlock[s.fmt] >> s.gshift, halves = count < 2 ? 2 : count;
+    if (al(p.scales, halves * 2) && p.lds % halves == 0) s.flags |= kSegScaleAligned;
+    if (p.outliers && al(p.outlier_w, 16) && p.ldow % 8 == 0 && p.outliers % 8 == 0) s.flags |= kSegOutlierAligned;
+    if (p.rank && al(p.res_v, 16) && p.ldv % 8 == 0) s.flags |= kSegVAligned;
+    if (p.rank && al(p.res_u, 16) && p.ldu % 8 == 0 && p.rank % 8 == 0) s.flags |= kSegUAligned;
+    // Split sums from the start of the scratch; words of residual projections in a region of their own at its end, below
+    // the one of the other kernels: a word is recognised by its launch tag, and no other data, nor tags of another count,
+    // may ever be taken for one.
+    if (partial_floats < kTPartFloats + kStreamWordFloats) return false;
+    const size_t floor = partial_floats - kTPartFloats - kStreamWordFloats, tail = partial_floats - kTPartFloats;
     // Half-SM CTAs let two launches of a chain share an SM (the next one fetches its weights while this one runs); a
     // whole-SM CTA has 16 warps and a deep ring: for few rows of activations it pays once a launch streams so much that its
     // start and end no longer count, for more than 8 rows (whose fragments need the registers) always.
-    int order[2], tries = 0;
-    const bool big = total_bytes / sms >= 400 * 1024;
-    { order[0] = m > 4 || big; order[1] = !order[0]; tries = m > 8 ? 1 : 2; }
-    for (int t = 0; t < tries; ++t) {
-        const bool whole = order[t] != 0;
+    const bool big = (size_t)p.n * s.row_bytes / sms >= 400 * 1024, first = m > 4 || big;
+    for (int t = 0; t < (m > 8 ? 1 : 2); ++t) {
+        const bool whole = t == 0 ? first : !first;
         const int nw = mode == 2 || !whole ? 8 : 16, cap = whole ? kStreamMaxSmem : kHalfSmem;
-        int cta = 0, smem = 0, counters = 0;
-        // Split sums from the start of the scratch; words of residual projections in a region of their own at its end, below
-        // the one of the other kernels: a word is recognised by its launch tag, and no other data, nor tags of another count,
-        // may ever be taken for one.
-        if (partial_floats < kTPartFloats + kStreamWordFloats) return false;
-        const size_t floor = partial_floats - kTPartFloats - kStreamWordFloats;
-        size_t tail = partial_floats - kTPartFloats, head = 0;
-        bool ok = true, epoch = false;
-        for (int i = 0; i < count && ok; ++i) {
-            const qgemv_problem& p = *probs[i];
-            StreamSeg& s = a.seg[i];
-            int share = count == 1 ? sms : (int)((double)sms * bytes[i] / total_bytes + 0.5);
-            if (share < 1) share = 1;
-            if (i == count - 1 && cta + share > sms && sms - cta >= 1) share = sms - cta;
-            int need = 0;
-            ok = plan_segment(p, m, mode, bf16, nw, share, cap, floor - head, tail - floor, s, need);
-            if (!ok) break;
-            s.cta0 = cta;
-            cta += s.groups * s.ksplit;
-            if (need > smem) smem = need;
-            const size_t words = (size_t)s.t_parts * s.rank * m * 2;
-            tail = (tail - words) & ~(size_t)1;
-            out->t_off[i] = kWsPartialOff + tail * sizeof(float);
-            out->part_off[i] = kWsPartialOff + head * sizeof(float);
-            out->cnt_off[i] = kWsCounterOff + counters * sizeof(int);
-            if (s.ksplit > 1) { head += (size_t)s.ksplit * s.n * s.mp; counters += s.groups; }
-            epoch = epoch || s.rank > 0;
-        }
-        if (!ok || cta > 256) continue;
-        a.x = p0.x; a.ldx = p0.ldx; a.m = m; a.korig = p0.k_original; a.nw = nw; a.nseg = count;
-        a.xaligned = p0.ldx % 8 == 0 ? 1 : 0;
-        a.debug = p0.debug;
-        out->epoch = epoch;
-        out->grid = cta; out->threads = (nw + 1) * 32; out->smem = smem; out->mode = mode;
+        int smem = 0;
+        if (!plan_segment(p, m, mode, bf16, nw, sms, cap, floor, tail - floor, s, smem)) continue;
+        const int ctas = s.groups * s.ksplit;
+        if (ctas > 256) continue;
+        out->t_off = kWsPartialOff + ((tail - (size_t)s.t_parts * s.rank * m * 2) & ~(size_t)1) * sizeof(float);
+        out->part_off = kWsPartialOff;
+        out->cnt_off = kWsCounterOff;
+        a.x = p.x; a.ldx = p.ldx; a.m = m; a.korig = p.k_original; a.nw = nw;
+        a.xaligned = p.ldx % 8 == 0 ? 1 : 0;
+        a.debug = p.debug;
+        out->epoch = s.rank > 0;
+        out->grid = ctas; out->threads = (nw + 1) * 32; out->smem = smem; out->mode = mode;
         out->ok = true;
         return true;
     }
@@ -224,11 +192,9 @@ int launch_stream(StreamPlan& plan, bool bf16, bool dependent, void* workspace, 
     int* cnt = reinterpret_cast<int*>(ws + kWsCounterOff);
     a.status = cnt + kWsStatusIdx;
     a.epoch = plan.epoch ? reinterpret_cast<unsigned long long*>(cnt + kWsStreamEpochIdx) : nullptr;
-    for (int i = 0; i < a.nseg; ++i) {
-        a.seg[i].tparts = reinterpret_cast<unsigned long long*>(ws + plan.t_off[i]);
-        a.seg[i].partial = reinterpret_cast<float*>(ws + plan.part_off[i]);
-        a.seg[i].counters = reinterpret_cast<int*>(ws + plan.cnt_off[i]);
-    }
+    a.seg.tparts = reinterpret_cast<unsigned long long*>(ws + plan.t_off);
+    a.seg.partial = reinterpret_cast<float*>(ws + plan.part_off);
+    a.seg.counters = reinterpret_cast<int*>(ws + plan.cnt_off);
     decltype(&launch_stream_mode<0, false>) fn[3][2] = {{launch_stream_mode<0, false>, launch_stream_mode<0, true>},
                                                         {launch_stream_mode<1, false>, launch_stream_mode<1, true>},
                                                         {launch_stream_mode<2, false>, launch_stream_mode<2, true>}};

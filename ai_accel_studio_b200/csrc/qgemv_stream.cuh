@@ -12,16 +12,15 @@ constexpr int kSlotRowBytes = 128;     // bytes of one weight row in a ring slot
 constexpr int kTileBytes = kStreamTileRows * kSlotRowBytes;
 constexpr int kSlotBytes = kTileBytes + kStreamTileRows * 16;   // the weights of a tile and 16 bytes of scales per row
 constexpr int kMaxTiles = 2;           // tiles a warp keeps accumulators for (one row block)
-constexpr int kMaxSegments = 4;        // weight matrices one launch can serve
 constexpr int kMaxDepth = 4;           // ring depth in batches (one batch = one slot per tile of a row block)
 constexpr int kHalfSmem = 115712;      // 113 KB: two CTAs per SM, so that the next launch is resident while this one runs
 constexpr size_t kStreamWordFloats = size_t(1) << 17;     // scratch kept for {value, launch tag} words, in 32-bit units
 constexpr int kProjectionK = 256;      // K columns of one round of an in-kernel residual projection
 
-// Weight formats: packed codes by the scale groups per 128-column block, or plain 16-bit rows.
-enum StreamFormat { kInt2G128 = 0, kInt2G64 = 1, kInt4G128 = 2, kInt4G64 = 3, kInt4G32 = 4, kDense16 = 5 };
+// Weight formats: packed codes by the scale groups per 128-column block.
+enum StreamFormat { kInt2G128 = 0, kInt2G64 = 1, kInt4G128 = 2, kInt4G64 = 3, kInt4G32 = 4 };
 
-// One weight matrix of a launch: its operands and the share of the grid that works on it.
+// The weight matrix of a launch: its operands and how it is cut.
 struct StreamSeg {
     const uint8_t* w;         long long ldw;      // weight rows, leading dimension in bytes
     const __half* sc;         long long lds;
@@ -40,7 +39,7 @@ struct StreamSeg {
     int rank, t_parts, t_parts_split, t_rounds;   // residual: K parts (all / per split), rounds of kProjectionK columns per part
     int flags;
     // geometry
-    int cta0, groups, ksplit, rows_per;           // first CTA, row groups, K splits, rows of one row group
+    int groups, ksplit, rows_per;                 // row groups, K splits, rows of one row group
     int ns, ns_split;                             // weight slots per row, and per K split
     int wk, wr;                                   // warps along K, warps along the rows
     int tiles_w, nrb, T, depth;                   // tiles per warp, row blocks per warp, tiles per row block, ring depth
@@ -54,22 +53,22 @@ enum { kSegScaleAligned = 1, kSegOutlierAligned = 2, kSegVAligned = 4, kSegUAlig
 
 struct StreamArgs {
     const void* x;            long long ldx;
-    int m, korig, nw, nseg;
+    int m, korig, nw;
     int xaligned, debug;
     int* status;                                  // wait-timeout status word
     unsigned long long* epoch;                    // launches of the workspace with residual projections, times 256
-    StreamSeg seg[kMaxSegments];
+    StreamSeg seg;
 };
 
 // The plan of a launch: everything but the addresses that change from call to call (x, y, scratch).
 struct StreamPlan {
     bool ok, epoch;
     int grid, threads, smem, mode;                // mode: 0 integer path (1 - 2 rows), 1 fp16 path (to 8), 2 (to 16)
-    size_t t_off[kMaxSegments], part_off[kMaxSegments], cnt_off[kMaxSegments];   // bytes from the workspace base
+    size_t t_off, part_off, cnt_off;              // bytes from the workspace base
     StreamArgs args;
 };
-// Up to kMaxSegments matrices that share x (same pointer, rows and columns).  `partial_floats`: capacity of the workspace's scratch area.
-bool plan_stream(const qgemv_problem* const* probs, int count, size_t partial_floats, StreamPlan* out);
+// `partial_floats`: capacity of the workspace's scratch area.
+bool plan_stream(const qgemv_problem& p, size_t partial_floats, StreamPlan* out);
 // `dependent`: may start before the preceding kernel of the stream has finished (the weights are final).
 int launch_stream(StreamPlan& plan, bool bf16, bool dependent, void* workspace, cudaStream_t s);
 
