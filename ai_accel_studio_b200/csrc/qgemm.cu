@@ -7,15 +7,17 @@
 // column = two K neighbours).  B is a tile of up to 256 activation rows, brought into shared memory by TMA (128-byte
 // swizzle); the accumulator (128 x 256 fp32) takes the other half of tensor memory.
 //
-//   bound      tensor pipe: 128 x 256 x 128 MACs take 1024 clocks per SM; making 128 x 128 weights takes 8 warps about 260
-//              issue slots per scheduler of those (INT4 1.6, INT2 1.3 instructions per weight, from a byte permute of the
-//              four scaled levels), reading B takes 64 of shared memory's 128 bytes a clock.
+//   bound      a unit of 128 K columns takes some 1070 clocks whatever the width of the tile: at 256 rows that is the tensor
+//              pipe (128 x 256 x 128 MACs, 1024 clocks at 8192 flop a clock), at fewer the weights, of which a warpgroup makes
+//              128 x 128 in 3300 - 4000 clocks (INT4 1.6, INT2 1.3 instructions per weight, from a byte permute of the four
+//              scaled levels); three or four take turns.  Then a tile's end: some 30 k clocks to store 128 x 256 results, during
+//              which the tensor pipe is idle.
 //   A in TMEM  keeps the converted weights out of shared memory, whose bandwidth B and the TMA writes need.
 //   terms      base, outlier columns and residual are three products, and the framework's expression rounds each of them to the
 //              activation type before it adds them.  So do the results here: this kernel stores the rounded base, and a third
 //              one (terms_kernel) adds the two small products to it.  As further K columns of one sum they cost next to nothing,
 //              but that is another number (512 rows, bf16: 3.4e-3 apart), and a decoder's layers make 1e-2 of it.
-//   split      units of 128 K columns are dealt out evenly over the SMs when whole tiles would leave more than that idle; the
+//   split      where whole tiles would leave too much of the chip idle, a tile's K is cut between CTAs (see plan_gemm); the
 //              contributions of a tile then meet in scratch memory and whichever CTA comes last adds them in CTA order.
 //
 // A first small kernel lays x out for this: K columns permuted the way the codes leave a word, padded with zeros to
@@ -37,7 +39,7 @@ constexpr int kUnit = 128;                 // K columns of one stage (A: 64 colu
 constexpr int kChunk = 64;                 // K columns of one TMA box: 128 bytes of a 16-bit row
 constexpr int kMaxStages = 6;
 constexpr int kMaxWidth = 256;             // activation rows of a tile
-constexpr int kGroups = 4;                 // warpgroups that dequantise (every fourth unit each) and finish tiles
+constexpr int kGroups = 4;                 // warpgroups that dequantise (in turn; as many as there are stages) and finish tiles
 constexpr int kGemmThreads = kGroups * 128 + 64;     // and one warp that issues TMA, one that issues the mma
 constexpr int kTmaWarp = kGroups * 4, kMmaWarp = kTmaWarp + 1;
 constexpr int kSmemCtl = 512;              // barriers, at the end of shared memory
@@ -57,7 +59,7 @@ struct GemmArgs {
     int stages, ring;                         // stages of A and B (one barrier for both: a wait costs the mma warp 200 clocks); units of codes the ring holds (power of two)
     int ctl_off;                              // barriers in shared memory
     int groups;                               // warpgroups that dequantise: at most `stages`, see the wait for a stage
-    int split;                                // 1: units dealt out evenly, 0: whole tiles
+    int split;                                // 1: units dealt out over the CTAs, 0: whole tiles
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -41,7 +41,7 @@ int simt_unit_bytes(const qgemv_problem& p) {
 int validate(const qgemv_problem* p, size_t need, int max_m = QGEMV_MAX_M) {
     if (!p) { set_error("qgemv_run: problem is NULL"); return QGEMV_ERR_BAD_ARG; }
     if (p->bits != 2 && p->bits != 4) { set_error("qgemv_run: bits must be 2 or 4 (got %d)", p->bits); return QGEMV_ERR_BAD_ARG; }
-    if (p->m < 1 || p->m > max_m) { set_error("qgemv_run: M must be 1..%d (got %d); larger batches use the dequantise + GEMM path", max_m, p->m); return QGEMV_ERR_BAD_ARG; }
+    if (p->m < 1 || p->m > max_m) { set_error("qgemv_run: M must be 1..%d (got %d); more rows: qgemv_prepare, qgemv_run_batch", max_m, p->m); return QGEMV_ERR_BAD_ARG; }
     if (p->n < 1 || p->k_padded < 1 || p->k_original < 1 || p->k_original > p->k_padded) { set_error("qgemv_run: bad N / K (n=%d, k_padded=%d, k_original=%d)", p->n, p->k_padded, p->k_original); return QGEMV_ERR_BAD_ARG; }
     if (!p->x || !p->packed || !p->scales || !p->y) { set_error("qgemv_run: x, packed, scales and y must be non-null"); return QGEMV_ERR_BAD_ARG; }
     if (p->act < QGEMV_ACT_NONE || p->act > QGEMV_ACT_SILU_MUL) { set_error("qgemv_run: unknown activation %d", p->act); return QGEMV_ERR_BAD_ARG; }

@@ -35,7 +35,8 @@ constexpr int kBlocksPerSlot[5] = {4, 4, 2, 2, 2};               // 128-column b
 constexpr int kGroupsPerBlock[5] = {1, 2, 1, 2, 4};
 
 // Instructions of a warp per tile and slot, and per slot and row block (fetching activations), by path and format: counted
-// from the main loop (ncu agrees within 10 %).  Only their ratios to each other and to the bytes matter here.
+// from the main loop.  A whole launch executes about half as many again (14336 x 4096 INT2, 16 rows: 7.7 M warp instructions by
+// counter, 5 M by these), so only their ratios to each other and to the bytes matter here.
 constexpr int kTileCost[2][5] = {{220, 260, 110, 130, 170}, {320, 400, 170, 210, 300}};
 constexpr int kSlotCost[2][5] = {{180, 180, 110, 110, 110}, {220, 240, 130, 140, 150}};
 
@@ -79,7 +80,8 @@ bool plan_segment(const qgemv_problem& p, int m, int mode, bool bf16, int nw, in
                 s.t_parts_split = cdiv(slice, kProjectionK * s.t_rounds);
                 s.t_parts = s.t_parts_split * S;
                 words = (size_t)s.t_parts * p.rank * m;
-                // in the first CTAs of a split: those are resident whenever a CTA that waits for them is
+                // in the first CTAs of a split: they start first.  One of them may still wait for words of a later one that is
+                // not resident yet; every wait is bounded, and running out is reported by the workspace's status word.
                 if ((words <= 1024 && rtiles * s.t_parts_split <= (s.groups < kMaxJobs ? s.groups : kMaxJobs)) || s.t_parts_split == 1) break;
             }
         }

@@ -1,14 +1,14 @@
-// Streaming fused GEMV for packed groupwise INT2 / INT4 (and 16-bit) weights, up to 16 activation rows, sm_100a.
+// Streaming fused GEMV for packed groupwise INT2 / INT4 weights, up to 16 activation rows, sm_100a.
 //
 // A decode GEMV is a few microseconds of weight stream wrapped in a chain of short dependent phases; the chain, not HBM,
 // is what bounds it.  This kernel keeps the chain short and the instruction count per weight low:
 //
-//  * Everything that does not depend on x happens before the dependency wait.  Each warp owns a ring of 1 KB slots
-//    (16 weight rows x 64 bytes) filled by cp.async and has it full before `griddepcontrol.wait`.  A CTA takes half an
-//    SM's shared memory and registers, so the next launch of a decode loop is resident beside the running one and
-//    its first ~10 MB of weights are in shared memory when x arrives.
+//  * Everything that does not depend on x happens before the dependency wait.  Each warp owns a ring of slots (16 weight rows
+//    x 128 bytes and their scales) filled by cp.async and has it full before `griddepcontrol.wait`.  For up to four rows a CTA
+//    takes half an SM's shared memory where it can, so the next launch of a decode loop is resident beside the running one and
+//    its first weights are in shared memory when x arrives; for more rows, or very large matrices, it takes a whole SM.
 //  * The warps cut K between them and keep the activations of the 128 columns they work on in registers (mma B fragments),
-//    used for up to four 16-row tiles.  There is no CTA barrier inside the main loop.
+//    used for up to two 16-row tiles.  There is no CTA barrier inside the main loop.
 //  * One or two activation rows run on integer tensor cores (mma.m16n8k32, u8 x s8 -> s32; as fast per instruction as the
 //    fp16 one and twice the K).  x is staged as four signed base-256 digits of a 31-bit fixed-point number per 128 columns
 //    -- exact for every element above 2^-20 of the block's largest -- and the digits are columns of B.  A code byte
@@ -21,8 +21,12 @@
 //    all-ones A.  bf16 activations become fp16 with a power of two per 128 columns (exact).
 //  * Outlier columns (16-bit weights against the gathered x) are two more mma per tile and 32 columns at the end; the
 //    residual's projections V.x are computed by single warps of a few CTAs and travel as {value, launch tag} words.
-//  * The main loop is kept below the instruction cache of an SM partition (a body of about 16 KB measured 1.8 of 5.8
-//    cycles per instruction waiting for instructions).
+//  * The main loop is kept below the instruction cache of an SM partition.
+//
+// What is left (counters of cold launches): few warps and a short life.  14336 x 4096 INT2, 16 rows: 7.7 M warp instructions,
+// 23 % of the issue slots used by 9 warps an SM; of the 7 clocks between two instructions of a warp 2 are fixed latency, 1.9
+// waiting for instructions, 1.8 for the CTA's barrier.  8192 x 28672 INT4, 8 rows: 24 M, 40 % of the slots, 17 warps an SM, 2.5
+// clocks at the barrier (warps that are done wait for the others), 2.4 of latency; DRAM at a quarter.
 //
 // Replaces _decode_gemv (ai_accel_lab/kernels/decode_int2.py:43-96) and _decode_int4_gemv
 // (ai_accel_lab/kernels/groupwise_int4.py:85-107) of the reference project.
