@@ -216,7 +216,7 @@ class HybridPackedLinear(nn.Module):
             from .. import ops
             has_o = self.outlier_idx.numel() > 0
             state = ops.native().Linear(self.bits, self.original_k, self.group_size, 3 if self.gated_pairs else 0, self._kernel_code(),
-                                       self.in_features, self.out_features, min(self.chunked_max_rows, 16), packed, self.scales, self.bias,
+                                       self.in_features, self.out_features, max(4, min(self.chunked_max_rows, 16)), packed, self.scales, self.bias,
                                        self.outlier_idx if has_o else None, self.outlier_weight if has_o else None,
                                        self.res_u if self.residual_rank else None, self.res_v if self.residual_rank else None)
         d["_native_call"], d["_native_state"], d["_native_packed"] = state if self.prefetch_next is None else None, state, packed

@@ -197,3 +197,15 @@ def test_operands_given_other_memory_are_taken_up(rows):
     mod.scales.data = mod.scales.data * 2
     # a power of two is exact but for results among fp16's subnormals, which are 2^-24 apart
     assert float((mod(x).float() - 2 * want.float()).abs().max()) <= 2.0 ** -23
+
+
+def test_row_limit_leaves_the_decode_path_alone():
+    """``chunked_max_rows`` moves batches of 5 - 16 rows to the prompt route; one to four rows are the fused GEMV's whatever it says."""
+    torch.manual_seed(8)
+    mod = HybridInt4Linear(torch.nn.Linear(1024, 512), 128, None, 8)
+    mod.set_residual(torch.randn(512, 8) * 0.1, torch.randn(8, 1024) * 0.1)
+    mod = mod.cuda()
+    x = torch.randn(4, 1024).bfloat16().cuda()
+    want = mod(x)
+    mod.chunked_max_rows = 0
+    assert torch.equal(mod(x), want)
