@@ -3,22 +3,23 @@
 // The torch expression of the same algorithm (kernels/groupwise_int2.py, groupwise_int4.py) makes a temporary of the
 // matrix's size for every step of every candidate scale -- some 150 passes over memory at 13 candidates.  Here a group's
 // weights stay in registers: 16 consecutive columns per lane (times V for groups above 128), 2 - 8 lanes per group.  Bound
-// by instruction issue, not by HBM: 126 M warp instructions for 4096 x 4096 INT2, 18 per weight and candidate, at 63 % of the
-// issue slots with 12 warps an SM.
+// by instructions and their latency, not by HBM.
 // Measured, 4096 x 4096 INT2 with activation statistics (B200): torch expression 17.7 ms; 349 us with a decision per weight
-// by quotient or estimate; 228 us with the decision per candidate as below.
+// by quotient or estimate; 228 us with a decision per weight and candidate; 80 us as below.  INT4: 170 -> 110 us.
 //
-// Results are the expression's own: every operation is rounded as there (IEEE division, no contraction), and the squared
-// errors are added in the order in which the framework's reduction adds a contiguous row (four neighbours, then a binary
-// tree), so equal candidates are resolved alike.  Quotients are only computed for a candidate with an estimate too close to
-// a decision boundary to be sure (margins an order above the estimates' error); everywhere else |w| / s is estimated, and
-// the error follows from magnitudes alone: levels are symmetric.
+// Results are the expression's own: where it matters every operation is rounded as there (IEEE division, no contraction), and
+// the squared errors are added in the order in which the framework's reduction adds a contiguous row (four neighbours, then a
+// binary tree), so equal candidates are resolved alike.  But it rarely matters.  The candidates' errors are estimated first --
+// INT2: from a histogram of the weights over all candidates' decision boundaries, one pass instead of thirteen; INT4: candidate by
+// candidate, without looking at how close a decision was -- and only candidates that the estimate cannot tell apart are compared
+// by the exact sums (exact_search).  Codes likewise: a quotient only where the estimate is too close to a decision boundary.
 #include "qgemv_common.cuh"
 
 namespace qgemv {
 namespace {
 
 constexpr float kThird = 0.3333333432674408f;         // float32(1/3)
+constexpr float kMagic = 12582912.0f;                 // 1.5 * 2^23: adding and subtracting it rounds to an integer
 
 // Index of the closest level of x in (-1, -1/3, 1/3, 1), the first one on ties of the rounded distances.
 __device__ __noinline__ int closest_exact(float x) {
@@ -57,12 +58,42 @@ __device__ __forceinline__ float magnitude(float a, float w, float cand, float c
         margin = fminf(margin, fabsf(a - edge));
         return a > edge ? cand : cand3;
     } else {
-        const float t = a * inv, r = (t + 12582912.0f) - 12582912.0f;      // round to nearest even
+        const float t = a * inv, r = (t + kMagic) - kMagic;                // round to nearest even
         margin = fminf(margin, fabsf(fabsf(t - r) - 0.5f));
         return __fmul_rn(fminf(r, w < 0.0f ? 8.0f : 7.0f), cand);
     }
 }
 constexpr float kMargin = 1e-5f;
+
+// Code of w at scale s (edge = 2 / 3 s, inv ~ 1 / s) by estimate; false if it is too close to a decision boundary to be sure.
+template <int BITS>
+__device__ __forceinline__ bool code_estimate(float w, float s, float edge, float inv, int& c) {
+    const float a = fabsf(w);
+    if constexpr (BITS == 2) {
+        const int hi = a > edge ? 1 : 0;
+        c = a == 0.0f ? 1 : w < 0.0f ? 1 - hi : 2 + hi;                    // level -1/3 wins the tie at zero
+        return (a == 0.0f || a > kMargin * s) && fabsf(a - edge) > kMargin * s;
+    } else {
+        const float t = a * inv, r = (t + kMagic) - kMagic;
+        c = w < 0.0f ? -(int)fminf(r, 8.0f) : (int)fminf(r, 7.0f);
+        return fabsf(fabsf(t - r) - 0.5f) > kMargin && t < 65536.0f;
+    }
+}
+
+// Candidates whose estimated errors lie within this share of the group's energy (INT2: sum of aw w^2) or of the smallest error
+// (INT4) of the best one are compared by their exact errors.  Sums of at most 512 terms in fp32 are off by less than 1e-6 of
+// these figures, and a weight that an estimate puts on the wrong side of a decision boundary lies within 1e-6 of it, where
+// both sides give the same error.
+constexpr float kContender = 1e-5f;
+constexpr int kMaxFast = 16;                          // most candidates of a search by estimates
+
+// First candidate, and candidates per unit, if they are evenly spaced, ascending and positive; else {0, 0}.
+__device__ __forceinline__ float2 even_grid(const float* factors, int steps) {
+    const float f0 = factors[0], h = (factors[steps - 1] - f0) / (float)max(steps - 1, 1);
+    bool even = steps > 1 && f0 > 0.0f && h > 1e-3f;
+    for (int s = 1; s < steps; ++s) even = even && fabsf(factors[s] - (f0 + s * h)) <= 5e-7f * factors[steps - 1];
+    return even ? make_float2(f0, 1.0f / h) : make_float2(0.0f, 0.0f);
+}
 
 // max(x, 1e-8) that leaves NaN as it is, as the framework's clamp does.
 __device__ __forceinline__ float at_least_tiny(float x) { return x < 1e-8f ? 1e-8f : x; }
@@ -73,119 +104,270 @@ template <int DT> __device__ __forceinline__ float load_w(const void* w, size_t 
     else return static_cast<const float*>(w)[i];
 }
 
-// lg lanes per group, each 16 consecutive columns of every 128 (V of them).
+struct PackArgs {
+    const void* w;            long long ldw;
+    const float* rms;         const float* factors;
+    uint8_t* packed;          __half* scales;
+    int n, k, ng, group, lg, steps;           // lg: lanes per group, each 16 consecutive columns of every 128
+    bool vec, vec_rms;                        // 16-byte loads of w, rms
+};
+
+// Sixteen weights of a row from column k0, zero past the last one.
+template <int DT>
+__device__ __forceinline__ void load_weights(const PackArgs& p, int row, int k0, float (&f)[16]) {
+    if (p.vec && k0 + 16 <= p.k) {
+        if constexpr (DT == QGEMV_F32) {
+            const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(p.w) + (size_t)row * p.ldw + k0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { const float4 a = src[q]; f[q * 4] = a.x; f[q * 4 + 1] = a.y; f[q * 4 + 2] = a.z; f[q * 4 + 3] = a.w; }
+        } else {
+            const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __half*>(p.w) + (size_t)row * p.ldw + k0);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const uint4 a = src[q];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[q * 8 + e] = load_w<DT>(&a, e);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) f[e] = k0 + e < p.k ? load_w<DT>(p.w, (size_t)row * p.ldw + k0 + e) : 0.0f;
+    }
+}
+// What the squared errors of four columns from c count: the square of the statistics, at least 1e-8.
+__device__ __forceinline__ float4 load_energy(const PackArgs& p, int c) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.vec_rms && c + 4 <= p.k) a = __ldg(reinterpret_cast<const float4*>(p.rms + c));
+    else { if (c < p.k) a.x = p.rms[c]; if (c + 1 < p.k) a.y = p.rms[c + 1]; if (c + 2 < p.k) a.z = p.rms[c + 2]; if (c + 3 < p.k) a.w = p.rms[c + 3]; }
+    return make_float4(at_least_tiny(__fmul_rn(a.x, a.x)), at_least_tiny(__fmul_rn(a.y, a.y)), at_least_tiny(__fmul_rn(a.z, a.z)), at_least_tiny(__fmul_rn(a.w, a.w)));
+}
+
+// The best of the candidates in `mine`, by errors in which every operation is rounded as in the expression.  `visit`: the
+// candidates of all groups of the warp (the shuffles need it converged).  Out of line, with loads of its own: one group in a
+// hundred needs it, and its registers would halve the number of warps.
 template <int BITS, int V, int DT>
-__global__ void __launch_bounds__(256) pack_kernel(const void* __restrict__ w, long long ldw, int n, int k, int ng, int group, int lg,
-                                                   const float* __restrict__ rms, const float* __restrict__ factors, int steps,
-                                                   uint8_t* __restrict__ packed, __half* __restrict__ scales, bool vec, bool vec_rms) {
-    const long long groups = (long long)n * ng;
+__device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, float base, uint32_t visit, uint32_t mine, bool every) {
+    float f[V][16], aw[V][16], tiny = 3.0e38f;         // tiny: smallest magnitude that is not zero
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        load_weights<DT>(p, row, k0 + v * 128, f[v]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 a = load_energy(p, k0 + v * 128 + q * 4);
+            aw[v][q * 4] = a.x; aw[v][q * 4 + 1] = a.y; aw[v][q * 4 + 2] = a.z; aw[v][q * 4 + 3] = a.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) tiny = f[v][e] != 0.0f ? fminf(tiny, fabsf(f[v][e])) : tiny;
+    }
+    float best = 0.0f, chosen = base;
+    bool first = true;
+#pragma unroll 1
+    for (int s = 0; s < p.steps; ++s) {
+        if (!every && !(visit >> s & 1)) continue;
+        const float cand = __fmul_rn(base, p.factors[s]);
+        const float div = BITS == 2 ? fmaxf(cand, 1e-8f) : cand, inv = __fdividef(1.0f, div);
+        const float cand3 = __fmul_rn(kThird, cand), edge = 0.6666667f * div;
+        float e4[4][4];                                // [neighbour quadruple][element]: the framework's per-thread accumulators
+        float margin = BITS == 2 ? tiny : 1.0f;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float a = fabsf(f[v][e]);
+                const float d = __fsub_rn(magnitude<BITS>(a, f[v][e], cand, cand3, edge, inv, margin), a);
+                const float x = __fmul_rn(__fmul_rn(d, d), aw[v][e]);
+                e4[e >> 2][e & 3] = v == 0 ? x : __fadd_rn(e4[e >> 2][e & 3], x);
+            }
+        if (margin < (BITS == 2 ? kMargin * div : kMargin)) {       // rare: this lane's columns again, by quotients
+#pragma unroll 1
+            for (int e = 0; e < 16; ++e) {
+                float x = 0.0f;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    float w1 = 0.0f, b = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) if (i == e) { w1 = f[v][i]; b = aw[v][i]; }
+                    const float d = __fsub_rn(__fmul_rn(level_of<BITS>(code_exact<BITS>(w1, div, false)), cand), w1);
+                    const float y = __fmul_rn(__fmul_rn(d, d), b);
+                    x = v == 0 ? y : __fadd_rn(x, y);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) if (i == e) e4[i >> 2][i & 3] = x;
+            }
+        }
+        float t[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) t[q] = __fadd_rn(__fadd_rn(__fadd_rn(e4[q][0], e4[q][1]), e4[q][2]), e4[q][3]);
+        float err = __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
+        for (int o = 1; o < p.lg; o <<= 1) err = __fadd_rn(err, __shfl_xor_sync(0xffffffffu, err, o));
+        if (!every && !(mine >> s & 1)) continue;
+        if (first || err < best) { best = err; chosen = cand; }
+        first = false;
+    }
+    return chosen;
+}
+
+// Blocks of an SM, by registers: what a thread keeps is its weights.
+__host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ? (bits == 2 ? 4 : 3) : v == 2 ? (bits == 2 ? 3 : 2) : bits == 2 ? 2 : 1; }
+
+template <int BITS, int V, int DT>
+__global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const __grid_constant__ PackArgs p) {
+    __shared__ float2 bins[(kMaxFast + 1) * 256];      // [bin][thread]: (sum aw, sum aw |w|) of the thread's columns
+    float2* const mine = bins + threadIdx.x;
+    const int lg = p.lg, steps = p.steps;
+    float2 grid = make_float2(0.0f, 0.0f);
+    if (p.rms && steps <= kMaxFast) grid = even_grid(p.factors, steps);
+    const long long groups = (long long)p.n * p.ng;
     const int per_block = 256 / lg;
     const int sub = threadIdx.x / lg, l = threadIdx.x - sub * lg;
     const long long trips = (groups + per_block - 1) / per_block;
-    const int row_bytes = ng * group * BITS / 8;
+    const int row_bytes = p.ng * p.group * BITS / 8;
+    auto row_of = [&](long long i) { return groups < 0x80000000ll ? (int)((uint32_t)i / (uint32_t)p.ng) : (int)(i / p.ng); };
     for (long long trip = blockIdx.x; trip < trips; trip += gridDim.x) {
         const long long gi = min(trip * per_block + sub, groups - 1);       // the last block repeats a group: shuffles stay converged
-        const int row = (int)(gi / ng), grp = (int)(gi - (long long)row * ng);
-        float f[V][16], aw[V][16], tiny = 3.0e38f;                          // tiny: smallest magnitude that is not zero
+        const int row = row_of(gi), grp = (int)(gi - (long long)row * p.ng), k0 = grp * p.group + l * 16;
+        if (trip + gridDim.x < trips) {                // the next trip's weights to L2 meanwhile
+            const long long gn = min((trip + gridDim.x) * per_block + sub, groups - 1);
+            const int rn = row_of(gn), kn = (int)(gn - (long long)rn * p.ng) * p.group + l * 16;
+            if (kn < p.k) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p.w) + ((size_t)rn * p.ldw + kn) * (DT == QGEMV_F32 ? 4 : 2)));
+        }
+        float f[V][16];
         uint32_t peak_bits = 0;                                             // largest magnitude; by its bits, above which NaN's are
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            const int k0 = grp * group + v * 128 + l * 16;
-            if (vec && k0 + 16 <= k) {
-                if constexpr (DT == QGEMV_F32) {
-                    const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(w) + (size_t)row * ldw + k0);
+            load_weights<DT>(p, row, k0 + v * 128, f[v]);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) { const float4 a = src[q]; f[v][q * 4] = a.x; f[v][q * 4 + 1] = a.y; f[v][q * 4 + 2] = a.z; f[v][q * 4 + 3] = a.w; }
-                } else {
-                    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __half*>(w) + (size_t)row * ldw + k0);
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const uint4 a = src[q];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) f[v][q * 8 + e] = load_w<DT>(&a, e);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < 16; ++e) f[v][e] = k0 + e < k ? load_w<DT>(w, (size_t)row * ldw + k0 + e) : 0.0f;
-            }
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                peak_bits = max(peak_bits, __float_as_uint(fabsf(f[v][e])));
-                tiny = f[v][e] != 0.0f ? fminf(tiny, fabsf(f[v][e])) : tiny;
-            }
-            if (rms) {
-                const bool whole = k0 + 16 <= k && vec_rms;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-                    const int c = k0 + q * 4;
-                    if (whole) a = __ldg(reinterpret_cast<const float4*>(rms + c));
-                    else { if (c < k) a.x = rms[c]; if (c + 1 < k) a.y = rms[c + 1]; if (c + 2 < k) a.z = rms[c + 2]; if (c + 3 < k) a.w = rms[c + 3]; }
-                    aw[v][q * 4] = at_least_tiny(__fmul_rn(a.x, a.x)); aw[v][q * 4 + 1] = at_least_tiny(__fmul_rn(a.y, a.y));
-                    aw[v][q * 4 + 2] = at_least_tiny(__fmul_rn(a.z, a.z)); aw[v][q * 4 + 3] = at_least_tiny(__fmul_rn(a.w, a.w));
-                }
-            }
+            for (int e = 0; e < 16; ++e) peak_bits = max(peak_bits, __float_as_uint(fabsf(f[v][e])));
         }
         for (int o = 1; o < lg; o <<= 1) peak_bits = max(peak_bits, __shfl_xor_sync(0xffffffffu, peak_bits, o));
         const float peak = __uint_as_float(peak_bits), base = at_least_tiny(BITS == 2 ? peak : __fmul_rn(peak, 1.0f / 7.0f));
         float chosen = base;
-        if (rms) {
-            float best = 0.0f;
-            for (int s = 0; s < steps; ++s) {
-                const float cand = __fmul_rn(base, factors[s]);
-                const float div = BITS == 2 ? fmaxf(cand, 1e-8f) : cand, inv = __fdividef(1.0f, div);
-                const float cand3 = __fmul_rn(kThird, cand), edge = 0.6666667f * div;
-                float e4[4][4];                        // [neighbour quadruple][element]: the framework's per-thread accumulators
-                float margin = BITS == 2 ? tiny : 1.0f;
+        if (p.rms) {
+            // ---- which candidates can have the smallest error (a bit each), by estimates -------------------------
+            uint32_t contenders = 0xffffffffu;
+            const bool fast = grid.y > 0.0f;
+            if (fast) {
+                float lowest = 3.0e38f;
+                if constexpr (BITS == 2) {
+                    // The error of a candidate s follows from A = sum aw and B = sum aw |w| over |w| > 2/3 s: those take the level s,
+                    // the others s / 3.  A histogram over all candidates' boundaries gives every A and B in one pass.
+                    const float c1 = 1.5f * grid.y / base, c0 = 0.5f - grid.x * grid.y;      // rounds to the number of boundaries below
+                    __syncwarp();                       // the group's lanes have read the previous group's sums
+                    for (int s = 0; s <= steps; ++s) mine[s * 256] = make_float2(0.0f, 0.0f);
+                    float energy = 0.0f;
 #pragma unroll
-                for (int v = 0; v < V; ++v)
+                    for (int v = 0; v < V; ++v)
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        const float a = fabsf(f[v][e]);
-                        const float d = __fsub_rn(magnitude<BITS>(a, f[v][e], cand, cand3, edge, inv, margin), a);
-                        const float x = __fmul_rn(__fmul_rn(d, d), aw[v][e]);
-                        e4[e >> 2][e & 3] = v == 0 ? x : __fadd_rn(e4[e >> 2][e & 3], x);
-                    }
-                if (margin < (BITS == 2 ? kMargin * div : kMargin)) {       // rare: this lane's columns again, by quotients
-#pragma unroll 1
-                    for (int e = 0; e < 16; ++e) {
-                        float x = 0.0f;
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 x4 = load_energy(p, k0 + v * 128 + q * 4);
+                            const float x[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-                        for (int v = 0; v < V; ++v) {
-                            float w1 = 0.0f, b = 0.0f;
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) if (i == e) { w1 = f[v][i]; b = aw[v][i]; }
-                            const float d = __fsub_rn(__fmul_rn(level_of<BITS>(code_exact<BITS>(w1, div, false)), cand), w1);
-                            const float y = __fmul_rn(__fmul_rn(d, d), b);
-                            x = v == 0 ? y : __fadd_rn(x, y);
+                            for (int e = 0; e < 4; ++e) {
+                                const float a = fabsf(f[v][q * 4 + e]), xa = x[e] * a, t = fminf(fmaxf(fmaf(a, c1, c0), 0.0f), (float)steps);
+                                float2* const at = mine + (__float_as_int(t + kMagic) - __float_as_int(kMagic)) * 256;
+                                const float2 h = *at;
+                                *at = make_float2(h.x + x[e], h.y + xa);
+                                energy = fmaf(xa, a, energy);
+                            }
                         }
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) if (i == e) e4[i >> 2][i & 3] = x;
+                    for (int o = 1; o < lg; o <<= 1) energy += __shfl_xor_sync(0xffffffffu, energy, o);
+                    // sums from the top: lane l adds bin hi - l over the group's lanes, a scan over the lanes does the rest
+                    float2* const lane0 = mine - l;
+                    float2 carry = make_float2(0.0f, 0.0f);
+                    __syncwarp();
+                    for (int hi = steps; hi >= 0; hi -= lg) {
+                        const int b = hi - l;
+                        float2 r = make_float2(0.0f, 0.0f);
+                        if (b >= 0)
+                            for (int i = 0; i < lg; ++i) { const float2 h = lane0[b * 256 + ((l + i) & (lg - 1))]; r.x += h.x; r.y += h.y; }
+                        for (int o = 1; o < lg; o <<= 1) {
+                            const float x = __shfl_up_sync(0xffffffffu, r.x, o, lg), y = __shfl_up_sync(0xffffffffu, r.y, o, lg);
+                            if (l >= o) { r.x += x; r.y += y; }
+                        }
+                        r.x += carry.x; r.y += carry.y;
+                        carry = make_float2(__shfl_sync(0xffffffffu, r.x, lg - 1, lg), __shfl_sync(0xffffffffu, r.y, lg - 1, lg));
+                        __syncwarp();
+                        if (b >= 0) lane0[b * 256] = r;
                     }
-                }
-                float t[4];
+                    __syncwarp();
+                    auto error = [&](int s) {           // carry: the totals
+                        const float2 r = lane0[(s + 1) * 256];
+                        const float cand = base * p.factors[s], third = cand * kThird, ra = carry.x - r.x, rb = carry.y - r.y;
+                        return fmaf(cand, fmaf(cand, r.x, -2.0f * r.y), fmaf(third, fmaf(third, ra, -2.0f * rb), energy));
+                    };
+                    for (int s = l; s < steps; s += lg) lowest = fminf(lowest, error(s));
+                    for (int o = 1; o < lg; o <<= 1) lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
+                    contenders = 0;
+                    for (int s = l; s < steps; s += lg) contenders |= (error(s) <= lowest + kContender * energy ? 1u : 0u) << s;
+                    for (int o = 1; o < lg; o <<= 1) contenders |= __shfl_xor_sync(0xffffffffu, contenders, o);
+                    if (!(energy > 1e-30f && energy < 1e30f)) contenders = 0xffffffffu;
+                } else {
+                    float count[V][16];                 // what the columns count
 #pragma unroll
-                for (int q = 0; q < 4; ++q) t[q] = __fadd_rn(__fadd_rn(__fadd_rn(e4[q][0], e4[q][1]), e4[q][2]), e4[q][3]);
-                float err = __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
-                for (int o = 1; o < lg; o <<= 1) err = __fadd_rn(err, __shfl_xor_sync(0xffffffffu, err, o));
-                if (s == 0 || err < best) { best = err; chosen = cand; }
+                    for (int v = 0; v < V; ++v)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 x = load_energy(p, k0 + v * 128 + q * 4);
+                            count[v][q * 4] = x.x; count[v][q * 4 + 1] = x.y; count[v][q * 4 + 2] = x.z; count[v][q * 4 + 3] = x.w;
+                        }
+#pragma unroll 1
+                    for (int s = 0; s < steps; ++s) {
+                        const float cand = base * p.factors[s], inv = __fdividef(1.0f, cand);
+                        float e0 = 0.0f, e1 = 0.0f;
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) {
+                                const float a = fabsf(f[v][e]), r = fminf(fmaf(a, inv, kMagic) - kMagic, f[v][e] < 0.0f ? 8.0f : 7.0f);
+                                const float d = fmaf(r, cand, -a);
+                                if (e & 1) e1 = fmaf(d * count[v][e], d, e1); else e0 = fmaf(d * count[v][e], d, e0);
+                            }
+                        float err = e0 + e1;
+                        for (int o = 1; o < lg; o <<= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
+                        mine[s * 256].x = err;
+                        lowest = fminf(lowest, err);
+                    }
+                    contenders = 0;
+                    for (int s = 0; s < steps; ++s) contenders |= (mine[s * 256].x <= lowest + kContender * lowest ? 1u : 0u) << s;
+                    if (!(lowest > 1e-30f && lowest < 1e30f)) contenders = 0xffffffffu;
+                }
+            }
+            const bool decided = fast && __popc(contenders) == 1;
+            if (decided) chosen = __fmul_rn(base, p.factors[__ffs(contenders) - 1]);
+            const uint32_t visit = __reduce_or_sync(0xffffffffu, decided ? 0u : contenders);
+            if (visit) {
+                const float exact = exact_search<BITS, V, DT>(p, row, k0, base, visit, contenders, !fast);
+                if (!decided) chosen = exact;
             }
         }
-        if (l == 0) scales[(size_t)row * ng + grp] = __float2half_rn(chosen);
+        if (l == 0) p.scales[(size_t)row * p.ng + grp] = __float2half_rn(chosen);
+        const float edge = 0.6666667f * chosen, inv = __fdividef(1.0f, chosen);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            uint32_t word[BITS == 2 ? 1 : 2];
+            uint32_t word[BITS == 2 ? 1 : 2], unsure = 0;
 #pragma unroll
             for (int i = 0; i < (BITS == 2 ? 1 : 2); ++i) {
                 word[i] = 0;
 #pragma unroll
                 for (int e = 0; e < 32 / BITS; ++e) {
-                    const int c = code_exact<BITS>(f[v][i * (32 / BITS) + e], chosen, true) + (BITS == 4 ? 8 : 0);
-                    word[i] |= (uint32_t)c << (BITS * e);
+                    const int at = i * (32 / BITS) + e;
+                    int c;
+                    if (!code_estimate<BITS>(f[v][at], chosen, edge, inv, c)) unsure |= 1u << at;
+                    word[i] |= (uint32_t)(c + (BITS == 4 ? 8 : 0)) << (BITS * e);
                 }
             }
-            uint8_t* out = packed + (size_t)row * row_bytes + (size_t)(grp * group + v * 128 + l * 16) * BITS / 8;
+#pragma unroll 1
+            for (; unsure; unsure &= unsure - 1) {     // rare: by the quotient
+                const int e = __ffs(unsure) - 1, at = (BITS * e) & 31;
+                float w1 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) if (i == e) w1 = f[v][i];
+                const uint32_t c = (uint32_t)(code_exact<BITS>(w1, chosen, true) + (BITS == 4 ? 8 : 0)) << at;
+                const uint32_t keep = ~((BITS == 2 ? 3u : 15u) << at);
+                if (BITS == 4 && e >= 8) word[BITS == 2 ? 0 : 1] = (word[BITS == 2 ? 0 : 1] & keep) | c;
+                else word[0] = (word[0] & keep) | c;
+            }
+            uint8_t* out = p.packed + (size_t)row * row_bytes + (size_t)(k0 + v * 128) * BITS / 8;
             if constexpr (BITS == 2) *reinterpret_cast<uint32_t*>(out) = word[0];
             else *reinterpret_cast<uint2*>(out) = make_uint2(word[0], word[1]);
         }
@@ -214,10 +396,11 @@ extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int
     const int esize = w_dtype == QGEMV_F32 ? 4 : 2;
     const bool vec = reinterpret_cast<uintptr_t>(w) % 16 == 0 && ldw * esize % 16 == 0;
     const long long trips = ((long long)n * ng + 256 / lg - 1) / (256 / lg);
-    const int grid = (int)(trips < 148 * 16 ? trips : 148 * 16);
+    const int most = 148 * pack_blocks(bits, v);       // as many blocks as are resident
+    const int grid = (int)(trips < most ? trips : most);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    __half* sc = static_cast<__half*>(scales);
-#define QP(B, V, D) pack_kernel<B, V, D><<<grid, 256, 0, s>>>(w, ldw, n, k, ng, group, lg, rms, factors, steps, packed, sc, vec, reinterpret_cast<uintptr_t>(rms) % 16 == 0)
+    const PackArgs a{w, ldw, rms, factors, packed, static_cast<__half*>(scales), n, k, ng, group, lg, steps, vec, reinterpret_cast<uintptr_t>(rms) % 16 == 0};
+#define QP(B, V, D) pack_kernel<B, V, D><<<grid, 256, 0, s>>>(a)
 #define QP_D(B, V) do { if (w_dtype == QGEMV_F16) QP(B, V, QGEMV_F16); else if (w_dtype == QGEMV_BF16) QP(B, V, QGEMV_BF16); else QP(B, V, QGEMV_F32); } while (0)
 #define QP_V(B) do { if (v == 1) QP_D(B, 1); else if (v == 2) QP_D(B, 2); else QP_D(B, 4); } while (0)
     if (bits == 2) QP_V(2); else QP_V(4);

@@ -74,3 +74,35 @@ def test_pack_of_values_that_are_not_finite(monkeypatch, bits):
         assert torch.equal(got.scales.isnan(), want.scales.isnan()) and torch.equal(got.scales.nan_to_num(), want.scales.nan_to_num())
         finite = want.scales.isfinite().repeat_interleave(64 * bits // 8, dim=1)      # NaN has no code
         assert torch.equal(got.packed[finite], want.packed[finite])
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("steps", [1, 2, 16, 17, 40])
+def test_pack_searches_any_number_of_candidates(monkeypatch, bits, steps):
+    """Up to 16 candidates are told apart by estimates, more are all compared exactly; heavy tails, exact ties between candidates
+    (weights on a coarse grid) and groups of zeros leave several that the estimates cannot tell apart."""
+    mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
+    g = torch.Generator(device="cuda").manual_seed(steps)
+    w = torch.empty((96, 640), device="cuda").normal_(0, 0.02, generator=g)
+    w[32:64] = (w[32:64] * 100).round() / 100
+    w[64:] *= torch.empty((32, 640), device="cuda").log_normal_(0, 2, generator=g)
+    w[5] = 0
+    rms = torch.empty(640, device="cuda").log_normal_(0, 2, generator=g)
+    got = fn(w, 128, rms, steps)
+    with monkeypatch.context() as m:
+        m.setattr(mod, "_pack_on_device", lambda *a: None)
+        want = fn(w, 128, rms, steps)
+    differ = got.scales != want.scales
+    same = ~differ.repeat_interleave(16 * bits, dim=1)
+    assert torch.equal(got.packed[same], want.packed[same])
+    # Where another candidate was taken, its error in 64 bits is as small as far as sums of 128 terms in 32 bits can tell: 128 * 2^-24.
+    group = w.view(96, 5, 128)[differ]
+    base = (group.abs().amax(-1) / (1 if bits == 2 else 7)).clamp_min(1e-8)
+    factors = torch.linspace(*((0.55, 1.15) if bits == 2 else (0.72, 1.18)), steps, device="cuda")
+    cand = (base[:, None] * factors).double()
+    x = group.double()[:, None, :] / cand[..., None]
+    level = ((x.clamp(-1, 1) * 3 + 3) / 2).round() * 2 / 3 - 1 if bits == 2 else x.round().clamp(-8, 7)
+    energy = rms.view(5, 128).square().clamp_min(1e-8).double().expand(96, 5, 128)[differ][:, None, :]
+    error = ((level * cand[..., None] - group.double()[:, None, :]).square() * energy).sum(-1)
+    taken = [error.gather(1, (cand - q.scales[differ].double()[:, None]).abs().argmin(1, keepdim=True)) for q in (got, want)]
+    assert bool(((taken[0] - taken[1]).abs() <= 128 * 2.0 ** -24 * taken[1]).all())
