@@ -153,8 +153,9 @@ extern "C" const char* qgemv_plan_name(const qgemv_problem* p) {
 namespace {
 
 // Validate, pick a kernel, launch.  `partial_floats` is the capacity of the partial-sum area of
-// the workspace the problem points at; `ordered`: the launch must not overlap the work issued before it.
-int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t partial_floats, bool ordered) {
+// the workspace the problem points at; `ordered`: the launch must not overlap the work issued before it; `x_follows`: align_x_kernel
+// has just been launched for it.
+int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t partial_floats, bool ordered, bool x_follows = false) {
     const int v = validate(p, need_bytes);
     if (v != QGEMV_OK) return v;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -164,6 +165,7 @@ int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t 
     bool missing = false;
     MmaPlan plan = choose(*p, partial_floats, &missing);
     plan.ordered = ordered;
+    plan.x_follows = x_follows;
     const bool use_mma = plan.ok;
     {
         if (missing) {
@@ -173,7 +175,7 @@ int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t 
             return QGEMV_ERR_SHAPE;
         }
     }
-    if (a.rank > 0 && !(use_mma && plan.t_inline)) {
+    if (a.rank > 0 && !(use_mma && plan.t_inline) && !x_follows) {
         const int r = launch_residual_t(a, bf16, s);
         if (r != QGEMV_OK) return r;
     }
@@ -308,8 +310,12 @@ extern "C" int qgemv_run_ordered(const qgemv_problem* p, void* stream) {
 namespace {
 struct Prepared {                                  // what qgemv_prepare writes into the caller's buffer
     qgemv_problem problem;
+    int pitch;                                     // > 0: qgemv_run on a copy of x with rows of this many elements, in the workspace
+    bool project;                                  // the copying launch also makes the residual projections
     StreamPlan plan;                               // ok == false: as qgemv_run, four rows at a time
 };
+// The copy of x: inside the scratch for partial sums, behind what the tensor-core kernel uses of it for itself.
+constexpr size_t kCopyOff = kWsPartialOff + (size_t(2) << 20), kCopyBytes = size_t(1) << 20;
 }  // namespace
 
 extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
@@ -332,6 +338,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     Prepared* q = static_cast<Prepared*>(prepared);
     q->problem = *p;
     q->plan = StreamPlan{};
+    q->pitch = 0; q->project = false;
     const bool padded = p->ldx >= p->k_padded && p->k_padded == p->k_original;
     bool starved = false;
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && padded) {
@@ -339,6 +346,24 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         const MmaPlan plan = choose(*p, kMaxPartialFloats, &none);
         const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
+    }
+    // One to four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of its
+    // 16 warps (see align_x_kernel).  Rows that leave it fewer stay with the streaming kernel, whose one launch takes x as it is (512 x 10001
+    // INT4, M = 4: 20 us either way), and so do calls that it finishes in less than the 8 us that two launches cost an eager caller on the
+    // host: no residual (with one it takes 8.4 us and more, the two launches 6.2 on the GPU) and few bytes (8192 x 1500 INT4, M = 1: 6.2 us;
+    // 8192 x 4300: 11.3, two launches 10.5; 4096 x 10001 INT2 14.4 and 10.6), unless three or four long rows make it slow (512 x 4300: 9.3).
+    if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && (!padded || p->ldx % 8)) {
+        qgemv_problem c = *p;                          // (as the streaming kernel, only x that starts on 16 bytes)
+        c.ldx = ((int64_t)p->k_padded + 7) / 8 * 8;
+        c.x = static_cast<char*>(p->workspace) + kCopyOff;
+        bool none = false;
+        const MmaPlan plan = choose(c, kMaxPartialFloats, &none);
+        const bool pays = p->rank > 0 || (size_t)p->n * p->k_padded * p->bits / 8 >= (size_t(8) << 20) || (p->m >= 3 && p->k_original >= 4096);
+        if (aligned(p->x, 16) && plan.ok && plan.variant == 1 && plan.nw >= 16 && pays && (size_t)c.m * c.ldx * 2 <= kCopyBytes) {
+            q->pitch = (int)c.ldx;
+            q->project = p->rank > 0 && !plan.t_inline;
+            return QGEMV_OK;
+        }
     }
     if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8 || starved) &&
         plan_stream(*p, kMaxPartialFloats, &q->plan))
@@ -364,6 +389,16 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
     }
     qgemv_problem p = q->problem;
     p.workspace = workspace;
+    if (q->pitch) {
+        if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
+        cudaStream_t s = static_cast<cudaStream_t>(stream);
+        char* const copy = static_cast<char*>(workspace) + kCopyOff;
+        p.x = x; p.y = y;
+        const int r = launch_align_x(make_args(p, kMaxPartialFloats), p.x_dtype == QGEMV_BF16, copy, q->pitch, q->project, !ordered, s);
+        if (r != QGEMV_OK) return r;
+        p.x = copy; p.ldx = q->pitch;
+        return run_checked(&p, stream, 0, kMaxPartialFloats, false, true);      // overlaps the copying launch only
+    }
     for (int lo = 0; lo < q->problem.m; lo += QGEMV_MAX_M) {
         p.m = q->problem.m - lo < QGEMV_MAX_M ? q->problem.m - lo : QGEMV_MAX_M;
         p.x = static_cast<const char*>(x) + (size_t)lo * p.ldx * 2;

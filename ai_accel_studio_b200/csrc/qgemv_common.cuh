@@ -76,10 +76,13 @@ int  check_launch(const char* what);
 size_t gemm_scratch_bytes(const qgemv_problem& p);
 int run_gemm(const qgemv_problem& p, void* scratch, size_t scratch_bytes, cudaStream_t s);
 int launch_residual_t(const Args& a, bool bf16, cudaStream_t s);
+// x to rows of `pitch` at `to` and, if asked, the residual projections; `dependent`: the weights (V) are final.
+int launch_align_x(const Args& a, bool bf16, void* to, int pitch, bool project, bool dependent, cudaStream_t s);
 int launch_simt(const Args& a, int bits, bool bf16, int unit_bytes, cudaStream_t s);
 const char* simt_name(int bits, int m, int unit_bytes);
 
 struct MmaPlan {
+    bool x_follows;         // x, and residual projections that are not made inside, come from the launch just before this one
     bool ordered;           // the launch must not overlap the preceding kernel of the stream, which may be writing the weights
     bool ok;
     int gb;                 // packed bytes per group per row (16, 32 or 64)

@@ -865,7 +865,7 @@ int launch_mma(const Args& a, int bits, bool bf16, const MmaPlan& pl, int debug,
     p.off_xo = pl.off_xo; p.off_gx = pl.off_gx; p.off_slots = pl.off_slots; p.off_epi = pl.off_epi;
     p.off_meta = pl.off_meta; p.off_xs = pl.off_xs; p.off_ring = pl.off_ring;
     p.t_inline = pl.t_inline; p.t_parts = pl.t_parts; p.off_tt = pl.off_tt;
-    p.wait_for_x = (a.rank > 0 && !pl.t_inline) ? 0 : pl.ordered ? 2 : 1;
+    p.wait_for_x = pl.x_follows ? 1 : (a.rank > 0 && !pl.t_inline) ? 0 : pl.ordered ? 2 : 1;
     p.debug = debug;
     p.tile_aligned = pl.tile_aligned;
     return bits == 2 ? launch_mma_int2(p, pl.gb, bf16, pl.grid, pl.smem_bytes, s)

@@ -264,6 +264,60 @@ __global__ void __launch_bounds__(256) residual_t_kernel(const Args a) {
     }
 }
 
+// x whose rows end before the padded K, or are not 16-byte aligned, as the tensor-core kernel wants it: the first `project` CTAs
+// project a residual row each, the others copy 2048 columns of a row of x into `to` (rows of `pitch`, zeros past the last column).
+// Latency is its bound: two-byte loads, but all of a thread's at once, those of V before the dependency wait.  It stands before a kernel
+// that then needs no code for odd x: 4999 x 4300 INT4, three bf16 rows, odd rank 17.1 us as one streaming launch, 13.0 as these two
+// (15.1 with 512 threads a CTA, whose loads came in two rounds); 8192 x 8200 INT4, four rows 37.0 -> 19.8; 3000 x 5001 INT2, three rows
+// 26.1 -> 12.2.
+template <bool BF16>
+__global__ void __launch_bounds__(1024) align_x_kernel(const Args a, unsigned short* to, int pitch, int project) {
+    using XT = typename Act16<BF16>::T;
+    constexpr int B = 6;                               // columns a thread projects at a time
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int r = blockIdx.x, tid = threadIdx.x;
+    if (r >= project) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const int chunks = (pitch + 2047) / 2048, c = r - project, m = c / chunks, k = (c - m * chunks) * 2048 + tid * 2;
+        const unsigned short* x = static_cast<const unsigned short*>(a.x) + (size_t)m * a.ldx;
+        const uint32_t lo = k < a.korig ? x[k] : 0, hi = k + 1 < a.korig ? x[k + 1] : 0;
+        if (k < pitch) *reinterpret_cast<uint32_t*>(to + (size_t)m * pitch + k) = lo | hi << 16;      // the pitch is even
+        return;
+    }
+    const __half* v = a.rv + (size_t)r * a.ldv;
+    const XT* x = static_cast<const XT*>(a.x);
+    float s[QGEMV_MAX_M] = {0.f, 0.f, 0.f, 0.f};
+    for (int k0 = tid; k0 - tid < a.korig; k0 += B * 1024) {
+        float f[B], g[B][QGEMV_MAX_M];
+#pragma unroll
+        for (int i = 0; i < B; ++i) f[i] = k0 + i * 1024 < a.korig ? __half2float(v[k0 + i * 1024]) : 0.0f;
+        if (k0 == tid) asm volatile("griddepcontrol.wait;" ::: "memory");             // V is a weight
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+            for (int m = 0; m < QGEMV_MAX_M; ++m)
+                g[i][m] = m < a.m && k0 + i * 1024 < a.korig ? Act16<BF16>::to_float(x[(size_t)m * a.ldx + k0 + i * 1024]) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+            for (int m = 0; m < QGEMV_MAX_M; ++m) s[m] = fmaf(f[i], g[i][m], s[m]);
+    }
+    __shared__ float red[32][QGEMV_MAX_M];
+#pragma unroll
+    for (int m = 0; m < QGEMV_MAX_M; ++m) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[m] += __shfl_xor_sync(0xffffffffu, s[m], o);
+        if ((tid & 31) == 0) red[tid >> 5][m] = s[m];
+    }
+    __syncthreads();
+    if (tid < a.m) {
+        float tot = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) tot += red[i][tid];
+        a.t[tid * kMaxRank + r] = tot;
+    }
+}
+
 template <int BITS, int M, int U>
 int launch_simt_bmu(const Args& a, bool bf16, cudaStream_t s) {
     dim3 grid((a.n + kRowsPerBlock - 1) / kRowsPerBlock), block(kThreads);
@@ -296,6 +350,23 @@ int launch_residual_t(const Args& a, bool bf16, cudaStream_t s) {
     if (bf16) residual_t_kernel<true><<<grid, block, 0, s>>>(a);
     else      residual_t_kernel<false><<<grid, block, 0, s>>>(a);
     return check_launch("residual_t_kernel");
+}
+
+int launch_align_x(const Args& a, bool bf16, void* to, int pitch, bool project, bool dependent, cudaStream_t s) {
+    const int rows = project ? a.rank : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows + a.m * ((pitch + 2047) / 2048));
+    cfg.blockDim = dim3(1024);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    unsigned short* const dst = static_cast<unsigned short*>(to);
+    if (bf16) (void)cudaLaunchKernelEx(&cfg, align_x_kernel<true>, a, dst, pitch, rows);
+    else (void)cudaLaunchKernelEx(&cfg, align_x_kernel<false>, a, dst, pitch, rows);
+    return check_launch("align_x_kernel");
 }
 
 int launch_simt(const Args& a, int bits, bool bf16, int unit_bytes, cudaStream_t s) {

@@ -7,8 +7,8 @@ import torch
 
 from conftest import ABS_TOL, REL_TOL, c_forward
 from ai_accel_studio_b200 import ops
-from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2
-from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4
+from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2, unpack_groupwise_int2
+from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4, unpack_groupwise_int4
 from ai_accel_studio_b200.optimize import HybridInt2Linear, HybridInt4Linear
 
 pytestmark = pytest.mark.gpu
@@ -209,3 +209,34 @@ def test_row_limit_leaves_the_decode_path_alone():
     want = mod(x)
     mod.chunked_max_rows = 0
     assert torch.equal(mod(x), want)
+
+
+# one column short of, at and past a copying CTA's 2048 columns and a projecting CTA's 6144; K a multiple of 8 but not of the group (projections made
+# inside the GEMV) and not (made by the copying launch); rows of x that are not 16-byte aligned
+@pytest.mark.parametrize("bits,n,k,group,oc,rank", [(4, 40, 2047, 128, 0, 1), (2, 17, 2049, 64, 3, 5), (4, 200, 6143, 64, 8, 8), (2, 200, 6145, 256, 0, 64),
+                                                    (4, 64, 4104, 128, 32, 8), (2, 2400, 1003, 128, 16, 0)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_rows_of_odd_x_are_copied_first(bits, n, k, group, oc, rank, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    w = torch.empty((n, k), device="cuda").normal_(0, 0.05, generator=g)
+    pw = (pack_groupwise_int2 if bits == 2 else pack_groupwise_int4)(w, group)
+    oidx = torch.randperm(k, generator=g, device="cuda")[:oc].to(torch.int32)
+    ow = torch.empty((n, oc), device="cuda").normal_(0, 0.05, generator=g).half()
+    ru = torch.empty((n, rank), device="cuda").normal_(0, 0.05, generator=g).half()
+    rv = torch.empty((rank, k), device="cuda").normal_(0, 0.05, generator=g).half()
+    cls = HybridInt2Linear if bits == 2 else HybridInt4Linear
+    mod = cls.from_buffers(pw.packed, pw.scales, k, group, oidx, ow, None, *((ru, rv) if rank else (None, None)))
+    dense = (unpack_groupwise_int2 if bits == 2 else unpack_groupwise_int4)(pw).double()[:, :k]
+    for rows in (1, 2, 3, 4):
+        x = torch.empty((rows, k), device="cuda").normal_(0, 1, generator=g).to(dtype)
+        xd = x.double()
+        ref = xd @ dense.T + xd[:, oidx.long()] @ ow.double().T + (xd @ rv.double().T) @ ru.double().T
+        rel = REL_TOL if dtype == torch.float16 else 2.0 ** -8
+        y = mod(x)
+        assert float((y.double() - ref).norm()) <= rel * float(ref.norm()), rows
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = mod(x)
+        graph.replay()
+        assert torch.equal(captured, y) and torch.equal(mod(x), y)
+    assert ops.workspace_status("cuda") == 0
