@@ -88,12 +88,13 @@ __device__ __forceinline__ bool code_estimate(float w, float s, float edge, floa
 constexpr float kContender = 1e-5f;
 constexpr int kMaxFast = 16;                          // most candidates of a search by estimates
 
-// First candidate, and candidates per unit, if they are evenly spaced, ascending and positive; else {0, 0}.
+// First candidate, and candidates per unit, if they are evenly spaced, ascending and positive; else {0, 0}.  A lane checks one of at most
+// kMaxFast, so that small matrices wait for one load, not for a row of them.  All lanes of the warp call it.
 __device__ __forceinline__ float2 even_grid(const float* factors, int steps) {
     const float f0 = factors[0], h = (factors[steps - 1] - f0) / (float)max(steps - 1, 1);
-    bool even = steps > 1 && f0 > 0.0f && h > 1e-3f;
-    for (int s = 1; s < steps; ++s) even = even && fabsf(factors[s] - (f0 + s * h)) <= 5e-7f * factors[steps - 1];
-    return even ? make_float2(f0, 1.0f / h) : make_float2(0.0f, 0.0f);
+    const int s = min((int)(threadIdx.x & 31), steps - 1);
+    const bool even = steps > 1 && f0 > 0.0f && h > 1e-3f && fabsf(factors[s] - (f0 + s * h)) <= 5e-7f * factors[steps - 1];
+    return __all_sync(0xffffffffu, even) ? make_float2(f0, 1.0f / h) : make_float2(0.0f, 0.0f);
 }
 
 // max(x, 1e-8) that leaves NaN as it is, as the framework's clamp does.
@@ -214,8 +215,8 @@ __host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ?
 
 template <int BITS, int V, int DT>
 __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const __grid_constant__ PackArgs p) {
-    __shared__ float2 bins[(kMaxFast + 1) * 256];      // [bin][thread]: (sum aw, sum aw |w|) of the thread's columns
-    float2* const mine = bins + threadIdx.x;
+    __shared__ float2 bins[BITS == 2 ? (kMaxFast + 1) * 256 : 1];        // INT2: [bin][thread], (sum aw, sum aw |w|) of the thread's columns
+    [[maybe_unused]] float2* const mine = bins + (BITS == 2 ? threadIdx.x : 0);
     const int lg = p.lg, steps = p.steps;
     float2 grid = make_float2(0.0f, 0.0f);
     if (p.rms && steps <= kMaxFast) grid = even_grid(p.factors, steps);
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                             const float4 x = load_energy(p, k0 + v * 128 + q * 4);
                             count[v][q * 4] = x.x; count[v][q * 4 + 1] = x.y; count[v][q * 4 + 2] = x.z; count[v][q * 4 + 3] = x.w;
                         }
+                    contenders = 0;
 #pragma unroll 1
                     for (int s = 0; s < steps; ++s) {
                         const float cand = base * p.factors[s], inv = __fdividef(1.0f, cand);
@@ -326,11 +328,11 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                             }
                         float err = e0 + e1;
                         for (int o = 1; o < lg; o <<= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
-                        mine[s * 256].x = err;
+                        // all within reach of the lowest so far; a lower one drops those that it has left behind.  What stays of a slow
+                        // descent is compared by exact errors, too, which cannot change the choice.
+                        if (err <= lowest + kContender * lowest) contenders = (lowest <= err + kContender * err ? contenders : 0u) | 1u << s;
                         lowest = fminf(lowest, err);
                     }
-                    contenders = 0;
-                    for (int s = 0; s < steps; ++s) contenders |= (mine[s * 256].x <= lowest + kContender * lowest ? 1u : 0u) << s;
                     if (!(lowest > 1e-30f && lowest < 1e30f)) contenders = 0xffffffffu;
                 }
             }
