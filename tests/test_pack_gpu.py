@@ -106,3 +106,19 @@ def test_pack_searches_any_number_of_candidates(monkeypatch, bits, steps):
     error = ((level * cand[..., None] - group.double()[:, None, :]).square() * energy).sum(-1)
     taken = [error.gather(1, (cand - q.scales[differ].double()[:, None]).abs().argmin(1, keepdim=True)) for q in (got, want)]
     assert bool(((taken[0] - taken[1]).abs() <= 128 * 2.0 ** -24 * taken[1]).all())
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("group", [64, 256])
+def test_pack_with_statistics_whose_sums_overflow(monkeypatch, bits, group):
+    """Statistics whose squares add up beyond the type's range, over weights so small that the squared errors do not: the search
+    goes by the errors, as in the torch expression."""
+    mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
+    g = torch.Generator(device="cuda").manual_seed(group)
+    w = torch.empty((256, 1024), device="cuda").normal_(0, 1e-5, generator=g)
+    rms = torch.empty(1024, device="cuda").uniform_(4e18, 1.8e19, generator=g)
+    got = fn(w, group, rms)
+    with monkeypatch.context() as m:
+        m.setattr(mod, "_pack_on_device", lambda *a: None)
+        want = fn(w, group, rms)
+    assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
