@@ -303,8 +303,9 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                     contenders = 0;
                     for (int s = l; s < steps; s += lg) contenders |= (error(s) <= lowest + kContender * energy ? 1u : 0u) << s;
                     for (int o = 1; o < lg; o <<= 1) contenders |= __shfl_xor_sync(0xffffffffu, contenders, o);
-                    // out of range, or sums of aw that overflowed where those of aw w^2 did not: no estimate
-                    if (!(energy > 1e-30f && energy < 1e30f && lowest < 1e30f) || !contenders) contenders = 0xffffffffu;
+                    // No estimate: out of range; sums of aw that overflowed where those of aw w^2 did not; candidates below 1e-8,
+                    // where the expression divides by 1e-8 instead and so has other decision boundaries.
+                    if (!(energy > 1e-30f && energy < 1e30f && lowest < 1e30f && base * grid.x >= 1e-8f) || !contenders) contenders = 0xffffffffu;
                 } else {
                     float count[V][16];                 // what the columns count
 #pragma unroll

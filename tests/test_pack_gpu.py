@@ -122,3 +122,20 @@ def test_pack_with_statistics_whose_sums_overflow(monkeypatch, bits, group):
         m.setattr(mod, "_pack_on_device", lambda *a: None)
         want = fn(w, group, rms)
     assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("group", [32, 128])
+def test_pack_of_groups_near_the_smallest_scale(monkeypatch, bits, group):
+    """Peaks from below to well above 1e-8: the expression divides by no less than that, whatever the candidate is."""
+    mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
+    g = torch.Generator(device="cuda").manual_seed(group)
+    w = torch.empty((512, 512), device="cuda").normal_(0, 1, generator=g)
+    w *= torch.logspace(-9.5, -6, 512, device="cuda")[:, None]
+    rms = torch.empty(512, device="cuda").log_normal_(0, 1, generator=g)
+    for dtype in (torch.float32, torch.bfloat16):
+        got = fn(w.to(dtype), group, rms)
+        with monkeypatch.context() as m:
+            m.setattr(mod, "_pack_on_device", lambda *a: None)
+            want = fn(w.to(dtype), group, rms)
+        assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
