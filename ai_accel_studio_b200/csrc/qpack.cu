@@ -81,11 +81,18 @@ __device__ __forceinline__ bool code_estimate(float w, float s, float edge, floa
     }
 }
 
-// Candidates whose estimated errors lie within this share of the group's energy (INT2: sum of aw w^2) or of the smallest error
-// (INT4) of the best one are compared by their exact errors.  Sums of at most 512 terms in fp32 are off by less than 1e-6 of
-// these figures, and a weight that an estimate puts on the wrong side of a decision boundary lies within 1e-6 of it, where
-// both sides give the same error.
-constexpr float kContender = 1e-5f;
+// Candidates whose estimated errors exceed the smallest one by no more than kErrorShare of it plus kEnergyShare of the group's energy
+// N = sum of aw w^2 are compared by their exact errors E.  What separates estimates and exact errors (u = 2^-24):
+// INT4: the expression rounds the level times the candidate, which can change E by 2 u sqrt(E N), 4 u sqrt(E N) <= 28 u E + u N / 7 for two
+//   candidates; it decides by a rounded quotient, the estimate by a reciprocal within u, so that a weight within 16 u of a decision
+//   boundary may get the other level, which changes its term by 128 u; the sums' roundings come to a few u E.  (With 1e-5 E alone, no N and
+//   a reciprocal within 4 u, the best of two candidates was dropped whose levels lie on either side of a weight, close to it.)
+// INT2: the estimate is a sum of terms of up to 12.5 N + 4 E altogether, since the weights below a decision boundary enter by
+//   aw s^2 / 9 <= 2 aw (s / 3 - |w|)^2 + 2 aw w^2.  They are sums of up to 16 V + 17 steps, whose roundings (not their bound, which is
+//   tenfold) come to 1 - 1.5 u of a term: some 4 u E + 12 u N between two candidates, a tenth of what is allowed for.  A weight on the wrong side of a
+//   boundary lies within 25 u of it and changes its term by 50 u aw w^2.
+constexpr float kErrorShare = 1e-5f;
+template <int BITS> constexpr float kEnergyShare = BITS == 4 ? 1e-8f : 1e-5f;
 constexpr int kMaxFast = 16;                          // most candidates of a search by estimates
 
 // First candidate, and candidates per unit, if they are evenly spaced, ascending and positive; else {0, 0}.  A lane checks one of at most
@@ -300,25 +307,30 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                     };
                     for (int s = l; s < steps; s += lg) lowest = fminf(lowest, error(s));
                     for (int o = 1; o < lg; o <<= 1) lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
+                    const float reach = lowest + (kErrorShare * lowest + kEnergyShare<BITS> * energy);
                     contenders = 0;
-                    for (int s = l; s < steps; s += lg) contenders |= (error(s) <= lowest + kContender * energy ? 1u : 0u) << s;
+                    for (int s = l; s < steps; s += lg) contenders |= (error(s) <= reach ? 1u : 0u) << s;
                     for (int o = 1; o < lg; o <<= 1) contenders |= __shfl_xor_sync(0xffffffffu, contenders, o);
                     // No estimate: out of range; sums of aw that overflowed where those of aw w^2 did not; candidates below 1e-8,
                     // where the expression divides by 1e-8 instead and so has other decision boundaries.
                     if (!(energy > 1e-30f && energy < 1e30f && lowest < 1e30f && base * grid.x >= 1e-8f) || !contenders) contenders = 0xffffffffu;
                 } else {
-                    float count[V][16];                 // what the columns count
+                    float count[V][16], energy = 0.0f;  // what the columns count
 #pragma unroll
                     for (int v = 0; v < V; ++v)
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             const float4 x = load_energy(p, k0 + v * 128 + q * 4);
                             count[v][q * 4] = x.x; count[v][q * 4 + 1] = x.y; count[v][q * 4 + 2] = x.z; count[v][q * 4 + 3] = x.w;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) energy = fmaf(count[v][q * 4 + e] * f[v][q * 4 + e], f[v][q * 4 + e], energy);
                         }
+                    for (int o = 1; o < lg; o <<= 1) energy += __shfl_xor_sync(0xffffffffu, energy, o);
+                    const float always = kEnergyShare<BITS> * energy;
                     contenders = 0;
 #pragma unroll 1
                     for (int s = 0; s < steps; ++s) {
-                        const float cand = base * p.factors[s], inv = __fdividef(1.0f, cand);
+                        const float cand = base * p.factors[s], near = __fdividef(1.0f, cand), inv = fmaf(fmaf(-cand, near, 1.0f), near, near);
                         float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
                         for (int v = 0; v < V; ++v)
@@ -332,7 +344,8 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                         for (int o = 1; o < lg; o <<= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
                         // all within reach of the lowest so far; a lower one drops those that it has left behind.  What stays of a slow
                         // descent is compared by exact errors, too, which cannot change the choice.
-                        if (err <= lowest + kContender * lowest) contenders = (lowest <= err + kContender * err ? contenders : 0u) | 1u << s;
+                        if (err <= lowest + (kErrorShare * lowest + always))
+                            contenders = (lowest <= err + (kErrorShare * err + always) ? contenders : 0u) | 1u << s;
                         lowest = fminf(lowest, err);
                     }
                     if (!(lowest > 1e-30f && lowest < 1e30f)) contenders = 0xffffffffu;

@@ -139,3 +139,27 @@ def test_pack_of_groups_near_the_smallest_scale(monkeypatch, bits, group):
             m.setattr(mod, "_pack_on_device", lambda *a: None)
             want = fn(w.to(dtype), group, rms)
         assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
+
+
+@pytest.mark.parametrize("group,steps", [(16, 11), (128, 11), (128, 16), (512, 16)])
+def test_pack_int4_of_weights_between_the_levels_of_two_candidates(monkeypatch, group, steps):
+    """One weight decides a group's scale and lies midway, to a few units in the last place, between the levels that two candidates give
+    it, which are within 1 % of each other: its differences from them are so small that the roundings of the levels count."""
+    levels = (torch.linspace(0.72, 1.18, steps).double()[:, None] * torch.arange(1, 8)).flatten()
+    lower, upper = levels[:, None], levels[None, :]
+    near = (lower < upper) & (upper - lower < 0.01 * lower) & (lower + upper < 14)
+    middles = ((lower + upper) / 2)[near].cuda()
+    g = torch.Generator(device="cuda").manual_seed(group + steps)
+    rows = 1 << 14
+    base = torch.empty(rows, device="cuda").uniform_(0.01, 1, generator=g)
+    middle = (middles[torch.randint(0, len(middles), (rows,), generator=g, device="cuda")] * base.double()).float()
+    w = torch.zeros((rows, group), device="cuda")
+    w[:, 0] = base * 7
+    w[:, 5] = (middle.view(torch.int32) + torch.randint(-4, 5, (rows,), generator=g, device="cuda", dtype=torch.int32)).view(torch.float32)
+    rms = torch.full((group,), 1e-4, device="cuda")
+    rms[5] = 1
+    got = groupwise_int4.pack_groupwise_int4(w, group, rms, steps)
+    with monkeypatch.context() as m:
+        m.setattr(groupwise_int4, "_pack_on_device", lambda *a: None)
+        want = groupwise_int4.pack_groupwise_int4(w, group, rms, steps)
+    assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
