@@ -50,21 +50,32 @@ template <int BITS> __device__ __forceinline__ float level_of(int c) {
     if constexpr (BITS == 2) return c == 0 ? -1.0f : c == 1 ? -kThird : c == 2 ? kThird : 1.0f;
     else return (float)c;
 }
-// Magnitude of a = |w| quantised at scale cand (cand3 = cand / 3, edge = 2 / 3 cand, inv ~ 1 / cand), and by how much a
-// misses the nearest decision boundary (INT2: in units of w, INT4: of cand).  INT2's boundary at 0 (level -1/3 wins the tie)
-// changes the sign only of values that are handled apart (`tiny`).
+// Distance of w from its level at scale cand (cand3 = cand / 3, edge = 2 / 3 cand, inv ~ 1 / cand), up to its sign, and in `miss` how near w
+// comes to a decision boundary: INT2 the smallest distance from one, INT4 the largest distance of |w| / cand from an integer.
+// INT2's boundary at 0 (level -1/3 wins the tie) changes the sign only of values that are handled apart (kTiny).
 template <int BITS>
-__device__ __forceinline__ float magnitude(float a, float w, float cand, float cand3, float edge, float inv, float& margin) {
+__device__ __forceinline__ float distance(float w, float cand, float cand3, float edge, float inv, float& miss) {
     if constexpr (BITS == 2) {
-        margin = fminf(margin, fabsf(a - edge));
-        return a > edge ? cand : cand3;
+        const float a = fabsf(w);
+        miss = fminf(miss, fabsf(a - edge));
+        return __fsub_rn(a > edge ? cand : cand3, a);
     } else {
-        const float t = a * inv, r = (t + kMagic) - kMagic;                // round to nearest even
-        margin = fminf(margin, fabsf(fabsf(t - r) - 0.5f));
-        return __fmul_rn(fminf(r, w < 0.0f ? 8.0f : 7.0f), cand);
+        const float t = w * inv, r = (t + kMagic) - kMagic;                // round to nearest even
+        miss = fmaxf(miss, fabsf(t - r));
+        return __fsub_rn(__fmul_rn(fminf(fmaxf(r, -8.0f), 7.0f), cand), w);
     }
 }
-constexpr float kMargin = 1e-5f;
+// Closer to a boundary than this (of the scale) the quotient decides.  INT2: quotient, distances and edge are rounded within 2e-7; INT4: the
+// last boundary is 7.5, where products with a reciprocal from reciprocal() and quotients differ by up to 3 units of 2^-24, 1.4e-6.  A positive quotient of 2^-25 and more is nearer to the level
+// 1/3 than to -1/3 after rounding, too: only below kTiny may the first one win.
+template <int BITS> constexpr float kMargin = BITS == 2 ? 1e-6f : 2e-6f;
+constexpr float kTiny = 6e-8f;
+
+// 1 / x within 2^-24 of itself (1e-8 <= x < 2^126).
+__device__ __forceinline__ float reciprocal(float x) {
+    const float near = __fdividef(1.0f, x);            // within 2^-22
+    return fmaf(fmaf(-x, near, 1.0f), near, near);
+}
 
 // Code of w at scale s (edge = 2 / 3 s, inv ~ 1 / s) by estimate; false if it is too close to a decision boundary to be sure.
 template <int BITS>
@@ -73,11 +84,11 @@ __device__ __forceinline__ bool code_estimate(float w, float s, float edge, floa
     if constexpr (BITS == 2) {
         const int hi = a > edge ? 1 : 0;
         c = a == 0.0f ? 1 : w < 0.0f ? 1 - hi : 2 + hi;                    // level -1/3 wins the tie at zero
-        return (a == 0.0f || a > kMargin * s) && fabsf(a - edge) > kMargin * s;
+        return (a == 0.0f || a > kTiny * s) && fabsf(a - edge) > kMargin<2> * s;
     } else {
         const float t = a * inv, r = (t + kMagic) - kMagic;
         c = w < 0.0f ? -(int)fminf(r, 8.0f) : (int)fminf(r, 7.0f);
-        return fabsf(fabsf(t - r) - 0.5f) > kMargin && t < 65536.0f;
+        return fabsf(fabsf(t - r) - 0.5f) > kMargin<4> && t < 65536.0f;
     }
 }
 
@@ -151,10 +162,37 @@ __device__ __forceinline__ float4 load_energy(const PackArgs& p, int c) {
     return make_float4(at_least_tiny(__fmul_rn(a.x, a.x)), at_least_tiny(__fmul_rn(a.y, a.y)), at_least_tiny(__fmul_rn(a.z, a.z)), at_least_tiny(__fmul_rn(a.w, a.w)));
 }
 
+// A lane's share of the squared errors of a candidate, decided by quotients: weights and statistics are loaded one by one, because the
+// callers have them in registers, which cannot be indexed.
+template <int BITS, int V, int DT>
+__device__ __noinline__ float error_by_quotients(const PackArgs& p, int row, int k0, float cand, float div) {
+    float t[4];
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        float sum = 0.0f;
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            float x = 0.0f;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int k = k0 + v * 128 + q * 4 + e;
+                const float w = k < p.k ? load_w<DT>(p.w, (size_t)row * p.ldw + k) : 0.0f, a = k < p.k ? p.rms[k] : 0.0f;
+                const float d = __fsub_rn(__fmul_rn(level_of<BITS>(code_exact<BITS>(w, div, false)), cand), w);
+                const float y = __fmul_rn(__fmul_rn(d, d), at_least_tiny(__fmul_rn(a, a)));
+                x = v == 0 ? y : __fadd_rn(x, y);
+            }
+            sum = e == 0 ? x : __fadd_rn(sum, x);
+        }
+        if (q == 0) t[0] = sum; else if (q == 1) t[1] = sum; else if (q == 2) t[2] = sum; else t[3] = sum;
+    }
+    return __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
+}
+
 // The best of the candidates in `mine`, by errors in which every operation is rounded as in the expression.  `visit`: the
 // candidates of all groups of the warp (the shuffles need it converged).  Out of line, with loads of its own: of
 // normal weights in groups of 128, one group in 800 (INT2, 13 candidates) or in 10 000 (INT4, 11) needs it, and its registers
-// would halve the number of warps.
+// would halve the number of warps.  A column's terms are added up as they are made: kept until it is known whether a decision was
+// close, they would not fit the registers beside weights and energies.
 template <int BITS, int V, int DT>
 __device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, float base, uint32_t visit, uint32_t mine, bool every) {
     float f[V][16], aw[V][16], tiny = 3.0e38f;         // tiny: smallest magnitude that is not zero
@@ -169,47 +207,34 @@ __device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, f
 #pragma unroll
         for (int e = 0; e < 16; ++e) tiny = f[v][e] != 0.0f ? fminf(tiny, fabsf(f[v][e])) : tiny;
     }
+    const float* const factors = p.factors;
+    const int steps = p.steps, lg = p.lg;
     float best = 0.0f, chosen = base;
     bool first = true;
 #pragma unroll 1
-    for (int s = 0; s < p.steps; ++s) {
+    for (int s = 0; s < steps; ++s) {
         if (!every && !(visit >> s & 1)) continue;
-        const float cand = __fmul_rn(base, p.factors[s]);
-        const float div = BITS == 2 ? fmaxf(cand, 1e-8f) : cand, inv = __fdividef(1.0f, div);
+        const float cand = __fmul_rn(base, factors[s]);
+        const float div = BITS == 2 ? fmaxf(cand, 1e-8f) : cand, inv = BITS == 2 ? 0.0f : reciprocal(div);
         const float cand3 = __fmul_rn(kThird, cand), edge = 0.6666667f * div;
-        float e4[4][4];                                // [neighbour quadruple][element]: the framework's per-thread accumulators
-        float margin = BITS == 2 ? tiny : 1.0f;
+        float miss = BITS == 2 ? 3.0e38f : 0.0f, t[4];
 #pragma unroll
-        for (int v = 0; v < V; ++v)
+        for (int q = 0; q < 4; ++q)                    // the framework's per-thread accumulators: four neighbours, V of each
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float a = fabsf(f[v][e]);
-                const float d = __fsub_rn(magnitude<BITS>(a, f[v][e], cand, cand3, edge, inv, margin), a);
-                const float x = __fmul_rn(__fmul_rn(d, d), aw[v][e]);
-                e4[e >> 2][e & 3] = v == 0 ? x : __fadd_rn(e4[e >> 2][e & 3], x);
-            }
-        if (margin < (BITS == 2 ? kMargin * div : kMargin)) {       // rare: this lane's columns again, by quotients
-#pragma unroll 1
-            for (int e = 0; e < 16; ++e) {
+            for (int e = 0; e < 4; ++e) {
                 float x = 0.0f;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    float w1 = 0.0f, b = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) if (i == e) { w1 = f[v][i]; b = aw[v][i]; }
-                    const float d = __fsub_rn(__fmul_rn(level_of<BITS>(code_exact<BITS>(w1, div, false)), cand), w1);
-                    const float y = __fmul_rn(__fmul_rn(d, d), b);
+                    const float d = distance<BITS>(f[v][q * 4 + e], cand, cand3, edge, inv, miss);
+                    const float y = __fmul_rn(__fmul_rn(d, d), aw[v][q * 4 + e]);
                     x = v == 0 ? y : __fadd_rn(x, y);
                 }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) if (i == e) e4[i >> 2][i & 3] = x;
+                t[q] = e == 0 ? x : __fadd_rn(t[q], x);
             }
-        }
-        float t[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) t[q] = __fadd_rn(__fadd_rn(__fadd_rn(e4[q][0], e4[q][1]), e4[q][2]), e4[q][3]);
         float err = __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
-        for (int o = 1; o < p.lg; o <<= 1) err = __fadd_rn(err, __shfl_xor_sync(0xffffffffu, err, o));
+        const bool unsure = BITS == 2 ? miss < kMargin<2> * div || tiny < kTiny * div : miss > 0.5f - kMargin<4>;
+        if (unsure) err = error_by_quotients<BITS, V, DT>(p, row, k0, cand, div);       // rare
+        for (int o = 1; o < lg; o <<= 1) err = __fadd_rn(err, __shfl_xor_sync(0xffffffffu, err, o));
         if (!every && !(mine >> s & 1)) continue;
         if (first || err < best) { best = err; chosen = cand; }
         first = false;
@@ -330,7 +355,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                     contenders = 0;
 #pragma unroll 1
                     for (int s = 0; s < steps; ++s) {
-                        const float cand = base * p.factors[s], near = __fdividef(1.0f, cand), inv = fmaf(fmaf(-cand, near, 1.0f), near, near);
+                        const float cand = base * p.factors[s], inv = reciprocal(cand);
                         float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
                         for (int v = 0; v < V; ++v)
@@ -360,7 +385,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
             }
         }
         if (l == 0) p.scales[(size_t)row * p.ng + grp] = __float2half_rn(chosen);
-        const float edge = 0.6666667f * chosen, inv = __fdividef(1.0f, chosen);
+        const float edge = 0.6666667f * chosen, inv = BITS == 2 ? 0.0f : reciprocal(chosen);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             uint32_t word[BITS == 2 ? 1 : 2], unsure = 0;

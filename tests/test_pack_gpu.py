@@ -163,3 +163,36 @@ def test_pack_int4_of_weights_between_the_levels_of_two_candidates(monkeypatch, 
         m.setattr(groupwise_int4, "_pack_on_device", lambda *a: None)
         want = groupwise_int4.pack_groupwise_int4(w, group, rms, steps)
     assert torch.equal(got.scales, want.scales) and torch.equal(got.packed, want.packed)
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("steps", [7, 17])
+@pytest.mark.parametrize("group", [64, 256, 512])
+def test_pack_of_weights_at_decision_boundaries(monkeypatch, bits, steps, group):
+    """Weights within a few units in the last place of a candidate's decision boundaries, and weights so small beside the scale that the
+    rounded distances to the two inner levels are equal or nearly so: few candidates (estimates first) and many (exact errors only)."""
+    mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
+    g = torch.Generator(device="cuda").manual_seed(bits + steps + group)
+    n, k = 256, 1024
+    peak = torch.empty((n, k // group, 1), device="cuda").uniform_(0.01, 1, generator=g)
+    factors = torch.linspace(*((0.55, 1.15) if bits == 2 else (0.72, 1.18)), steps, device="cuda")
+    cand = (peak if bits == 2 else peak / 7) * factors[torch.randint(0, steps, (n, k // group, group), generator=g, device="cuda")]
+    halves = 2 / 3 if bits == 2 else torch.randint(0, 8, cand.shape, generator=g, device="cuda") + 0.5
+    edge = torch.minimum(cand * halves, peak)
+    edge = (edge.view(torch.int32) + torch.randint(-6, 7, edge.shape, generator=g, device="cuda", dtype=torch.int32)).view(torch.float32)
+    small = peak * torch.exp2(torch.empty(cand.shape, device="cuda").uniform_(-34, -14, generator=g))
+    w = torch.where(torch.rand(cand.shape, generator=g, device="cuda") < 0.5, edge, small)
+    w = w * (torch.randint(0, 2, w.shape, generator=g, device="cuda") * 2 - 1)
+    w[..., 0] = peak[..., 0]
+    w = w.reshape(n, k)
+    rms = torch.empty(k, device="cuda").log_normal_(0, 1, generator=g)
+    for arms in (None, rms):
+        got = fn(w, group, arms, steps)
+        with monkeypatch.context() as m:
+            m.setattr(mod, "_pack_on_device", lambda *a: None)
+            want = fn(w, group, arms, steps)
+        # equal but for sums of a group that the framework adds in another order (at most one in a thousand)
+        differ = got.scales != want.scales
+        assert int(differ.sum()) <= differ.numel() // 1000
+        same = ~differ.repeat_interleave(group * bits // 8, dim=1)
+        assert torch.equal(got.packed[same], want.packed[same])
