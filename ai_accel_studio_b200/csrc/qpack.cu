@@ -245,13 +245,14 @@ __device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, f
 // Blocks of an SM, by registers: what a thread keeps is its weights.
 __host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ? (bits == 2 ? 4 : 3) : v == 2 ? (bits == 2 ? 3 : 2) : bits == 2 ? 2 : 1; }
 
-template <int BITS, int V, int DT>
+// SEARCH: there are statistics, the scale is searched for.
+template <int BITS, int V, int DT, bool SEARCH>
 __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const __grid_constant__ PackArgs p) {
-    __shared__ float2 bins[BITS == 2 ? (kMaxFast + 1) * 256 : 1];        // INT2: [bin][thread], (sum aw, sum aw |w|) of the thread's columns
-    [[maybe_unused]] float2* const mine = bins + (BITS == 2 ? threadIdx.x : 0);
+    __shared__ float2 bins[SEARCH && BITS == 2 ? (kMaxFast + 1) * 256 : 1];        // INT2: [bin][thread], (sum aw, sum aw |w|) of the thread's columns
+    [[maybe_unused]] float2* const mine = bins + (SEARCH && BITS == 2 ? threadIdx.x : 0);
     const int lg = p.lg, steps = p.steps;
     float2 grid = make_float2(0.0f, 0.0f);
-    if (p.rms && steps <= kMaxFast) grid = even_grid(p.factors, steps);
+    if (SEARCH && steps <= kMaxFast) grid = even_grid(p.factors, steps);
     const long long groups = (long long)p.n * p.ng;
     const int per_block = 256 / lg;
     const int sub = threadIdx.x / lg, l = threadIdx.x - sub * lg;
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
         for (int o = 1; o < lg; o <<= 1) peak_bits = max(peak_bits, __shfl_xor_sync(0xffffffffu, peak_bits, o));
         const float peak = __uint_as_float(peak_bits), base = at_least_tiny(BITS == 2 ? peak : __fmul_rn(peak, 1.0f / 7.0f));
         float chosen = base;
-        if (p.rms) {
+        if constexpr (SEARCH) {
             // ---- which candidates can have the smallest error (a bit each), by estimates -------------------------
             uint32_t contenders = 0xffffffffu;
             const bool fast = grid.y > 0.0f;
@@ -444,7 +445,7 @@ extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int
     const int grid = (int)(trips < most ? trips : most);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const PackArgs a{w, ldw, rms, factors, packed, static_cast<__half*>(scales), n, k, ng, group, lg, steps, vec, reinterpret_cast<uintptr_t>(rms) % 16 == 0};
-#define QP(B, V, D) pack_kernel<B, V, D><<<grid, 256, 0, s>>>(a)
+#define QP(B, V, D) do { if (rms) pack_kernel<B, V, D, true><<<grid, 256, 0, s>>>(a); else pack_kernel<B, V, D, false><<<grid, 256, 0, s>>>(a); } while (0)
 #define QP_D(B, V) do { if (w_dtype == QGEMV_F16) QP(B, V, QGEMV_F16); else if (w_dtype == QGEMV_BF16) QP(B, V, QGEMV_BF16); else QP(B, V, QGEMV_F32); } while (0)
 #define QP_V(B) do { if (v == 1) QP_D(B, 1); else if (v == 2) QP_D(B, 2); else QP_D(B, 4); } while (0)
     if (bits == 2) QP_V(2); else QP_V(4);
