@@ -347,18 +347,22 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
     }
-    // One to four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of its
-    // 16 warps (see align_x_kernel).  Rows that leave it fewer stay with the streaming kernel, whose one launch takes x as it is (512 x 10001
-    // INT4, M = 4: 20 us either way), and so do calls that it finishes in less than the 8 us that two launches cost an eager caller on the
-    // host: no residual (with one it takes 8.4 us and more, the two launches 6.2 on the GPU) and few bytes (8192 x 1500 INT4, M = 1: 6.2 us;
-    // 8192 x 4300: 11.3, two launches 10.5; 4096 x 10001 INT2 14.4 and 10.6), unless three or four long rows make it slow (512 x 4300: 9.3).
-    if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && (!padded || p->ldx % 8)) {
+    // Three or four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of
+    // its 16 warps (see align_x_kernel) and loses no precision against the streaming kernel, which takes x as it is.  One and two rows
+    // stay with that: it adds them up as integers (error of a result before it is rounded 1e-7, in the phased kernel 5e-7 to 2e-5, 1024 rows
+    // of 4100 to 7000 columns), and so do INT2 groups above 64, whose chains of products in one accumulator are longer in the phased kernel
+    // (3.3e-6 against 3.0e-6; INT2 groups of 64 and INT4 are equal).  Rows that leave fewer warps stay as well (512 x 10001 INT4,
+    // M = 4: 20 us either way), and calls that one launch finishes in less than the 8 us that two cost an eager caller on the host: no residual
+    // (with one it takes 8.4 us and more, the two launches 6.2 on the GPU) and few bytes (INT4, M = 3 and 4: 8575 x 776 5.5 us, 11574 x 1336
+    // 9.3; 8209 x 2928, 12 MB, 10.0 against 9.2 of two launches), unless the rows are long (1462 x 4323 INT2, M = 3: 9.3 against 5.1).
+    const bool as_exact = p->m >= 3 && (p->bits == 4 || p->group <= 64);
+    if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && as_exact && (!padded || p->ldx % 8)) {
         qgemv_problem c = *p;                          // (as the streaming kernel, only x that starts on 16 bytes)
         c.ldx = ((int64_t)p->k_padded + 7) / 8 * 8;
         c.x = static_cast<char*>(p->workspace) + kCopyOff;
         bool none = false;
         const MmaPlan plan = choose(c, kMaxPartialFloats, &none);
-        const bool pays = p->rank > 0 || (size_t)p->n * p->k_padded * p->bits / 8 >= (size_t(8) << 20) || (p->m >= 3 && p->k_original >= 4096);
+        const bool pays = p->rank > 0 || (size_t)p->n * p->k_padded * p->bits / 8 >= (size_t(8) << 20) || p->k_original >= 4096;
         if (aligned(p->x, 16) && plan.ok && plan.variant == 1 && plan.nw >= 16 && pays && (size_t)c.m * c.ldx * 2 <= kCopyBytes) {
             q->pitch = (int)c.ldx;
             q->project = p->rank > 0 && !plan.t_inline;

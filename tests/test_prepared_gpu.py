@@ -7,8 +7,8 @@ import torch
 
 from conftest import ABS_TOL, REL_TOL, c_forward
 from ai_accel_studio_b200 import ops
-from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2, unpack_groupwise_int2
-from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4, unpack_groupwise_int4
+from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2, unpack_codes_int2, unpack_groupwise_int2
+from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4, unpack_codes_int4, unpack_groupwise_int4
 from ai_accel_studio_b200.optimize import HybridInt2Linear, HybridInt4Linear
 
 pytestmark = pytest.mark.gpu
@@ -209,6 +209,56 @@ def test_row_limit_leaves_the_decode_path_alone():
     want = mod(x)
     mod.chunked_max_rows = 0
     assert torch.equal(mod(x), want)
+
+
+def _launches(call):
+    """Kernels in a graph captured from ``call``."""
+    import ctypes
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    rt, raw, n = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(n)) == 0
+    nodes, kind = (ctypes.c_void_p * n.value)(), ctypes.c_int()
+    assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(n)) == 0
+    kinds = []
+    for node in nodes:
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        kinds.append(kind.value)
+    return kinds.count(0)                                              # cudaGraphNodeTypeKernel
+
+
+def _random_module(g, bits, n, k, group, oc=0, rank=0):
+    """A packed Linear of random weights, and its dense matrix with outlier columns and residual, in 64 bits."""
+    w = torch.empty((n, k), device="cuda").normal_(0, 0.05, generator=g)
+    pw = (pack_groupwise_int2 if bits == 2 else pack_groupwise_int4)(w, group)
+    oidx = torch.randperm(k, generator=g, device="cuda")[:oc].to(torch.int32)
+    ow = torch.empty((n, oc), device="cuda").normal_(0, 0.05, generator=g).half()
+    ru = torch.empty((n, rank), device="cuda").normal_(0, 0.05, generator=g).half()
+    rv = torch.empty((rank, k), device="cuda").normal_(0, 0.05, generator=g).half()
+    cls = HybridInt2Linear if bits == 2 else HybridInt4Linear
+    make = lambda bias=None: cls.from_buffers(pw.packed, pw.scales, k, group, oidx, ow, bias, *((ru, rv) if rank else (None, None)))
+    codes = (unpack_codes_int2 if bits == 2 else unpack_codes_int4)(pw).double()
+    dense = ((codes * 2 / 3 - 1) if bits == 2 else codes - 8) * pw.scales.double().repeat_interleave(group, dim=1)
+    dense = dense[:, :k] + ru.double() @ rv.double()
+    dense[:, oidx.long()] += ow.double()
+    return make, dense
+
+
+@pytest.mark.parametrize("bits,group", [(2, 64), (2, 128), (2, 256), (4, 32), (4, 64), (4, 128)])
+@pytest.mark.parametrize("rows", [1, 2])
+def test_one_and_two_rows_of_odd_x_are_summed_exactly(bits, group, rows):
+    """Unpadded x of one and two rows: sums of integers, so that what is left are the roundings of some hundred group sums, outlier
+    columns and residual in 32 bits, 2^-24 times the root of their number: below 2^-21.  A bias that cancels the first row's results keeps
+    the rounding of the output out of it."""
+    g = torch.Generator(device="cuda").manual_seed(group + rows)
+    make, dense = _random_module(g, bits, 1024, 6001, group, 16, 8)
+    x = (torch.empty((rows, 6001), device="cuda").normal_(0, 1, generator=g) * torch.empty(6001, device="cuda").log_normal_(0, 1, generator=g)).half()
+    ref = x.double() @ dense.T
+    bias = -ref[0].half()
+    mod = make(bias)
+    assert float((mod(x)[0].double() - (ref[0] + bias.double())).norm()) <= 2.0 ** -21 * float(ref[0].norm())
+    assert _launches(lambda: mod(x)) == 1
 
 
 # one column short of, at and past a copying CTA's 2048 columns and a projecting CTA's 6144; K a multiple of 8 but not of the group (projections made
