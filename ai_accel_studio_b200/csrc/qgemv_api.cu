@@ -314,8 +314,9 @@ struct Prepared {                                  // what qgemv_prepare writes 
     bool project;                                  // the copying launch also makes the residual projections
     StreamPlan plan;                               // ok == false: as qgemv_run, four rows at a time
 };
-// The copy of x: inside the scratch for partial sums, behind what the tensor-core kernel uses of it for itself.
-constexpr size_t kCopyOff = kWsPartialOff + (size_t(2) << 20), kCopyBytes = size_t(1) << 20;
+static_assert(kWsTraceOff + kWsTraceBytes <= kWsPartialOff + (kMaxPartialFloats - kTPartFloats - kStreamWordFloats) * sizeof(float) &&
+              kWsCopyOff + kWsCopyBytes <= kWsPartialOff + (kMaxPartialFloats - kTPartFloats - kStreamWordFloats) * sizeof(float),
+              "the copy of x or the time stamps reach into the words at the end of the workspace");
 }  // namespace
 
 extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
@@ -359,11 +360,11 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && as_exact && (!padded || p->ldx % 8)) {
         qgemv_problem c = *p;                          // (as the streaming kernel, only x that starts on 16 bytes)
         c.ldx = ((int64_t)p->k_padded + 7) / 8 * 8;
-        c.x = static_cast<char*>(p->workspace) + kCopyOff;
+        c.x = static_cast<char*>(p->workspace) + kWsCopyOff;
         bool none = false;
         const MmaPlan plan = choose(c, kMaxPartialFloats, &none);
         const bool pays = p->rank > 0 || (size_t)p->n * p->k_padded * p->bits / 8 >= (size_t(8) << 20) || p->k_original >= 4096;
-        if (aligned(p->x, 16) && plan.ok && plan.variant == 1 && plan.nw >= 16 && pays && (size_t)c.m * c.ldx * 2 <= kCopyBytes) {
+        if (aligned(p->x, 16) && plan.ok && plan.variant == 1 && plan.nw >= 16 && pays && (size_t)c.m * c.ldx * 2 <= kWsCopyBytes) {
             q->pitch = (int)c.ldx;
             q->project = p->rank > 0 && !plan.t_inline;
             return QGEMV_OK;
@@ -396,7 +397,7 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
     if (q->pitch) {
         if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        char* const copy = static_cast<char*>(workspace) + kCopyOff;
+        char* const copy = static_cast<char*>(workspace) + kWsCopyOff;
         p.x = x; p.y = y;
         const int r = launch_align_x(make_args(p, kMaxPartialFloats), p.x_dtype == QGEMV_BF16, copy, q->pitch, q->project, !ordered, s);
         if (r != QGEMV_OK) return r;

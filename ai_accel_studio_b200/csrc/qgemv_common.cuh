@@ -14,7 +14,13 @@ namespace qgemv {
 // Workspace layout (bytes from the 256-byte aligned base the caller passes):
 //   [0, 1024)            residual projections t[m][r] = sum_k V[r,k] x[m,k], fp32, QGEMV_MAX_M x 64
 //   [1024, 1024+4*16384) arrival counters, one int32 per 16-row tile (zero between calls)
-//   [kWsPartialOff, ..)   partial sums of tiles shared by several warps, fp32 [warp][2][4][32]
+//   [kWsPartialOff, ..)   partial sums, kMaxPartialFloats fp32 in all:
+//     from its start        tiles shared by CTAs of the tensor-core kernels [CTA][2][4][32], or split sums of the streaming kernel
+//     [kWsCopyOff, ..)      x in padded rows for the tensor-core kernel (align_x_kernel), kWsCopyBytes
+//     [kWsTraceOff, ..)     time stamps of a build with QGEMV_TRACE, kWsTraceBytes
+//     at its end            {value, launch tag} words of the streaming kernel (kStreamWordFloats) and of the others (kTPartFloats)
+//   The tensor-core kernels read a copy of x while they write partial sums, time stamps and words; split sums of the streaming kernel may lie
+//   over all but the words, since it takes no copy and writes none of the others.
 constexpr int    kMaxRank        = 64;
 constexpr size_t kWsTOff         = 0;
 constexpr size_t kWsCounterOff   = 1024;
@@ -28,6 +34,12 @@ constexpr int    kMaxTParts      = 8;              // K-parts of an in-kernel re
 // tail of the partial-sum area: {fp32 value, launch tag} per (K-part, m, rank column), in 32-bit words
 constexpr int    kTPartFloats    = 2 * kMaxTParts * QGEMV_MAX_M * kMaxRank;
 constexpr size_t kMaxPartialFloats = size_t(1) << 20;                             // 4 MiB of fp32 partial sums
+constexpr int    kMaxCtas        = 512;           // of a tensor-core kernel; one per SM are launched
+constexpr size_t kCtaPartialBytes = 2 * 4 * 32 * sizeof(float);
+constexpr size_t kWsCopyOff      = kWsPartialOff + (size_t(1) << 20), kWsCopyBytes = size_t(1) << 20;
+constexpr size_t kWsTraceOff     = kWsPartialOff + (size_t(2) << 20), kWsTraceBytes = kMaxCtas * size_t(16 * 16 * 8);      // [CTA][warp][16] times
+static_assert(kWsPartialOff + kMaxCtas * kCtaPartialBytes <= kWsCopyOff && kWsCopyOff + kWsCopyBytes <= kWsTraceOff && kWsCopyOff % 256 == 0,
+              "regions of the workspace that one launch uses overlap");
 
 // Device-side view of one problem; a trivially copyable kernel parameter.
 struct Args {

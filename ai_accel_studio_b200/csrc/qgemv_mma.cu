@@ -809,7 +809,7 @@ MmaPlan plan_mma(const qgemv_problem& p, size_t partial_floats) {
     }
     if (pl.tile_aligned) slot_cap = ((pl.nt + grid - 1) / grid) * rpt;
     if (slot_cap * slot_bytes > 65536) return pl;
-    if ((size_t)grid * 2 * 4 * 32 + kTPartFloats > partial_floats) return pl;
+    if (grid > kMaxCtas || grid * kCtaPartialBytes / sizeof(float) + kTPartFloats > partial_floats) return pl;
 
     pl.scales_async = (p.lds % cg == 0) && al(p.scales, (size_t)cg * 2) ? 1 : 0;
     pl.ocb = align_up(p.outliers * 2, 16);

@@ -125,14 +125,14 @@ __device__ __forceinline__ float ld_cg_f32(const float* p) {
 }
 
 // Optional phase trace (build with -DQGEMV_TRACE): lane 0 of every warp stores the global
-// nanosecond timer at a few points into the upper half of the partial-sum scratch.
+// nanosecond timer at a few points into a region of the scratch (kWsTraceOff).
 #ifdef QGEMV_TRACE
 #define QTRACE(slot)                                                                            \
     do {                                                                                        \
         if ((threadIdx.x & 31) == 0) {                                                          \
             unsigned long long t_;                                                              \
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_) :: "memory");                  \
-            reinterpret_cast<unsigned long long*>(p.a.partial + (kMaxPartialFloats / 2))        \
+            reinterpret_cast<unsigned long long*>(p.a.partial + (kWsTraceOff - kWsPartialOff) / 4) \
                 [((size_t)blockIdx.x * 16 + (threadIdx.x >> 5)) * 16 + (slot)] = t_;            \
         }                                                                                       \
     } while (0)
