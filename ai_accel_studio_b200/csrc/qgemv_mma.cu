@@ -172,13 +172,13 @@ __device__ __forceinline__ void stage_activations(const MmaArgs& p, unsigned cha
             part += __shfl_xor_sync(0xffffffffu, part, 2);
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-            int e2 = 0;
-            if (big > 0.0f && big < 3.0e38f) e2 = (int)((__float_as_uint(big) >> 23) & 0xffu) - 127 - 13;   // floor(log2) - 13
-            e2 = max(-60, min(100, e2));
-            const float down = __int_as_float((127 - e2) << 23);         // 2^-e : multiplier for x
-            const float up = __int_as_float((127 + 24 + e2) << 23);      // 2^(24+e): undoes subnormal unit and group scale
+            // 2^e: power of two below the largest, over 2^13.  Any finite bf16 (-126 <= e <= 114): the sums are kept times kSumScale, so that `up` is finite.
+            const int top = (int)((__float_as_uint(big) >> 23) & 0xffu);
+            const int e2 = big > 0.0f && top < 255 ? max(-126, top - 127 - 13) : 0;
+            const float down = __int_as_float((127 - e2) << 23);                              // 2^-e : multiplier for x
+            const float up = __int_as_float((127 + 24 - kSumShift + e2) << 23);               // undoes subnormal unit and group scale
             if (live) {
-                if (tq == 0) gx[grp * M + mrow] = make_float2(BITS == 2 ? part : 8.0f * part,
+                if (tq == 0) gx[grp * M + mrow] = make_float2((BITS == 2 ? kSumScale : 8.0f * kSumScale) * part,
                                                               BITS == 2 ? up * (2.0f / 3.0f) : up);
 #pragma unroll
                 for (int i = 0; i < GE::TW; ++i) {            // one 32-bit code word of this lane
@@ -225,8 +225,8 @@ __device__ __forceinline__ void stage_activations(const MmaArgs& p, unsigned cha
             const int pos = (qq & 1) * 2 + (qq >> 1);
             const size_t h = ((((size_t)(grp * GE::TW + ii) * (GE::NCLS / 2) + (c >> 1)) * M + m) * 4 + t) * 8 +
                              (c & 1) * 4 + pos;
-            const float up = gx[grp * M + m].y * (BITS == 2 ? 1.5f : 1.0f);      // 2^(24 + e)
-            val = __half2float(xs[h]) * __int_as_float((127 - 24 + BITS * c) << 23) * up;
+            const float up = gx[grp * M + m].y * (BITS == 2 ? 1.5f : 1.0f);      // 2^(24 - kSumShift + e)
+            val = __half2float(xs[h]) * __int_as_float((127 - 24 + kSumShift + BITS * c) << 23) * up;
         }
         xo[i] = val;
     }

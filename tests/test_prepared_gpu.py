@@ -290,3 +290,19 @@ def test_rows_of_odd_x_are_copied_first(bits, n, k, group, oc, rank, dtype):
         graph.replay()
         assert torch.equal(captured, y) and torch.equal(mod(x), y)
     assert ops.workspace_status("cuda") == 0
+
+
+@pytest.mark.parametrize("bits,group", [(2, 64), (4, 128)])
+@pytest.mark.parametrize("k", [5001, 5120])
+def test_bf16_activations_of_any_magnitude(bits, group, k):
+    """Groups of activations are normalised to fp16 and back, from bf16's smallest normal numbers on.  The largest: the sum of 128 codes
+    of 15 times 1e35 is still below the largest number of 32 bits."""
+    g = torch.Generator(device="cuda").manual_seed(group + k)
+    make, dense = _random_module(g, bits, 512, k, group, 8)
+    mod = make()
+    for rows in (1, 3, 4, 8):
+        for magnitude in (1e-35, 1e-30, 1e-24, 1e-20, 1.0, 1e20, 1e30, 1e35):
+            x = (torch.empty((rows, k), device="cuda").normal_(0, 1, generator=g) * magnitude).bfloat16()
+            ref = x.double() @ dense.T
+            assert float((mod(x).double() - ref).norm()) <= 2.0 ** -8 * float(ref.norm()), (rows, magnitude)
+    assert ops.workspace_status("cuda") == 0
