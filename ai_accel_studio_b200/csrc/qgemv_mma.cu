@@ -172,9 +172,9 @@ __device__ __forceinline__ void stage_activations(const MmaArgs& p, unsigned cha
             part += __shfl_xor_sync(0xffffffffu, part, 2);
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-            // 2^e: power of two below the largest, over 2^13.  Any finite bf16 (-126 <= e <= 114): the sums are kept times kSumScale, so that `up` is finite.
-            const int top = (int)((__float_as_uint(big) >> 23) & 0xffu);
-            const int e2 = big > 0.0f && top < 255 ? max(-126, top - 127 - 13) : 0;
+            // 2^e: power of two below the largest, over 2^13, of any bf16: the sums are kept times kSumScale, so that `up` is finite.  (No
+            // largest but zero: zeros whatever e is.  Infinity: the level offset makes NaN of the group's sums whatever e is.)
+            const int e2 = max(-126, (int)(__float_as_uint(big) >> 23) - 127 - 13);
             const float down = __int_as_float((127 - e2) << 23);                              // 2^-e : multiplier for x
             const float up = __int_as_float((127 + 24 - kSumShift + e2) << 23);               // undoes subnormal unit and group scale
             if (live) {
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qgemv_mma_kernel(const __gr
         if (t < TT) {
             for (int r = lo; r < hi; ++r) {
                 const float4 v = *reinterpret_cast<const float4*>(slots + (size_t)(r - r0) * SLOT_BYTES + (g * TT + t) * 16);
-                y[0] += v.x; y[1] += v.y; y[2] += v.z; y[3] += v.w;
+                y[0] = fmaf(v.x, 1 / kSumScale, y[0]); y[1] = fmaf(v.y, 1 / kSumScale, y[1]); y[2] = fmaf(v.z, 1 / kSumScale, y[2]); y[3] = fmaf(v.w, 1 / kSumScale, y[3]);
             }
         }
         const bool whole = lo == tile * p.rpt && hi == (tile + 1) * p.rpt;

@@ -290,8 +290,8 @@ __device__ __forceinline__ float4 tile_extras(const MmaArgs& p, const unsigned c
     return make_float4(y[0], y[1], y[2], y[3]);
 }
 
-// Sums of code products are kept times 2^-12 until a tile is finished: the power of two that undoes the normalisation of a group of
-// activations is then finite for the largest bf16 (2^(24 + 114 - 12)), and results of the smallest lose nothing that 16 bits hold.
+// Sums of code products are kept times 2^-12 until the runs of a tile are added up: the power of two that undoes the normalisation of a group of
+// activations is then finite for the largest bf16 (2^(24 + 115 - 12)), and results of the smallest lose nothing that 16 bits hold.
 constexpr int   kSumShift = 12;
 constexpr float kSumScale = 1.0f / (1 << kSumShift);
 
@@ -304,8 +304,6 @@ __device__ __forceinline__ void finish_tile(const MmaArgs& p, const unsigned cha
     const int g = row_in_tile >= 0 ? row_in_tile : lane >> 2;      // tile row of this lane's first output row (second: + 8)
     const int r0 = tile * kTileRows + g, r1 = r0 + 8;
     const int c0 = min(r0, a.n - 1), c1 = min(r1, a.n - 1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) y[i] *= 1.0f / kSumScale;
     if constexpr (EX) {
         const float4 e = tile_extras<M>(p, smem, tile, pre, row_in_tile);
         y[0] += e.x; y[1] += e.y; y[2] += e.z; y[3] += e.w;

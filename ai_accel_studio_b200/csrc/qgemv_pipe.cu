@@ -235,9 +235,9 @@ __device__ __forceinline__ void pipe_stage_x(const MmaArgs& p, unsigned char* sm
             part += __shfl_xor_sync(0xffffffffu, part, 2);
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
             big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-            // 2^e: power of two below the largest, over 2^13.  Any finite bf16 (-126 <= e <= 114): the sums are kept times kSumScale, so that `up` is finite.
-            const int top = (int)((__float_as_uint(big) >> 23) & 0xffu);
-            const int e2 = big > 0.0f && top < 255 ? max(-126, top - 127 - 13) : 0;
+            // 2^e: power of two below the largest, over 2^13, of any bf16: the sums are kept times kSumScale, so that `up` is finite.  (No
+            // largest but zero: zeros whatever e is.  Infinity: the level offset makes NaN of the group's sums whatever e is.)
+            const int e2 = max(-126, (int)(__float_as_uint(big) >> 23) - 127 - 13);
             const float down = __int_as_float((127 - e2) << 23);                              // 2^-e : multiplier for x
             const float up = __int_as_float((127 + 24 - kSumShift + e2) << 23);               // undoes subnormal unit and group scale
             if (live) {
@@ -703,7 +703,8 @@ __global__ void __launch_bounds__(kPipeWarps * 32, 1) qgemv_pipe_kernel(const __
                     const uint32_t s0 = slots_u32 + (uint32_t)(lt * p.rpt) * SLOT_BYTES;
                     for (int j = 0; j < p.rpt; ++j) {
                         const float4 v = lds128f(s0 + j * SLOT_BYTES);
-                        yy[0] += v.x; yy[1] += v.y; yy[2] += v.z; yy[3] += v.w;
+                        yy[0] = fmaf(v.x, 1 / kSumScale, yy[0]); yy[1] = fmaf(v.y, 1 / kSumScale, yy[1]);
+                        yy[2] = fmaf(v.z, 1 / kSumScale, yy[2]); yy[3] = fmaf(v.w, 1 / kSumScale, yy[3]);
                     }
                 }
                 if (EX && a.rank > 0) {             // the table of t is built by the reader warp early on
