@@ -79,7 +79,7 @@ def test_pack_of_values_that_are_not_finite(monkeypatch, bits):
 @pytest.mark.parametrize("bits", [2, 4])
 @pytest.mark.parametrize("steps", [1, 2, 16, 17, 40])
 def test_pack_searches_any_number_of_candidates(monkeypatch, bits, steps):
-    """Up to 16 candidates are told apart by estimates, more are all compared exactly; heavy tails, exact ties between candidates
+    """Two to 16 candidates are told apart by estimates, one or more than 16 are all compared exactly; heavy tails, exact ties between candidates
     (weights on a coarse grid) and groups of zeros leave several that the estimates cannot tell apart."""
     mod, fn = (groupwise_int2, groupwise_int2.pack_groupwise_int2) if bits == 2 else (groupwise_int4, groupwise_int4.pack_groupwise_int4)
     g = torch.Generator(device="cuda").manual_seed(steps)
@@ -93,6 +93,9 @@ def test_pack_searches_any_number_of_candidates(monkeypatch, bits, steps):
         m.setattr(mod, "_pack_on_device", lambda *a: None)
         want = fn(w, 128, rms, steps)
     differ = got.scales != want.scales
+    # One group of the 480 may differ: of sums that the framework adds in another order than the kernel (measured: one, among the heavy tails,
+    # INT4 with 40 candidates, as it did when every candidate of every search was compared exactly).
+    assert int(differ.sum()) <= 1
     same = ~differ.repeat_interleave(16 * bits, dim=1)
     assert torch.equal(got.packed[same], want.packed[same])
     # Where another candidate was taken, its error in 64 bits is as small as far as sums of 128 terms in 32 bits can tell: 128 * 2^-24.

@@ -1,5 +1,5 @@
 """The streaming kernel behind qgemv_prepare / the modules' prepared launches: 5 - 16 rows in one launch, and any row count
-where x's rows are not padded or not aligned.  Sizes at the edges of its tiles (16 rows, 128-column blocks, slots of 128
+where x's rows are not padded or not aligned; three and four such rows that are copied for the phased kernel instead.  Sizes at the edges of its tiles (16 rows, 128-column blocks, slots of 128
 bytes), of the row blocks (a warp takes one or two tiles), of K splits between CTAs, and of the scale copies."""
 import numpy as np
 import pytest
@@ -7,8 +7,8 @@ import torch
 
 from conftest import ABS_TOL, REL_TOL, c_forward
 from ai_accel_studio_b200 import ops
-from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2, unpack_codes_int2, unpack_groupwise_int2
-from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4, unpack_codes_int4, unpack_groupwise_int4
+from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2, unpack_codes_int2
+from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4, unpack_codes_int4
 from ai_accel_studio_b200.optimize import HybridInt2Linear, HybridInt4Linear
 
 pytestmark = pytest.mark.gpu
@@ -261,26 +261,30 @@ def test_one_and_two_rows_of_odd_x_are_summed_exactly(bits, group, rows):
     assert _launches(lambda: mod(x)) == 1
 
 
-# one column short of, at and past a copying CTA's 2048 columns and a projecting CTA's 6144; K a multiple of 8 but not of the group (projections made
-# inside the GEMV) and not (made by the copying launch); rows of x that are not 16-byte aligned
-@pytest.mark.parametrize("bits,n,k,group,oc,rank", [(4, 40, 2047, 128, 0, 1), (2, 17, 2049, 64, 3, 5), (4, 200, 6143, 64, 8, 8), (2, 200, 6145, 256, 0, 64),
-                                                    (4, 64, 4104, 128, 32, 8), (2, 2400, 1003, 128, 16, 0)])
+# Launches of three and of four rows: two where x is copied first, one where the streaming kernel takes it as it is.
+@pytest.mark.parametrize("bits,n,k,group,oc,rank,launches", [
+    (4, 40, 2047, 128, 0, 1, (2, 2)),        # one column short of a copying CTA's 2048 columns
+    (2, 17, 2049, 64, 3, 5, (2, 2)),         # one past it
+    (4, 200, 6143, 64, 8, 8, (2, 2)),        # one column short of a projecting CTA's 6144
+    (4, 200, 6145, 32, 0, 64, (2, 1)),       # one past it, largest rank: 16 x 11.4 KB of rings and rows of U beside 70 KB are too much for four rows
+    (4, 64, 4104, 128, 32, 8, (2, 2)),       # 16-byte rows, but K padded: 4 CTAs of the GEMV, too few to make 16 parts of the projections
+    (4, 320, 4104, 128, 32, 8, (2, 2)),      # 20 CTAs: the GEMV makes them
+    (4, 512, 4300, 128, 0, 0, (2, 2)),       # no residual: long rows
+    (2, 512, 4103, 64, 3, 0, (2, 2)),
+    (4, 6000, 2900, 64, 0, 0, (2, 2)),       # no residual: 8.8 MB of codes
+    (2, 2400, 1003, 64, 16, 0, (1, 1)),      # no residual, short rows, few bytes
+    (4, 512, 10001, 128, 3, 8, (2, 1)),      # four rows of x leave the phased kernel 12 warps
+    (2, 200, 6145, 256, 0, 64, (1, 1)),      # INT2 groups above 64
+    (2, 2400, 1003, 128, 16, 5, (1, 1)),
+])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_rows_of_odd_x_are_copied_first(bits, n, k, group, oc, rank, dtype):
+def test_rows_of_odd_x_are_copied_first(bits, n, k, group, oc, rank, launches, dtype):
     g = torch.Generator(device="cuda").manual_seed(n + k)
-    w = torch.empty((n, k), device="cuda").normal_(0, 0.05, generator=g)
-    pw = (pack_groupwise_int2 if bits == 2 else pack_groupwise_int4)(w, group)
-    oidx = torch.randperm(k, generator=g, device="cuda")[:oc].to(torch.int32)
-    ow = torch.empty((n, oc), device="cuda").normal_(0, 0.05, generator=g).half()
-    ru = torch.empty((n, rank), device="cuda").normal_(0, 0.05, generator=g).half()
-    rv = torch.empty((rank, k), device="cuda").normal_(0, 0.05, generator=g).half()
-    cls = HybridInt2Linear if bits == 2 else HybridInt4Linear
-    mod = cls.from_buffers(pw.packed, pw.scales, k, group, oidx, ow, None, *((ru, rv) if rank else (None, None)))
-    dense = (unpack_groupwise_int2 if bits == 2 else unpack_groupwise_int4)(pw).double()[:, :k]
+    make, dense = _random_module(g, bits, n, k, group, oc, rank)
+    mod = make()
     for rows in (1, 2, 3, 4):
         x = torch.empty((rows, k), device="cuda").normal_(0, 1, generator=g).to(dtype)
-        xd = x.double()
-        ref = xd @ dense.T + xd[:, oidx.long()] @ ow.double().T + (xd @ rv.double().T) @ ru.double().T
+        ref = x.double() @ dense.T
         rel = REL_TOL if dtype == torch.float16 else 2.0 ** -8
         y = mod(x)
         assert float((y.double() - ref).norm()) <= rel * float(ref.norm()), rows
@@ -289,7 +293,51 @@ def test_rows_of_odd_x_are_copied_first(bits, n, k, group, oc, rank, dtype):
             captured = mod(x)
         graph.replay()
         assert torch.equal(captured, y) and torch.equal(mod(x), y)
+        assert _launches(lambda: mod(x)) == (1, 1, *launches)[rows - 1], rows
     assert ops.workspace_status("cuda") == 0
+
+
+def test_copies_of_odd_x_follow_each_other_in_one_workspace():
+    """The copy is written again by every launch, beside launches that may start early: each sees its own x.  In between, a kernel that
+    uses the same workspace otherwise (8 rows) and weights that are written in place."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    mods = [_random_module(g, 4, 700, 5001, 64, 3, 5)[0](), _random_module(g, 4, 300, 1003, 128, 0, 8)[0]()]
+    xs = [[torch.empty((rows, k), device="cuda").normal_(0, 1, generator=g).half() for rows in (3, 4, 8, 3)] for k in (5001, 1003)]
+    want = [[mod(x).clone() for x in x2] for mod, x2 in zip(mods, xs)]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(25):
+        for i in range(4):
+            for mod, x2 in zip(mods, xs):
+                got.append(mod(x2[i]))
+    torch.cuda.synchronize()
+    for j, y in enumerate(got):
+        assert torch.equal(y, want[j % 2][j // 2 % 4]), j
+    kept = mods[0].scales.clone()
+    for _ in range(10):
+        mods[0].scales.zero_()
+        zero = mods[0](xs[0][0])
+        mods[0].scales.copy_(kept)
+        assert torch.equal(mods[0](xs[0][0]), want[0][0]) and not torch.equal(zero, want[0][0])
+
+
+def test_copies_of_odd_x_overlap_their_predecessor_only_over_settled_weights():
+    """The copying launch starts after a kernel that may be writing the weights, though it reads none itself but V: the launch behind it
+    reads weights before it waits for the copy."""
+    g = torch.Generator(device="cuda").manual_seed(10)
+    mod = _random_module(g, 4, 512, 1003, 128, 0, 8)[0]()
+    x = torch.empty((3, 1003), device="cuda").normal_(0, 1, generator=g).half()
+
+    def calls(write):
+        x.mul_(1)
+        if write:
+            mod.scales.mul_(1)
+        mod(x)
+        mod(x)
+
+    mod(x)
+    assert _overlapping_launches(lambda: calls(False)) == 4            # every launch its predecessor
+    assert _overlapping_launches(lambda: calls(True)) == 3             # but the first copy
 
 
 @pytest.mark.parametrize("bits,group", [(2, 64), (4, 128)])
