@@ -310,7 +310,7 @@ extern "C" int qgemv_run_ordered(const qgemv_problem* p, void* stream) {
 namespace {
 struct Prepared {                                  // what qgemv_prepare writes into the caller's buffer
     qgemv_problem problem;
-    int pitch;                                     // > 0: qgemv_run on a copy of x with rows of this many elements, in the workspace
+    int pitch;                                     // > 0: two launches, the second on a copy of x with rows of this many elements, in the workspace
     bool project;                                  // the copying launch also makes the residual projections
     StreamPlan plan;                               // ok == false: as qgemv_run, four rows at a time
 };
@@ -322,7 +322,8 @@ static_assert(kWsTraceOff + kWsTraceBytes <= kWsPartialOff + (kMaxPartialFloats 
 extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
 
 // The streaming kernel takes what qgemv_run cannot take in one launch -- more than four rows, and x whose rows are not
-// padded to k_padded columns or not 16-byte aligned -- and leaves one to four aligned rows to the kernels above: those
+// padded to k_padded columns or not 16-byte aligned, unless three or four of them are copied (see below) -- and leaves one to four aligned
+// rows to the kernels above: those
 // launches last about as long as their code takes to arrive in the instruction caches (some 3.5 clocks per instruction on
 // a first pass), and the streaming kernel has more of it (4096 x 4096 INT4, M = 1: 10.8 against 7.1 us).  The exception are
 // rows so long that their activations leave the phased kernel few of its 16 warps, or do not fit beside it at all (M = 4,
@@ -352,9 +353,9 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     // its 16 warps (see align_x_kernel) and loses no precision against the streaming kernel, which takes x as it is.  One and two rows
     // stay with that: it adds them up as integers (error of a result before it is rounded 1e-7, in the phased kernel 5e-7 to 2e-5, 1024 rows
     // of 4100 to 7000 columns), and so do INT2 groups above 64, whose chains of products in one accumulator are longer in the phased kernel
-    // (3.3e-6 against 3.0e-6; INT2 groups of 64 and INT4 are equal).  Rows that leave fewer warps stay as well (512 x 10001 INT4,
-    // M = 4: 20 us either way), and calls that one launch finishes in less than the 8 us that two cost an eager caller on the host: no residual
-    // (with one it takes 8.4 us and more, the two launches 6.2 on the GPU) and few bytes (INT4, M = 3 and 4: 8575 x 776 5.5 us, 11574 x 1336
+    // (errors 8 to 33 % larger, groups of 128 and 256; INT2 groups of 64 and INT4 are equal to 1 %).  Rows that leave fewer warps stay as well (512 x 10001 INT4,
+    // M = 4: 20 us either way), and calls that one launch finishes in less than the 8 us that two cost an eager caller on the host: no
+    // residual (with one it takes 10.7 us and more, the two launches 6.6 on the GPU: 512 x 1500 INT4, M = 3) and few bytes (INT4, M = 3 and 4: 8575 x 776 5.5 us, 11574 x 1336
     // 9.3; 8209 x 2928, 12 MB, 10.0 against 9.2 of two launches), unless the rows are long (1462 x 4323 INT2, M = 3: 9.3 against 5.1).
     const bool as_exact = p->m >= 3 && (p->bits == 4 || p->group <= 64);
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && as_exact && (!padded || p->ldx % 8)) {

@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(256) residual_t_kernel(const Args a) {
 // x whose rows end before the padded K, or are not 16-byte aligned, as the tensor-core kernel wants it: the first `project` CTAs
 // project a residual row each, the others copy 2048 columns of a row of x into `to` (rows of `pitch`, zeros past the last column).
 // Latency is its bound: two-byte loads, but all of a thread's at once, those of V before the dependency wait.  It stands before a kernel
-// that then needs no code for odd x: 4999 x 4300 INT4, three bf16 rows, odd rank 17.1 us as one streaming launch, 13.0 as these two
-// (15.1 with 512 threads a CTA, whose loads came in two rounds); 8192 x 8200 INT4, four rows 37.0 -> 19.8; 3000 x 5001 INT2, three rows
-// 26.1 -> 12.2.
+// that then needs no code for odd x.  One streaming launch and these two, chains over weights from DRAM, us: 4999 x 4300 INT4, three
+// bf16 rows, odd rank 18.2 and 13.6 (15.1 with 512 threads a CTA, whose loads came in two rounds); 10150 x 6255 INT4, three rows 32.3 and
+// 15.4; 3000 x 5001 INT2, groups of 64, three rows, odd rank 16.2 and 12.7; 512 x 1500 INT4, three rows, rank 8 10.8 and 6.6.
 template <bool BF16>
 __global__ void __launch_bounds__(1024) align_x_kernel(const Args a, unsigned short* to, int pitch, int project) {
     using XT = typename Act16<BF16>::T;

@@ -3,10 +3,11 @@
 // The torch expression of the same algorithm (kernels/groupwise_int2.py, groupwise_int4.py) makes a temporary of the
 // matrix's size for every step of every candidate scale -- some 150 passes over memory at 13 candidates.  Here a group's
 // weights stay in registers: 16 consecutive columns per lane (times V for groups above 128), 2 - 8 lanes per group.  Bound
-// by instructions, not by HBM: 8192 x 8192 INT2 takes 201 M warp instructions at 67 % of the issue slots with 29 warps an SM,
-// INT4 372 M at 78 % with 21.
-// Measured, 4096 x 4096 INT2 with activation statistics (B200): torch expression 17.7 ms; 349 us with a decision per weight
-// by quotient or estimate; 228 us with a decision per weight and candidate; 80 us as below.  INT4: 170 -> 110 us.
+// by instructions, not by HBM: 8192 x 8192 INT2 takes 202 M warp instructions at 70 % of the issue slots with 28 warps an SM,
+// INT4 358 M at 78 % with 21 (groups of 128).
+// Measured, 4096 x 4096 with activation statistics (B200): torch expression 17.7 ms; INT2 225 us with a decision per weight and
+// candidate, 74 us as below; INT4 172 and 105; without statistics 41 and 22 - 23.  More than 16 candidates, all compared exactly: 40 of INT2
+// 532 and 360, of INT4 449 and 430.
 //
 // Results are the expression's own: where it matters every operation is rounded as there (IEEE division, no contraction), and
 // the squared errors are added in the order in which the framework's reduction adds a contiguous row (four neighbours, then a
@@ -190,7 +191,7 @@ __device__ __noinline__ float error_by_quotients(const PackArgs& p, int row, int
 
 // The best of the candidates in `mine`, by errors in which every operation is rounded as in the expression.  `visit`: the
 // candidates of all groups of the warp (the shuffles need it converged).  Out of line, with loads of its own: of
-// normal weights in groups of 128, one group in 800 (INT2, 13 candidates) or in 10 000 (INT4, 11) needs it, and its registers
+// normal weights in groups of 128, one group in 700 (INT2, 13 candidates) or in 12 000 (INT4, 11) needs it, and its registers
 // would halve the number of warps.  A column's terms are added up as they are made: kept until it is known whether a decision was
 // close, they would not fit the registers beside weights and energies.
 template <int BITS, int V, int DT>
@@ -242,7 +243,9 @@ __device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, f
     return chosen;
 }
 
-// Blocks of an SM, by registers: what a thread keeps is its weights.
+// Blocks of an SM, by registers: what a thread keeps is its weights.  The caps spill a little (76 bytes of stores a thread for INT4, 208 and
+// up for INT2), which costs less than the warps would in most: 4096 x 4096 fp16 with these / with one block fewer, us: groups of 128
+// INT4 106 / 114, INT2 74.6 / 70.0, 256 INT4 95 / 111, INT2 69 / 65, 512 INT2 76 / 80; without statistics 23 - 26 / 24 - 34.
 __host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ? (bits == 2 ? 4 : 3) : v == 2 ? (bits == 2 ? 3 : 2) : bits == 2 ? 2 : 1; }
 
 // SEARCH: there are statistics, the scale is searched for.

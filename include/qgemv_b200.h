@@ -176,7 +176,8 @@ int qgemv_workspace_status(const void* workspace, void* stream, int32_t* host_ou
 
 /* The same GEMV for loops that issue it again and again, and for up to QGEMV_MAX_BATCH rows: qgemv_prepare validates and plans
  * once, into a caller-owned host buffer of qgemv_prepared_bytes() bytes; qgemv_launch_prepared only launches.  x and y may
- * change from call to call (same shape, strides and alignment), and so may the workspace.  x needs only k_original columns
+ * change from call to call (same shape, strides and alignment), and so may the workspace.  A launch may be two kernels: three or
+ * four rows of x that are not padded or not 16-byte aligned may be copied into the workspace first.  x needs only k_original columns
  * (ldx >= k_original) except for the CUDA-core kernel, which qgemv_prepare reports with QGEMV_ERR_ALIGN (pad x, and pass
  * k_original = k_padded with res_v padded likewise, or use qgemv_run).  `ordered` != 0: the
  * preceding kernel of the stream may still be writing the weights, so the launch does not overlap it, whichever kernel was
