@@ -32,6 +32,8 @@ UNITS = [
     ("qgemv_pipe.cu", ["-DQGEMV_INST_BITS=4"], "qgemv_pipe_int4.o"),
     ("qgemv_plan.cu", [], "qgemv_plan.o"),
     *(("qgemv_stream.cu", [f"-DQGEMV_STREAM_MODE={m}", f"-DQGEMV_STREAM_BF16={b}"], f"qgemv_stream_{m}{b}.o") for m in range(3) for b in range(2)),
+    ("qgemv_held_plan.cu", [], "qgemv_held_plan.o"),
+    *(("qgemv_held.cu", [f"-DQGEMV_HELD_FMT={f}", f"-DQGEMV_HELD_BF16={b}"], f"qgemv_held_{f}{b}.o") for f in range(5) for b in range(2)),
 ]
 OBJDIR = CSRC / "build"
 NVCC_FLAGS = [

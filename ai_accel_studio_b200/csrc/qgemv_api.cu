@@ -2,7 +2,7 @@
 #include <cstdarg>
 #include <cstdio>
 
-#include "qgemv_stream.cuh"
+#include "qgemv_held.cuh"
 
 namespace qgemv {
 
@@ -139,10 +139,25 @@ MmaPlan choose(const qgemv_problem& p, size_t partial_floats, bool* forced_missi
     return plan;
 }
 
+// Up to four rows of short K: the kernel that holds its activations in registers instead of staging them.  Every CTA makes the residual
+// projections itself then, where the phased kernel passes them on between CTAs; without a residual it still wins for groups of 128 and more,
+// whose scales cost it least.  It has the longer way per 16 weight rows, so not where an SM gets more than two such tiles.  In a chain, M = 1,
+// held against phased kernel: 896 x 896 INT2 with residual 4.0 against 5.1 us, INT4 3.9 against 4.6; 4864 x 896 5.7 against 6.3 and 5.8 against
+// 6.2; 9728 x 896 INT2 9.1 against 6.2; 2048 x 2048 5.8 against 5.1; without residual 2048 x 768 INT2 2.7 against 3.7, groups of 64 1024 x 1024
+// 2.7 against 2.4, of 32 INT4 2.8 against 2.1.
+bool choose_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* plan) {
+    if (p.kernel != QGEMV_KERNEL_AUTO || p.m > QGEMV_MAX_M || p.k_padded > 1024 || p.k_original != p.k_padded) return false;
+    const int tiles = (p.n + kStreamTileRows - 1) / kStreamTileRows, sms = sm_count();
+    if (tiles * 4 > sms * 9 || (p.rank == 0 && p.group < 128) || (p.group == 32 && tiles > sms)) return false;
+    return plan_held(p, partial_floats, plan);
+}
+
 }  // namespace
 
 extern "C" const char* qgemv_plan_name(const qgemv_problem* p) {
     if (validate(p, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0)) != QGEMV_OK) return nullptr;
+    HeldPlan held;
+    if (choose_held(*p, kMaxPartialFloats, &held)) return "qgemv_held_kernel";
     bool missing = false;
     const MmaPlan plan = choose(*p, kMaxPartialFloats, &missing);
     if (plan.ok) return plan.name;
@@ -162,6 +177,10 @@ int run_checked(const qgemv_problem* p, void* stream, size_t need_bytes, size_t 
     Args a = make_args(*p, partial_floats);
     const bool bf16 = p->x_dtype == QGEMV_BF16;
 
+    if (!x_follows) {
+        HeldPlan held;
+        if (choose_held(*p, partial_floats, &held)) return launch_held(held, bf16, !ordered, p->workspace, s);
+    }
     bool missing = false;
     MmaPlan plan = choose(*p, partial_floats, &missing);
     plan.ordered = ordered;
@@ -242,6 +261,24 @@ extern "C" int qgemv_plan_describe(const qgemv_problem* p, qgemv_plan_info* out)
     if (!out) { set_error("qgemv_plan_describe: out is NULL"); return QGEMV_ERR_BAD_ARG; }
     const int v = validate(p, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0));
     if (v != QGEMV_OK) return v;
+    HeldPlan held;
+    if (choose_held(*p, kMaxPartialFloats, &held)) {
+        *out = qgemv_plan_info{};
+        out->family = QGEMV_KERNEL_MMA;
+        out->variant = 3;
+        out->launches = 1;
+        out->grid = held.groups * held.args.ksplit;
+        out->warps = held.wk * held.wr;
+        out->smem_bytes = held.smem;
+        out->tile_aligned = 1;
+        out->inline_projections = p->rank > 0;
+        out->ctas_per_sm = 1;
+        out->stages = held_depth(p->bits, held.kbw);
+        out->chunk_bytes = 128;
+        out->run_chunks = (held.args.row_bytes + 127) / 128;
+        out->runs_per_tile = 1;
+        return QGEMV_OK;
+    }
     bool missing = false;
     const MmaPlan plan = choose(*p, kMaxPartialFloats, &missing);
     if (missing) { set_error("qgemv_plan_describe: the tensor-core-assisted kernels do not support this shape"); return QGEMV_ERR_SHAPE; }
@@ -313,6 +350,7 @@ struct Prepared {                                  // what qgemv_prepare writes 
     int pitch;                                     // > 0: two launches, the second on a copy of x with rows of this many elements, in the workspace
     bool project;                                  // the copying launch also makes the residual projections
     StreamPlan plan;                               // ok == false: as qgemv_run, four rows at a time
+    HeldPlan held;
 };
 static_assert(kWsTraceOff + kWsTraceBytes <= kWsPartialOff + (kMaxPartialFloats - kTPartFloats - kStreamWordFloats) * sizeof(float) &&
               kWsCopyOff + kWsCopyBytes <= kWsPartialOff + (kMaxPartialFloats - kTPartFloats - kStreamWordFloats) * sizeof(float),
@@ -341,6 +379,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     q->problem = *p;
     q->plan = StreamPlan{};
     q->pitch = 0; q->project = false;
+    q->held.ok = false;
     const bool padded = p->ldx >= p->k_padded && p->k_padded == p->k_original;
     bool starved = false;
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && padded) {
@@ -349,6 +388,9 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
     }
+    if (choose_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
+    if (p->kernel == QGEMV_KERNEL_AUTO && (p->m > QGEMV_MAX_M || (starved && p->m > 2)) && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
+    q->held.ok = false;
     // Three or four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of
     // its 16 warps (see align_x_kernel) and loses no precision against the streaming kernel, which takes x as it is.  One and two rows
     // stay with that: it adds them up as integers (error of a result before it is rounded 1e-7, in the phased kernel 5e-7 to 2e-5, 1024 rows
@@ -387,6 +429,12 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
 extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspace, int ordered, void* stream) {
     Prepared* q = static_cast<Prepared*>(prepared);
     if (!q || !x || !y || !workspace) { set_error("qgemv_launch_prepared: null pointer"); return QGEMV_ERR_BAD_ARG; }
+    if (q->held.ok) {
+        if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
+        q->held.args.x = x;
+        q->held.args.y = y;
+        return launch_held(q->held, q->problem.x_dtype == QGEMV_BF16, !ordered, workspace, static_cast<cudaStream_t>(stream));
+    }
     if (q->plan.ok) {
         if (!aligned(x, 16)) { set_error("qgemv_launch_prepared: x must be 16-byte aligned, as it was for qgemv_prepare"); return QGEMV_ERR_ALIGN; }
         q->plan.args.x = x;

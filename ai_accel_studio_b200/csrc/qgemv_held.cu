@@ -1,0 +1,768 @@
+// Fused GEMV for packed groupwise INT2 / INT4 weights with the activations held in registers, up to 16 rows, sm_100a.
+//
+// The warps of a CTA cut K between them.  A warp loads its columns of x straight into mma B fragments (16 registers per 128 columns
+// and 8 activation rows) and keeps them for all weight rows of the CTA, so x is neither staged in shared memory nor read
+// again per tile, and nearly all of the SM's shared memory is ring: every warp copies its 128 to 512 columns of the next 16-row tiles with
+// cp.async.  What a warp adds up for a tile meets the other warps' sums in shared memory, once per batch of tiles; the batch
+// before is finished (outliers, residual, bias, activation, store) while the next one streams.
+//
+//  * Codes are not converted: `word & mask` leaves one code in the low mantissa bits of each 16-bit half, an fp16 subnormal worth
+//    code * radix^c * 2^-24.  The classes c accumulate apart and are weighed in fp32.  x is fp16 as it comes (bf16: a power of two per 128
+//    columns, exact).
+//  * One more warp serves the others: group scales of the next batch (each row's are one contiguous piece), outlier columns as one
+//    more partial sum, rows of U, the projections t = V x.
+//  * t comes from the fragments, by mma with the rows of V as A.  With few columns every CTA makes all of it; else the first CTAs
+//    make a row or more each and pass them on as {value, launch tag} words.
+//  * K is split between CTAs where a row's activations do not fit the registers of a CTA's warps, or where there are few rows;
+//    the last CTA to arrive adds the splits in order.
+//
+// Replaces _decode_gemv (ai_accel_lab/kernels/decode_int2.py:43-96) and _decode_int4_gemv
+// (ai_accel_lab/kernels/groupwise_int4.py:85-107) of the reference project.
+#include <type_traits>
+
+#include "qgemv_frag.cuh"
+#include "qgemv_held.cuh"
+
+namespace qgemv {
+namespace {
+
+__device__ __forceinline__ void mbarrier_init(uint32_t mb, int count) { asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(mb), "r"(count) : "memory"); }
+// This thread's arrival, once its asynchronous copies so far have landed.
+__device__ __forceinline__ void mbarrier_arrive_copies(uint32_t mb) { asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(mb) : "memory"); }
+// Bounded: copies always land, so running out (about a second) would mean a lost copy.
+__device__ __forceinline__ bool mbarrier_wait(uint32_t mb, int parity) {
+    for (int i = 0; i < (1 << 20); ++i) {
+        uint32_t ok;
+        asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.shared.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }" : "=r"(ok) : "r"(mb), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// Two 64-bit registers: an mma wants a B pair in neighbouring ones, and values that live through the main loop are else moved there before every use.
+__device__ __forceinline__ void lds128(uint32_t a, uint64_t& x, uint64_t& y) { asm("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory"); }
+__device__ __forceinline__ void sts128(uint32_t a, const uint4& v) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory"); }
+__device__ __forceinline__ void sts_half(uint32_t a, __half v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(__half_as_ushort(v)) : "memory"); }
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+    uint16_t v; asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory"); return v;
+}
+
+template <int FMT, int KBW> struct Held {
+    using F = Fmt<FMT>;
+    static constexpr int BW = F::BITS == 2 ? 32 : 64;                 // bytes of a block in a weight row
+    static constexpr int SB = held_stage_blocks(F::BITS, KBW);        // blocks of a ring stage
+    static constexpr int NS = KBW / SB;                               // stages of a tile
+    static constexpr int PITCH = SB * BW;                             // bytes of a weight row in a stage: 32, 64 or 128
+    static constexpr int STAGE = 16 * PITCH;
+    static constexpr int DEPTH = held_depth(F::BITS, KBW);
+    static constexpr int PPR = PITCH / 16, RPI = 32 / PPR, COPIES = 16 / RPI;
+};
+
+// XOR for the 16-byte pieces of a 128-byte line, so that the rows one shared-memory read touches fall into different banks.
+template <int PITCH> __device__ __forceinline__ int stage_swizzle(int r) {
+    if constexpr (PITCH == 32) return (r >> 2) & 1;
+    else if constexpr (PITCH == 64) return (r & 2) | ((r >> 2) & 1);
+    else return row_swizzle(r);
+}
+template <int PITCH> __device__ __forceinline__ uint32_t stage_offset(int r, int byte) {
+    const int at = r * PITCH;
+    return (uint32_t)((at & ~127) + (((at & 127) + byte) ^ (stage_swizzle<PITCH>(r) << 4)));
+}
+
+// Float index of (activation column c, weight row r) in a partial sum of hp * 2 columns per 8: writes of the mma layout and reads
+// of four rows are free of bank conflicts.
+__device__ __forceinline__ int part_index(int hp, int c, int r) {
+    const int p = ((c & 7) >> 1) + hp * (c & 1);
+    return (c >> 3) * 128 + p * 16 + (r ^ (((p >> 1) & 1) * 8));
+}
+
+// Producer side of a warp's ring: stages in the order (tile, part of the columns).
+template <typename H> struct Ring {
+    const uint8_t* src;                               // this lane's row and piece of the next tile, first stage
+    long long step;                                   // to the warp's next tile
+    int ldw, row, row_step, last, end_row;            // weight row of that tile, the last one a tile may start at, end of the CTA's rows
+    int left;                                         // bytes from this lane's piece to the end of the warp's columns
+    uint32_t dst, at;
+
+    __device__ __forceinline__ void issue() {         // all stages of a tile
+        const bool more = row < end_row;
+        if (more && row > last) { src -= (long long)(row - last) * ldw; row = last; end_row = last; }      // the last tile of all ends with the matrix
+#pragma unroll
+        for (int st = 0; st < H::NS; ++st) {
+            if (more && left > st * H::PITCH) {
+                const uint32_t d = dst + at;
+#pragma unroll
+                for (int i = 0; i < H::COPIES; ++i) cp_async16((H::PITCH == 128 && (i & 1) ? d ^ 16u : d) + i * 512, src + (long long)(i * H::RPI) * ldw + st * H::PITCH);
+            }
+            cp_async_commit();
+            at = at + H::STAGE == H::DEPTH * H::STAGE ? 0u : at + H::STAGE;
+        }
+        src += step;
+        row += row_step;
+    }
+};
+
+__device__ __forceinline__ void mma_pair(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint64_t b) {
+    asm("{ .reg .b32 b0, b1; mov.b64 {b0, b1}, %8; mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%0,%1,%2,%3}; }"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(b));
+}
+__device__ __forceinline__ void mma_pair(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint64_t b, const float (&c)[4]) {
+    asm("{ .reg .b32 b0, b1; mov.b64 {b0, b1}, %8; mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%9,%10,%11,%12}; }"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(b), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+// y += scale * level sum of scale group j of block kb (16 weight rows).  ci: offset of the levels times the sums of x.  Every class is a chain of
+// its own from zero, weighed in fp32: one accumulator for all, with the offset in it, has 2 to 6 times the error, because the tensor cores
+// cut what they add to the size of what is there.  The A operands of all activations' mma come from the same registers, so these follow each other.
+template <int FMT, int NB, bool BF16>
+__device__ __forceinline__ void group_block(const uint32_t (&w0)[Fmt<FMT>::W], const uint32_t (&w1)[Fmt<FMT>::W], int j, const uint64_t (&fr)[NB][8],
+                                            const float (&zero)[4], const float4 (&ci)[NB], float s0, float s1, float (&y)[NB][4]) {
+    using F = Fmt<FMT>;
+    constexpr int CL = F::BITS == 4 ? 2 : 4;          // position classes of a code in a 16-bit half: the masks that need no shift
+    constexpr float kDown = F::BITS == 4 ? 1.0f / 16.0f : 0.25f;
+    float sum[NB][4];
+#pragma unroll
+    for (int cl = CL - 1; cl >= 0; --cl) {
+        const uint32_t mk = F::BITS == 4 ? 0x000f000fu << (4 * cl) : 0x00030003u << (2 * cl);
+        float c[NB][4];
+#pragma unroll
+        for (int i = 0; i < F::WG; ++i) {
+            const int q = j * F::WG + i;
+            const uint32_t a0 = w0[q] & mk, a1 = w1[q] & mk, a2 = (w0[q] >> 8) & mk, a3 = (w1[q] >> 8) & mk;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                if (i == 0) mma_pair(c[b], a0, a1, a2, a3, fr[b][q * CL + cl], zero);
+                else mma_pair(c[b], a0, a1, a2, a3, fr[b][q * CL + cl]);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[b][e] = cl == CL - 1 ? c[b][e] : fmaf(sum[b][e], kDown, c[b][e]);
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        // INT2 levels are 2/3 c - 1, INT4 levels c - 8; codes carry the subnormal unit 2^-24
+        constexpr float kUnit = F::BITS == 4 ? 16777216.0f : 16777216.0f * (2.0f / 3.0f);
+        sum[b][0] = fmaf(sum[b][0], kUnit, ci[b].x); sum[b][1] = fmaf(sum[b][1], kUnit, ci[b].y);
+        sum[b][2] = fmaf(sum[b][2], kUnit, ci[b].x); sum[b][3] = fmaf(sum[b][3], kUnit, ci[b].y);
+        if constexpr (BF16) { sum[b][0] *= ci[b].z; sum[b][1] *= ci[b].w; sum[b][2] *= ci[b].z; sum[b][3] *= ci[b].w; }
+        y[b][0] = fmaf(s0, sum[b][0], y[b][0]); y[b][1] = fmaf(s0, sum[b][1], y[b][1]);
+        y[b][2] = fmaf(s1, sum[b][2], y[b][2]); y[b][3] = fmaf(s1, sum[b][3], y[b][3]);
+    }
+}
+
+template <int FMT> __device__ __forceinline__ int piece_of(int t, int q) {          // the lane's q-th piece of 8 columns of a block
+    constexpr int NG = Fmt<FMT>::NG;
+    if constexpr (NG == 1) return t * 4 + q;
+    else if constexpr (NG == 2) return (q >> 1) * 8 + t * 2 + (q & 1);
+    else return q * 4 + t;
+}
+// Sixteen bf16 values of a lane (eight lanes hold the 128 of a row and block) to fp16 with a power of two; returns what to multiply by.
+__device__ __forceinline__ float bf16_to_scaled(uint4 (&v)[2]) {
+    uint32_t big = 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const uint32_t e[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) big = max(big, max((e[i] << 16) & 0x7fffffffu, e[i] & 0x7fff0000u));
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+    const int e = block_exponent(big);
+    const float down = pow2f(13 - e);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float f[8];
+        widen8<true>(v[q], f);
+        uint32_t h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 hh = __floats2half2_rn(f[2 * i] * down, f[2 * i + 1] * down);
+            h[i] = *reinterpret_cast<const uint32_t*>(&hh);
+        }
+        v[q] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    return big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
+}
+
+// Bias, activation and store of four weight rows (r on, of the tile at row n0) of one activation column.  Called by whole warps.
+template <bool BF16>
+__device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], uint32_t bias, bool live, int m, int n0, int r) {
+    using XT = typename Act16<BF16>::T;
+    if (bias) {
+        const uint2 b = lds64(bias);
+        const __half2 lo = *reinterpret_cast<const __half2*>(&b.x), hi = *reinterpret_cast<const __half2*>(&b.y);
+        v[0] += __low2float(lo); v[1] += __high2float(lo); v[2] += __low2float(hi); v[3] += __high2float(hi);
+    }
+    int n = n0 + r;
+    if (p.act != QGEMV_ACT_NONE) {
+        if (p.act == QGEMV_ACT_SILU_MUL) {             // rows r and r + 8 of a tile are a (gate, up) pair: one output
+            auto r16 = [](float f) { return Act16<BF16>::to_float(Act16<BF16>::from_float(f)); };
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float up = r16(__shfl_xor_sync(0xffffffffu, v[e], 2)), gate = r16(v[e]);
+                v[e] = r16(gate / (1.0f + __expf(-gate))) * up;
+            }
+            live = live && r < 8;
+            n = n0 / 2 + r;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = apply_act(v[e], p.act);
+        }
+    }
+    if (!live) return;
+    XT o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = Act16<BF16>::from_float(v[e]);
+    XT* y = static_cast<XT*>(p.y) + (long long)m * p.ldy + n;
+    if ((p.flags & kHeldYVector) && (n & 3) == 0) {
+        *reinterpret_cast<uint2*>(y) = *reinterpret_cast<const uint2*>(o);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = o[e];
+    }
+}
+
+// Phase trace of a build with QGEMV_TRACE: lane 0 of every warp stores the clock.
+#ifdef QGEMV_TRACE
+#define QGEMV_HELD_STAMP(i) do { if ((threadIdx.x & 31) == 0 && (i) < 16) reinterpret_cast<long long*>(reinterpret_cast<char*>(p.partial) + (kWsTraceOff - kWsPartialOff))[((blockIdx.x + blockIdx.y * gridDim.x) * 16 + threadIdx.y + threadIdx.z * blockDim.y) * 16 + (i)] = clock64(); } while (0)
+#else
+#define QGEMV_HELD_STAMP(i) do {} while (0)
+#endif
+
+template <int FMT, int KBW, int NB, bool BF16>
+__global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const __grid_constant__ HeldArgs p) {
+    using F = Fmt<FMT>;
+    using H = Held<FMT, KBW>;
+    using XT = typename Act16<BF16>::T;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long full[kHeldMaxWarps * kHeldMaxBatch + 3];      // outlier weights of a batch's tiles have landed; U; scales, two buffers
+    QGEMV_HELD_STAMP(0);
+    pdl_launch_dependents();
+    const int lane = threadIdx.x, kw = threadIdx.y, wrow = threadIdx.z, wk = blockDim.y, wr = blockDim.z;
+    const int warp = wrow * wk + kw, tid = warp * 32 + lane, threads = wk * wr * 32;
+    const int g = lane >> 2, t = lane & 3, M = p.m;
+    const int grp = blockIdx.x, split = blockIdx.y;
+    const int rowbase = grp * p.rows_per, rowend = min(rowbase + p.rows_per, p.n), last = p.n - 16;
+    const int kb0 = split * p.blocks_split + kw * KBW;                   // this warp's first block
+    const uint32_t sm = smem_u32(smem), ring_at = sm + (uint32_t)warp * (H::DEPTH * H::STAGE);
+    const bool exchange = p.per_cta < p.rank;
+    const int nr = exchange ? min(p.per_cta, p.rank - grp * p.per_cta) : p.rank;      // ranks that this CTA projects
+    const int r0 = exchange ? grp * p.per_cta : 0;
+    float* const part = reinterpret_cast<float*>(smem + p.off_part);
+    float* const tpart = reinterpret_cast<float*>(smem + p.off_tpart);                   // a warp's share of them [8][mp]
+    float* const tt = reinterpret_cast<float*>(smem + p.off_tt);                         // residual projections [m][rank8]
+    constexpr int part_floats = NB * 128;
+    const int batch_rows = wr * p.tb * 16;
+    const bool has_o = p.noc && split == 0;
+
+    // ---- before the dependency wait: all that does not depend on x ----------------------------------------------------
+    Ring<H> ring;
+    {
+        const int r = lane / H::PPR, piece = lane % H::PPR;
+        ring.ldw = (int)p.ldw;
+        ring.left = min(p.row_bytes, (split + 1) * p.blocks_split * H::BW) - kb0 * H::BW - piece * 16;
+        ring.row = rowbase + wrow * 16; ring.row_step = wr * 16; ring.last = last; ring.end_row = rowend;
+        ring.src = p.w + (long long)(ring.row + r) * p.ldw + kb0 * H::BW + piece * 16;
+        ring.step = (long long)(wr * 16) * p.ldw;
+        ring.dst = ring_at + stage_offset<H::PITCH>(r, piece * 16);
+        ring.at = 0;
+    }
+#pragma unroll 1
+    for (int d = 0; d < H::DEPTH / H::NS; ++d) ring.issue();
+    QGEMV_HELD_STAMP(1);
+    constexpr int kFullU = kHeldMaxWarps * kHeldMaxBatch, kFullScales = kFullU + 1;
+    if (tid < p.tb * wr) mbarrier_init(smem_u32(full + tid), 32);
+    if (tid < 3) mbarrier_init(smem_u32(full + kFullU + tid), threads);
+    __syncthreads();
+    // Scales of sc_rows rows (all of the CTA's, or a batch's), from the 4- or 16-byte word that holds the K slice's first; past the row's end zero.
+    const int sc_lds = (int)p.lds, sc_first = split * p.sc_split;
+    auto stage_scales = [&](int row0, int buf) {
+        const int nrow = min(p.sc_rows, (rowend - row0 + 15) & ~15), u = tid & ((1 << p.sc_log) - 1), per = p.sc_unit >> 1;
+        if (u < p.sc_units) {
+            const uint32_t to = sm + p.off_sc + buf * p.sc_bytes + u * p.sc_unit;
+#pragma unroll 1
+            for (int r = tid >> p.sc_log; r < nrow; r += threads >> p.sc_log) {
+                const int off = (min(row0 + (r & ~15), last) + (r & 15)) * sc_lds + sc_first, odd = off & 1, n = max(0, min(per, p.ng - sc_first + odd - u * per)) * 2;
+                const __half* from = n ? p.sc + (off - odd + u * per) : p.sc;
+                if (per == 8) cp_async16z(to + r * p.sc_pitch, from, n);
+                else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + r * p.sc_pitch), "l"(from), "r"(n) : "memory");
+            }
+        }
+        mbarrier_arrive_copies(smem_u32(full + kFullScales + buf));
+    };
+    stage_scales(rowbase, 0);
+    // Outlier weights of a batch's tiles, each fetched and multiplied by one warp of its row of warps, another one from batch to batch.
+    int turn = kw;                                     // this warp has tile `turn` of its row's batch, and every wk-th after it
+    auto stage_outliers = [&](int row0) {
+        const uint32_t to = sm + p.off_ow;
+        const int units = p.noc * 4;
+#pragma unroll 1
+        for (int i = turn; i < p.tb; i += wk) {
+            const int jt = i * wr + wrow, row = row0 + jt * 16;
+            if (row >= rowend) break;
+#pragma unroll 1
+            for (int e = lane; e < 16 << p.ow_log; e += 32) {
+                const int r = e >> p.ow_log, u = e & ((1 << p.ow_log) - 1), left = min(8, p.oc - u * 8);
+                if (u >= units) continue;
+                const uint32_t d = to + (uint32_t)((jt * 16 + r) * units + u) * 16;
+                const __half* from = p.ow + (long long)(min(row, last) + r) * p.ldow + u * 8;
+                if (p.flags & kHeldOutlierAligned) cp_async16z(d, left > 0 ? from : p.ow, left > 0 ? left * 2 : 0);
+                else
+                    for (int q = 0; q < 8; ++q) sts_half(d + q * 2, q < left ? __ldg(from + q) : __half(0.0f));
+            }
+            mbarrier_arrive_copies(smem_u32(full + jt));
+        }
+    };
+    if (has_o) stage_outliers(rowbase);
+    {                                                  // rows of U (padded to 8 columns) and bias of all the CTA's tiles
+        const int nrow = (rowend - rowbase + 15) & ~15, pieces = p.rank8 >> 3;
+        for (int i = tid; i < nrow; i += threads) {
+            const int n = min(rowbase + (i & ~15), last) + (i & 15);
+            for (int q = 0; q < pieces; ++q) {
+                const __half* from = p.ru + (long long)n * p.ldu + q * 8;
+                const uint32_t d = sm + p.off_u + (uint32_t)(i * pieces + q) * 16;
+                if (p.flags & kHeldUAligned) cp_async16z(d, from, 16);
+                else
+                    for (int k = 0; k < 8; ++k) sts_half(d + k * 2, q * 8 + k < p.rank ? __ldg(from + k) : __half(0.0f));
+            }
+            if (p.bias) sts_half(sm + p.off_bias + i * 2, __ldg(p.bias + n));
+        }
+        mbarrier_arrive_copies(smem_u32(full + kFullU));
+    }
+    const int n_xo = has_o ? M << p.oc_log : 0, xo_mask = (1 << p.oc_log) - 1;      // activations of the outlier columns, [m][column]
+    int xcol = -1;
+    if (tid < n_xo && (tid & xo_mask) < p.oc) xcol = __ldg(p.oidx + (tid & xo_mask));
+    for (int i = tid; i < p.rank8 * M; i += threads) tt[i] = 0.0f;
+    QGEMV_HELD_STAMP(2);
+    pdl_wait();
+    QGEMV_HELD_STAMP(3);
+
+    // ---- activations of this warp's columns as B fragments, and what the offset of the levels makes of their sums ----------
+    // Columns of B past the last activation row repeat it: their sums are not used.
+    float zero[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) asm volatile("mov.b32 %0, 0;" : "=f"(zero[e]));
+    uint64_t fr[KBW][NB][8];
+    float4* const tab = reinterpret_cast<float4*>(smem + p.off_tab) + (size_t)warp * (KBW * F::NG * NB * 4) + t;
+    // Rows of 128 columns come 32 bytes a lane, four rows a load, are permuted to code order and change hands through the warp's part of shared
+    // memory (16-byte pieces, swizzled): a fragment loaded directly would touch 16 lines a load, and the SM looks up about one a clock.
+    const int kend = min(p.korig, (split + 1) * p.blocks_split * kHeldBlock);
+    const uint32_t scratch = sm + p.off_part + (uint32_t)warp * 2048;
+    auto load_rows = [&](const unsigned short* base, long long ld, int nrow, int kb, uint4 (&v)[2][2]) {
+        const int k = (kb0 + kb) * kHeldBlock + (lane & 7) * 16;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (i * 4 >= nrow) continue;
+            const unsigned short* from = base + (long long)min(i * 4 + (lane >> 3), nrow - 1) * ld + k;
+            if ((kb0 + kb + 1) * kHeldBlock <= kend) {
+                v[i][0] = *reinterpret_cast<const uint4*>(from);
+                v[i][1] = *reinterpret_cast<const uint4*>(from + 8);
+            } else {
+                v[i][0] = v[i][1] = make_uint4(0u, 0u, 0u, 0u);
+                if (k < kend) v[i][0] = *reinterpret_cast<const uint4*>(from);
+                if (k + 8 < kend) v[i][1] = *reinterpret_cast<const uint4*>(from + 8);
+            }
+        }
+    };
+    constexpr int kRowBit = F::NG == 1 ? 2 : F::NG == 2 ? 1 : 4;       // what an odd row flips of a piece's position
+    auto to_frag = [&](uint4 (&v)[2][2], int nrow, uint64_t (&f)[8]) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = i * 4 + (lane >> 3), pc = (lane & 7) * 2;
+            const uint32_t at = scratch + (uint32_t)(r * 256 + (pc ^ ((pc >> 3) & 1) ^ ((r & 1) * kRowBit)) * 16);
+            if (i * 4 < nrow) {
+                to_frag_order<F::BITS>(v[i][0], v[i][1]);
+                sts128(at, v[i][0]);
+                sts128(at ^ 16u, v[i][1]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int pc = piece_of<FMT>(t, q);
+            lds128(scratch + (uint32_t)(g * 256 + (pc ^ ((pc >> 3) & 1) ^ ((g & 1) * kRowBit)) * 16), f[q * 2], f[q * 2 + 1]);
+        }
+        __syncwarp();
+    };
+    uint4 xv[NB][KBW][2][2];
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int kb = 0; kb < KBW; ++kb) load_rows(static_cast<const unsigned short*>(p.x) + (long long)(b * 8) * p.ldx, p.ldx, M - b * 8, kb, xv[b][kb]);
+    {
+        XT xval = XT(0.0f);
+        if (xcol >= 0 && xcol < p.korig) xval = static_cast<const XT*>(p.x)[(long long)(tid >> p.oc_log) * p.ldx + xcol];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+#pragma unroll
+            for (int kb = 0; kb < KBW; ++kb) {
+                if constexpr (BF16) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const float up = bf16_to_scaled(xv[b][kb][i]);
+                        const int r = i * 4 + (lane >> 3);
+                        if ((lane & 7) == 0) {
+                            float* u = reinterpret_cast<float*>(tab - t + (kb * F::NG * NB + b) * 4 + (r >> 1)) + 2 + (r & 1);
+#pragma unroll
+                            for (int j = 0; j < F::NG; ++j) u[j * NB * 16] = up;
+                        }
+                    }
+                }
+                to_frag(xv[b][kb], M - b * 8, fr[kb][b]);
+            }
+        }
+#pragma unroll 1
+        for (int i = tid; i < n_xo; i += threads) {    // whole warps: a power of two of 32 and more columns per row
+            const int j = i & xo_mask, m = i >> p.oc_log;
+            if (i != tid) {
+                const int col = j < p.oc ? __ldg(p.oidx + j) : -1;
+                xval = col >= 0 && col < p.korig ? static_cast<const XT*>(p.x)[(long long)m * p.ldx + col] : XT(0.0f);
+            }
+            float f = Act16<BF16>::to_float(xval);
+            if constexpr (BF16) {                      // a power of two per 32 columns keeps fp16 exact
+                uint32_t big = __float_as_uint(f) & 0x7fffffffu;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+                const int e = block_exponent(big);
+                f *= pow2f(13 - e);
+                if (lane == 0 && j < p.noc * 32)
+                    reinterpret_cast<float*>(smem + p.off_upo)[(j >> 5) * M + m] = big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
+            }
+            if (j < p.noc * 32) *reinterpret_cast<__half*>(smem + p.off_xo + (size_t)m * (p.noc * 64 + 16) + j * 2) = __float2half_rn(f);
+        }
+        constexpr float kOffset = F::BITS == 4 ? -8.0f : -1.0f;
+#pragma unroll
+        for (int kb = 0; kb < KBW; ++kb)
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                float2 sx[F::NG];
+#pragma unroll
+                for (int j = 0; j < F::NG; ++j) {
+                    float a[4];
+                    mma_pair(a, kOnesF16, kOnesF16, kOnesF16, kOnesF16, fr[kb][b][j * (8 / F::NG)], zero);
+#pragma unroll
+                    for (int i = 1; i < 8 / F::NG; ++i) mma_pair(a, kOnesF16, kOnesF16, kOnesF16, kOnesF16, fr[kb][b][j * (8 / F::NG) + i]);
+                    sx[j] = make_float2(a[0], a[1]);
+                }
+                if (g == 0) {
+#pragma unroll
+                    for (int j = 0; j < F::NG; ++j) *reinterpret_cast<float2*>(tab + ((kb * F::NG + j) * NB + b) * 4) = make_float2(sx[j].x * kOffset, sx[j].y * kOffset);
+                }
+            }
+        __syncwarp();
+    }
+    QGEMV_HELD_STAMP(4);
+    if (nr > 0 && wrow == 0) {                         // residual projections of this warp's columns, up to eight ranks
+        float acc[NB][4];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) acc[b][0] = acc[b][1] = 0.0f;
+        const unsigned short* const vr = reinterpret_cast<const unsigned short*>(p.rv) + (long long)r0 * p.ldv;
+#pragma unroll
+        for (int kb = 0; kb < KBW; ++kb) {
+            uint4 a[2][2];
+            uint64_t fa[8];
+            load_rows(vr, p.ldv, nr, kb, a);
+            to_frag(a, nr, fa);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                float c[4];
+                mma_pair(c, (uint32_t)fa[0], 0u, (uint32_t)(fa[0] >> 32), 0u, fr[kb][b][0], zero);
+#pragma unroll
+                for (int i = 1; i < 8; ++i) mma_pair(c, (uint32_t)fa[i], 0u, (uint32_t)(fa[i] >> 32), 0u, fr[kb][b][i]);
+                float ua = 1.0f, ub = 1.0f;
+                if constexpr (BF16) { const float4 f = tab[((kb * F::NG) * NB + b) * 4]; ua = f.z; ub = f.w; }
+                acc[b][0] = fmaf(c[0], ua, acc[b][0]); acc[b][1] = fmaf(c[1], ub, acc[b][1]);
+            }
+        }
+        float* const mine = tpart + (kw * 8 + g) * p.mp + 2 * t;
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            if (b * 8 + 2 * t < p.mp) *reinterpret_cast<float2*>(mine + b * 8) = make_float2(acc[b][0], acc[b][1]);
+    }
+    __syncthreads();                                   // projections, outlier activations, all that was stored without an asynchronous copy
+    unsigned long long* const words = p.words + (size_t)split * p.rank * M;
+    if (nr > 0 && tid < nr * M) {                      // the warps' shares in order
+        const unsigned tag = exchange ? (unsigned)(ld_relaxed_u64(p.epoch) >> 8) + 1u : 0u;
+        for (int i = tid; i < nr * M; i += threads) {
+            const int r = i / M, m = i - r * M;
+            float v = 0.0f;
+#pragma unroll 4
+            for (int k = 0; k < wk; ++k) v += tpart[(k * 8 + r) * p.mp + m];
+            if (!exchange) tt[m * p.rank8 + r] = v;
+            else if (!(p.debug & QGEMV_DEBUG_DROP_PROJECTIONS))
+                st_relaxed_u64(words + (r0 + r) * M + m, ((unsigned long long)tag << 32) | __float_as_uint(v));
+        }
+    }
+
+    QGEMV_HELD_STAMP(5);
+    // ---- main loop -----------------------------------------------------------------------------------------------------
+    uint32_t co[F::NG];                                // the lane's code words of row g in a stage
+#pragma unroll
+    for (int j = 0; j < F::NG; ++j) {
+        const int byte = F::WG == 4 ? t * 16 : F::WG == 2 ? j * 32 + t * 8 : j * 16 + t * 4;
+        co[j] = stage_offset<H::PITCH>(g, byte);       // the piece bits of block b: XOR, they do not overlap
+    }
+    uint32_t sc_off[KBW];                              // a row's scales: warp's first one at byte 0 or, from an odd one on, 2
+#pragma unroll
+    for (int kb = 0; kb < KBW; ++kb) sc_off[kb] = F::NG > 1 ? (uint32_t)(kb * F::NG * 2) : (uint32_t)((kb >> p.gshift) * 2);
+    const int hp = p.mp < 8 ? p.mp >> 1 : 4;
+    const int po0 = part_index(hp, 2 * t, g), po1 = part_index(hp, 2 * t + 1, g);      // rows g + 8: XOR 8
+    uint32_t slot = ring_at;
+    int row = rowbase + wrow * 16, bt = 0, turn0 = 0;
+    const uint32_t sc_lane = sm + p.off_sc + (uint32_t)((wrow * 16 + g) * p.sc_pitch + (F::NG > 1 ? kw * KBW * F::NG : kw * KBW >> p.gshift) * 2);
+    for (int row0 = rowbase; row0 < rowend; row0 += batch_rows, ++bt) {
+        const int buf = bt & 1;
+        const int sb = p.sc_all ? 0 : buf;
+        if (!p.sc_all && row0 + batch_rows < rowend) stage_scales(row0 + batch_rows, buf ^ 1);      // every warp is done with that buffer's last batch
+        if (bt > 0 && has_o) stage_outliers(row0);
+        if (!mbarrier_wait(smem_u32(full + kFullScales + sb), p.sc_all ? 0 : (bt >> 1) & 1) && lane == 0) atomicExch(p.status, 2);
+        uint32_t sc_tile = sc_lane + (p.sc_all ? (uint32_t)((row0 - rowbase) * p.sc_pitch) : (uint32_t)(buf * p.sc_bytes));
+        float* dst = part + (size_t)buf * (p.part_bytes / 4) + (size_t)warp * part_floats;
+        const int batch_end = min(row0 + batch_rows, rowend);
+#pragma unroll 1
+        for (; row < batch_end; row += wr * 16) {
+            float y[NB][4];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) y[b][0] = y[b][1] = y[b][2] = y[b][3] = 0.0f;
+            const uint32_t sc = sc_tile + (((uint32_t)((min(row, last) + g) * sc_lds + sc_first) & 1u) << 1);
+#pragma unroll
+            for (int st = 0; st < H::NS; ++st) {
+                if (st == 0) cp_async_wait_n<H::DEPTH - 1>(); else cp_async_wait_n<H::DEPTH - 2>();      // a tile's stages are refilled together
+                __syncwarp();
+                uint32_t s0[H::SB * F::NG], s1[H::SB * F::NG];
+#pragma unroll
+                for (int sb = 0; sb < H::SB; ++sb) {
+                    const int kb = st * H::SB + sb;
+                    uint32_t w0[F::W], w1[F::W];
+#pragma unroll
+                    for (int j = 0; j < F::NG; ++j) {
+                        const uint32_t at = slot + (co[j] ^ (uint32_t)(sb * H::BW));
+                        if constexpr (F::WG == 4) {
+                            const uint4 a = lds128(at), d = lds128(at + 8 * H::PITCH);
+                            w0[0] = a.x; w0[1] = a.y; w0[2] = a.z; w0[3] = a.w;
+                            w1[0] = d.x; w1[1] = d.y; w1[2] = d.z; w1[3] = d.w;
+                        } else if constexpr (F::WG == 2) {
+                            const uint2 a = lds64(at), d = lds64(at + 8 * H::PITCH);
+                            w0[j * 2] = a.x; w0[j * 2 + 1] = a.y;
+                            w1[j * 2] = d.x; w1[j * 2 + 1] = d.y;
+                        } else {
+                            w0[j] = lds32(at);
+                            w1[j] = lds32(at + 8 * H::PITCH);
+                        }
+                        s0[sb * F::NG + j] = lds_u16(sc + sc_off[kb] + j * 2);
+                        s1[sb * F::NG + j] = lds_u16(sc + sc_off[kb] + j * 2 + 8 * p.sc_pitch);
+                    }
+#pragma unroll
+                    for (int j = 0; j < F::NG; ++j) {
+                        const float f0 = __half2float(__ushort_as_half((unsigned short)s0[sb * F::NG + j])), f1 = __half2float(__ushort_as_half((unsigned short)s1[sb * F::NG + j]));
+                        float4 ci[NB];
+#pragma unroll
+                        for (int b = 0; b < NB; ++b) {
+                            if constexpr (BF16) ci[b] = tab[((kb * F::NG + j) * NB + b) * 4];
+                            else { const float2 c2 = *reinterpret_cast<const float2*>(tab + ((kb * F::NG + j) * NB + b) * 4); ci[b] = make_float4(c2.x, c2.y, 1.0f, 1.0f); }
+                        }
+                        group_block<FMT, NB, BF16>(w0, w1, j, fr[kb], zero, ci, f0, f1, y);
+                    }
+                }
+                if (st == H::NS - 1) {
+                    __syncwarp();                      // every lane has read the tile before it is refilled
+                    ring.issue();
+                }
+                slot = slot + H::STAGE == ring_at + H::DEPTH * H::STAGE ? ring_at : slot + H::STAGE;
+            }
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                if (b * 8 + 2 * t < p.mp) {
+                    dst[b * 128 + po0] = y[b][0];
+                    dst[b * 128 + po1] = y[b][1];
+                    dst[b * 128 + (po0 ^ 8)] = y[b][2];
+                    dst[b * 128 + (po1 ^ 8)] = y[b][3];
+                }
+            }
+            dst += threads / 32 * part_floats;
+            sc_tile += (uint32_t)(wr * 16 * p.sc_pitch);
+        }
+        QGEMV_HELD_STAMP(6 + bt * 2);
+        if (has_o) {                                   // outlier columns, 32 per two mma, onto the warp's own sums
+#pragma unroll 1
+            for (int i = turn; i < p.tb; i += wk) {
+                const int jt = i * wr + wrow;
+                if (row0 + jt * 16 >= rowend) break;
+                if (!mbarrier_wait(smem_u32(full + jt), bt & 1) && lane == 0) atomicExch(p.status, 2);
+                __syncwarp();
+                const uint32_t ow = sm + p.off_ow + (uint32_t)((jt * 16 + g) * (p.noc * 64) + t * 16);
+                float v[NB][4];
+#pragma unroll
+                for (int b = 0; b < NB; ++b) v[b][0] = v[b][1] = v[b][2] = v[b][3] = 0.0f;
+#pragma unroll 1
+                for (int blk = 0; blk < p.noc; ++blk) {
+                    const uint4 a = lds128(ow + blk * 64), d = lds128(ow + blk * 64 + 8 * p.noc * 64);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        const uint4 xv = lds128(sm + p.off_xo + (uint32_t)min(b * 8 + g, M - 1) * (p.noc * 64 + 16) + blk * 64 + t * 16);
+                        if constexpr (BF16) {
+                            float acc[4];
+                            mma_f16(acc, a.x, d.x, a.y, d.y, xv.x, xv.y, zero);
+                            mma_f16(acc, a.z, d.z, a.w, d.w, xv.z, xv.w);
+                            const float* upo = reinterpret_cast<const float*>(smem + p.off_upo) + blk * M;
+                            const float ua = upo[min(b * 8 + 2 * t, M - 1)], ub = upo[min(b * 8 + 2 * t + 1, M - 1)];
+                            v[b][0] = fmaf(acc[0], ua, v[b][0]); v[b][1] = fmaf(acc[1], ub, v[b][1]);
+                            v[b][2] = fmaf(acc[2], ua, v[b][2]); v[b][3] = fmaf(acc[3], ub, v[b][3]);
+                        } else {
+                            mma_f16(v[b], a.x, d.x, a.y, d.y, xv.x, xv.y);
+                            mma_f16(v[b], a.z, d.z, a.w, d.w, xv.z, xv.w);
+                        }
+                    }
+                }
+                float* const o = part + (size_t)buf * (p.part_bytes / 4) + (size_t)(i * (threads / 32) + warp) * part_floats;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    if (b * 8 + 2 * t < p.mp) {
+                        o[b * 128 + po0] += v[b][0]; o[b * 128 + po1] += v[b][1];
+                        o[b * 128 + (po0 ^ 8)] += v[b][2]; o[b * 128 + (po1 ^ 8)] += v[b][3];
+                    }
+                }
+            }
+            turn = turn >= p.tb ? turn - p.tb : turn - p.tb + wk;          // the next warps' turn (tb <= wk)
+        }
+        if (bt == 0 && exchange && warp == threads / 32 - 1) {     // all CTAs' projections of this K slice
+            const int limit = (p.debug & QGEMV_DEBUG_DROP_PROJECTIONS) ? (1 << 7) : (1 << 20);
+            const unsigned tag = (unsigned)(ld_relaxed_u64(p.epoch) >> 8) + 1u;
+            for (int i = lane; i < p.rank * M; i += 32) {
+                unsigned long long w = ld_relaxed_u64(words + i);
+                int spins = 0;
+                while ((unsigned)(w >> 32) != tag) {
+                    if (++spins > limit) { atomicExch(p.status, 1); break; }
+                    __nanosleep(32);
+                    w = ld_relaxed_u64(words + i);
+                }
+                const int r = i / M;
+                tt[(i - r * M) * p.rank8 + r] = __uint_as_float((unsigned)w);
+            }
+        }
+        if (bt == 0 && !mbarrier_wait(smem_u32(full + kFullU), 0) && lane == 0) atomicExch(p.status, 2);
+        __syncthreads();
+        QGEMV_HELD_STAMP(7 + bt * 2);
+        // ---- the batch's sums: a thread adds four weight rows of one activation column; other warps first in every batch -------
+        const int items = ((batch_end - row0 + 15) >> 4) * p.mp * 4;
+        int i0 = tid - turn0;
+        if (i0 < 0) i0 += threads;
+#pragma unroll 1
+        for (int i = i0; (i & ~31) < items; i += threads) {
+            const int quad = i & 3, pc = (i >> 2) & (p.mp - 1), jt = (i >> 2) >> p.mp_log, pp = pc & 7;
+            const int m = (pc & ~7) + (((pp & (hp - 1)) << 1) | (pp >= hp ? 1 : 0));
+            const bool live = i < items && m < M;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            const int rl = row0 - rowbase + jt * 16 + quad * 4;
+            if (live) {
+                uint32_t at = smem_u32(part) + (uint32_t)(buf * p.part_bytes) + (uint32_t)((jt * wk * part_floats + (pc >> 3) * 128 + pp * 16 + ((quad * 4) ^ (((pp >> 1) & 1) * 8))) * 4);
+#pragma unroll 4
+                for (int k = 0; k < wk; ++k, at += part_floats * 4) {
+                    const float4 a = lds128f(at);
+                    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+                }
+#pragma unroll 1
+                for (int q = 0; q < p.rank8; q += 8) {
+                    const float4 ta = lds128f(smem_u32(tt + m * p.rank8 + q)), tb4 = lds128f(smem_u32(tt + m * p.rank8 + q + 4));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float f[8];
+                        widen8<false>(lds128(sm + p.off_u + (uint32_t)((rl + e) * p.rank8 + q) * 2), f);
+                        v[e] = fmaf(f[0], ta.x, v[e]); v[e] = fmaf(f[1], ta.y, v[e]); v[e] = fmaf(f[2], ta.z, v[e]); v[e] = fmaf(f[3], ta.w, v[e]);
+                        v[e] = fmaf(f[4], tb4.x, v[e]); v[e] = fmaf(f[5], tb4.y, v[e]); v[e] = fmaf(f[6], tb4.z, v[e]); v[e] = fmaf(f[7], tb4.w, v[e]);
+                    }
+                }
+            }
+            if (p.ksplit > 1) {
+                if (live) *reinterpret_cast<float4*>(p.partial + (((size_t)split * gridDim.x + grp) * p.rows_pad + (row0 - rowbase) + jt * 16) * p.mp + pc * 16 + quad * 4) = make_float4(v[0], v[1], v[2], v[3]);
+                continue;
+            }
+            finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + rl * 2 : 0u, live, m, min(row0 + jt * 16, last), quad * 4);
+        }
+        turn0 += (items + 31) & ~31;
+        if (turn0 >= threads) turn0 %= threads;
+    }
+
+    if (p.ksplit > 1) {
+        __shared__ int arrived;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            arrived = atomicAdd(p.counters + grp, 1);
+            if (arrived == p.ksplit - 1) p.counters[grp] = 0;
+        }
+        __syncthreads();
+        if (arrived == p.ksplit - 1) {
+            __threadfence();
+            const int items = ((rowend - rowbase + 15) >> 4) * p.mp * 4;
+            const size_t stride = (size_t)gridDim.x * p.rows_pad * p.mp;
+#pragma unroll 1
+            for (int i = tid; (i & ~31) < items; i += threads) {
+                const int quad = i & 3, pc = (i >> 2) & (p.mp - 1), jt = (i >> 2) >> p.mp_log, pp = pc & 7;
+                const int m = (pc & ~7) + (((pp & (hp - 1)) << 1) | (pp >= hp ? 1 : 0));
+                const bool live = i < items && m < M;
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                const float* src = p.partial + ((size_t)grp * p.rows_pad + jt * 16) * p.mp + pc * 16 + quad * 4;
+                if (live)
+#pragma unroll 4
+                    for (int k = 0; k < p.ksplit; ++k) {
+                        const float4 a = __ldcg(reinterpret_cast<const float4*>(src + k * stride));
+                        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+                    }
+                finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + (jt * 16 + quad * 4) * 2 : 0u, live, m, min(rowbase + jt * 16, last), quad * 4);
+            }
+        }
+    }
+    QGEMV_HELD_STAMP(15);
+    // The launch count that tags the residual projections: every CTA adds one, the first one what is missing to 256, so
+    // count / 256 does not change while a CTA of this launch may still read it.
+    if (exchange && tid == 0) atomicAdd(p.epoch, grp + split == 0 ? 257ull - gridDim.x * gridDim.y : 1ull);
+}
+
+template <int FMT, int KBW, int NB, bool BF16>
+int launch_one(const HeldPlan& h, bool dependent, cudaStream_t s) {
+    auto kern = qgemv_held_kernel<FMT, KBW, NB, BF16>;
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!configured[dev]) {                            // the same carve-out for every kernel of a decode step, see the streaming kernel
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamMaxSmem - 2048) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
+            return check_launch("cudaFuncSetAttribute(qgemv_held_kernel)");
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(h.groups, h.args.ksplit);
+    cfg.blockDim = dim3(32, h.wk, h.wr);
+    cfg.dynamicSmemBytes = h.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kern, h.args) != cudaSuccess) return check_launch("qgemv_held_kernel");
+    return QGEMV_OK;
+}
+
+}  // namespace
+
+// One translation unit per format and activation type keeps the build parallel.
+#if !defined(QGEMV_HELD_FMT) || !defined(QGEMV_HELD_BF16)
+#error "compile with -DQGEMV_HELD_FMT=0..4 and -DQGEMV_HELD_BF16=0|1"
+#endif
+template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s) {
+    if (h.nb == 1) {
+        if (h.kbw == 1) return launch_one<FMT, 1, 1, BF16>(h, dependent, s);
+        if (h.kbw == 2) return launch_one<FMT, 2, 1, BF16>(h, dependent, s);
+        return launch_one<FMT, 4, 1, BF16>(h, dependent, s);
+    }
+    if (h.kbw == 1) return launch_one<FMT, 1, 2, BF16>(h, dependent, s);
+    return launch_one<FMT, 2, 2, BF16>(h, dependent, s);
+}
+template int launch_held_fmt<QGEMV_HELD_FMT, QGEMV_HELD_BF16>(const HeldPlan&, bool, cudaStream_t);
+
+}  // namespace qgemv

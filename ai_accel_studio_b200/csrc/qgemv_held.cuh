@@ -1,0 +1,62 @@
+// Declarations of the GEMV with register-held activations, shared by its planner / launcher (qgemv_held_plan.cu) and its kernel
+// (qgemv_held.cu).
+#pragma once
+#include "qgemv_stream.cuh"
+
+namespace qgemv {
+
+constexpr int kHeldBlock = 128;        // columns of K that one step of a warp covers for 16 weight rows
+constexpr int kHeldMaxWarps = 16;
+
+// Blocks of a ring stage of a warp that holds kbw blocks (at most 128 bytes of a weight row), and stages of its ring: 16 warps keep
+// 64 to 160 KB in flight.
+constexpr int held_stage_blocks(int bits, int kbw) { return bits == 2 || kbw < 2 ? kbw : 2; }
+constexpr int held_stage_codes(int bits, int kbw) { return held_stage_blocks(bits, kbw) * (bits == 2 ? 32 : 64) * 16; }
+constexpr int held_depth(int bits, int kbw) { return held_stage_codes(bits, kbw) == 2048 ? 4 : held_stage_codes(bits, kbw) == 1024 ? 6 : 8; }
+constexpr int kHeldGroups[5] = {1, 2, 1, 2, 4};       // scale groups per block by weight format, as Fmt<>::NG
+constexpr int kHeldMaxBatch = 4;       // tiles of a warp between two meetings of its CTA
+
+enum { kHeldOutlierAligned = 1, kHeldUAligned = 2, kHeldYVector = 4 };
+
+struct HeldArgs {
+    const void* x;            long long ldx;
+    const uint8_t* w;         long long ldw;      // weight rows, leading dimension in bytes
+    const __half* sc;         long long lds;
+    const __half* bias;
+    const int32_t* oidx;
+    const __half* ow;         long long ldow;
+    const __half* ru;         long long ldu;
+    const __half* rv;         long long ldv;
+    void* y;                  long long ldy;
+    unsigned long long* words;                    // {value, launch tag} words of the residual projections: [split][rank][m]
+    float* partial;                               // fp32 sums of a K split: [split][row group][rows_pad / 16][mp][16]
+    int* counters;                                // arrivals per row group of a K split
+    int* status;                                  // wait-timeout status word
+    unsigned long long* epoch;                    // launches of the workspace that exchange residual projections, times 256
+    int m, n, korig, row_bytes, act, flags, debug;
+    int ng, gshift;                               // scale groups per row; log2(group / 128) for groups of 128 and more
+    int oc, noc, oc_log;                          // outlier columns, blocks of 32 of them, log2 of those columns rounded up
+    int rank, rank8, per_cta;                     // residual rank, padded to 8, ranks a CTA projects (== rank: no exchange)
+    int ksplit, rows_per, rows_pad;               // K splits; rows of a row group, padded to 16
+    int blocks_split;                             // 128-column blocks of a K split
+    int tb;                                       // tiles of a warp per batch
+    int mp, mp_log;                               // columns of a partial sum (2, 4, 8 or 16)
+    int sc_split, sc_unit, sc_units, sc_log, sc_pitch;      // scales of a K split; bytes of one copy, copies of a row, log2 of those rounded up, bytes of a staged row
+    int sc_rows, sc_bytes, sc_all;                // rows staged at a time, bytes of a buffer; all of the CTA's rows in one
+    int ow_log;                                   // log2 of the 16-byte pieces of a row of outlier weights, rounded up
+    int off_part, off_tab, off_tpart, off_sc, off_ow, off_u, off_bias, off_xo, off_upo, off_tt;      // shared memory (rings start at 0)
+    int part_bytes;                               // one of the two buffers of partial sums
+};
+
+struct HeldPlan {
+    bool ok;
+    int fmt, kbw, nb;
+    int groups, wk, wr, smem;                     // row groups; warps along K and along the tiles
+    size_t t_off;                                 // bytes from the workspace base
+    HeldArgs args;
+};
+// `partial_floats`: capacity of the workspace's scratch area.
+bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out);
+int launch_held(HeldPlan& plan, bool bf16, bool dependent, void* workspace, cudaStream_t s);
+
+}  // namespace qgemv

@@ -1,0 +1,159 @@
+// Geometry of the GEMV with register-held activations: how K and the weight rows are cut for a given problem, and the launch.
+#include "qgemv_held.cuh"
+
+namespace qgemv {
+namespace {
+
+bool al(const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; }
+int up_to(int v, int a) { return (v + a - 1) / a * a; }
+int cdiv(int a, int b) { return (a + b - 1) / b; }
+
+constexpr int kHeldSmem = kStreamMaxSmem - 2048;      // dynamic shared memory beside the kernel's static words
+constexpr int kLocalBytes = 24 * 1024;                // of V: up to here every CTA makes all residual projections itself
+
+// Clocks of a scheduler for one warp's work on 16 weight rows: per 128 columns, and beside them (ring, scales, sums, its part of the epilogue);
+// up to 8 and up to 16 activation rows.
+constexpr double kBlockCost[2][5] = {{145, 165, 150, 175, 220}, {240, 270, 235, 270, 340}};
+constexpr double kTileCost[2] = {320, 370};
+
+int log2_up(int v) { int s = 0; while ((1 << s) < v) ++s; return s; }
+
+// Shared memory of a geometry; false if it does not fit.
+bool place(const qgemv_problem& p, int m, bool bf16, HeldPlan& h) {
+    HeldArgs& a = h.args;
+    const int nw = h.wk * h.wr, tiles_w = cdiv(a.rows_pad / 16, h.wr);
+    // scales of a K slice, wherever its first one lies in a word; an odd number of 16 bytes a row: 8 rows in 8 different bank groups
+    const int halves = cdiv(h.wk * h.kbw * kHeldGroups[h.fmt], 1 << a.gshift);
+    a.sc_unit = al(p.scales, 16) && p.lds % 8 == 0 && (a.ksplit == 1 || a.sc_split % 8 == 0) ? 16 : 4;
+    a.sc_units = a.sc_unit == 16 ? cdiv(halves, 8) : halves / 2 + 1;
+    a.sc_log = log2_up(a.sc_units);
+    a.sc_pitch = up_to(a.sc_units * a.sc_unit, 16);
+    if (a.sc_pitch / 16 % 2 == 0) a.sc_pitch += 16;
+    if ((nw * 32) >> a.sc_log == 0) return false;
+    for (int tb = tiles_w < kHeldMaxBatch ? tiles_w : kHeldMaxBatch; tb >= 1; --tb) {
+        if (tb > h.wk) continue;
+        for (a.sc_all = 1; a.sc_all >= 0; --a.sc_all) {
+            a.tb = tb;
+            a.sc_rows = a.sc_all ? a.rows_pad : h.wr * tb * 16;
+            a.sc_bytes = a.sc_rows * a.sc_pitch;
+            a.part_bytes = nw * tb * h.nb * 512;
+            int off = held_depth(p.bits, h.kbw) * nw * held_stage_codes(p.bits, h.kbw);
+            auto put = [&](int bytes) { const int at = off; off = up_to(off + bytes, 128); return at; };
+            a.off_part = put(2 * a.part_bytes > nw * 2048 ? 2 * a.part_bytes : nw * 2048);
+            a.off_tab = put(nw * h.kbw * kHeldGroups[h.fmt] * h.nb * 64);
+            a.off_tpart = put(a.rank ? h.wk * 8 * a.mp * 4 : 0);
+            a.off_sc = put((a.sc_all ? 1 : 2) * a.sc_bytes);
+            a.off_ow = put(h.wr * tb * 16 * a.noc * 64);
+            a.off_u = put(a.rows_pad * a.rank8 * 2);
+            a.off_bias = put(p.bias ? a.rows_pad * 2 : 0);
+            a.off_xo = put(a.noc ? m * (a.noc * 64 + 16) : 0);
+            a.off_upo = put(bf16 ? a.noc * m * 4 : 0);
+            a.off_tt = put(a.rank8 * m * 4);
+            h.smem = off;
+            if (off <= kHeldSmem) return true;
+        }
+    }
+    return false;
+}
+
+}  // namespace
+
+bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out) {
+    const int m = p.m, sms = sm_count();
+    out->ok = false;
+    if (m < 1 || m > 16 || p.n < 16 || !al(p.x, 16) || p.ldx % 8 || p.k_original % 8) return false;
+    HeldPlan h{};
+    HeldArgs& a = h.args;
+    h.fmt = stream_format(p.bits, p.group);
+    if (h.fmt < 0 || !al(p.packed, 16) || p.ldp % 16 || p.outliers > kStreamMaxOutliers || p.rank > kMaxRank) return false;
+    if (p.rank && (!al(p.res_v, 16) || p.ldv % 8)) return false;
+    if (!al(p.scales, 4) || p.ldp > 0x7fffffff || (long long)p.n * p.lds > 0x7fffffff) return false;
+    if (p.outliers && al(p.outlier_w, 16) && p.ldow % 8 == 0) a.flags |= kHeldOutlierAligned;
+    if (p.rank && al(p.res_u, 16) && p.ldu % 8 == 0 && p.rank % 8 == 0) a.flags |= kHeldUAligned;
+    const bool bf16 = p.x_dtype == QGEMV_BF16;
+    a.x = p.x; a.ldx = p.ldx;
+    a.w = p.packed; a.ldw = p.ldp;
+    a.sc = static_cast<const __half*>(p.scales); a.lds = p.lds;
+    a.bias = static_cast<const __half*>(p.bias);
+    a.oidx = p.outlier_idx; a.ow = static_cast<const __half*>(p.outlier_w); a.ldow = p.ldow;
+    a.ru = static_cast<const __half*>(p.res_u); a.ldu = p.ldu;
+    a.rv = static_cast<const __half*>(p.res_v); a.ldv = p.ldv;
+    a.y = p.y; a.ldy = p.ldy;
+    a.m = m; a.n = p.n; a.korig = p.k_original; a.act = p.act; a.debug = p.debug;
+    a.row_bytes = (int)((long long)p.k_padded * p.bits / 8);
+    a.ng = p.k_padded / p.group;
+    for (a.gshift = 0; p.group >= 128 && (128 << a.gshift) < p.group; ++a.gshift) {}
+    a.oc = p.outliers; a.noc = cdiv(p.outliers, 32); a.oc_log = log2_up(a.noc * 32); a.ow_log = log2_up(a.noc * 4);
+    a.rank = p.rank; a.rank8 = up_to(p.rank, 8);
+    h.nb = m > 8 ? 2 : 1;
+    a.mp = m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : 16;
+    a.mp_log = log2_up(a.mp);
+    const int blocks = cdiv(p.k_padded, kHeldBlock), tiles = cdiv(p.n, 16);
+    // split sums from the start of the scratch, words of residual projections where the streaming kernel has its own (none of the two fits the
+    // small scratch of qgemv_run_static, which gets neither splits nor, there, long words)
+    if (partial_floats < kTPartFloats) return false;
+    const size_t tail = partial_floats - kTPartFloats, floor = tail > kStreamWordFloats ? tail - kStreamWordFloats : 0, words = tail - floor > tail / 4 && floor == 0 ? tail / 4 : tail - floor;
+
+    double best = -1;
+    const int most_splits = m <= QGEMV_MAX_M && blocks <= kHeldMaxWarps ? 1 : 16;      // (short rows are planned for every call of qgemv_run)
+    for (int S = 1; S <= most_splits && S <= blocks; ++S) {
+        for (h.kbw = 1; h.kbw <= (h.nb == 1 ? 4 : 2); h.kbw *= 2) {
+            HeldPlan c = h;
+            HeldArgs& q = c.args;
+            // a split starts at a whole scale group and at a whole turn of a warp
+            q.blocks_split = S == 1 ? blocks : up_to(cdiv(blocks, S), 1 << a.gshift > h.kbw ? 1 << a.gshift : h.kbw);
+            if (cdiv(blocks, q.blocks_split) != S) continue;
+            c.wk = cdiv(q.blocks_split, c.kbw);
+            if (c.wk > kHeldMaxWarps) continue;
+            q.ksplit = S;
+            q.sc_split = q.blocks_split * kHeldGroups[h.fmt] >> a.gshift;
+            const int R = sms / S;
+            q.rows_per = R >= tiles ? 16 : up_to(cdiv(p.n, R), p.act == QGEMV_ACT_SILU_MUL ? 16 : 4);
+            q.rows_pad = up_to(q.rows_per, 16);
+            c.groups = cdiv(p.n, q.rows_per);
+            const int nt = q.rows_pad / 16;
+            if (c.groups * S > 256 || (S > 1 && (size_t)S * c.groups * q.rows_pad * q.mp > floor)) continue;
+            // residual projections: all in every CTA, or dealt to the first ones of a split
+            const size_t v_bytes = (size_t)(q.blocks_split * kHeldBlock < p.k_original ? q.blocks_split * kHeldBlock : p.k_original) * p.rank * 2;
+            q.per_cta = p.rank <= 8 && v_bytes <= (size_t)kLocalBytes ? p.rank : cdiv(p.rank, c.groups);
+            if (q.per_cta > 8 || (q.per_cta < p.rank && (size_t)S * p.rank * m * 2 > words)) continue;
+            const int all = kHeldMaxWarps / c.wk < nt ? kHeldMaxWarps / c.wk : nt;
+            for (c.wr = all; c.wr >= 1 && c.wr >= all / 2; c.wr = c.wr > 1 ? c.wr / 2 : 0) {
+                if (!place(p, m, bf16, c)) continue;
+                const int nw = c.wk * c.wr, tiles_w = cdiv(nt, c.wr);
+                const double bytes = (double)q.rows_per * q.blocks_split * (p.bits == 2 ? 32 : 64);
+                const double per = nw / 4.0, share = per >= 4 ? per : per < 1 ? 2.5 : 2.0 + per / 2;      // warps of a scheduler, what they slow each other down by
+                const double main = tiles_w * (c.kbw * kBlockCost[h.nb - 1][h.fmt] + kTileCost[h.nb - 1]) * share, stream = bytes / 22;
+                // a split's sums go to L2 and the last CTA of a row group reads them all
+                const double hand_over = S > 1 ? 2500 + (double)(S + 1) * q.rows_pad * q.mp * 4 / 20 : 0;
+                const double cost = (main > stream ? main + stream / 4 : stream + main / 4) + (double)q.blocks_split * kHeldBlock * m * 2 / 50 + hand_over;
+                if (best < 0 || cost < best) { best = cost; *out = c; }
+            }
+        }
+    }
+    if (best < 0) return false;
+    HeldArgs& q = out->args;
+    out->t_off = kWsPartialOff + ((tail - (size_t)q.ksplit * q.rank * m * 2) & ~(size_t)1) * sizeof(float);
+    out->ok = true;
+    return true;
+}
+
+template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s);
+
+int launch_held(HeldPlan& h, bool bf16, bool dependent, void* workspace, cudaStream_t s) {
+    HeldArgs& a = h.args;
+    char* ws = static_cast<char*>(workspace);
+    int* cnt = reinterpret_cast<int*>(ws + kWsCounterOff);
+    a.status = cnt + kWsStatusIdx;
+    a.epoch = reinterpret_cast<unsigned long long*>(cnt + kWsStreamEpochIdx);
+    a.words = reinterpret_cast<unsigned long long*>(ws + h.t_off);
+    a.partial = reinterpret_cast<float*>(ws + kWsPartialOff);
+    a.counters = cnt;
+    a.flags = al(a.y, 8) && a.ldy % 4 == 0 ? a.flags | kHeldYVector : a.flags & ~kHeldYVector;
+    decltype(&launch_held_fmt<0, false>) fn[5][2] = {{launch_held_fmt<0, false>, launch_held_fmt<0, true>}, {launch_held_fmt<1, false>, launch_held_fmt<1, true>},
+                                                     {launch_held_fmt<2, false>, launch_held_fmt<2, true>}, {launch_held_fmt<3, false>, launch_held_fmt<3, true>},
+                                                     {launch_held_fmt<4, false>, launch_held_fmt<4, true>}};
+    return fn[h.fmt][bf16 ? 1 : 0](h, dependent, s);
+}
+
+}  // namespace qgemv

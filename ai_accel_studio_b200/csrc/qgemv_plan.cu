@@ -2,11 +2,6 @@
 #include "qgemv_stream.cuh"
 
 namespace qgemv {
-namespace {
-
-bool al(const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; }
-int up_to(int v, int a) { return (v + a - 1) / a * a; }
-int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 int sm_count() {
     static int cached[64] = {0};
@@ -20,7 +15,10 @@ int sm_count() {
     return cached[dev];
 }
 
+namespace {
 int log2_exact(int v) { int s = 0; while ((1 << s) < v) ++s; return (1 << s) == v ? s : -1; }
+
+}  // namespace
 
 int stream_format(int bits, int group) {
     if (bits == 2 && group == 64) return kInt2G64;
@@ -29,6 +27,12 @@ int stream_format(int bits, int group) {
     if (group % 128 || log2_exact(group / 128) < 0) return -1;
     return bits == 2 ? kInt2G128 : kInt4G128;
 }
+
+namespace {
+
+bool al(const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; }
+int up_to(int v, int a) { return (v + a - 1) / a * a; }
+int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 constexpr int kCodesPerSlot[5] = {512, 512, 256, 256, 256};
 constexpr int kBlocksPerSlot[5] = {4, 4, 2, 2, 2};               // 128-column blocks

@@ -67,6 +67,8 @@ struct StreamPlan {
     size_t t_off, part_off, cnt_off;              // bytes from the workspace base
     StreamArgs args;
 };
+int sm_count();                                       // of the current device
+int stream_format(int bits, int group);               // -1: not built
 // `partial_floats`: capacity of the workspace's scratch area.
 bool plan_stream(const qgemv_problem& p, size_t partial_floats, StreamPlan* out);
 // `dependent`: may start before the preceding kernel of the stream has finished (the weights are final).

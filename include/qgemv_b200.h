@@ -214,7 +214,7 @@ int qgemv_plan_launches(const qgemv_problem* p);
  * Returns QGEMV_OK or a negative QGEMV_ERR_* if the problem is invalid. */
 typedef struct qgemv_plan_info {
     int32_t family;          /* QGEMV_KERNEL_SIMT or QGEMV_KERNEL_MMA */
-    int32_t variant;         /* MMA family: 1 = barrier-phased kernel, 2 = pipelined kernel; 0 otherwise */
+    int32_t variant;         /* MMA family: 1 = barrier-phased kernel, 2 = pipelined kernel, 3 = activations held in registers; 0 otherwise */
     int32_t launches;        /* as qgemv_plan_launches */
     int32_t grid;            /* CTAs */
     int32_t warps;           /* warps per CTA */
@@ -229,7 +229,7 @@ typedef struct qgemv_plan_info {
     int32_t epilogue_tiles;  /* pipelined kernel: tiles per CTA whose epilogue operands are prefetched */
     int32_t l2_chunks;       /* pipelined kernel: chunks per warp announced to L2 before the dependency wait */
     int32_t projection_parts;/* K parts of the in-kernel residual projections (0 when they are not inline) */
-    int32_t chunk_bytes;     /* MMA family: packed bytes per row per ring slot */
+    int32_t chunk_bytes;     /* MMA family: packed bytes per row per ring slot (variant 3: 128, a line; run_chunks: lines of a row) */
 } qgemv_plan_info;
 int qgemv_plan_describe(const qgemv_problem* p, qgemv_plan_info* out);
 

@@ -1,0 +1,103 @@
+"""The GEMV whose warps hold their activations in registers (qgemv_held.cu): 5 - 16 rows, and 1 - 4 rows of up to 1024 columns.  Sizes at the
+edges of its cuts: 16-row tiles (the last one ends with the matrix), 128-column blocks, K splits between CTAs, batches of tiles, scale rows that
+start at odd positions."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import ABS_TOL, REL_TOL, c_forward
+from ai_accel_studio_b200 import _cabi, ops
+from ai_accel_studio_b200.kernels.groupwise_int2 import pack_groupwise_int2
+from ai_accel_studio_b200.kernels.groupwise_int4 import pack_groupwise_int4
+from ai_accel_studio_b200.optimize import HybridInt2Linear, HybridInt4Linear
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # bits, n, k, group, outliers, rank, bias, rows
+    (2, 16, 128, 64, 0, 0, False, (5, 16)),              # one tile, one block
+    (4, 31, 160, 32, 3, 1, True, (5, 9)),                # two tiles that overlap, a block of 32 columns, scale rows of 5
+    (2, 2369, 4096, 64, 8, 5, True, (6, 16)),            # rows off vectors of four
+    (4, 7000, 1056, 32, 33, 8, False, (8, 13)),          # 33 scales a row: every other row starts inside a word; two outlier blocks
+    (4, 300, 8320, 64, 16, 8, True, (5, 10)),            # 65 blocks: K cut between CTAs
+    (2, 1200, 20480, 256, 0, 12, True, (7, 16)),         # splits at whole scale groups, projections dealt to several CTAs
+    (2, 40000, 512, 128, 64, 8, False, (8, 16)),         # many batches of tiles, scales staged batch by batch
+    (4, 4800, 3800, 40, 0, 0, False, (5,)),              # a group that is not built: four rows at a time, as before
+]
+
+
+def _module(bits, n, k, group, oc, rank, has_bias, g):
+    pw = (pack_groupwise_int2 if bits == 2 else pack_groupwise_int4)(torch.randn(n, k, generator=g) * 0.05, group)
+    h = {"packed": pw.packed, "scales": pw.scales,
+         "bias": (torch.randn(n, generator=g) * 0.1).half() if has_bias else None,
+         "oidx": torch.randperm(k, generator=g)[:oc].to(torch.int32) if oc else None,
+         "ow": (torch.randn(n, oc, generator=g) * 0.05).half() if oc else None,
+         "ru": (torch.randn(n, rank, generator=g) * 0.05).half() if rank else None,
+         "rv": (torch.randn(rank, k, generator=g) * 0.05).half() if rank else None}
+    d = {key: None if t is None else t.cuda() for key, t in h.items()}
+    cls = HybridInt2Linear if bits == 2 else HybridInt4Linear
+    return cls.from_buffers(d["packed"], d["scales"], k, group, d["oidx"], d["ow"], d["bias"], d["ru"], d["rv"]), h, d, pw.padded_k
+
+
+def _reference(coracle, bits, k, group, h, xp):
+    np_ = lambda t: None if t is None else t.numpy()
+    bf16 = xp.dtype == torch.bfloat16
+    raw = xp.view(torch.int16).numpy().view(np.uint16) if bf16 else xp.numpy()
+    return np.concatenate([c_forward(coracle, raw[i:i + 4], bits, np_(h["packed"]), np_(h["scales"]), k, group, np_(h["bias"]), np_(h["oidx"]),
+                                     np_(h["ow"]), np_(h["ru"]), np_(h["rv"]), x_is_bf16=bf16) for i in range(0, xp.shape[0], 4)])
+
+
+def _close(got, ref, dtype):
+    rel = REL_TOL if dtype == torch.float16 else 2.0 ** -8       # as for the other kernels; bf16 results are rounded to 2^-9 relative
+    got = got.float().cpu().numpy()
+    assert (np.abs(got - ref) <= ABS_TOL + rel * np.abs(ref)).all(), np.abs(got - ref).max()
+    assert np.linalg.norm(got - ref) <= rel * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("bits,n,k,group,oc,rank,has_bias,rows", CASES)
+def test_batches_against_oracle(bits, n, k, group, oc, rank, has_bias, rows, coracle):
+    g = torch.Generator().manual_seed(n + k)
+    mod, h, _, kp = _module(bits, n, k, group, oc, rank, has_bias, g)
+    for m in rows:
+        for dtype in (torch.float16, torch.bfloat16):
+            x = (torch.randn(m, k, generator=g) * torch.exp(torch.randn(k, generator=g))).to(dtype)
+            y = mod(x.cuda())
+            _close(y, _reference(coracle, bits, k, group, h, torch.nn.functional.pad(x, (0, kp - k)).contiguous()), dtype)
+            assert torch.equal(mod(x.cuda()), y)                   # fixed summation order
+    assert ops.workspace_status("cuda") == 0
+
+
+@pytest.mark.parametrize("bits,n,k,group,oc,rank,act", [
+    (4, 128, 896, 128, 8, 8, 0), (2, 17, 128, 64, 0, 3, 1), (2, 4864, 896, 128, 8, 8, 3), (4, 2048, 1024, 32, 33, 16, 0), (4, 999, 768, 128, 0, 0, 2)])
+def test_few_rows_of_short_k(bits, n, k, group, oc, rank, act, coracle):
+    """One kernel whatever the way to it: qgemv_run, the built-in scratch, a prepared launch."""
+    lib, stream = _cabi.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    g = torch.Generator().manual_seed(n)
+    mod, h, d, _ = _module(bits, n, k, group, oc, rank, True, g)
+    ws = ops.ensure_workspace("cuda")
+    for m in (1, 4):
+        x = torch.randn(m, k, generator=g).half()
+        xd, width = x.cuda(), n // 2 if act == 3 else n
+        ys = [torch.full((m, width), float("nan"), dtype=torch.float16, device="cuda") for _ in range(3)]
+        p = ops._problem(xd, d["packed"], d["scales"], d["bias"], d["oidx"], d["ow"], d["ru"], d["rv"], ys[0], ws, bits, group, k, act, 0, None)
+        assert _cabi.plan_describe(p).variant == 3
+        assert lib.qgemv_run(ctypes.byref(p), stream) == 0, _cabi.last_error()
+        p.y = ys[1].data_ptr()
+        assert lib.qgemv_run_static(ctypes.byref(p), stream) == 0, _cabi.last_error()
+        blob = ctypes.create_string_buffer(lib.qgemv_prepared_bytes())
+        assert lib.qgemv_prepare(ctypes.byref(p), blob) == 0, _cabi.last_error()
+        assert lib.qgemv_launch_prepared(blob, ctypes.c_void_p(xd.data_ptr()), ctypes.c_void_p(ys[2].data_ptr()), ctypes.c_void_p(ws.data_ptr()), 0, stream) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+        ref = torch.from_numpy(_reference(coracle, bits, k, group, h, x)).float()
+        if act == 1:
+            ref = ref.relu()
+        elif act == 2:
+            ref = torch.nn.functional.silu(ref)
+        elif act == 3:                                               # rows 16 b + j and 16 b + 8 + j are a gate and its up projection
+            pairs = ref.half().float().view(m, -1, 2, 8)
+            ref = (torch.nn.functional.silu(pairs[:, :, 0]).half().float() * pairs[:, :, 1]).reshape(m, -1)
+        _close(ys[0], ref.numpy(), torch.float16)
+    assert ops.workspace_status("cuda") == 0
