@@ -512,8 +512,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
         while (unit >= p.units) { unit -= p.units; ++tile; }
 #pragma unroll 1
         for (int i = wg < G ? wg : count; i < count; i += G, ++q) {
-            for (; done < tile && ok; ++done) ok = finish_tile<BF16>(p, e, done, p.units - 1);      // tiles that ended with others' units
-            if (!ok) break;
             landed();
             // A parity cannot tell a release from the one two before it.  This warpgroup's last unit was G <= stages ago and waited
             // for a release no older than that, so the one before the awaited release has happened.
@@ -533,6 +531,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * stage);
+            // Tiles that ended before this unit, which is in its stage already for the mma to go on with.  (The wait for the stage was for a unit at
+            // least G before this one: all that its mma waited for was finished by this warpgroup behind its unit before.)
+            for (; done < tile && ok; ++done) ok = finish_tile<BF16>(p, e, done, p.units - 1);
+            if (!ok) break;
             stage += G;
             if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
             unit += G;
