@@ -723,8 +723,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prepare_kernel(const __grid_c
 // takes 16 activation rows x 32 weight rows, four mma.m16n8k16 side by side whose columns are dealt so that a lane of a quad holds
 // eight neighbours of y: 16-byte accesses, 64 bytes a row.  K comes 32 columns at a time, eight neighbours a lane (any order of K does,
 // as long as both operands use it), straight from memory.  Bound by latency and instructions around its traffic, y in and out.
-// Two terms take 28 of 117 us at 512 x 14336 (K 4096, bf16), 80 of 470 at 1000 x 28672 (K 8192, fp16), the projections V x included;
-// with 32 activation rows a warp (128 registers, two CTAs an SM) the same within 5 %, and 4 us more on 32 x 4096.
+// For more than 64 outlier columns or rank 32; the usual ones have a kernel of their own below.
 // ---------------------------------------------------------------------------------------------
 struct TermArgs {
     const unsigned short* x;                           // extra columns of the laid out x: [m][ke], outliers, then projections
@@ -755,6 +754,36 @@ __device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
     if constexpr (BF16) asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     else asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
+}
+
+// Activation and store of a lane's eight results: activation row `row`, weight rows nl on.  Called by whole warps.
+template <bool BF16>
+__device__ __forceinline__ void store_terms(const TermArgs& p, uint4 w, int row, int nl, int t) {
+    using XT = typename Act16<BF16>::T;
+    XT* e = reinterpret_cast<XT*>(&w);
+    int col = nl;
+    bool mine = row < p.m;
+    if (p.act == QGEMV_ACT_SILU_MUL) {                 // lanes of even t hold eight gate rows, their neighbours the eight up rows
+        col = nl / 16 * 8;
+        mine = mine && !(t & 1) && nl < p.n;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float gate = Act16<BF16>::to_float(e[q]), up = __shfl_down_sync(0xffffffffu, gate, 1);
+            e[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(Act16<BF16>::from_float(gate / (1.0f + __expf(-gate)))) * up);
+        }
+    } else if (p.act != QGEMV_ACT_NONE) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) e[q] = Act16<BF16>::from_float(apply_act(Act16<BF16>::to_float(e[q]), p.act));
+    }
+    if (!mine) return;
+    XT* dst = static_cast<XT*>(p.y) + (size_t)row * p.ldy + col;
+    const int left = p.act == QGEMV_ACT_SILU_MUL ? 8 : p.n - nl;
+    if (p.vec && left >= 8) {
+        *reinterpret_cast<uint4*>(dst) = w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) if (q < left) dst[q] = e[q];
+    }
 }
 
 template <bool BF16>
@@ -861,36 +890,158 @@ __global__ void __launch_bounds__(kTermWarps * 32, 3) terms_kernel(const __grid_
                     w = add2<BF16>(w, term);
                 }
         }
-        XT* y = static_cast<XT*>(p.y);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            uint4 w = raw[i];
-            XT* e = reinterpret_cast<XT*>(&w);
-            int col = nl;
-            bool mine = arow(i) < p.m;
-            if (p.act == QGEMV_ACT_SILU_MUL) {         // lanes of even t hold eight gate rows, their neighbours the eight up rows
-                col = nl / 16 * 8;
-                mine = mine && !(t & 1) && nl < p.n;
+        for (int i = 0; i < 2; ++i) store_terms<BF16>(p, raw[i], arow(i), nl, t);
+    }
+}
+
+// The same for up to 64 outlier columns and rank 32, which is what a module has as a rule.  The kernel above asks for both operands of every
+// product again for each 16 activation rows; eight lines a request, its 22 requests kept the SM's line look-ups busy for 35 of the 63 us it took at
+// 1000 x 28672. Here a warp keeps the fragments of its 32 weight rows for all the activation rows of its CTA, the CTA's warps share
+// a tile of x in shared memory (three buffers: one barrier a tile), and a tile's base is asked for one tile ahead.  Same sums in the same order.
+template <bool BF16, int OB, int RB>
+__global__ void __launch_bounds__(kTermWarps * 32, 2) terms_held_kernel(const __grid_constant__ TermArgs p) {
+    using XT = typename Act16<BF16>::T;
+    constexpr int PIECES = (OB + RB) * 4, PITCH = ((OB + RB) | 1) * 64;      // 16-byte pieces of a row of x; an odd number of half lines
+    __shared__ __align__(128) unsigned char xs[3][kTermRows * PITCH];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int n0 = (blockIdx.x * kTermWarps + warp) * kTermTile, nl = n0 + t * 8;
+    const int tiles = (p.m + kTermRows - 1) / kTermRows, step = gridDim.y;
+    // weights are final: the first kernel of the call started in stream order
+    uint4 bo[OB > 0 ? OB : 1][4], br[4];
+    auto weights = [&](const __half* w, long long ldw, int cols, int k, int j, bool wide) {
+        const int row = n0 + (g >> 1) * 8 + 2 * j + (g & 1);
+        const unsigned short* src = reinterpret_cast<const unsigned short*>(w) + (size_t)min(row, p.n - 1) * ldw + k;
+        if (k >= cols) return make_uint4(0u, 0u, 0u, 0u);
+        if (wide && k + 8 <= cols) return __ldg(reinterpret_cast<const uint4*>(src));
+        uint32_t e[4];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const float gate = Act16<BF16>::to_float(e[q]), up = __shfl_down_sync(0xffffffffu, gate, 1);
-                    e[q] = Act16<BF16>::from_float(Act16<BF16>::to_float(Act16<BF16>::from_float(gate / (1.0f + __expf(-gate)))) * up);
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t lo = k + 2 * q < cols ? __ldg(src + 2 * q) : 0, hi = k + 2 * q + 1 < cols ? __ldg(src + 2 * q + 1) : 0;
+            e[q] = lo | hi << 16;
+        }
+        return make_uint4(e[0], e[1], e[2], e[3]);
+    };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int o = 0; o < OB; ++o) {
+            bo[o][j] = weights(p.ow, p.ldow, p.oc, o * 32 + t * 8, j, p.ow_vec);
+            if constexpr (BF16) {
+                uint32_t* e = reinterpret_cast<uint32_t*>(&bo[o][j]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(e + q));
+                    e[q] = pack2<true>(f.x, f.y);
                 }
-            } else if (p.act != QGEMV_ACT_NONE) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) e[q] = Act16<BF16>::from_float(apply_act(Act16<BF16>::to_float(e[q]), p.act));
-            }
-            if (!mine) continue;
-            XT* dst = y + (size_t)arow(i) * p.ldy + col;
-            const int left = p.act == QGEMV_ACT_SILU_MUL ? 8 : p.n - nl;
-            if (p.vec && left >= 8) {
-                *reinterpret_cast<uint4*>(dst) = w;
-            } else {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) if (q < left) dst[q] = e[q];
             }
         }
+        if (RB) br[j] = weights(p.ru, p.ldu, p.rank, t * 8, j, p.ru_vec);
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto fetch = [&](int tile, int buf) {              // 16 rows of the extra columns of x; rows past the end repeat the last one
+        if (tile < tiles)
+            for (int i = tid; i < kTermRows * PIECES; i += kTermWarps * 32) {
+                const int r = i / PIECES, q = i - r * PIECES;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&xs[buf][r * PITCH + q * 16])),
+                             "l"(p.x + (size_t)min(tile * kTermRows + r, p.m - 1) * p.ke + q * 8) : "memory");
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto base = [&](int tile, uint4 (&raw)[2]) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = tile * kTermRows + i * 8 + g;
+            raw[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row >= p.m) continue;
+            const XT* src = static_cast<const XT*>(p.base) + (size_t)row * p.ldb + nl;
+            if (p.vec && nl + 8 <= p.n) {
+                raw[i] = *reinterpret_cast<const uint4*>(src);
+            } else {
+                XT* e = reinterpret_cast<XT*>(&raw[i]);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) if (nl + q < p.n) e[q] = src[q];
+            }
+        }
+    };
+    fetch(blockIdx.y, 0);
+    fetch(blockIdx.y + step, 1);
+    uint4 raw[2], next[2];
+    base(blockIdx.y, raw);
+    int buf = 0;
+#pragma unroll 1
+    for (int tile = blockIdx.y; tile < tiles; tile += step) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                               // the tile is there, and nobody reads the one before it any more
+        fetch(tile + 2 * step, buf == 0 ? 2 : buf - 1);
+        if (tile + step < tiles) base(tile + step, next);
+        const uint32_t at = smem_u32(xs[buf]) + g * PITCH + t * 16;
+        auto frag = [&](int blk, uint4 (&a)[2]) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a[i].x), "=r"(a[i].y), "=r"(a[i].z), "=r"(a[i].w) : "r"(at + i * 8 * PITCH + blk * 64) : "memory");
+        };
+        float acc[4][4];
+        if (OB > 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
+#pragma unroll
+            for (int o = 0; o < OB; ++o) {
+                uint4 a[2];
+                frag(o, a);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 b = bo[o][j];
+                    if constexpr (BF16) {
+                        mma_bf16(acc[j], a[0].x, a[1].x, a[0].y, a[1].y, b.x, b.y);
+                        mma_bf16(acc[j], a[0].z, a[1].z, a[0].w, a[1].w, b.z, b.w);
+                    } else {
+                        mma16816(acc[j], a[0].x, a[1].x, a[0].y, a[1].y, b.x, b.y);
+                        mma16816(acc[j], a[0].z, a[1].z, a[0].w, a[1].w, b.z, b.w);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t& w = reinterpret_cast<uint32_t*>(&raw[i])[j];
+                    w = add2<BF16>(w, pack2<BF16>(acc[j][i * 2], acc[j][i * 2 + 1]));
+                }
+        }
+        if (RB > 0) {                                  // an fp16 product for either activation type
+            uint4 a[2];
+            frag(OB, a);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
+                mma16816(acc[j], a[0].x, a[1].x, a[0].y, a[1].y, br[j].x, br[j].y);
+                mma16816(acc[j], a[0].z, a[1].z, a[0].w, a[1].w, br[j].z, br[j].w);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t& w = reinterpret_cast<uint32_t*>(&raw[i])[j];
+                    uint32_t term = pack2<false>(acc[j][i * 2], acc[j][i * 2 + 1]);
+                    if constexpr (BF16) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&term));
+                        term = pack2<true>(f.x, f.y);
+                    }
+                    w = add2<BF16>(w, term);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store_terms<BF16>(p, raw[i], tile * kTermRows + i * 8 + g, nl, t);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) raw[i] = next[i];
+        buf = buf == 2 ? 0 : buf + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 struct GemmPlan { GemmArgs a; int grid, smem, kw, ke, oc32, groups, shares; bool terms; size_t x_bytes, t_bytes, b_bytes, scratch; };
@@ -1033,10 +1184,23 @@ int launch_terms(const qgemv_problem& p, const GemmPlan& g, const void* scratch,
     a.ow_vec = p.outliers > 0 && al(p.outlier_w) && p.ldow % 8 == 0;
     a.ru_vec = p.rank > 0 && al(p.res_u) && p.ldu % 8 == 0;
     a.vec = al(a.base) && a.ldb % 8 == 0 && al(p.y) && p.ldy % 8 == 0;
-    // three CTAs fit an SM; up to two rounds of them, so that a CTA's weights serve several tiles of activation rows
-    const int cols = (p.n + kTermWarps * kTermTile - 1) / (kTermWarps * kTermTile), tiles = (p.m + kTermRows - 1) / kTermRows, fit = 6 * sms() / cols;
+    const int cols = (p.n + kTermWarps * kTermTile - 1) / (kTermWarps * kTermTile), tiles = (p.m + kTermRows - 1) / kTermRows;
+    const bool held = p.outliers <= 64 && p.rank <= 32;
+    int rows;                                          // CTAs over the activation rows
+    if (held) {                                        // two CTAs fit an SM; whole rounds of them, a CTA's start counted as two tiles
+        const int slots = 2 * sms();
+        int best = 0x7fffffff;
+        rows = 1;
+        for (int r = 1; r <= tiles && (r == 1 || cols * r <= 4 * slots); ++r) {
+            const int cost = (cols * r + slots - 1) / slots * ((tiles + r - 1) / r + 2);
+            if (cost < best) { best = cost; rows = r; }
+        }
+    } else {                                           // three CTAs fit an SM; up to two rounds of them, so that a CTA's weights serve several tiles of activation rows
+        const int fit = 6 * sms() / cols;
+        rows = fit < 1 ? 1 : fit < tiles ? fit : tiles;
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cols, fit < 1 ? 1 : fit < tiles ? fit : tiles);
+    cfg.gridDim = dim3(cols, rows);
     cfg.blockDim = dim3(kTermWarps * 32);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1044,7 +1208,10 @@ int launch_terms(const qgemv_problem& p, const GemmPlan& g, const void* scratch,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, terms_kernel<BF16>, a);
+    if (!held) (void)cudaLaunchKernelEx(&cfg, terms_kernel<BF16>, a);
+    else if (p.outliers == 0) (void)cudaLaunchKernelEx(&cfg, terms_held_kernel<BF16, 0, 1>, a);
+    else if (p.outliers <= 32) (void)(p.rank ? cudaLaunchKernelEx(&cfg, terms_held_kernel<BF16, 1, 1>, a) : cudaLaunchKernelEx(&cfg, terms_held_kernel<BF16, 1, 0>, a));
+    else (void)(p.rank ? cudaLaunchKernelEx(&cfg, terms_held_kernel<BF16, 2, 1>, a) : cudaLaunchKernelEx(&cfg, terms_held_kernel<BF16, 2, 0>, a));
     return check_launch("terms_kernel");
 }
 

@@ -170,3 +170,19 @@ def test_two_rows_of_long_k_on_either_side_of_the_route(bits, n):
     want = x.double() @ mod.effective_weight().double().t() + mod.bias.double()
     assert float((mod(x).double() - want).norm() / want.norm()) <= 2.0 ** -11      # one rounding of a 32-bit sum, and its own error
     assert ops.workspace_status("cuda") == 0
+
+
+@pytest.mark.parametrize("rows,n,oc,rank", [(17, 250, 32, 0), (33, 512, 64, 32), (49, 264, 1, 1), (20, 256, 0, 32), (31, 300, 65, 1), (18, 256, 8, 33)])
+def test_terms_at_the_edges_of_their_kernels(monkeypatch, rows, n, oc, rank):
+    """Up to 64 outlier columns and rank 32 have a kernel that keeps the weights in registers, more of either the general one: 16 activation rows a
+    tile, 256 weight rows a CTA, blocks of 32 columns."""
+    mod = _module(4, n, 512, 128, oc, rank, True, torch.Generator().manual_seed(n + rows))
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    for name in ("fp16", "bf16"):
+        monkeypatch.setattr(torch.backends.cuda.matmul, f"allow_{name}_reduced_precision_reduction", False)
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(rows, 512, generator=gen, device="cuda").to(dtype)
+        y, want = mod(x), mod._dense(x)
+        u = 2.0 ** (-11 if dtype == torch.float16 else -8)
+        assert float((y != want).float().mean()) < 0.04          # as in test_batch_rounds_as_the_expression_does
+        assert float((y.double() - want.double()).norm() / want.double().norm()) < 0.3 * u
