@@ -19,7 +19,7 @@ MAX_M = 4
 MAX_BATCH = 16
 ABI_VERSION = 6
 
-EXPORTS = ("qgemv_run", "qgemv_run_ordered", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_describe", "qgemv_workspace_status", "qgemv_workspace_bytes", "qgemv_plan_name", "qdequant", "qunpack_codes", "qgemv_pack",
+EXPORTS = ("qgemv_run", "qgemv_run_ordered", "qgemv_run_static", "qgemv_plan_launches", "qgemv_plan_describe", "qgemv_workspace_status", "qgemv_workspace_bytes", "qgemv_plan_name", "qdequant", "qunpack_codes", "qgemv_pack", "qgemv_pack_spaced",
            "qgemv_prepared_bytes", "qgemv_prepare", "qgemv_launch_prepared", "qgemv_batch_scratch_bytes", "qgemv_run_batch", "qgemv_error_string", "qgemv_abi_version", "qgemv_sizeof_problem",
            "qcomm_slot_bytes", "qcomm_flag_bytes", "qcomm_state_bytes", "qcomm_allreduce", "qcomm_allreduce_rmsnorm", "qcomm_status", "qcomm_alloc", "qcomm_free",
            "qcomm_ipc_export", "qcomm_ipc_open", "qcomm_ipc_close",
@@ -140,6 +140,8 @@ def lib():
     l.qunpack_codes.restype = C.c_int
     l.qgemv_pack.argtypes = [ci, vp, i64, ci, ci, ci, ci, vp, vp, ci, vp, vp, vp]
     l.qgemv_pack.restype = ci
+    l.qgemv_pack_spaced.argtypes = [ci, vp, i64, ci, ci, ci, ci, vp, C.c_float, C.c_float, ci, vp, vp, vp]
+    l.qgemv_pack_spaced.restype = ci
     l.qgemv_error_string.argtypes = []
     l.qgemv_error_string.restype = C.c_char_p
     l.qgemv_abi_version.argtypes = []

@@ -127,7 +127,8 @@ template <int DT> __device__ __forceinline__ float load_w(const void* w, size_t 
 
 struct PackArgs {
     const void* w;            long long ldw;
-    const float* rms;         const float* factors;
+    const float* rms;         const float* factors;           // factors NULL: evenly spaced, made by every block itself
+    float first, last, spacing;
     uint8_t* packed;          __half* scales;
     int n, k, ng, group, lg, steps;           // lg: lanes per group, each 16 consecutive columns of every 128
     bool vec, vec_rms;                        // 16-byte loads of w, rms
@@ -195,7 +196,7 @@ __device__ __noinline__ float error_by_quotients(const PackArgs& p, int row, int
 // would halve the number of warps.  A column's terms are added up as they are made: kept until it is known whether a decision was
 // close, they would not fit the registers beside weights and energies.
 template <int BITS, int V, int DT>
-__device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, float base, uint32_t visit, uint32_t mine, bool every) {
+__device__ __noinline__ float exact_search(const PackArgs& p, const float* factors, int row, int k0, float base, uint32_t visit, uint32_t mine, bool every) {
     float f[V][16], aw[V][16], tiny = 3.0e38f;         // tiny: smallest magnitude that is not zero
 #pragma unroll
     for (int v = 0; v < V; ++v) {
@@ -208,7 +209,6 @@ __device__ __noinline__ float exact_search(const PackArgs& p, int row, int k0, f
 #pragma unroll
         for (int e = 0; e < 16; ++e) tiny = f[v][e] != 0.0f ? fminf(tiny, fabsf(f[v][e])) : tiny;
     }
-    const float* const factors = p.factors;
     const int steps = p.steps, lg = p.lg;
     float best = 0.0f, chosen = base;
     bool first = true;
@@ -254,8 +254,17 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
     __shared__ float2 bins[SEARCH && BITS == 2 ? (kMaxFast + 1) * 256 : 1];        // INT2: [bin][thread], (sum aw, sum aw |w|) of the thread's columns
     [[maybe_unused]] float2* const mine = bins + (SEARCH && BITS == 2 ? threadIdx.x : 0);
     const int lg = p.lg, steps = p.steps;
+    // Evenly spaced candidates as torch.linspace spaces them (from both ends, one rounding), without a launch that makes them.
+    __shared__ float spaced[SEARCH ? QGEMV_PACK_MAX_SPACED : 1];
+    const float* factors = p.factors;
+    if (SEARCH && !factors) {
+        const int s = threadIdx.x;
+        if (s < steps) spaced[s] = s < steps / 2 || steps == 1 ? __fmaf_rn(p.spacing, (float)s, p.first) : __fmaf_rn(-p.spacing, (float)(steps - 1 - s), p.last);
+        __syncthreads();
+        factors = spaced;
+    }
     float2 grid = make_float2(0.0f, 0.0f);
-    if (SEARCH && steps <= kMaxFast) grid = even_grid(p.factors, steps);
+    if (SEARCH && steps <= kMaxFast) grid = even_grid(factors, steps);
     const long long groups = (long long)p.n * p.ng;
     const int per_block = 256 / lg;
     const int sub = threadIdx.x / lg, l = threadIdx.x - sub * lg;
@@ -331,7 +340,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                     __syncwarp();
                     auto error = [&](int s) {           // carry: the totals
                         const float2 r = lane0[(s + 1) * 256];
-                        const float cand = base * p.factors[s], third = cand * kThird, ra = carry.x - r.x, rb = carry.y - r.y;
+                        const float cand = base * factors[s], third = cand * kThird, ra = carry.x - r.x, rb = carry.y - r.y;
                         return fmaf(cand, fmaf(cand, r.x, -2.0f * r.y), fmaf(third, fmaf(third, ra, -2.0f * rb), energy));
                     };
                     for (int s = l; s < steps; s += lg) lowest = fminf(lowest, error(s));
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                     contenders = 0;
 #pragma unroll 1
                     for (int s = 0; s < steps; ++s) {
-                        const float cand = base * p.factors[s], inv = reciprocal(cand);
+                        const float cand = base * factors[s], inv = reciprocal(cand);
                         float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
                         for (int v = 0; v < V; ++v)
@@ -381,10 +390,10 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
                 }
             }
             const bool decided = fast && __popc(contenders) == 1;
-            if (decided) chosen = __fmul_rn(base, p.factors[__ffs(contenders) - 1]);
+            if (decided) chosen = __fmul_rn(base, factors[__ffs(contenders) - 1]);
             const uint32_t visit = __reduce_or_sync(0xffffffffu, decided ? 0u : contenders);
             if (visit) {
-                const float exact = exact_search<BITS, V, DT>(p, row, k0, base, visit, contenders, !fast);
+                const float exact = exact_search<BITS, V, DT>(p, factors, row, k0, base, visit, contenders, !fast);
                 if (!decided) chosen = exact;
             }
         }
@@ -427,11 +436,11 @@ __global__ void __launch_bounds__(256, pack_blocks(BITS, V)) pack_kernel(const _
 
 using namespace qgemv;
 
-extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, const float* factors,
-                          int steps, uint8_t* packed, void* scales, void* stream) {
+static int run_pack(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, const float* factors, float first,
+                    float last, int steps, uint8_t* packed, void* scales, void* stream) {
     if (!w || !packed || !scales || n < 1 || k < 1 || ldw < k || (bits != 2 && bits != 4) || w_dtype < QGEMV_F16 || w_dtype > QGEMV_F32 ||
-        (rms && (!factors || steps < 1))) {
-        set_error("qgemv_pack: null pointer, non-positive size or bad type");
+        (rms && (steps < 1 || (!factors && steps > QGEMV_PACK_MAX_SPACED)))) {
+        set_error("qgemv_pack: null pointer, non-positive size, bad type or too many candidates");
         return QGEMV_ERR_BAD_ARG;
     }
     const int v = group <= 128 ? 1 : group / 128, lg = group <= 128 ? group / 16 : 8;
@@ -447,7 +456,7 @@ extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int
     const int most = 148 * pack_blocks(bits, v);       // as many blocks as are resident
     const int grid = (int)(trips < most ? trips : most);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const PackArgs a{w, ldw, rms, factors, packed, static_cast<__half*>(scales), n, k, ng, group, lg, steps, vec, reinterpret_cast<uintptr_t>(rms) % 16 == 0};
+    const PackArgs a{w, ldw, rms, factors, first, last, steps > 1 ? (last - first) / (float)(steps - 1) : 0.0f, packed, static_cast<__half*>(scales), n, k, ng, group, lg, steps, vec, reinterpret_cast<uintptr_t>(rms) % 16 == 0};
 #define QP(B, V, D) do { if (rms) pack_kernel<B, V, D, true><<<grid, 256, 0, s>>>(a); else pack_kernel<B, V, D, false><<<grid, 256, 0, s>>>(a); } while (0)
 #define QP_D(B, V) do { if (w_dtype == QGEMV_F16) QP(B, V, QGEMV_F16); else if (w_dtype == QGEMV_BF16) QP(B, V, QGEMV_BF16); else QP(B, V, QGEMV_F32); } while (0)
 #define QP_V(B) do { if (v == 1) QP_D(B, 1); else if (v == 2) QP_D(B, 2); else QP_D(B, 4); } while (0)
@@ -456,4 +465,15 @@ extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int
 #undef QP_D
 #undef QP
     return check_launch("pack_kernel");
+}
+
+extern "C" int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, const float* factors,
+                          int steps, uint8_t* packed, void* scales, void* stream) {
+    if (rms && !factors) { set_error("qgemv_pack: rms needs factors"); return QGEMV_ERR_BAD_ARG; }
+    return run_pack(bits, w, ldw, w_dtype, n, k, group, rms, factors, 0.0f, 0.0f, steps, packed, scales, stream);
+}
+
+extern "C" int qgemv_pack_spaced(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, float first, float last,
+                                 int steps, uint8_t* packed, void* scales, void* stream) {
+    return run_pack(bits, w, ldw, w_dtype, n, k, group, rms, nullptr, first, last, steps, packed, scales, stream);
 }

@@ -448,6 +448,43 @@ PyObject* functional(PyObject*, PyObject* const* a, Py_ssize_t n) {
     catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
 }
 
+// ---- quantiser ------------------------------------------------------------------------------------------
+
+// pack(weight, bits, group, rms, first, last, steps) -> (packed, scales), or None where the caller has to prepare the operands (or raise)
+PyObject* pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "pack takes 7 arguments"); return nullptr; }
+    const long bits = PyLong_AsLong(a[1]), group = PyLong_AsLong(a[2]), steps = PyLong_AsLong(a[6]);
+    const double first = PyFloat_AsDouble(a[4]), last = PyFloat_AsDouble(a[5]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!THPVariable_CheckExact(a[0]) || (a[3] != Py_None && !THPVariable_CheckExact(a[3]))) Py_RETURN_NONE;
+    try {
+        const at::Tensor& w = THPVariable_Unpack(a[0]);
+        const auto type = w.scalar_type();
+        if (observed(w) || !w.is_cuda() || w.dim() != 2 || w.numel() == 0 || w.stride(1) != 1 || w.stride(0) < w.size(1) || w.size(0) > 0x7fffffff || w.size(1) > 0x7fffffff ||
+            (type != at::kHalf && type != at::kBFloat16 && type != at::kFloat) || steps < 1 || steps > QGEMV_PACK_MAX_SPACED || group < 1)
+            Py_RETURN_NONE;
+        const float* rms = nullptr;
+        if (a[3] != Py_None) {
+            const at::Tensor& r = THPVariable_Unpack(a[3]);
+            if (observed(r) || !r.is_cuda() || r.get_device() != w.get_device() || r.scalar_type() != at::kFloat || r.dim() != 1 || (r.numel() > 1 && r.stride(0) != 1) ||
+                r.numel() < w.size(1))
+                Py_RETURN_NONE;
+            rms = static_cast<const float*>(r.data_ptr());
+        }
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != w.get_device()) guard.set_index(w.get_device());
+        const int64_t rows = w.size(0), k = w.size(1), ng = (k + group - 1) / group;
+        at::Tensor packed = at::empty({rows, ng * group * bits / 8}, w.options().dtype(at::kByte)), scales = at::empty({rows, ng}, w.options().dtype(at::kHalf));
+        check(qgemv_pack_spaced((int)bits, w.data_ptr(), w.stride(0), type == at::kHalf ? QGEMV_F16 : type == at::kBFloat16 ? QGEMV_BF16 : QGEMV_F32, (int)rows, (int)k, (int)group,
+                                rms, (float)first, (float)last, (int)steps, static_cast<uint8_t*>(packed.data_ptr()), scales.data_ptr(),
+                                c10::cuda::getCurrentCUDAStream(w.get_device()).stream()));
+        PyObject* const pp = THPVariable_Wrap(std::move(packed));
+        PyObject* const ps = THPVariable_Wrap(std::move(scales));
+        return Py_BuildValue("(NN)", pp, ps);
+    } catch (const PyError&) { return nullptr; }
+    catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+}
+
 // setup(ensure_workspace, error_class)
 PyObject* setup(PyObject*, PyObject* args) {
     PyObject *fn, *err;
@@ -462,6 +499,7 @@ PyMethodDef module_methods[] = {
     {"forget", forget, METH_NOARGS, "no weights are settled any more"},
     {"settled", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(settled)), METH_FASTCALL, "whether launches have waited for these weights"},
     {"functional", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(functional)), METH_FASTCALL, "prepared-problem call of the decode_int*_linear functions"},
+    {"pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(pack)), METH_FASTCALL, "quantiser call for operands as the kernel takes them"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", "Host side of eager packed-Linear calls", -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -64,6 +64,9 @@ def _pack_on_device(weight, bits, group_size, activation_rms, first, last, steps
     if not weight.is_cuda or weight.ndim != 2 or weight.dtype not in ops._DT or group_size not in ops.PACK_GROUPS or \
             weight.numel() == 0 or not 1 <= steps <= 1024:
         return None
+    done = ops.native().pack(weight, bits, group_size, activation_rms, first, last, steps)      # most calls; the rest may need copies, or raise
+    if done is not None:
+        return *done, done[1].shape[1] * group_size
     w, rms = weight.detach(), None
     if activation_rms is not None:
         rms = activation_rms.detach().to(w.device).float().flatten()

@@ -250,6 +250,12 @@ int qdequant(int bits, const uint8_t* packed, int64_t ldp, const void* scales, i
 int qgemv_pack(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, const float* factors,
                int steps, uint8_t* packed, void* scales, void* stream);
 
+/* The same with candidates evenly spaced from `first` to `last`, both included (torch.linspace, to the bit): no array of them has to be made
+ * first.  At most QGEMV_PACK_MAX_SPACED steps. */
+#define QGEMV_PACK_MAX_SPACED 64
+int qgemv_pack_spaced(int bits, const void* w, int64_t ldw, int w_dtype, int n, int k, int group, const float* rms, float first, float last,
+                      int steps, uint8_t* packed, void* scales, void* stream);
+
 /* Expand packed bytes to one uint8 code per weight, [N, Kpad].
  * Replaces the code extraction of ai_accel_lab/kernels/groupwise_int2.py:123-124 and
  * ai_accel_lab/kernels/groupwise_int4.py:64-65. */
