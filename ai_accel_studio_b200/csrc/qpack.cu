@@ -243,10 +243,10 @@ __device__ __noinline__ float exact_search(const PackArgs& p, const float* facto
     return chosen;
 }
 
-// Blocks of an SM, by registers: what a thread keeps is its weights.  The caps spill a little (76 bytes of stores a thread for INT4, 208 and
-// up for INT2), which costs less than the warps would in most: 4096 x 4096 fp16 with these / with one block fewer, us: groups of 128
-// INT4 106 / 114, INT2 74.6 / 70.0, 256 INT4 95 / 111, INT2 69 / 65, 512 INT2 76 / 80; without statistics 23 - 26 / 24 - 34.
-__host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ? (bits == 2 ? 4 : 3) : v == 2 ? (bits == 2 ? 3 : 2) : bits == 2 ? 2 : 1; }
+// Blocks of an SM, by registers: what a thread keeps is its weights.  4096 x 4096 fp16 with these / with one block fewer, us: INT4 groups of 128
+// 106 / 114, 256 95 / 111; INT2 512 76 / 80.  INT2 up to 256 spills 208 bytes of stores a thread and more with one block more than
+// here: 128 72.5 against 67, 64 81 against 77, 1024 x 1024 13.1 against 9.6.
+__host__ __device__ constexpr int pack_blocks(int bits, int v) { return v == 1 ? 3 : v == 2 ? 2 : bits == 2 ? 2 : 1; }
 
 // SEARCH: there are statistics, the scale is searched for.
 template <int BITS, int V, int DT, bool SEARCH>
