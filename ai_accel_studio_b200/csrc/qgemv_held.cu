@@ -186,9 +186,11 @@ __device__ __forceinline__ float bf16_to_scaled(uint4 (&v)[2]) {
     return big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
 }
 
-// Bias, activation and store of four weight rows (r on, of the tile at row n0) of one activation column.  Called by whole warps.
+// Bias, activation and store of four weight rows (r on, of the tile at row n0) of one activation column.  A tile may reach
+// into its neighbours' rows, the matrix' last one below and a CTA's last one above: it stores rows [from, to) only, because the others' sums
+// may have their outlier columns in another place.  Called by whole warps.
 template <bool BF16>
-__device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], uint32_t bias, bool live, int m, int n0, int r) {
+__device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], uint32_t bias, bool live, int m, int n0, int r, int from, int to) {
     using XT = typename Act16<BF16>::T;
     if (bias) {
         const uint2 b = lds64(bias);
@@ -216,11 +218,12 @@ __device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], ui
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[e] = Act16<BF16>::from_float(v[e]);
     XT* y = static_cast<XT*>(p.y) + (long long)m * p.ldy + n;
-    if ((p.flags & kHeldYVector) && (n & 3) == 0) {
+    if ((p.flags & kHeldYVector) && (n & 3) == 0 && r >= from && r + 4 <= to) {
         *reinterpret_cast<uint2*>(y) = *reinterpret_cast<const uint2*>(o);
     } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = o[e];
+        for (int e = 0; e < 4; ++e)
+            if (r + e >= from && r + e < to) y[e] = o[e];
     }
 }
 
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     using H = Held<FMT, KBW>;
     using XT = typename Act16<BF16>::T;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) unsigned long long full[kHeldMaxWarps * kHeldMaxBatch + 3];      // outlier weights of a batch's tiles have landed; U; scales, two buffers
+    __shared__ __align__(8) unsigned long long full[2 * kHeldMaxWarps * kHeldMaxBatch + 3];      // outlier weights of a batch's tiles have landed, two buffers; U; scales, two buffers
     QGEMV_HELD_STAMP(0);
     pdl_launch_dependents();
     const int lane = threadIdx.x, kw = threadIdx.y, wrow = threadIdx.z, wk = blockDim.y, wr = blockDim.z;
@@ -257,6 +260,10 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     const int batch_rows = wr * p.tb * 16;
     const bool has_o = p.noc && split == 0;
 
+    if (tid < 2 * p.tb * wr) mbarrier_init(smem_u32(full + tid), 32);
+    constexpr int kFullU = 2 * kHeldMaxWarps * kHeldMaxBatch, kFullScales = kFullU + 1;
+    if (tid < 3) mbarrier_init(smem_u32(full + kFullU + tid), threads);
+    __syncthreads();
     // ---- before the dependency wait: all that does not depend on x ----------------------------------------------------
     Ring<H> ring;
     {
@@ -269,13 +276,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         ring.dst = ring_at + stage_offset<H::PITCH>(r, piece * 16);
         ring.at = 0;
     }
-#pragma unroll 1
-    for (int d = 0; d < H::DEPTH / H::NS; ++d) ring.issue();
-    QGEMV_HELD_STAMP(1);
-    constexpr int kFullU = kHeldMaxWarps * kHeldMaxBatch, kFullScales = kFullU + 1;
-    if (tid < p.tb * wr) mbarrier_init(smem_u32(full + tid), 32);
-    if (tid < 3) mbarrier_init(smem_u32(full + kFullU + tid), threads);
-    __syncthreads();
+    ring.issue();                                      // the first tile, then what is wanted with it, then the rest of the ring
     // Scales of sc_rows rows (all of the CTA's, or a batch's), from the 4- or 16-byte word that holds the K slice's first; past the row's end zero.
     const int sc_lds = (int)p.lds, sc_first = split * p.sc_split;
     auto stage_scales = [&](int row0, int buf) {
@@ -295,8 +296,8 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     stage_scales(rowbase, 0);
     // Outlier weights of a batch's tiles, each fetched and multiplied by one warp of its row of warps, another one from batch to batch.
     int turn = kw;                                     // this warp has tile `turn` of its row's batch, and every wk-th after it
-    auto stage_outliers = [&](int row0) {
-        const uint32_t to = sm + p.off_ow;
+    auto stage_outliers = [&](int row0, int buf, int turn) {
+        const uint32_t to = sm + p.off_ow + buf * p.ow_bytes;
         const int units = p.noc * 4;
 #pragma unroll 1
         for (int i = turn; i < p.tb; i += wk) {
@@ -312,10 +313,10 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 else
                     for (int q = 0; q < 8; ++q) sts_half(d + q * 2, q < left ? __ldg(from + q) : __half(0.0f));
             }
-            mbarrier_arrive_copies(smem_u32(full + jt));
+            mbarrier_arrive_copies(smem_u32(full + buf * (p.tb * wr) + jt));
         }
     };
-    if (has_o) stage_outliers(rowbase);
+    if (has_o) stage_outliers(rowbase, 0, turn);
     {                                                  // rows of U (padded to 8 columns) and bias of all the CTA's tiles
         const int nrow = (rowend - rowbase + 15) & ~15, pieces = p.rank8 >> 3;
         for (int i = tid; i < nrow; i += threads) {
@@ -331,6 +332,9 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         }
         mbarrier_arrive_copies(smem_u32(full + kFullU));
     }
+#pragma unroll 1
+    for (int d = 1; d < H::DEPTH / H::NS; ++d) ring.issue();
+    QGEMV_HELD_STAMP(1);
     const int n_xo = has_o ? M << p.oc_log : 0, xo_mask = (1 << p.oc_log) - 1;      // activations of the outlier columns, [m][column]
     int xcol = -1;
     if (tid < n_xo && (tid & xo_mask) < p.oc) xcol = __ldg(p.oidx + (tid & xo_mask));
@@ -516,7 +520,8 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         const int buf = bt & 1;
         const int sb = p.sc_all ? 0 : buf;
         if (!p.sc_all && row0 + batch_rows < rowend) stage_scales(row0 + batch_rows, buf ^ 1);      // every warp is done with that buffer's last batch
-        if (bt > 0 && has_o) stage_outliers(row0);
+        const int next_turn = turn >= p.tb ? turn - p.tb : turn - p.tb + wk;       // the next warps' turn (tb <= wk)
+        if (has_o && row0 + batch_rows < rowend) stage_outliers(row0 + batch_rows, buf ^ 1, next_turn);
         if (!mbarrier_wait(smem_u32(full + kFullScales + sb), p.sc_all ? 0 : (bt >> 1) & 1) && lane == 0) atomicExch(p.status, 2);
         uint32_t sc_tile = sc_lane + (p.sc_all ? (uint32_t)((row0 - rowbase) * p.sc_pitch) : (uint32_t)(buf * p.sc_bytes));
         float* dst = part + (size_t)buf * (p.part_bytes / 4) + (size_t)warp * part_floats;
@@ -590,9 +595,9 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
             for (int i = turn; i < p.tb; i += wk) {
                 const int jt = i * wr + wrow;
                 if (row0 + jt * 16 >= rowend) break;
-                if (!mbarrier_wait(smem_u32(full + jt), bt & 1) && lane == 0) atomicExch(p.status, 2);
+                if (!mbarrier_wait(smem_u32(full + buf * (p.tb * wr) + jt), (bt >> 1) & 1) && lane == 0) atomicExch(p.status, 2);
                 __syncwarp();
-                const uint32_t ow = sm + p.off_ow + (uint32_t)((jt * 16 + g) * (p.noc * 64) + t * 16);
+                const uint32_t ow = sm + p.off_ow + buf * p.ow_bytes + (uint32_t)((jt * 16 + g) * (p.noc * 64) + t * 16);
                 float v[NB][4];
 #pragma unroll
                 for (int b = 0; b < NB; ++b) v[b][0] = v[b][1] = v[b][2] = v[b][3] = 0.0f;
@@ -625,7 +630,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                     }
                 }
             }
-            turn = turn >= p.tb ? turn - p.tb : turn - p.tb + wk;          // the next warps' turn (tb <= wk)
+            turn = next_turn;
         }
         if (bt == 0 && exchange && warp == threads / 32 - 1) {     // all CTAs' projections of this K slice
             const int limit = (p.debug & QGEMV_DEBUG_DROP_PROJECTIONS) ? (1 << 7) : (1 << 20);
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 if (live) *reinterpret_cast<float4*>(p.partial + (((size_t)split * gridDim.x + grp) * p.rows_pad + (row0 - rowbase) + jt * 16) * p.mp + pc * 16 + quad * 4) = make_float4(v[0], v[1], v[2], v[3]);
                 continue;
             }
-            finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + rl * 2 : 0u, live, m, min(row0 + jt * 16, last), quad * 4);
+            finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + rl * 2 : 0u, live, m, min(row0 + jt * 16, last), quad * 4, max(0, row0 + jt * 16 - last), rowend - min(row0 + jt * 16, last));
         }
         turn0 += (items + 31) & ~31;
         if (turn0 >= threads) turn0 %= threads;
@@ -711,7 +716,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                         const float4 a = __ldcg(reinterpret_cast<const float4*>(src + k * stride));
                         v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
                     }
-                finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + (jt * 16 + quad * 4) * 2 : 0u, live, m, min(rowbase + jt * 16, last), quad * 4);
+                finish_rows<BF16>(p, v, p.bias ? sm + p.off_bias + (jt * 16 + quad * 4) * 2 : 0u, live, m, min(rowbase + jt * 16, last), quad * 4, max(0, rowbase + jt * 16 - last), rowend - min(rowbase + jt * 16, last));
             }
         }
     }

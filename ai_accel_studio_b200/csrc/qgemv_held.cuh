@@ -43,7 +43,7 @@ struct HeldArgs {
     int mp, mp_log;                               // columns of a partial sum (2, 4, 8 or 16)
     int sc_split, sc_unit, sc_units, sc_log, sc_pitch;      // scales of a K split; bytes of one copy, copies of a row, log2 of those rounded up, bytes of a staged row
     int sc_rows, sc_bytes, sc_all;                // rows staged at a time, bytes of a buffer; all of the CTA's rows in one
-    int ow_log;                                   // log2 of the 16-byte pieces of a row of outlier weights, rounded up
+    int ow_log, ow_bytes;                         // log2 of the 16-byte pieces of a row of outlier weights, rounded up; bytes of one of their two buffers
     int off_part, off_tab, off_tpart, off_sc, off_ow, off_u, off_bias, off_xo, off_upo, off_tt;      // shared memory (rings start at 0)
     int part_bytes;                               // one of the two buffers of partial sums
 };

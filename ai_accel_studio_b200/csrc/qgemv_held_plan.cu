@@ -43,7 +43,8 @@ bool place(const qgemv_problem& p, int m, bool bf16, HeldPlan& h) {
             a.off_tab = put(nw * h.kbw * kHeldGroups[h.fmt] * h.nb * 64);
             a.off_tpart = put(a.rank ? h.wk * 8 * a.mp * 4 : 0);
             a.off_sc = put((a.sc_all ? 1 : 2) * a.sc_bytes);
-            a.off_ow = put(h.wr * tb * 16 * a.noc * 64);
+            a.ow_bytes = up_to(h.wr * tb * 16 * a.noc * 64, 128);
+            a.off_ow = put(2 * a.ow_bytes);
             a.off_u = put(a.rows_pad * a.rank8 * 2);
             a.off_bias = put(p.bias ? a.rows_pad * 2 : 0);
             a.off_xo = put(a.noc ? m * (a.noc * 64 + 16) : 0);
