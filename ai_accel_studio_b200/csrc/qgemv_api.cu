@@ -146,7 +146,7 @@ MmaPlan choose(const qgemv_problem& p, size_t partial_floats, bool* forced_missi
 // 6.2; 9728 x 896 INT2 9.1 against 6.2; 2048 x 2048 5.8 against 5.1; without residual 2048 x 768 INT2 2.7 against 3.7, groups of 64 1024 x 1024
 // 2.7 against 2.4, of 32 INT4 2.8 against 2.1.
 bool choose_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* plan) {
-    if (p.kernel != QGEMV_KERNEL_AUTO || p.m > QGEMV_MAX_M || p.k_padded > 1024 || p.k_original != p.k_padded) return false;
+    if (p.kernel != QGEMV_KERNEL_AUTO || p.m > QGEMV_MAX_M || p.k_padded > 1024 || p.k_original != p.k_padded || p.ldx % 8 || p.k_original % 8 || (p.rank && (!aligned(p.res_v, 16) || p.ldv % 8))) return false;
     const int tiles = (p.n + kStreamTileRows - 1) / kStreamTileRows, sms = sm_count();
     if (tiles * 4 > sms * 9 || (p.rank == 0 && p.group < 128) || (p.group == 32 && tiles > sms)) return false;
     return plan_held(p, partial_floats, plan);
@@ -389,7 +389,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
     }
     if (choose_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
-    if (p->kernel == QGEMV_KERNEL_AUTO && (p->m > QGEMV_MAX_M || (starved && p->m > 2)) && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
+    if (p->kernel == QGEMV_KERNEL_AUTO && (p->m > QGEMV_MAX_M || (starved && p->m > 2 && p->ldx % 8 == 0)) && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
     q->held.ok = false;
     // Three or four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of
     // its 16 warps (see align_x_kernel) and loses no precision against the streaming kernel, which takes x as it is.  One and two rows

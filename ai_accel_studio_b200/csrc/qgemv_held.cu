@@ -186,6 +186,36 @@ __device__ __forceinline__ float bf16_to_scaled(uint4 (&v)[2]) {
     return big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(e - 13);
 }
 
+// Rows of 128 columns that are not on 16-byte boundaries (or end off one), element by element, to where to_frag leaves aligned ones: the
+// permutation of to_frag_order, and the swizzle.  up: what bf16 rows are to be multiplied by, [row] (NULL: fp16 values).
+template <int BITS, int ROWBIT>
+__device__ __noinline__ void fill_odd(uint32_t scratch, const unsigned short* base, long long ld, int nrow, int left, float* up, int up_groups, int up_step) {
+    const int lane = threadIdx.x;
+#pragma unroll 1
+    for (int r = 0; r < nrow; ++r) {
+        unsigned short e[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[i] = lane + 32 * i < left ? base[r * ld + lane + 32 * i] : (unsigned short)0;
+        if (up) {
+            uint32_t big = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) big = max(big, (uint32_t)(e[i] & 0x7fff) << 16);
+            big = __reduce_max_sync(0xffffffffu, big);
+            const int x = block_exponent(big);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e[i] = __half_as_ushort(__float2half_rn(__uint_as_float((uint32_t)e[i] << 16) * pow2f(13 - x)));
+            if (lane < up_groups) up[lane * up_step + (r >> 1) * 4 + (r & 1)] = big >= kInfBits ? __int_as_float(0x7fffffff) : pow2f(x - 13);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = lane + 32 * i;
+            const int at = BITS == 4 ? (c & ~7) + (c & 1) * 4 + (c & 2) + ((c >> 2) & 1) : (c & ~15) + (c & 2) * 4 + (c & 1) * 4 + ((c >> 1) & 2) + ((c >> 3) & 1);
+            const int pc = at >> 3;
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(scratch + (uint32_t)(r * 256 + (pc ^ ((pc >> 3) & 1) ^ ((r & 1) * ROWBIT)) * 16 + (at & 7) * 2)), "h"(e[i]) : "memory");
+        }
+    }
+}
+
 // Bias, activation and store of four weight rows (r on, of the tile at row n0) of one activation column.  A tile may reach
 // into its neighbours' rows, the matrix' last one below and a CTA's last one above: it stores rows [from, to) only, because the others' sums
 // may have their outlier columns in another place.  Called by whole warps.
@@ -234,7 +264,8 @@ __device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], ui
 #define QGEMV_HELD_STAMP(i) do {} while (0)
 #endif
 
-template <int FMT, int KBW, int NB, bool BF16>
+// ODD: rows of x or V may lie off 16 bytes (an instance of its own: beside the usual ones the code costs 2 - 3 %).
+template <int FMT, int KBW, int NB, bool BF16, bool ODD>
 __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const __grid_constant__ HeldArgs p) {
     using F = Fmt<FMT>;
     using H = Held<FMT, KBW>;
@@ -371,7 +402,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         }
     };
     constexpr int kRowBit = F::NG == 1 ? 2 : F::NG == 2 ? 1 : 4;       // what an odd row flips of a piece's position
-    auto to_frag = [&](uint4 (&v)[2][2], int nrow, uint64_t (&f)[8]) {
+    auto to_scratch = [&](uint4 (&v)[2][2], int nrow) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = i * 4 + (lane >> 3), pc = (lane & 7) * 2;
@@ -382,6 +413,8 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 sts128(at ^ 16u, v[i][1]);
             }
         }
+    };
+    auto from_scratch = [&](uint64_t (&f)[8]) {
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -390,7 +423,9 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         }
         __syncwarp();
     };
+    const bool odd_x = ODD && (p.flags & kHeldXOdd) != 0;
     uint4 xv[NB][KBW][2][2];
+    if (!odd_x)
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
@@ -402,19 +437,25 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         for (int b = 0; b < NB; ++b) {
 #pragma unroll
             for (int kb = 0; kb < KBW; ++kb) {
-                if constexpr (BF16) {
+                float* const ups = reinterpret_cast<float*>(tab - t + (kb * F::NG * NB + b) * 4) + 2;
+                if (odd_x) {
+                    fill_odd<F::BITS, kRowBit>(scratch, static_cast<const unsigned short*>(p.x) + (long long)(b * 8) * p.ldx + (kb0 + kb) * kHeldBlock, p.ldx, min(8, M - b * 8),
+                                               kend - (kb0 + kb) * kHeldBlock, BF16 ? ups : nullptr, F::NG, NB * 16);
+                } else {
+                    if constexpr (BF16) {
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const float up = bf16_to_scaled(xv[b][kb][i]);
-                        const int r = i * 4 + (lane >> 3);
-                        if ((lane & 7) == 0) {
-                            float* u = reinterpret_cast<float*>(tab - t + (kb * F::NG * NB + b) * 4 + (r >> 1)) + 2 + (r & 1);
+                        for (int i = 0; i < 2; ++i) {
+                            const float up = bf16_to_scaled(xv[b][kb][i]);
+                            const int r = i * 4 + (lane >> 3);
+                            if ((lane & 7) == 0) {
 #pragma unroll
-                            for (int j = 0; j < F::NG; ++j) u[j * NB * 16] = up;
+                                for (int j = 0; j < F::NG; ++j) ups[j * NB * 16 + (r >> 1) * 4 + (r & 1)] = up;
+                            }
                         }
                     }
+                    to_scratch(xv[b][kb], M - b * 8);
                 }
-                to_frag(xv[b][kb], M - b * 8, fr[kb][b]);
+                from_scratch(fr[kb][b]);
             }
         }
 #pragma unroll 1
@@ -467,8 +508,13 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         for (int kb = 0; kb < KBW; ++kb) {
             uint4 a[2][2];
             uint64_t fa[8];
-            load_rows(vr, p.ldv, nr, kb, a);
-            to_frag(a, nr, fa);
+            if (ODD && (p.flags & kHeldVOdd)) {
+                fill_odd<F::BITS, kRowBit>(scratch, vr + (kb0 + kb) * kHeldBlock, p.ldv, nr, kend - (kb0 + kb) * kHeldBlock, nullptr, 0, 0);
+            } else {
+                load_rows(vr, p.ldv, nr, kb, a);
+                to_scratch(a, nr);
+            }
+            from_scratch(fa);
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 float c[4];
@@ -726,9 +772,9 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     if (exchange && tid == 0) atomicAdd(p.epoch, grp + split == 0 ? 257ull - gridDim.x * gridDim.y : 1ull);
 }
 
-template <int FMT, int KBW, int NB, bool BF16>
+template <int FMT, int KBW, int NB, bool BF16, bool ODD>
 int launch_one(const HeldPlan& h, bool dependent, cudaStream_t s) {
-    auto kern = qgemv_held_kernel<FMT, KBW, NB, BF16>;
+    auto kern = qgemv_held_kernel<FMT, KBW, NB, BF16, ODD>;
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -759,14 +805,19 @@ int launch_one(const HeldPlan& h, bool dependent, cudaStream_t s) {
 #if !defined(QGEMV_HELD_FMT) || !defined(QGEMV_HELD_BF16)
 #error "compile with -DQGEMV_HELD_FMT=0..4 and -DQGEMV_HELD_BF16=0|1"
 #endif
-template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s) {
+namespace {
+template <int FMT, bool BF16, bool ODD> int launch_odd(const HeldPlan& h, bool dependent, cudaStream_t s) {
     if (h.nb == 1) {
-        if (h.kbw == 1) return launch_one<FMT, 1, 1, BF16>(h, dependent, s);
-        if (h.kbw == 2) return launch_one<FMT, 2, 1, BF16>(h, dependent, s);
-        return launch_one<FMT, 4, 1, BF16>(h, dependent, s);
+        if (h.kbw == 1) return launch_one<FMT, 1, 1, BF16, ODD>(h, dependent, s);
+        if (h.kbw == 2) return launch_one<FMT, 2, 1, BF16, ODD>(h, dependent, s);
+        return launch_one<FMT, 4, 1, BF16, ODD>(h, dependent, s);
     }
-    if (h.kbw == 1) return launch_one<FMT, 1, 2, BF16>(h, dependent, s);
-    return launch_one<FMT, 2, 2, BF16>(h, dependent, s);
+    if (h.kbw == 1) return launch_one<FMT, 1, 2, BF16, ODD>(h, dependent, s);
+    return launch_one<FMT, 2, 2, BF16, ODD>(h, dependent, s);
+}
+}  // namespace
+template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s) {
+    return h.args.flags & (kHeldXOdd | kHeldVOdd) ? launch_odd<FMT, BF16, true>(h, dependent, s) : launch_odd<FMT, BF16, false>(h, dependent, s);
 }
 template int launch_held_fmt<QGEMV_HELD_FMT, QGEMV_HELD_BF16>(const HeldPlan&, bool, cudaStream_t);
 

@@ -62,13 +62,14 @@ bool place(const qgemv_problem& p, int m, bool bf16, HeldPlan& h) {
 bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out) {
     const int m = p.m, sms = sm_count();
     out->ok = false;
-    if (m < 1 || m > 16 || p.n < 16 || !al(p.x, 16) || p.ldx % 8 || p.k_original % 8) return false;
+    if (m < 1 || m > 16 || p.n < 16 || !al(p.x, 16)) return false;
     HeldPlan h{};
     HeldArgs& a = h.args;
     h.fmt = stream_format(p.bits, p.group);
     if (h.fmt < 0 || !al(p.packed, 16) || p.ldp % 16 || p.outliers > kStreamMaxOutliers || p.rank > kMaxRank) return false;
-    if (p.rank && (!al(p.res_v, 16) || p.ldv % 8)) return false;
     if (!al(p.scales, 4) || p.ldp > 0x7fffffff || (long long)p.n * p.lds > 0x7fffffff) return false;
+    if (p.ldx % 8 || p.k_original % 8) a.flags |= kHeldXOdd;
+    if (p.rank && (!al(p.res_v, 16) || p.ldv % 8 || p.k_original % 8)) a.flags |= kHeldVOdd;
     if (p.outliers && al(p.outlier_w, 16) && p.ldow % 8 == 0) a.flags |= kHeldOutlierAligned;
     if (p.rank && al(p.res_u, 16) && p.ldu % 8 == 0 && p.rank % 8 == 0) a.flags |= kHeldUAligned;
     const bool bf16 = p.x_dtype == QGEMV_BF16;

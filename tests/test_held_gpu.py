@@ -24,6 +24,8 @@ CASES = [
     (4, 300, 8320, 64, 16, 8, True, (5, 10)),            # 65 blocks: K cut between CTAs
     (2, 1200, 20480, 256, 0, 12, True, (7, 16)),         # splits at whole scale groups, projections dealt to several CTAs
     (2, 40000, 512, 128, 64, 8, False, (8, 16)),         # many batches of tiles, scales staged batch by batch
+    (2, 300, 1003, 64, 8, 5, True, (5, 16)),             # rows of x and V off 16 bytes, K padded
+    (4, 200, 8197, 128, 16, 9, False, (6, 12)),          # the same over two K splits
     (4, 4800, 3800, 40, 0, 0, False, (5,)),              # a group that is not built: four rows at a time, as before
 ]
 
