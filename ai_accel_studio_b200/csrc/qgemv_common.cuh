@@ -33,7 +33,7 @@ constexpr size_t kWsPartialOff   = kWsCounterOff + sizeof(int) * kWsMaxCounters;
 constexpr int    kMaxTParts      = 8;              // K-parts of an in-kernel residual projection
 // tail of the partial-sum area: {fp32 value, launch tag} per (K-part, m, rank column), in 32-bit words
 constexpr int    kTPartFloats    = 2 * kMaxTParts * QGEMV_MAX_M * kMaxRank;
-constexpr size_t kMaxPartialFloats = size_t(1) << 21;                             // 8 MiB of fp32 partial sums: two K splits of 16 x 28672 results need 3.7
+constexpr size_t kMaxPartialFloats = size_t(9) << 19;                             // 18 MiB of fp32 partial sums: eight K splits of 28672 x 16 results need 14, two of 128256 x 16 need 15.7
 constexpr int    kMaxCtas        = 512;           // of a tensor-core kernel; one per SM are launched
 constexpr size_t kCtaPartialBytes = 2 * 4 * 32 * sizeof(float);
 constexpr size_t kWsCopyOff      = kWsPartialOff + (size_t(1) << 20), kWsCopyBytes = size_t(1) << 20;
