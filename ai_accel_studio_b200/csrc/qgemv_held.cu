@@ -191,11 +191,15 @@ __device__ __forceinline__ float bf16_to_scaled(uint4 (&v)[2]) {
 template <int BITS, int ROWBIT>
 __device__ __noinline__ void fill_odd(uint32_t scratch, const unsigned short* base, long long ld, int nrow, int left, float* up, int up_groups, int up_step) {
     const int lane = threadIdx.x;
-#pragma unroll 1
-    for (int r = 0; r < nrow; ++r) {
-        unsigned short e[4];
+    unsigned short v[8][4];                            // all rows at once: one after the other each waits out its loads' latency
 #pragma unroll
-        for (int i = 0; i < 4; ++i) e[i] = lane + 32 * i < left ? base[r * ld + lane + 32 * i] : (unsigned short)0;
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[r][i] = r < nrow && lane + 32 * i < left ? base[r * ld + lane + 32 * i] : (unsigned short)0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (r >= nrow) break;
+        unsigned short (&e)[4] = v[r];
         if (up) {
             uint32_t big = 0;
 #pragma unroll
