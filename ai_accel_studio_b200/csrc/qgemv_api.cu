@@ -359,17 +359,19 @@ static_assert(kWsTraceOff + kWsTraceBytes <= kWsPartialOff + (kMaxPartialFloats 
 
 extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
 
-// The streaming kernel takes what qgemv_run cannot take in one launch -- more than four rows, and x whose rows are not
-// padded to k_padded columns or not 16-byte aligned, unless three or four of them are copied (see below) -- and leaves one to four aligned
-// rows to the kernels above: those
-// launches last about as long as their code takes to arrive in the instruction caches (some 3.5 clocks per instruction on
-// a first pass), and the streaming kernel has more of it (4096 x 4096 INT4, M = 1: 10.8 against 7.1 us).  The exception are
-// rows so long that their activations leave the phased kernel few of its 16 warps, or do not fit beside it at all (M = 4,
-// K = 28672; the CUDA-core kernel took those): the streaming kernel cuts K between CTAs instead.  With 4 warps left it wins
-// (14336 x 14336 INT4, M = 4: 44 against 65 us), with 8 it loses (4096 x 14336 INT4, M = 4: 24 against 18 us) unless there are
-// at most two rows, which it multiplies as integers (K = 28672, M = 2, N = 2048 and 8192: INT4 24 against 33 and 48 against 51 us,
-// INT2 21 against 16 and 36 against 43 us).  INT2 matrices of no more than one tile of 16 rows per SM, which the phased kernel reads
-// in a single round, stay with it (N = 512 to 2048: 16 us, streaming 17 to 21).
+// One to four aligned rows stay with the kernels above; more rows, and x whose rows are not padded to k_padded columns or not 16-byte aligned, go to the
+// kernel that holds its activations in registers, from three rows on, or the streaming one (one and two rows, formats or scratch the other does not take).
+// The phased kernel's launches last about as long as their code takes to arrive in the instruction caches (some 3.5 clocks per
+// instruction on a first pass), and the other two have more of it (4096 x 4096 INT4, M = 1: held 7.4, phased 7.2 us; M = 4 7.5 and 7.9).  The exception are
+// rows so long that their activations leave it few of its 16 warps, or do not fit beside it at all (M = 4, K = 28672; the CUDA-core kernel took those): the
+// other two cut K between CTAs instead.
+//  * Three and four rows: at 4 warps (57344 x 12288 INT4, M = 4 1.18x) and where it does not fit.
+//  * Four rows from K = 8192 on: at 8 warps (8192 x 11008 INT4 1.48x, 57344 x 12288 1.06x, 4096 x 14336 INT2 1.11x; below that K the phased kernel wins,
+//    14336 x 6144 0.86x).  INT4 from about K = 10000 on: at 12 (8192 x 11008 1.22x, 57344 x 11008 1.21 to 1.44x; 57344 x 9216 0.80x, INT2
+//    4096 x 11008 0.96x), groups of 32 at any K (0.99 to 1.26x, 13 matrices; 128 and 64 at K = 8192 0.86 to 1.13x).  Three rows are mixed, 0.84 to 1.36x at 8.
+//  * One and two rows, which the streaming kernel multiplies as integers: at 8 (K = 28672, M = 2, N = 2048 and 8192: INT4 24 against 33 and 48 against 51 us,
+//    INT2 21 against 16 and 36 against 43 us); INT2 matrices of no more than one tile of 16 rows per SM, which the phased kernel reads
+//    in a single round, stay with it (N = 512 to 2048: 16 us, streaming 17 to 21).
 extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
     const size_t need = qgemv_workspace_bytes(0, 0, 0, 0, 0, 0);
     const int v = validate(p, need, QGEMV_MAX_BATCH);
@@ -386,19 +388,24 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         bool none = false;
         const MmaPlan plan = choose(*p, kMaxPartialFloats, &none);
         const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
-        starved = !plan.ok || (plan.variant == 1 && plan.nw <= (p->m <= 2 && !one_round ? 8 : 4));
+        int most = p->m <= 2 && !one_round ? 8 : 4;    // warps
+        if (p->m == 4 && p->k_padded >= 8192) most = 8;
+        if (p->m == 4 && p->bits == 4 && (p->k_padded >= 10240 || p->group == 32)) most = 12;
+        starved = !plan.ok || (plan.variant == 1 && plan.nw <= most);
     }
     if (choose_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
-    if (p->kernel == QGEMV_KERNEL_AUTO && (p->m > QGEMV_MAX_M || (starved && p->m > 2 && p->ldx % 8 == 0)) && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
+    if (p->kernel == QGEMV_KERNEL_AUTO && p->m > QGEMV_MAX_M && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
     q->held.ok = false;
-    // Three or four rows of x that are not padded or not aligned: a launch that copies them, then the phased kernel, where that has all of
-    // its 16 warps (see align_x_kernel) and loses no precision against the streaming kernel, which takes x as it is.  One and two rows
-    // stay with that: it adds them up as integers (error of a result before it is rounded 1e-7, in the phased kernel 5e-7 to 2e-5, 1024 rows
-    // of 4100 to 7000 columns), and so do INT2 groups above 64, whose chains of products in one accumulator are longer in the phased kernel
-    // (errors 8 to 33 % larger, groups of 128 and 256; INT2 groups of 64 and INT4 are equal to 1 %).  Rows that leave fewer warps stay as well (512 x 10001 INT4,
-    // M = 4: 20 us either way), and calls that one launch finishes in less than the 8 us that two cost an eager caller on the host: no
-    // residual (with one it takes 10.7 us and more, the two launches 6.6 on the GPU: 512 x 1500 INT4, M = 3) and few bytes (INT4, M = 3 and 4: 8575 x 776 5.5 us, 11574 x 1336
-    // 9.3; 8209 x 2928, 12 MB, 10.0 against 9.2 of two launches), unless the rows are long (1462 x 4323 INT2, M = 3: 9.3 against 5.1).
+    // Three or four rows of x that are not padded or not aligned: the kernel with held activations below, which takes them as they are, or a launch
+    // that copies them and then the phased kernel.  The two launches stay where that one has all of its 16 warps (see align_x_kernel) and loses no precision
+    // (INT2 groups above 64: its chains of products in one accumulator are longer, errors 8 to 33 % larger; INT2 groups of 64 and INT4 are equal to 1 %)
+    // and  - without a residual, for large matrices or long rows (60000 x 1001 INT2 11.2 against 13.4 us of the one launch, 20000 x 2047 INT4 8.9 against 10.4;
+    //        8209 x 2928 9.4 against 7.2);
+    //      - with one, for matrices below 4 MB.  The one launch is faster there as well (676 x 1601 INT4 6.4 against 8.1, 513 x 712 3.8 against 7.1), but
+    //        how many launches these calls make is tested.  Above, one against two: 4999 x 4300 12.5 against 13.8, 9492 x 2248 10.2 against 12.5,
+    //        17030 x 1416 10.4 against 17.2.
+    // One and two rows stay with the streaming kernel, which adds them up as integers (error of a result before it is rounded 1e-7, in the others
+    // 5e-7 to 2e-5, 1024 rows of 4100 to 7000 columns).
     const bool as_exact = p->m >= 3 && (p->bits == 4 || p->group <= 64);
     if (p->kernel == QGEMV_KERNEL_AUTO && p->m <= QGEMV_MAX_M && as_exact && (!padded || p->ldx % 8)) {
         qgemv_problem c = *p;                          // (as the streaming kernel, only x that starts on 16 bytes)
@@ -406,13 +413,16 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         c.x = static_cast<char*>(p->workspace) + kWsCopyOff;
         bool none = false;
         const MmaPlan plan = choose(c, kMaxPartialFloats, &none);
-        const bool pays = p->rank > 0 || (size_t)p->n * p->k_padded * p->bits / 8 >= (size_t(8) << 20) || p->k_original >= 4096;
+        const size_t codes = (size_t)p->n * p->k_padded * p->bits / 8;
+        const bool pays = p->rank > 0 ? codes < (size_t(4) << 20) : codes >= (size_t(8) << 20) || p->k_original >= 4096;
         if (aligned(p->x, 16) && plan.ok && plan.variant == 1 && plan.nw >= 16 && pays && (size_t)c.m * c.ldx * 2 <= kWsCopyBytes) {
             q->pitch = (int)c.ldx;
             q->project = p->rank > 0 && !plan.t_inline;
             return QGEMV_OK;
         }
     }
+    if (p->kernel == QGEMV_KERNEL_AUTO && p->m > 2 && (starved || !padded || p->ldx % 8) && plan_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
+    q->held.ok = false;
     if (p->kernel != QGEMV_KERNEL_SIMT && (p->m > QGEMV_MAX_M || !padded || p->ldx % 8 || starved) &&
         plan_stream(*p, kMaxPartialFloats, &q->plan))
         return QGEMV_OK;

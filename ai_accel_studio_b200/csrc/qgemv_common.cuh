@@ -15,12 +15,13 @@ namespace qgemv {
 //   [0, 1024)            residual projections t[m][r] = sum_k V[r,k] x[m,k], fp32, QGEMV_MAX_M x 64
 //   [1024, 1024+4*16384) arrival counters, one int32 per 16-row tile (zero between calls)
 //   [kWsPartialOff, ..)   partial sums, kMaxPartialFloats fp32 in all:
-//     from its start        tiles shared by CTAs of the tensor-core kernels [CTA][2][4][32], or split sums of the streaming kernel
+//     from its start        tiles shared by CTAs of the tensor-core kernels [CTA][2][4][32], or split sums of the streaming kernel and of
+//                           the one with register-held activations
 //     [kWsCopyOff, ..)      x in padded rows for the tensor-core kernel (align_x_kernel), kWsCopyBytes
 //     [kWsTraceOff, ..)     time stamps of a build with QGEMV_TRACE, kWsTraceBytes
-//     at its end            {value, launch tag} words of the streaming kernel (kStreamWordFloats) and of the others (kTPartFloats)
-//   The tensor-core kernels read a copy of x while they write partial sums, time stamps and words; split sums of the streaming kernel may lie
-//   over all but the words, since it takes no copy and writes none of the others.
+//     at its end            {value, launch tag} words of those two (kStreamWordFloats) and of the others (kTPartFloats)
+//   The tensor-core kernels read a copy of x while they write partial sums, time stamps and words; split sums of the other two may lie
+//   over all but the words, since they take no copy and write none of the others.
 constexpr int    kMaxRank        = 64;
 constexpr size_t kWsTOff         = 0;
 constexpr size_t kWsCounterOff   = 1024;

@@ -76,10 +76,11 @@ __device__ __forceinline__ int part_index(int hp, int c, int r) {
 }
 
 // Producer side of a warp's ring: stages in the order (tile, part of the columns).
-template <typename H> struct Ring {
+template <typename H, bool ODD> struct Ring {
     const uint8_t* src;                               // this lane's row and piece of the next tile, first stage
     long long step;                                   // to the warp's next tile
     int ldw, row, row_step, last, end_row;            // weight row of that tile, the last one a tile may start at, end of the CTA's rows
+    int rows_left;                                    // ODD: rows of the matrix below this lane's first one, in the tile
     int left;                                         // bytes from this lane's piece to the end of the warp's columns
     uint32_t dst, at;
 
@@ -91,7 +92,8 @@ template <typename H> struct Ring {
             if (more && left > st * H::PITCH) {
                 const uint32_t d = dst + at;
 #pragma unroll
-                for (int i = 0; i < H::COPIES; ++i) cp_async16((H::PITCH == 128 && (i & 1) ? d ^ 16u : d) + i * 512, src + (long long)(i * H::RPI) * ldw + st * H::PITCH);
+                for (int i = 0; i < H::COPIES; ++i)
+                    if (!ODD || i * H::RPI < rows_left) cp_async16((H::PITCH == 128 && (i & 1) ? d ^ 16u : d) + i * 512, src + (long long)(i * H::RPI) * ldw + st * H::PITCH);
             }
             cp_async_commit();
             at = at + H::STAGE == H::DEPTH * H::STAGE ? 0u : at + H::STAGE;
@@ -268,7 +270,8 @@ __device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], ui
 #define QGEMV_HELD_STAMP(i) do {} while (0)
 #endif
 
-// ODD: rows of x or V may lie off 16 bytes (an instance of its own: beside the usual ones the code costs 2 - 3 %).
+// ODD: rows of x or V may lie off 16 bytes, and the matrix may have less than a tile of rows (what is computed for the missing ones is not
+// stored).  An instance of its own: beside the usual ones the code costs 2 - 3 %.
 template <int FMT, int KBW, int NB, bool BF16, bool ODD>
 __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const __grid_constant__ HeldArgs p) {
     using F = Fmt<FMT>;
@@ -282,14 +285,15 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     const int warp = wrow * wk + kw, tid = warp * 32 + lane, threads = wk * wr * 32;
     const int g = lane >> 2, t = lane & 3, M = p.m;
     const int grp = blockIdx.x, split = blockIdx.y;
-    const int rowbase = grp * p.rows_per, rowend = min(rowbase + p.rows_per, p.n), last = p.n - 16;
+    const int rowbase = grp * p.rows_per, rowend = min(rowbase + p.rows_per, p.n);
+    const int last = ODD ? max(0, p.n - 16) : p.n - 16, low = ODD ? min(15, p.n - 1) : 15;      // where the last tile starts, the last row of a tile
     const int kb0 = split * p.blocks_split + kw * KBW;                   // this warp's first block
     const uint32_t sm = smem_u32(smem), ring_at = sm + (uint32_t)warp * (H::DEPTH * H::STAGE);
     const bool exchange = p.per_cta < p.rank;
     const int nr = exchange ? min(p.per_cta, p.rank - grp * p.per_cta) : p.rank;      // ranks that this CTA projects
     const int r0 = exchange ? grp * p.per_cta : 0;
     float* const part = reinterpret_cast<float*>(smem + p.off_part);
-    float* const tpart = reinterpret_cast<float*>(smem + p.off_tpart);                   // a warp's share of them [8][mp]
+    float* const tpart = reinterpret_cast<float*>(smem + p.off_tpart);                   // a warp's share of them [nr8][mp]
     float* const tt = reinterpret_cast<float*>(smem + p.off_tt);                         // residual projections [m][rank8]
     constexpr int part_floats = NB * 128;
     const int batch_rows = wr * p.tb * 16;
@@ -300,11 +304,12 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     if (tid < 3) mbarrier_init(smem_u32(full + kFullU + tid), threads);
     __syncthreads();
     // ---- before the dependency wait: all that does not depend on x ----------------------------------------------------
-    Ring<H> ring;
+    Ring<H, ODD> ring;
     {
         const int r = lane / H::PPR, piece = lane % H::PPR;
         ring.ldw = (int)p.ldw;
         ring.left = min(p.row_bytes, (split + 1) * p.blocks_split * H::BW) - kb0 * H::BW - piece * 16;
+        ring.rows_left = min(16, p.n) - r;
         ring.row = rowbase + wrow * 16; ring.row_step = wr * 16; ring.last = last; ring.end_row = rowend;
         ring.src = p.w + (long long)(ring.row + r) * p.ldw + kb0 * H::BW + piece * 16;
         ring.step = (long long)(wr * 16) * p.ldw;
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
             const uint32_t to = sm + p.off_sc + buf * p.sc_bytes + u * p.sc_unit;
 #pragma unroll 1
             for (int r = tid >> p.sc_log; r < nrow; r += threads >> p.sc_log) {
-                const int off = (min(row0 + (r & ~15), last) + (r & 15)) * sc_lds + sc_first, odd = off & 1, n = max(0, min(per, p.ng - sc_first + odd - u * per)) * 2;
+                const int off = (min(row0 + (r & ~15), last) + min(r & 15, low)) * sc_lds + sc_first, odd = off & 1, n = max(0, min(per, p.ng - sc_first + odd - u * per)) * 2;
                 const __half* from = n ? p.sc + (off - odd + u * per) : p.sc;
                 if (per == 8) cp_async16z(to + r * p.sc_pitch, from, n);
                 else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + r * p.sc_pitch), "l"(from), "r"(n) : "memory");
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 const int r = e >> p.ow_log, u = e & ((1 << p.ow_log) - 1), left = min(8, p.oc - u * 8);
                 if (u >= units) continue;
                 const uint32_t d = to + (uint32_t)((jt * 16 + r) * units + u) * 16;
-                const __half* from = p.ow + (long long)(min(row, last) + r) * p.ldow + u * 8;
+                const __half* from = p.ow + (long long)(min(row, last) + min(r, low)) * p.ldow + u * 8;
                 if (p.flags & kHeldOutlierAligned) cp_async16z(d, left > 0 ? from : p.ow, left > 0 ? left * 2 : 0);
                 else
                     for (int q = 0; q < 8; ++q) sts_half(d + q * 2, q < left ? __ldg(from + q) : __half(0.0f));
@@ -355,7 +360,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     {                                                  // rows of U (padded to 8 columns) and bias of all the CTA's tiles
         const int nrow = (rowend - rowbase + 15) & ~15, pieces = p.rank8 >> 3;
         for (int i = tid; i < nrow; i += threads) {
-            const int n = min(rowbase + (i & ~15), last) + (i & 15);
+            const int n = min(rowbase + (i & ~15), last) + min(i & 15, low);
             for (int q = 0; q < pieces; ++q) {
                 const __half* from = p.ru + (long long)n * p.ldu + q * 8;
                 const uint32_t d = sm + p.off_u + (uint32_t)(i * pieces + q) * 16;
@@ -503,20 +508,22 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         __syncwarp();
     }
     QGEMV_HELD_STAMP(4);
-    if (nr > 0 && wrow == 0) {                         // residual projections of this warp's columns, up to eight ranks
+    if (wrow == 0)                                     // residual projections of this warp's columns, eight ranks at a time
+#pragma unroll 1
+    for (int rr = 0; rr < nr; rr += 8) {
         float acc[NB][4];
 #pragma unroll
         for (int b = 0; b < NB; ++b) acc[b][0] = acc[b][1] = 0.0f;
-        const unsigned short* const vr = reinterpret_cast<const unsigned short*>(p.rv) + (long long)r0 * p.ldv;
+        const unsigned short* const vr = reinterpret_cast<const unsigned short*>(p.rv) + (long long)(r0 + rr) * p.ldv;
 #pragma unroll
         for (int kb = 0; kb < KBW; ++kb) {
             uint4 a[2][2];
             uint64_t fa[8];
             if (ODD && (p.flags & kHeldVOdd)) {
-                fill_odd<F::BITS, kRowBit>(scratch, vr + (kb0 + kb) * kHeldBlock, p.ldv, nr, kend - (kb0 + kb) * kHeldBlock, nullptr, 0, 0);
+                fill_odd<F::BITS, kRowBit>(scratch, vr + (kb0 + kb) * kHeldBlock, p.ldv, min(8, nr - rr), kend - (kb0 + kb) * kHeldBlock, nullptr, 0, 0);
             } else {
-                load_rows(vr, p.ldv, nr, kb, a);
-                to_scratch(a, nr);
+                load_rows(vr, p.ldv, min(8, nr - rr), kb, a);
+                to_scratch(a, min(8, nr - rr));
             }
             from_scratch(fa);
 #pragma unroll
@@ -530,7 +537,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 acc[b][0] = fmaf(c[0], ua, acc[b][0]); acc[b][1] = fmaf(c[1], ub, acc[b][1]);
             }
         }
-        float* const mine = tpart + (kw * 8 + g) * p.mp + 2 * t;
+        float* const mine = tpart + (kw * p.nr8 + rr + g) * p.mp + 2 * t;
 #pragma unroll
         for (int b = 0; b < NB; ++b)
             if (b * 8 + 2 * t < p.mp) *reinterpret_cast<float2*>(mine + b * 8) = make_float2(acc[b][0], acc[b][1]);
@@ -543,7 +550,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
             const int r = i / M, m = i - r * M;
             float v = 0.0f;
 #pragma unroll 4
-            for (int k = 0; k < wk; ++k) v += tpart[(k * 8 + r) * p.mp + m];
+            for (int k = 0; k < wk; ++k) v += tpart[(k * p.nr8 + r) * p.mp + m];
             if (!exchange) tt[m * p.rank8 + r] = v;
             else if (!(p.debug & QGEMV_DEBUG_DROP_PROJECTIONS))
                 st_relaxed_u64(words + (r0 + r) * M + m, ((unsigned long long)tag << 32) | __float_as_uint(v));
@@ -821,7 +828,7 @@ template <int FMT, bool BF16, bool ODD> int launch_odd(const HeldPlan& h, bool d
 }
 }  // namespace
 template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s) {
-    return h.args.flags & (kHeldXOdd | kHeldVOdd) ? launch_odd<FMT, BF16, true>(h, dependent, s) : launch_odd<FMT, BF16, false>(h, dependent, s);
+    return h.args.flags & (kHeldXOdd | kHeldVOdd | kHeldFewRows) ? launch_odd<FMT, BF16, true>(h, dependent, s) : launch_odd<FMT, BF16, false>(h, dependent, s);
 }
 template int launch_held_fmt<QGEMV_HELD_FMT, QGEMV_HELD_BF16>(const HeldPlan&, bool, cudaStream_t);
 

@@ -16,7 +16,7 @@ constexpr int held_depth(int bits, int kbw) { return held_stage_codes(bits, kbw)
 constexpr int kHeldGroups[5] = {1, 2, 1, 2, 4};       // scale groups per block by weight format, as Fmt<>::NG
 constexpr int kHeldMaxBatch = 4;       // tiles of a warp between two meetings of its CTA
 
-enum { kHeldOutlierAligned = 1, kHeldUAligned = 2, kHeldYVector = 4, kHeldXOdd = 8, kHeldVOdd = 16 };
+enum { kHeldOutlierAligned = 1, kHeldUAligned = 2, kHeldYVector = 4, kHeldXOdd = 8, kHeldVOdd = 16, kHeldFewRows = 32 };
 
 struct HeldArgs {
     const void* x;            long long ldx;
@@ -36,7 +36,7 @@ struct HeldArgs {
     int m, n, korig, row_bytes, act, flags, debug;
     int ng, gshift;                               // scale groups per row; log2(group / 128) for groups of 128 and more
     int oc, noc, oc_log;                          // outlier columns, blocks of 32 of them, log2 of those columns rounded up
-    int rank, rank8, per_cta;                     // residual rank, padded to 8, ranks a CTA projects (== rank: no exchange)
+    int rank, rank8, per_cta, nr8;                // residual rank, padded to 8; ranks a CTA projects (== rank: no exchange), padded to 8
     int ksplit, rows_per, rows_pad;               // K splits; rows of a row group, padded to 16
     int blocks_split;                             // 128-column blocks of a K split
     int tb;                                       // tiles of a warp per batch

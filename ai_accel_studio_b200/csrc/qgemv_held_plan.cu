@@ -47,7 +47,7 @@ bool place(const qgemv_problem& p, int m, bool bf16, HeldPlan& h) {
             auto put = [&](int bytes) { const int at = off; off = up_to(off + bytes, 128); return at; };
             a.off_part = put(2 * a.part_bytes > nw * 2048 ? 2 * a.part_bytes : nw * 2048);
             a.off_tab = put(nw * h.kbw * kHeldGroups[h.fmt] * h.nb * 64);
-            a.off_tpart = put(a.rank ? h.wk * 8 * a.mp * 4 : 0);
+            a.off_tpart = put(h.wk * a.nr8 * a.mp * 4);
             a.off_sc = put((a.sc_all ? 1 : 2) * a.sc_bytes);
             a.ow_bytes = up_to(h.wr * tb * 16 * a.noc * 64, 128);
             a.off_ow = put(2 * a.ow_bytes);
@@ -68,12 +68,13 @@ bool place(const qgemv_problem& p, int m, bool bf16, HeldPlan& h) {
 bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out) {
     const int m = p.m, sms = sm_count();
     out->ok = false;
-    if (m < 1 || m > 16 || p.n < 16 || !al(p.x, 16)) return false;
+    if (m < 1 || m > 16 || !al(p.x, 16)) return false;
     HeldPlan h{};
     HeldArgs& a = h.args;
     h.fmt = stream_format(p.bits, p.group);
     if (h.fmt < 0 || !al(p.packed, 16) || p.ldp % 16 || p.outliers > kStreamMaxOutliers || p.rank > kMaxRank) return false;
     if (!al(p.scales, 4) || p.ldp > 0x7fffffff || (long long)p.n * p.lds > 0x7fffffff) return false;
+    if (p.n < 16) a.flags |= kHeldFewRows;
     if (p.ldx % 8 || p.k_original % 8) a.flags |= kHeldXOdd;
     if (p.rank && (!al(p.res_v, 16) || p.ldv % 8 || p.k_original % 8)) a.flags |= kHeldVOdd;
     if (p.outliers && al(p.outlier_w, 16) && p.ldow % 8 == 0) a.flags |= kHeldOutlierAligned;
@@ -124,7 +125,8 @@ bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out) {
             // residual projections: all in every CTA, or dealt to the first ones of a split
             const size_t v_bytes = (size_t)(q.blocks_split * kHeldBlock < p.k_original ? q.blocks_split * kHeldBlock : p.k_original) * p.rank * 2;
             q.per_cta = p.rank <= 8 && v_bytes <= (size_t)kLocalBytes ? p.rank : cdiv(p.rank, c.groups);
-            if (q.per_cta > 8 || (q.per_cta < p.rank && (size_t)S * p.rank * m * 2 > words)) continue;
+            q.nr8 = up_to(q.per_cta, 8);
+            if (q.per_cta < p.rank && (size_t)S * p.rank * m * 2 > words) continue;
             const int all = kHeldMaxWarps / c.wk < nt ? kHeldMaxWarps / c.wk : nt;
             for (c.wr = all; c.wr >= 1; c.wr /= 2) {
                 const int nw = c.wk * c.wr, tiles_w = cdiv(nt, c.wr);

@@ -1,4 +1,5 @@
-"""The GEMV whose warps hold their activations in registers (qgemv_held.cu): 5 - 16 rows, and 1 - 4 rows of up to 1024 columns.  Sizes at the
+"""The GEMV whose warps hold their activations in registers (qgemv_held.cu): 5 - 16 rows, 3 and 4 rows that are not padded, 4 rows of long K,
+and 1 - 4 rows of up to 1024 columns.  Sizes at the
 edges of its cuts: 16-row tiles (the last one ends with the matrix), 128-column blocks, K splits between CTAs, batches of tiles, scale rows that
 start at odd positions."""
 import ctypes
@@ -24,8 +25,11 @@ CASES = [
     (4, 300, 8320, 64, 16, 8, True, (5, 10)),            # 65 blocks: K cut between CTAs
     (2, 1200, 20480, 256, 0, 12, True, (7, 16)),         # splits at whole scale groups, projections dealt to several CTAs
     (2, 40000, 512, 128, 64, 8, False, (8, 16)),         # many batches of tiles, scales staged batch by batch
-    (2, 300, 1003, 64, 8, 5, True, (5, 16)),             # rows of x and V off 16 bytes, K padded
-    (4, 200, 8197, 128, 16, 9, False, (6, 12)),          # the same over two K splits
+    (2, 300, 1003, 64, 8, 5, True, (3, 5, 16)),             # rows of x and V off 16 bytes, K padded
+    (4, 200, 8197, 128, 16, 9, False, (4, 6, 12)),          # the same over two K splits
+    (2, 33, 4300, 128, 0, 31, False, (3, 8)),            # more ranks than eight for every CTA
+    (2, 15, 1536, 64, 5, 9, True, (3, 9)),               # less than a tile of rows
+    (4, 1, 3001, 32, 16, 8, True, (4, 6)),
     (4, 4800, 3800, 40, 0, 0, False, (5,)),              # a group that is not built: four rows at a time, as before
 ]
 
@@ -102,4 +106,18 @@ def test_few_rows_of_short_k(bits, n, k, group, oc, rank, act, coracle):
             pairs = ref.half().float().view(m, -1, 2, 8)
             ref = (torch.nn.functional.silu(pairs[:, :, 0]).half().float() * pairs[:, :, 1]).reshape(m, -1)
         _close(ys[0], ref.numpy(), torch.float16)
+    assert ops.workspace_status("cuda") == 0
+
+
+@pytest.mark.parametrize("bits,n,k,group,oc,rank", [(4, 300, 11008, 128, 16, 8), (2, 2400, 14336, 64, 64, 3), (4, 4096, 10240, 64, 0, 0), (4, 1003, 6144, 32, 64, 8)])
+def test_four_rows_of_long_k(bits, n, k, group, oc, rank, coracle):
+    """Aligned rows whose activations leave the phased kernel few warps, beside the same through qgemv_run, which stays with it."""
+    g = torch.Generator().manual_seed(n)
+    mod, h, _, _ = _module(bits, n, k, group, oc, rank, True, g)
+    x = torch.randn(4, k, generator=g).half()
+    xd, ref = x.cuda(), _reference(coracle, bits, k, group, h, x)
+    y = mod(xd)
+    _close(y, ref, torch.float16)
+    assert torch.equal(mod(xd), y)
+    _close(mod.forward_into(xd, torch.empty_like(y)), ref, torch.float16)
     assert ops.workspace_status("cuda") == 0
