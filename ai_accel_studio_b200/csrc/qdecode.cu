@@ -4,6 +4,7 @@
 // one launch per step of the layer, coalesced 8 / 16-byte accesses, enough CTAs for the attention
 // to spread the cache over the SMs, and no waiting between CTAs (the attention's slices meet through
 // an arrival counter: whoever comes last merges).
+#include <atomic>
 #include <type_traits>
 
 #include "qgemv_common.cuh"
@@ -150,9 +151,10 @@ constexpr int kAttMaxSlices = 16;
 constexpr int kAttBlock = 16;                    // positions of a warp's turn
 constexpr int kAttSlice = kAttWarps * kAttBlock; // one turn of a CTA
 constexpr int kAttMaxHeads = 8;                  // query heads per kv head
+constexpr int kAttCluster = 8;                   // slices of a cluster: what every device can place
 
-// Slices the sequence axis is cut into: as many CTAs as fit the SMs one each, each with a turn's positions at least.  Meeting
-// again (fence, counter, reading the parts back) costs 2.5 us, a turn well under 1: shorter slices only pay the former, and a
+// Slices the sequence axis is cut into where they meet through global memory: as many CTAs as fit the SMs one each, each with a turn's positions at
+// least.  Meeting there (fence, counter, reading the parts back) costs 2.5 us, a turn well under 1 to 1.7: shorter slices only pay the former, and a
 // second wave (9 slices for 32 (sequence, kv head) pairs) measured slower than more turns.
 inline int attention_slices(int batch, int kv_heads, int max_len) {
     const int ctas = batch * kv_heads, by_len = max_len / kAttSlice;
@@ -179,6 +181,17 @@ __device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, u
                      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// A float of the same shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ float load_peer(const float* mine, int rank) {
+    float v;
+    asm volatile("{ .reg .u32 a; mapa.shared::cluster.u32 a, %1, %2; ld.shared::cluster.f32 %0, [a]; }"
+                 : "=f"(v) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank) : "memory");
+    return v;
+}
+
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     const typename Act16<BF16>::T a = Act16<BF16>::from_float(lo), b = Act16<BF16>::from_float(hi);
@@ -186,22 +199,24 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // Lane t of a quad holds, of a row of D elements, the eight from 32 c + 8 t in word c of v: so the partner of every element
-// under the rotation (D / 2 away) is the same lane's, D / 64 words further on.
+// under the rotation (D / 2 away) is the same lane's, D / 64 words further on.  The tables' words lie alike.
 template <int D, bool BF16>
-__device__ __forceinline__ void rotate_row(uint4 (&v)[D / 32], const void* cos_, const void* sin_, int t) {
+__device__ __forceinline__ void rotate_row(uint4 (&v)[D / 32], const uint4 (&cos_)[D / 32], const uint4 (&sin_)[D / 32]) {
     using T = typename Act16<BF16>::T;
     constexpr int H = D / 64;
 #pragma unroll
     for (int c = 0; c < H; ++c) {
         T* lo = reinterpret_cast<T*>(&v[c]);
         T* hi = reinterpret_cast<T*>(&v[c + H]);
-        const T* cs = static_cast<const T*>(cos_) + c * 32 + t * 8;
-        const T* sn = static_cast<const T*>(sin_) + c * 32 + t * 8;
+        const T* cl = reinterpret_cast<const T*>(&cos_[c]);
+        const T* ch = reinterpret_cast<const T*>(&cos_[c + H]);
+        const T* sl = reinterpret_cast<const T*>(&sin_[c]);
+        const T* sh = reinterpret_cast<const T*>(&sin_[c + H]);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float a = Act16<BF16>::to_float(lo[q]), b = Act16<BF16>::to_float(hi[q]);
-            lo[q] = Act16<BF16>::from_float(r16<BF16>(a * Act16<BF16>::to_float(cs[q])) + r16<BF16>(-b * Act16<BF16>::to_float(sn[q])));
-            hi[q] = Act16<BF16>::from_float(r16<BF16>(b * Act16<BF16>::to_float(cs[q + D / 2])) + r16<BF16>(a * Act16<BF16>::to_float(sn[q + D / 2])));
+            lo[q] = Act16<BF16>::from_float(r16<BF16>(a * Act16<BF16>::to_float(cl[q])) + r16<BF16>(-b * Act16<BF16>::to_float(sl[q])));
+            hi[q] = Act16<BF16>::from_float(r16<BF16>(b * Act16<BF16>::to_float(ch[q])) + r16<BF16>(a * Act16<BF16>::to_float(sh[q])));
         }
     }
 }
@@ -212,6 +227,7 @@ struct NewToken {
     const void* v; long long ldv;
     const void* cos; const void* sin;
     int table_rows; int* status;
+    bool wide;                                    // the tables' rows are on 16 bytes
 };
 
 // With the lanes of a warp along D this kernel spent its time in shuffles (five per position and query head: 36 us for 4
@@ -222,13 +238,15 @@ struct NewToken {
 // precision is lost against fp32 weights.  With it and the announcement to L2, fp16, in a chain of launches over caches that
 // come from DRAM, rope and append included: 34.3 -> 12.1 us at the size above, 11.6 -> 7.6 us for 8 kv heads x 4 over 577
 // positions, 7.1 -> 5.1 us for 2 x 7 of 64 elements over 162.  What is left is the chain position -> rows -> products ->
-// softmax -> meeting, and the launch.  One CTA per SM: with registers for two (128) the rotation spilled, 18.4 us above.
+// softmax -> meeting, and the launch.  The slices of a sequence meet in the shared memory of a cluster where the device can place that, and what does not hang on
+// the position (queries, new key and value) is asked for before it has arrived, the tables' rows 16 bytes at a time: 7.6 -> 6.2 us, 5.1 -> 4.1 and, at the
+// first size, 12.4 -> 12.0.  One CTA per SM: with registers for two (128) the rotation spilled, 18.4 us above.
 // ROPE: the queries are rotated on their way to fragments; the warp whose turn holds the new position takes that row from the
 // projections instead of the cache, rotates the key, and writes both to the cache.
 template <int D, bool BF16, bool ROPE>
 __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void* q_, long long ldq, void* kc_, void* vc_,
                                                                    const long long* pos_, void* out_, long long ldo, int heads, int hkv,
-                                                                   int max_len, float scale, float* parts, int* counters, bool wide,
+                                                                   int max_len, float scale, float* parts, int* counters, bool wide, bool clustered,
                                                                    const NewToken nt) {
     using T = typename Act16<BF16>::T;
     constexpr int C = D / 32;                     // 16-byte words of a row per lane
@@ -254,17 +272,6 @@ __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void
         for (int c = 0; c < D; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const long long pos = *static_cast<const volatile long long*>(pos_);
-    cut(pos);
-    bool append = false;
-    if constexpr (ROPE) {
-        append = pos >= 0 && pos < max_len && pos < nt.table_rows;
-        if (!append && nt.status && tid == 0) atomicExch(nt.status, 1);
-    }
-    const T* cs = nullptr;
-    const T* sn = nullptr;
-    if (append) { cs = static_cast<const T*>(nt.cos) + (size_t)pos * D; sn = static_cast<const T*>(nt.sin) + (size_t)pos * D; }
-
     auto load_row = [&](const T* row, uint4 (&v)[C]) {      // row points at the lane's first element
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -292,34 +299,71 @@ __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void
         for (int c = 0; c < C; ++c) v[c] = make_uint4(0u, 0u, 0u, 0u);
     };
 
+    // What does not hang on the position first: the queries, the new key and value (every warp, one will want them).
+    uint4 qf[C], nk[C], nv[C];                    // head g of the group; the new row
+    clear(qf);
+    const long long pos = *static_cast<const volatile long long*>(pos_);
+    if (g < heads) load_row(static_cast<const T*>(q_) + (size_t)b * ldq + (size_t)(kvh * heads + g) * D + t * 8, qf);
+    if constexpr (ROPE) {
+        load_row(static_cast<const T*>(nt.k) + (size_t)b * nt.ldk + (size_t)kvh * D + t * 8, nk);
+        load_row(static_cast<const T*>(nt.v) + (size_t)b * nt.ldv + (size_t)kvh * D + t * 8, nv);
+    }
+    cut(pos);
+    bool append = false;
+    uint4 cs[C], sn[C];
+    if constexpr (ROPE) {
+        append = pos >= 0 && pos < max_len && pos < nt.table_rows;
+        if (!append && nt.status && tid == 0) atomicExch(nt.status, 1);
+        if (append) {
+            const T* const cr = static_cast<const T*>(nt.cos) + (size_t)pos * D + t * 8;
+            const T* const sr = static_cast<const T*>(nt.sin) + (size_t)pos * D + t * 8;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                if (nt.wide) {
+                    cs[c] = *reinterpret_cast<const uint4*>(cr + c * 32);
+                    sn[c] = *reinterpret_cast<const uint4*>(sr + c * 32);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        reinterpret_cast<T*>(&cs[c])[e] = cr[c * 32 + e];
+                        reinterpret_cast<T*>(&sn[c])[e] = sr[c * 32 + e];
+                    }
+                }
+            }
+        }
+    }
+
     uint4 ka[C], kb[C], va[C], vb[C];             // positions p + g and p + g + 8 of the turn
     auto fetch = [&](int p) {
         const int pa = p + g, pb = p + g + 8;
         clear(ka); clear(kb); clear(va); clear(vb);
-        const bool na = append && pa == (int)pos, nb = append && pb == (int)pos;
-        if (pa < s1 && !na) { load_row(kbase + (size_t)pa * D, ka); load_row(vbase + (size_t)pa * D, va); }
-        if (pb < s1 && !nb) { load_row(kbase + (size_t)pb * D, kb); load_row(vbase + (size_t)pb * D, vb); }
+        if (pa < s1 && !(append && pa == (int)pos)) { load_row(kbase + (size_t)pa * D, ka); load_row(vbase + (size_t)pa * D, va); }
+        if (pb < s1 && !(append && pb == (int)pos)) { load_row(kbase + (size_t)pb * D, kb); load_row(vbase + (size_t)pb * D, vb); }
+    };
+    auto take_new = [&](int p) {                  // the turn's new row, if it has it
         if constexpr (ROPE) {
-            auto fresh = [&](uint4 (&k)[C], uint4 (&v)[C]) {
-                load_row(static_cast<const T*>(nt.k) + (size_t)b * nt.ldk + (size_t)kvh * D + t * 8, k);
-                load_row(static_cast<const T*>(nt.v) + (size_t)b * nt.ldv + (size_t)kvh * D + t * 8, v);
-                rotate_row<D, BF16>(k, cs, sn, t);
-                store_row(kbase + (size_t)pos * D, k);
-                store_row(vbase + (size_t)pos * D, v);
-            };
-            if (na && pa < s1) fresh(ka, va);
-            if (nb && pb < s1) fresh(kb, vb);
+            if (append && p <= (int)pos && (int)pos < p + kAttBlock && (int)pos < s1) {
+                const bool na = p + g == (int)pos, nb = p + g + 8 == (int)pos;
+                if (na || nb) {
+                    store_row(kbase + (size_t)pos * D, nk);
+                    store_row(vbase + (size_t)pos * D, nv);
+                }
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    if (na) { ka[c] = nk[c]; va[c] = nv[c]; }
+                    if (nb) { kb[c] = nk[c]; vb[c] = nv[c]; }
+                }
+            }
         }
         __syncwarp();
     };
     int p = s0 + warp * kAttBlock;
-    uint4 qf[C];                                  // head g of the group
-    clear(qf);
-    if (g < heads) {
-        load_row(static_cast<const T*>(q_) + (size_t)b * ldq + (size_t)(kvh * heads + g) * D + t * 8, qf);
-    }
     if (p < s1) fetch(p);                         // before anything waits for the queries
-    if (append) rotate_row<D, BF16>(qf, cs, sn, t);
+    if constexpr (ROPE) {
+        if (append && (int)pos >= s0 && (int)pos < s1 && ((int)pos - s0) / kAttBlock % kAttWarps == warp) rotate_row<D, BF16>(nk, cs, sn);      // its turn will come here
+        if (append) rotate_row<D, BF16>(qf, cs, sn);
+    }
+    if (p < s1) take_new(p);
     float m0 = -1.0e30f, m1 = -1.0e30f, l0 = 0.0f, l1 = 0.0f;      // heads 2t, 2t + 1; the sums of this lane's positions
     float o[D / 16][4];                           // rows: elements, see below; columns: heads 2t, 2t + 1
 #pragma unroll
@@ -370,7 +414,7 @@ __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void
             }
         }
         p += kAttWarps * kAttBlock;
-        if (p < s1) fetch(p);
+        if (p < s1) { fetch(p); take_new(p); }
     }
 #pragma unroll
     for (int off = 4; off < 32; off <<= 1) {
@@ -381,6 +425,7 @@ __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void
     // the CTA's warps meet in shared memory
     __shared__ float sm_m[kAttWarps][kAttMaxHeads], sm_l[kAttWarps][kAttMaxHeads];
     __shared__ float sm_o[kAttWarps][kAttMaxHeads][D];
+    __shared__ float cl_m[kAttMaxHeads], cl_l[kAttMaxHeads], cl_o[kAttMaxHeads * D];      // of the CTA, for its cluster
     __shared__ int is_last;
     const int active = max(1, min(kAttWarps, (s1 - s0 + kAttBlock - 1) / kAttBlock));      // warps that had a turn
     if (warp < active) {
@@ -411,12 +456,40 @@ __global__ void __launch_bounds__(kAttWarps * 32, 1) attention_kernel(const void
         }
         if (slices == 1) {
             out[i] = Act16<BF16>::from_float(ll > 0.0f ? acc * (1.0f / ll) : 0.0f);
+        } else if (clustered) {
+            cl_o[i] = acc;
+            if (dd == 0) { cl_m[h] = mm; cl_l[h] = ll; }
         } else {
             mine[h * STRIDE + 4 + dd] = acc;
             if (dd == 0) { mine[h * STRIDE] = mm; mine[h * STRIDE + 1] = ll; }
         }
     }
     if (slices == 1) return;
+    if (clustered) {                              // the slices are a cluster: each CTA makes a share of the results, from the shared memory of all, in order
+        cluster_barrier();
+        for (int i = slice * (kAttWarps * 32) + tid; i < heads * D; i += slices * (kAttWarps * 32)) {
+            const int h = i / D;
+            float mv[kAttCluster], lv[kAttCluster], ov[kAttCluster];
+#pragma unroll
+            for (int s = 0; s < kAttCluster; ++s) {
+                mv[s] = -1.0e30f; lv[s] = ov[s] = 0.0f;
+                if (s < slices) { mv[s] = load_peer(&cl_m[h], s); lv[s] = load_peer(&cl_l[h], s); ov[s] = load_peer(&cl_o[i], s); }
+            }
+            float mm = mv[0];
+#pragma unroll
+            for (int s = 1; s < kAttCluster; ++s) mm = fmaxf(mm, mv[s]);
+            float ll = 0.0f, acc = 0.0f;
+#pragma unroll
+            for (int s = 0; s < kAttCluster; ++s) {
+                const float f = __expf(mv[s] - mm);
+                ll = fmaf(lv[s], f, ll);
+                acc = fmaf(ov[s], f, acc);
+            }
+            out[i] = Act16<BF16>::from_float(ll > 0.0f ? acc * (1.0f / ll) : 0.0f);
+        }
+        cluster_barrier();                        // nobody leaves before the others have read its sums
+        return;
+    }
     // arrival: the last CTA of this (sequence, kv head) merges the slices; nobody waits
     __threadfence();
     __syncthreads();
@@ -506,30 +579,75 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 // Launch with the programmatic-stream-serialisation attribute: the kernels above release their
 // successor at entry and wait for their predecessor before they touch memory.
 template <typename... KArgs, typename... Args>
-int launch_pdl(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+int launch_clusters(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
     return check_launch(what);
+}
+template <typename... KArgs, typename... Args>
+int launch_pdl(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+    return launch_clusters(what, kern, grid, block, 1, s, args...);
 }
 
 template <bool ROPE>
 int launch_attention(bool bf16, int head_dim, dim3 grid, cudaStream_t s, const void* q, long long ldq, void* kc, void* vc, const long long* pos,
-                     void* out, long long ldo, int heads, int hkv, int max_len, float scale, float* parts, int* counters, bool wide,
+                     void* out, long long ldo, int heads, int hkv, int max_len, float scale, float* parts, int* counters, bool wide, bool clustered,
                      const NewToken& nt) {
     const dim3 block(kAttWarps * 32);
-#define QDEC_ATT(D, B) launch_pdl("attention_kernel", attention_kernel<D, B, ROPE>, grid, block, s, q, ldq, kc, vc, pos, out, ldo, heads, hkv, \
-                                  max_len, scale, parts, counters, wide, nt)
+#define QDEC_ATT(D, B) launch_clusters("attention_kernel", attention_kernel<D, B, ROPE>, grid, block, clustered ? (int)grid.x : 1, s, q, ldq, kc, vc, pos, out, ldo, heads, hkv, \
+                                  max_len, scale, parts, counters, wide, clustered, nt)
     if (head_dim == 64) return bf16 ? QDEC_ATT(64, true) : QDEC_ATT(64, false);
     return bf16 ? QDEC_ATT(128, true) : QDEC_ATT(128, false);
 #undef QDEC_ATT
+}
+
+// Clusters of `size` CTAs that the device places at a time, by the largest of the kernels (all take an SM to themselves).
+int attention_clusters(int size) {
+    static std::atomic<int> known[64][kAttCluster + 1];      // + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return 0; }
+    int n = known[dev][size].load(std::memory_order_relaxed) - 1;
+    if (n >= 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(kAttWarps * 32);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, attention_kernel<128, true, true>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+    known[dev][size].store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
+// Slices of a cluster, 0 where the global meeting is better.  The meeting in shared memory costs some 1 us (one slice 3.1 us, two 4.1, chains over 112
+// positions of 64 elements), so slices pay from about 192 positions on and down to 24 each: 8 instead of 5 over 576 positions of 8 heads x 128 6.2 against
+// 7.0 us (global meeting 7.6), instead of 1 over 300 4.2 against 5.6 (7.2).  As many as the device places at once for all (sequence, kv head) pairs: the
+// next larger ones go in two waves (16 pairs: 6 slices 10.3 us, 7 18.9).  More slices of the other kind win where a CTA of the cluster gets so many turns more
+// that they outweigh the meeting, us: 2 x 64 elements, 3072 positions 7.0 in the cluster, 7.5 in 16 slices; 4072 8.3 and 7.9; 8 x 128, 1772 8.3 and 9.0,
+// 2072 8.5 and 8.1; 16 x 128 (6 slices against 8) 1072 8.3 and 8.1, 372 5.9 and 9.6.
+int cluster_slices(int batch, int kv_heads, int head_dim, int max_len) {
+    if (max_len < 192) return 0;
+    const int pairs = batch * kv_heads, global = attention_slices(batch, kv_heads, max_len);
+    for (int c = kAttCluster; c >= 2; --c) {
+        if (attention_clusters(c) < pairs) continue;
+        const float turns = (float)max_len / kAttSlice * (1.0f / c - 1.0f / global);        // more of them than in global slices
+        return turns <= (c < kAttCluster ? 0.15f : head_dim == 64 ? 1.5f : 0.7f) ? c : 0;
+    }
+    return 0;
 }
 
 size_t attention_parts_floats(int batch, int q_heads, int kv_heads, int head_dim, int max_len) {
@@ -609,9 +727,10 @@ int run_attention(const char* name, const void* q, int64_t ldq, void* kcache, vo
     }
     int* counters = static_cast<int*>(workspace);
     float* parts = reinterpret_cast<float*>(static_cast<char*>(workspace) + ((size_t)batch * kv_heads * sizeof(int) + 255) / 256 * 256);
-    const dim3 grid(attention_slices(batch, kv_heads, max_len), kv_heads, batch);
+    const int cluster = cluster_slices(batch, kv_heads, head_dim, max_len);
+    const dim3 grid(cluster ? cluster : attention_slices(batch, kv_heads, max_len), kv_heads, batch);
     return (nt.k ? launch_attention<true> : launch_attention<false>)(dtype == QGEMV_BF16, head_dim, grid, static_cast<cudaStream_t>(stream), q, ldq, kcache,
-        vcache, reinterpret_cast<const long long*>(pos), out, ldo, q_heads / kv_heads, kv_heads, max_len, scale, parts, counters, all(16), nt);
+        vcache, reinterpret_cast<const long long*>(pos), out, ldo, q_heads / kv_heads, kv_heads, max_len, scale, parts, counters, all(16), cluster != 0, nt);
 }
 }  // namespace
 
@@ -630,7 +749,7 @@ extern "C" int qdec_rope_attention(const void* q, int64_t ldq, const void* k, in
     if (!k || !v || !cos_table || !sin_table || table_rows < 1) { set_error("qdec_rope_attention: null pointer or empty table"); return QGEMV_ERR_BAD_ARG; }
     if (ldk < (int64_t)kv_heads * head_dim || ldv < (int64_t)kv_heads * head_dim) { set_error("qdec_rope_attention: a leading dimension is smaller than its row"); return QGEMV_ERR_SHAPE; }
     return run_attention("qdec_rope_attention", q, ldq, kcache, vcache, pos, out, ldo, batch, q_heads, kv_heads, head_dim, max_len, scale, workspace,
-                         workspace_bytes, dtype, NewToken{k, ldk, v, ldv, cos_table, sin_table, table_rows, status}, stream);
+                         workspace_bytes, dtype, NewToken{k, ldk, v, ldv, cos_table, sin_table, table_rows, status, aligned16(cos_table) && aligned16(sin_table)}, stream);
 }
 
 extern "C" int qdec_silu_mul(const void* gate, int64_t ldg, const void* up, int64_t ldu, void* y, int64_t ldy,
