@@ -368,7 +368,8 @@ extern "C" size_t qgemv_prepared_bytes(void) { return sizeof(Prepared); }
 //  * Three and four rows: at 4 warps (57344 x 12288 INT4, M = 4 1.18x) and where it does not fit.
 //  * Four rows from K = 8192 on: at 8 warps (8192 x 11008 INT4 1.48x, 57344 x 12288 1.06x, 4096 x 14336 INT2 1.11x; below that K the phased kernel wins,
 //    14336 x 6144 0.86x).  INT4 from about K = 10000 on: at 12 (8192 x 11008 1.22x, 57344 x 11008 1.21 to 1.44x; 57344 x 9216 0.80x, INT2
-//    4096 x 11008 0.96x), groups of 32 at any K (0.99 to 1.26x, 13 matrices; 128 and 64 at K = 8192 0.86 to 1.13x).  Three rows are mixed, 0.84 to 1.36x at 8.
+//    4096 x 11008 0.96x), groups of 32 at any K (0.99 to 1.26x, 13 matrices; 128 and 64 at K = 8192 0.86 to 1.03x) and the most rows (57344 and 128256, K = 7168
+//    and 8192: 1.01 to 1.32x; 40000 0.86 to 1.02x).  Three rows are mixed, 0.84 to 1.36x at 8.
 //  * One and two rows, which the streaming kernel multiplies as integers: at 8 (K = 28672, M = 2, N = 2048 and 8192: INT4 24 against 33 and 48 against 51 us,
 //    INT2 21 against 16 and 36 against 43 us); INT2 matrices of no more than one tile of 16 rows per SM, which the phased kernel reads
 //    in a single round, stay with it (N = 512 to 2048: 16 us, streaming 17 to 21).
@@ -390,7 +391,7 @@ extern "C" int qgemv_prepare(const qgemv_problem* p, void* prepared) {
         const bool one_round = p->bits == 2 && (p->n + kStreamTileRows - 1) / kStreamTileRows <= plan.grid;
         int most = p->m <= 2 && !one_round ? 8 : 4;    // warps
         if (p->m == 4 && p->k_padded >= 8192) most = 8;
-        if (p->m == 4 && p->bits == 4 && (p->k_padded >= 10240 || p->group == 32)) most = 12;
+        if (p->m == 4 && p->bits == 4 && (p->k_padded >= 10240 || p->group == 32 || (p->k_padded >= 7168 && p->n >= 49152))) most = 12;
         starved = !plan.ok || (plan.variant == 1 && plan.nw <= most);
     }
     if (choose_held(*p, kMaxPartialFloats, &q->held)) return QGEMV_OK;
