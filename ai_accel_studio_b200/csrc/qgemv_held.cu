@@ -80,11 +80,10 @@ template <typename H, bool ODD> struct Ring {
     const uint8_t* src;                               // this lane's row and piece of the next tile, first stage
     long long step;                                   // to the warp's next tile
     int ldw, row, row_step, last, end_row;            // weight row of that tile, the last one a tile may start at, end of the CTA's rows
-    int rows_left;                                    // ODD: rows of the matrix below this lane's first one, in the tile
     int left;                                         // bytes from this lane's piece to the end of the warp's columns
     uint32_t dst, at;
 
-    __device__ __forceinline__ void issue() {         // all stages of a tile
+    __device__ __forceinline__ void issue(int n) {    // all stages of a tile; n: rows of the matrix
         const bool more = row < end_row;
         if (more && row > last) { src -= (long long)(row - last) * ldw; row = last; end_row = last; }      // the last tile of all ends with the matrix
 #pragma unroll
@@ -93,7 +92,7 @@ template <typename H, bool ODD> struct Ring {
                 const uint32_t d = dst + at;
 #pragma unroll
                 for (int i = 0; i < H::COPIES; ++i)
-                    if (!ODD || i * H::RPI < rows_left) cp_async16((H::PITCH == 128 && (i & 1) ? d ^ 16u : d) + i * 512, src + (long long)(i * H::RPI) * ldw + st * H::PITCH);
+                    if (!ODD || (int)threadIdx.x / H::PPR + i * H::RPI < n) cp_async16((H::PITCH == 128 && (i & 1) ? d ^ 16u : d) + i * 512, src + (long long)(i * H::RPI) * ldw + st * H::PITCH);
             }
             cp_async_commit();
             at = at + H::STAGE == H::DEPTH * H::STAGE ? 0u : at + H::STAGE;
@@ -270,8 +269,8 @@ __device__ __forceinline__ void finish_rows(const HeldArgs& p, float (&v)[4], ui
 #define QGEMV_HELD_STAMP(i) do {} while (0)
 #endif
 
-// ODD: rows of x or V may lie off 16 bytes, and the matrix may have less than a tile of rows (what is computed for the missing ones is not
-// stored).  An instance of its own: beside the usual ones the code costs 2 - 3 %.
+// ODD: rows of x or V may lie off 16 bytes, the matrix may have less than a tile of rows (what is computed for the missing ones is not
+// stored), a CTA more than eight ranks to project.  An instance of its own: beside the usual ones the code costs 2 - 3 %.
 template <int FMT, int KBW, int NB, bool BF16, bool ODD>
 __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const __grid_constant__ HeldArgs p) {
     using F = Fmt<FMT>;
@@ -286,7 +285,8 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     const int g = lane >> 2, t = lane & 3, M = p.m;
     const int grp = blockIdx.x, split = blockIdx.y;
     const int rowbase = grp * p.rows_per, rowend = min(rowbase + p.rows_per, p.n);
-    const int last = ODD ? max(0, p.n - 16) : p.n - 16, low = ODD ? min(15, p.n - 1) : 15;      // where the last tile starts, the last row of a tile
+    const int last = ODD ? max(0, p.n - 16) : p.n - 16;                  // where the last tile starts
+    auto in_tile = [&](int r) { return ODD ? min(r, p.n - 1) : r; };     // a tile's row, if the matrix has it
     const int kb0 = split * p.blocks_split + kw * KBW;                   // this warp's first block
     const uint32_t sm = smem_u32(smem), ring_at = sm + (uint32_t)warp * (H::DEPTH * H::STAGE);
     const bool exchange = p.per_cta < p.rank;
@@ -309,14 +309,13 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         const int r = lane / H::PPR, piece = lane % H::PPR;
         ring.ldw = (int)p.ldw;
         ring.left = min(p.row_bytes, (split + 1) * p.blocks_split * H::BW) - kb0 * H::BW - piece * 16;
-        ring.rows_left = min(16, p.n) - r;
         ring.row = rowbase + wrow * 16; ring.row_step = wr * 16; ring.last = last; ring.end_row = rowend;
         ring.src = p.w + (long long)(ring.row + r) * p.ldw + kb0 * H::BW + piece * 16;
         ring.step = (long long)(wr * 16) * p.ldw;
         ring.dst = ring_at + stage_offset<H::PITCH>(r, piece * 16);
         ring.at = 0;
     }
-    ring.issue();                                      // the first tile, then what is wanted with it, then the rest of the ring
+    ring.issue(p.n);                                      // the first tile, then what is wanted with it, then the rest of the ring
     // Scales of sc_rows rows (all of the CTA's, or a batch's), from the 4- or 16-byte word that holds the K slice's first; past the row's end zero.
     const int sc_lds = (int)p.lds, sc_first = split * p.sc_split;
     auto stage_scales = [&](int row0, int buf) {
@@ -325,7 +324,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
             const uint32_t to = sm + p.off_sc + buf * p.sc_bytes + u * p.sc_unit;
 #pragma unroll 1
             for (int r = tid >> p.sc_log; r < nrow; r += threads >> p.sc_log) {
-                const int off = (min(row0 + (r & ~15), last) + min(r & 15, low)) * sc_lds + sc_first, odd = off & 1, n = max(0, min(per, p.ng - sc_first + odd - u * per)) * 2;
+                const int off = (min(row0 + (r & ~15), last) + in_tile(r & 15)) * sc_lds + sc_first, odd = off & 1, n = max(0, min(per, p.ng - sc_first + odd - u * per)) * 2;
                 const __half* from = n ? p.sc + (off - odd + u * per) : p.sc;
                 if (per == 8) cp_async16z(to + r * p.sc_pitch, from, n);
                 else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + r * p.sc_pitch), "l"(from), "r"(n) : "memory");
@@ -348,7 +347,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 const int r = e >> p.ow_log, u = e & ((1 << p.ow_log) - 1), left = min(8, p.oc - u * 8);
                 if (u >= units) continue;
                 const uint32_t d = to + (uint32_t)((jt * 16 + r) * units + u) * 16;
-                const __half* from = p.ow + (long long)(min(row, last) + min(r, low)) * p.ldow + u * 8;
+                const __half* from = p.ow + (long long)(min(row, last) + in_tile(r)) * p.ldow + u * 8;
                 if (p.flags & kHeldOutlierAligned) cp_async16z(d, left > 0 ? from : p.ow, left > 0 ? left * 2 : 0);
                 else
                     for (int q = 0; q < 8; ++q) sts_half(d + q * 2, q < left ? __ldg(from + q) : __half(0.0f));
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
     {                                                  // rows of U (padded to 8 columns) and bias of all the CTA's tiles
         const int nrow = (rowend - rowbase + 15) & ~15, pieces = p.rank8 >> 3;
         for (int i = tid; i < nrow; i += threads) {
-            const int n = min(rowbase + (i & ~15), last) + min(i & 15, low);
+            const int n = min(rowbase + (i & ~15), last) + in_tile(i & 15);
             for (int q = 0; q < pieces; ++q) {
                 const __half* from = p.ru + (long long)n * p.ldu + q * 8;
                 const uint32_t d = sm + p.off_u + (uint32_t)(i * pieces + q) * 16;
@@ -373,7 +372,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         mbarrier_arrive_copies(smem_u32(full + kFullU));
     }
 #pragma unroll 1
-    for (int d = 1; d < H::DEPTH / H::NS; ++d) ring.issue();
+    for (int d = 1; d < H::DEPTH / H::NS; ++d) ring.issue(p.n);
     QGEMV_HELD_STAMP(1);
     const int n_xo = has_o ? M << p.oc_log : 0, xo_mask = (1 << p.oc_log) - 1;      // activations of the outlier columns, [m][column]
     int xcol = -1;
@@ -508,9 +507,10 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
         __syncwarp();
     }
     QGEMV_HELD_STAMP(4);
-    if (wrow == 0)                                     // residual projections of this warp's columns, eight ranks at a time
+    if (nr > 0 && wrow == 0)                           // residual projections of this warp's columns, up to eight ranks (ODD: at a time)
 #pragma unroll 1
-    for (int rr = 0; rr < nr; rr += 8) {
+    for (int rr = 0; rr < (ODD ? nr : 1); rr += 8) {
+        const int count = ODD ? min(8, nr - rr) : nr;
         float acc[NB][4];
 #pragma unroll
         for (int b = 0; b < NB; ++b) acc[b][0] = acc[b][1] = 0.0f;
@@ -520,10 +520,10 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
             uint4 a[2][2];
             uint64_t fa[8];
             if (ODD && (p.flags & kHeldVOdd)) {
-                fill_odd<F::BITS, kRowBit>(scratch, vr + (kb0 + kb) * kHeldBlock, p.ldv, min(8, nr - rr), kend - (kb0 + kb) * kHeldBlock, nullptr, 0, 0);
+                fill_odd<F::BITS, kRowBit>(scratch, vr + (kb0 + kb) * kHeldBlock, p.ldv, count, kend - (kb0 + kb) * kHeldBlock, nullptr, 0, 0);
             } else {
-                load_rows(vr, p.ldv, min(8, nr - rr), kb, a);
-                to_scratch(a, min(8, nr - rr));
+                load_rows(vr, p.ldv, count, kb, a);
+                to_scratch(a, count);
             }
             from_scratch(fa);
 #pragma unroll
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(kHeldMaxWarps * 32, 1) qgemv_held_kernel(const
                 }
                 if (st == H::NS - 1) {
                     __syncwarp();                      // every lane has read the tile before it is refilled
-                    ring.issue();
+                    ring.issue(p.n);
                 }
                 slot = slot + H::STAGE == ring_at + H::DEPTH * H::STAGE ? ring_at : slot + H::STAGE;
             }
@@ -828,7 +828,7 @@ template <int FMT, bool BF16, bool ODD> int launch_odd(const HeldPlan& h, bool d
 }
 }  // namespace
 template <int FMT, bool BF16> int launch_held_fmt(const HeldPlan& h, bool dependent, cudaStream_t s) {
-    return h.args.flags & (kHeldXOdd | kHeldVOdd | kHeldFewRows) ? launch_odd<FMT, BF16, true>(h, dependent, s) : launch_odd<FMT, BF16, false>(h, dependent, s);
+    return h.args.flags & (kHeldXOdd | kHeldVOdd | kHeldFewRows | kHeldManyRanks) ? launch_odd<FMT, BF16, true>(h, dependent, s) : launch_odd<FMT, BF16, false>(h, dependent, s);
 }
 template int launch_held_fmt<QGEMV_HELD_FMT, QGEMV_HELD_BF16>(const HeldPlan&, bool, cudaStream_t);
 

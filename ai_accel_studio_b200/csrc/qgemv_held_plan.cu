@@ -20,6 +20,7 @@ constexpr double kBatchCost = 1.3;                                    // a meeti
 constexpr double kOutlierCost = 0.75;                                 // a turn of every warp with 32 outlier columns of a tile, per 8 activation rows
 constexpr double kStreamRate = 36000, kHeldLoadCost = 0.003;          // bytes of weights that reach a CTA; loading 128 activations
 constexpr double kSplitCost = 1.0, kSumCost = 0.0002;                 // handing a split over, and per fp32 sum
+constexpr double kOddCost = 1.0, kOddWide = 1.2;                       // filling in an odd block's fragments, per 8 activation rows; four blocks spill there
 constexpr double kWideCost = 1.2;                                     // four blocks a warp: longer until the first tile is through
 
 int log2_up(int v) { int s = 0; while ((1 << s) < v) ++s; return s; }
@@ -126,15 +127,17 @@ bool plan_held(const qgemv_problem& p, size_t partial_floats, HeldPlan* out) {
             const size_t v_bytes = (size_t)(q.blocks_split * kHeldBlock < p.k_original ? q.blocks_split * kHeldBlock : p.k_original) * p.rank * 2;
             q.per_cta = p.rank <= 8 && v_bytes <= (size_t)kLocalBytes ? p.rank : cdiv(p.rank, c.groups);
             q.nr8 = up_to(q.per_cta, 8);
+            if (q.per_cta > 8) q.flags |= kHeldManyRanks; else q.flags &= ~kHeldManyRanks;
             if (q.per_cta < p.rank && (size_t)S * p.rank * m * 2 > words) continue;
             const int all = kHeldMaxWarps / c.wk < nt ? kHeldMaxWarps / c.wk : nt;
             for (c.wr = all; c.wr >= 1; c.wr /= 2) {
                 const int nw = c.wk * c.wr, tiles_w = cdiv(nt, c.wr);
                 if (nw < 8 && c.wr < all) break;
                 const double stream = (double)q.rows_per * q.blocks_split * (p.bits == 2 ? 32 : 64) / kStreamRate;
-                const double main = tiles_w * c.kbw * kBlockCost[c.kbw] * (h.nb == 2 ? kSecondRows : 1) * (bf16 ? kBf16 : 1) * (3.2 + nw * 0.05);
+                const bool odd = (a.flags & (kHeldXOdd | kHeldVOdd)) != 0;
+                const double main = tiles_w * c.kbw * kBlockCost[c.kbw] * (odd && c.kbw == 4 ? kOddWide : 1) * (h.nb == 2 ? kSecondRows : 1) * (bf16 ? kBf16 : 1) * (3.2 + nw * 0.05);
                 double cost = (main > stream ? main : stream) + kOutlierCost * h.nb * a.noc * cdiv(nt, nw) + kHeldLoadCost * c.wr * q.blocks_split * m +
-                              (S > 1 ? kSplitCost + kSumCost * (S + 1) * q.rows_pad * q.mp : 0) + (c.kbw == 4 ? kWideCost : 0);
+                              (S > 1 ? kSplitCost + kSumCost * (S + 1) * q.rows_pad * q.mp : 0) + (c.kbw == 4 ? kWideCost : 0) + (odd ? kOddCost * c.kbw * h.nb : 0);
                 if ((best >= 0 && cost + kBatchCost * h.nb >= best) || !place(p, m, bf16, c)) continue;
                 cost += kBatchCost * h.nb * cdiv(tiles_w, q.tb);
                 if (best < 0 || cost < best) { best = cost; *out = c; }
