@@ -474,6 +474,19 @@ extern "C" int qgemv_launch_prepared(void* prepared, const void* x, void* y, voi
     return QGEMV_OK;
 }
 
+namespace {
+// 17 to 32 rows of a small matrix: two launches with held activations, the second over weights in L2.  The prompts' three kernels need 11 to 20 us before and
+// beside the multiplication.  40 outlier columns, rank 8, two against three, us: INT4 2048 x 2048 17 rows 14.2 and 21.1, 32 rows 15.7 and 21.2; 896 x 4864 24 rows 16.5
+// and 26.1; 4096 x 4096 24 rows 21.8 and 24.4, 32 rows 25.4 and 24.4; 14336 x 4096 24 rows 36.4 and 34.4.  INT2 prompts are faster: 2048 x 2048 17 rows 14.3
+// and 19.2, 4096 x 4096 20.4 and 21.7, 32 rows 23.6 and 21.6; many rows of weights, 11008 x 2048 24 rows 20.2 and 19.4, or short K, 4864 x 896 14.1 and 13.7.
+bool two_launches(const qgemv_problem& p) {
+    if (p.kernel != QGEMV_KERNEL_AUTO || p.m <= QGEMV_MAX_BATCH || p.m > 2 * QGEMV_MAX_BATCH) return false;
+    const double weights = (double)p.n * p.k_padded;
+    if (p.bits == 4) return weights <= (p.m <= 24 ? 48e6 : 16e6);
+    return p.k_padded >= 1024 && p.n <= 4LL * p.k_padded && weights <= (p.m <= 24 ? 32e6 : 13e6);
+}
+}  // namespace
+
 // ---- any number of rows ----------------------------------------------------------------------------------
 
 extern "C" size_t qgemv_batch_scratch_bytes(const qgemv_problem* p) {
@@ -484,5 +497,20 @@ extern "C" size_t qgemv_batch_scratch_bytes(const qgemv_problem* p) {
 extern "C" int qgemv_run_batch(const qgemv_problem* p, void* scratch, size_t scratch_bytes, void* stream) {
     const int v = validate(p, qgemv_workspace_bytes(0, 0, 0, 0, 0, 0), 0x7fffffff);
     if (v != QGEMV_OK) return v;
-    return run_gemm(*p, scratch, scratch_bytes, static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const size_t need = gemm_scratch_bytes(*p);      // what the prompts' kernels refuse stays refused
+    if (need && scratch && scratch_bytes >= need && two_launches(*p)) {
+        qgemv_problem a = *p, b = *p;
+        a.m = QGEMV_MAX_BATCH;
+        b.m = p->m - QGEMV_MAX_BATCH;
+        b.x = static_cast<const char*>(p->x) + (size_t)a.m * p->ldx * 2;
+        b.y = static_cast<char*>(p->y) + (size_t)a.m * p->ldy * 2;
+        const bool bf16 = p->x_dtype == QGEMV_BF16;
+        HeldPlan first, second;
+        if (plan_held(a, kMaxPartialFloats, &first) && plan_held(b, kMaxPartialFloats, &second)) {
+            const int r = launch_held(first, bf16, false, p->workspace, s);      // in stream order, as the prompts' first kernel: weights may still be being written
+            return r != QGEMV_OK ? r : launch_held(second, bf16, true, p->workspace, s);
+        }
+    }
+    return run_gemm(*p, scratch, scratch_bytes, s);
 }

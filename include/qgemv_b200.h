@@ -190,7 +190,8 @@ int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspac
 /* The same computation for any number of rows (prompts): one kernel lays x out, one dequantises the codes into tensor memory
  * and multiplies there; the dense matrix is never written.  Weights are rounded as qdequant rounds them to the activation
  * type; base (with the bias), outlier term and residual are fp32 sums, each rounded to the activation type (the residual, whose V x
- * is rounded to fp16, to fp16 first) before they are added in this order, as the expression over a dense matrix does.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
+ * is rounded to fp16, to fp16 first) before they are added in this order, as the expression over a dense matrix does.  17 to 32 rows of a small matrix are
+ * two launches as qgemv_prepare's, without these roundings, which use the workspace.  `scratch`: qgemv_batch_scratch_bytes(p) bytes of device memory, 256-byte aligned, any contents,
  * private to the call until it completes (0: this shape is not built -- groups other than 32 (INT4), 64 and multiples of
  * 128, unaligned packed rows, more than 8192 tiles of 128 weight rows x 256 rows of x, more than 4096 outlier columns --
  * dequantise and use a library GEMM).  x needs only k_original columns.
@@ -198,7 +199,7 @@ int qgemv_launch_prepared(void* prepared, const void* x, void* y, void* workspac
 size_t qgemv_batch_scratch_bytes(const qgemv_problem* p);
 int qgemv_run_batch(const qgemv_problem* p, void* scratch, size_t scratch_bytes, void* stream);
 
-/* Bytes of workspace qgemv_run needs for a problem of this shape (never 0; at most a few MB). */
+/* Bytes of workspace qgemv_run needs for a problem of this shape (never 0; 18.1 MB). */
 size_t qgemv_workspace_bytes(int bits, int m, int n, int k_padded, int group, int rank);
 
 /* Name of the kernel variant qgemv_run would launch for `p` (static string, host memory), or

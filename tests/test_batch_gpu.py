@@ -172,7 +172,7 @@ def test_two_rows_of_long_k_on_either_side_of_the_route(bits, n):
     assert ops.workspace_status("cuda") == 0
 
 
-@pytest.mark.parametrize("rows,n,oc,rank", [(17, 250, 32, 0), (33, 512, 64, 32), (49, 264, 1, 1), (20, 256, 0, 32), (31, 300, 65, 1), (18, 256, 8, 33)])
+@pytest.mark.parametrize("rows,n,oc,rank", [(33, 250, 32, 0), (33, 512, 64, 32), (49, 264, 1, 1), (36, 256, 0, 32), (47, 300, 65, 1), (34, 256, 8, 33)])
 def test_terms_at_the_edges_of_their_kernels(monkeypatch, rows, n, oc, rank):
     """Up to 64 outlier columns and rank 32 have a kernel that keeps the weights in registers, more of either the general one: 16 activation rows a
     tile, 256 weight rows a CTA, blocks of 32 columns."""
