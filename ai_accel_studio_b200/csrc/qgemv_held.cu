@@ -9,12 +9,18 @@
 //  * Codes are not converted: `word & mask` leaves one code in the low mantissa bits of each 16-bit half, an fp16 subnormal worth
 //    code * radix^c * 2^-24.  The classes c accumulate apart and are weighed in fp32.  x is fp16 as it comes (bf16: a power of two per 128
 //    columns, exact).
-//  * One more warp serves the others: group scales of the next batch (each row's are one contiguous piece), outlier columns as one
-//    more partial sum, rows of U, the projections t = V x.
+//  * The warps take turns at the rest: outlier columns of a batch's tiles (two mma per 32 onto the warp's own sums), the sums of the batch before.  A
+//    17th warp for it would leave each thread 96 registers.
 //  * t comes from the fragments, by mma with the rows of V as A.  With few columns every CTA makes all of it; else the first CTAs
 //    make a row or more each and pass them on as {value, launch tag} words.
 //  * K is split between CTAs where a row's activations do not fit the registers of a CTA's warps, or where there are few rows;
 //    the last CTA to arrive adds the splits in order.
+//
+// Bound: instructions and latency of the SM, not HBM.  16 warps over 2 x 128 columns and 16 rows of INT2 need 1470 clocks for 16 weight rows with nothing but
+// shared-memory loads, masks and mma (8.3 clocks each on a scheduler, nearly added to the other instructions); with copies, scales, sums and their meeting it is
+// 1600 to 2000 for one block (clock stamps, 14336 x 4096, 16 rows), of 38 k clocks in all: 3 k until the ring is filled, 3.5 k for x, 2 k for the last sums.
+// Streaming kernel -> this one, us over weights from DRAM, 40 to 64 outlier columns, rank 8: INT2 14336 x 4096 16 rows 29.1 -> 20.7, INT4 8192 x 28672
+// 8 rows 55 -> 38, 16 rows 876 -> 70, 28672 x 28672 16 rows 2602 -> 244, 8 x 4300 8 rows 86 -> 6.9.  Bytes alone: 2.7, 18.8, 18.8, 65, 0.02.
 //
 // Replaces _decode_gemv (ai_accel_lab/kernels/decode_int2.py:43-96) and _decode_int4_gemv
 // (ai_accel_lab/kernels/groupwise_int4.py:85-107) of the reference project.

@@ -1,4 +1,6 @@
-// Streaming fused GEMV for packed groupwise INT2 / INT4 weights, up to 16 activation rows, sm_100a.
+// Streaming fused GEMV for packed groupwise INT2 / INT4 weights, up to 16 activation rows, sm_100a.  It takes one and two rows of x that are not
+// padded or aligned, or so long that the phased kernel is starved, exactly; from three rows on qgemv_held.cu is 1.1 to 10 times as fast, and this one takes
+// what that cannot plan (9 to 16 rows of more than some 42000 x 16800 weights, whose split sums do not fit the scratch).
 //
 // A decode GEMV is a few microseconds of weight stream wrapped in a chain of short dependent phases; the chain, not HBM,
 // is what bounds it.  This kernel keeps the chain short and the instruction count per weight low:
@@ -23,7 +25,7 @@
 //    residual's projections V.x are computed by single warps of a few CTAs and travel as {value, launch tag} words.
 //  * The main loop is kept below the instruction cache of an SM partition.
 //
-// What is left (counters of cold launches): few warps and a short life.  14336 x 4096 INT2, 16 rows: 7.7 M warp instructions,
+// What is left (counters of cold launches, of shapes that qgemv_held.cu now takes in 21 and 38 us instead of 29 and 55): few warps and a short life.  14336 x 4096 INT2, 16 rows: 7.7 M warp instructions,
 // 23 % of the issue slots used by 9 warps an SM; of the 7 clocks between two instructions of a warp 2 are fixed latency, 1.9
 // waiting for instructions, 1.8 for the CTA's barrier.  8192 x 28672 INT4, 8 rows: 24 M, 40 % of the slots, 17 warps an SM, 2.5
 // clocks at the barrier (warps that are done wait for the others), 2.4 of latency; DRAM at a quarter.
